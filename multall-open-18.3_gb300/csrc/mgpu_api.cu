@@ -53,6 +53,18 @@ const int kNumArrays = sizeof(kArrays) / sizeof(kArrays[0]);
 
 }  // namespace
 
+// A captured LOOP iteration.
+struct StepGraph {
+    cudaGraph_t graph = nullptr;
+    cudaGraphExec_t exec = nullptr;
+    size_t nodes = 0;
+    void drop() {
+        if (exec) cudaGraphExecDestroy(exec);
+        if (graph) cudaGraphDestroy(graph);
+        *this = StepGraph();
+    }
+};
+
 struct mgpu_handle {
     Dev d;
     cudaStream_t stream = nullptr;
@@ -68,10 +80,8 @@ struct mgpu_handle {
     void *dptr[sizeof(kArrays) / sizeof(kArrays[0])] = {};
     size_t dbytes[sizeof(kArrays) / sizeof(kArrays[0])] = {};
     std::vector<void *> allocs;
-    cudaGraph_t graph = nullptr;
-    cudaGraphExec_t gexec = nullptr;
-    size_t graph_nodes = 0;
-    size_t loss_nodes = 0, tail_nodes = 0;   // kernels in the conditional bodies
+    StepGraph sg[4];             // one LOOP iteration by what it runs: 1 LOSS, 2 the tail
+    bool ctl_known = false;      // h_ctl mirrors the control block: nothing has run since it was read
     double *d_int = nullptr;     // integrals output (4 x JM)
     void *flush_buf = nullptr;   // > L2, rewritten between timed iterations
     size_t flush_bytes = 0;
@@ -265,10 +275,11 @@ struct SaBranch {
     cudaEvent_t start = nullptr, bc = nullptr, done = nullptr;
 };
 
-void enqueue_core(const Dev &d, Launch L, cudaEvent_t join = nullptr, const SaBranch *sa = nullptr) {
-    Launch L0 = L;        // follows the LOSS conditional node: plain stream order
+// Lf: how the first kernel follows what was launched before it
+void enqueue_core(const Dev &d, Launch L, Launch Lf, cudaEvent_t join = nullptr, const SaBranch *sa = nullptr) {
+    Launch L0 = L;        // follows a join of two branches: plain stream order
     L0.pdl = false;
-    launch_flux_mass_energy(d, L0);
+    launch_flux_mass_energy(d, Lf);
     launch_tstep(d, L, V_RO, 2);
     if (d.ILOS >= 100) launch_roavg_cell(d, L);     // 4255-4267, after TSTEP(RO)
     const bool sab = sa && sa->s && d.ILOS >= 200;
@@ -320,16 +331,16 @@ int enqueue_step(mgpu_handle *h, Prof *prof = nullptr) {
     launch_step_begin(d, L);
     launch_prim(d, L);
     launch_loss(d, L, false);
-    enqueue_core(d, L);
+    enqueue_core(d, L, L);
     enqueue_tail(d, L);
     CK(cudaGetLastError());
     return 0;
 }
 
 // appends an IF conditional node to the graph being captured on h->stream
-// and captures its body (fn) on the side stream; *nbody = the body's nodes
+// and captures its body (fn) on the side stream
 template <typename F>
-int add_conditional(mgpu_handle *h, cudaGraphConditionalHandle hnd, size_t *nbody, F fn) {
+int add_conditional(mgpu_handle *h, cudaGraphConditionalHandle hnd, F fn) {
     cudaStreamCaptureStatus st;
     cudaGraph_t cg = nullptr;
     const cudaGraphNode_t *deps = nullptr;
@@ -346,28 +357,31 @@ int add_conditional(mgpu_handle *h, cudaGraphConditionalHandle hnd, size_t *nbod
     fn(Launch{h->side, h->sm_count, nullptr});
     cudaGraph_t out = nullptr;
     CK(cudaStreamEndCapture(h->side, &out));
-    CK(cudaGraphGetNodes(body, nullptr, nbody));
     CK(cudaStreamUpdateCaptureDependencies(h->stream, &node, nullptr, 1, cudaStreamSetCaptureDependencies));
     return 0;
 }
 
 // Records one LOOP iteration of h on h->stream, which must be capturing
-// (alone, or as one branch of a batch graph): the LOSS and tail kernels sit
-// in conditional bodies that the step-control kernel switches on only on
-// the steps that need them.
-int capture_step(mgpu_handle *h) {
+// (alone, or as one branch of a batch graph).  what >= 0: the iteration that
+// runs LOSS (bit 0) and the tail (bit 1) or not, as the caller knows from
+// the control block; their kernels still test the device's own flags.
+// what < 0: the LOSS and tail kernels sit in conditional bodies that the
+// step-control kernel switches on only on the steps that need them.
+int capture_step(mgpu_handle *h, int what) {
     cudaStreamCaptureStatus st;
     cudaGraph_t cg = nullptr;
     CK(cudaStreamGetCaptureInfo(h->stream, &st, nullptr, &cg, nullptr, nullptr, nullptr));
     cudaGraphConditionalHandle hl = 0, ht = 0;
-    // every handle of a graph belongs to one conditional node: an inviscid
-    // problem (ILOS = 0), which has no LOSS node, creates no LOSS handle
-    if (h->d.ILOS != 0) CK(cudaGraphConditionalHandleCreate(&hl, cg, 0, cudaGraphCondAssignDefault));
-    CK(cudaGraphConditionalHandleCreate(&ht, cg, 0, cudaGraphCondAssignDefault));
     Dev dg = h->d;
-    dg.use_cond = 1;
-    dg.cond_loss = (unsigned long long)hl;
-    dg.cond_tail = (unsigned long long)ht;
+    if (what < 0) {
+        // every handle of a graph belongs to one conditional node: an inviscid
+        // problem (ILOS = 0), which has no LOSS node, creates no LOSS handle
+        if (h->d.ILOS != 0) CK(cudaGraphConditionalHandleCreate(&hl, cg, 0, cudaGraphCondAssignDefault));
+        CK(cudaGraphConditionalHandleCreate(&ht, cg, 0, cudaGraphCondAssignDefault));
+        dg.use_cond = 1;
+        dg.cond_loss = (unsigned long long)hl;
+        dg.cond_tail = (unsigned long long)ht;
+    }
     Launch L{h->stream, h->sm_count, nullptr};
     launch_step_begin(dg, L);
     L.pdl = true;          // kernel-to-kernel edges of the step are programmatic
@@ -378,19 +392,29 @@ int capture_step(mgpu_handle *h) {
     CK(cudaStreamWaitEvent(h->aux, h->ev_fork, 0));
     launch_bc_sums(dg, Launch{h->aux, h->sm_count, nullptr});
     CK(cudaEventRecord(h->ev_join, h->aux));
-    // an inviscid problem (ILOS = 0) has no LOSS node
-    int rc = dg.ILOS == 0 ? 0 : add_conditional(h, hl, &h->loss_nodes, [&](Launch L2) { launch_loss(dg, L2, false); });
     SaBranch sab{h->aux2, h->ev_sa0, h->ev_sa1, h->ev_sa2};
-    if (!rc) enqueue_core(dg, L, h->ev_join, &sab);
-    if (!rc) rc = add_conditional(h, ht, &h->tail_nodes, [&](Launch L2) { enqueue_tail(dg, L2); });
+    if (what >= 0) {
+        if (what & 1) launch_loss(dg, L, false);
+        enqueue_core(dg, L, L, h->ev_join, &sab);
+        if (what & 2) enqueue_tail(dg, L);
+        CK(cudaGetLastError());
+        return 0;
+    }
+    Launch L0 = L;         // follows a conditional node: plain stream order
+    L0.pdl = false;
+    // an inviscid problem (ILOS = 0) has no LOSS node
+    int rc = dg.ILOS == 0 ? 0 : add_conditional(h, hl, [&](Launch L2) { launch_loss(dg, L2, false); });
+    if (!rc) enqueue_core(dg, L, L0, h->ev_join, &sab);
+    if (!rc) rc = add_conditional(h, ht, [&](Launch L2) { enqueue_tail(dg, L2); });
     return rc;
 }
 
-// one LOOP iteration of h as a CUDA graph
-int build_graph(mgpu_handle *h) {
-    if (h->gexec) return 0;
+// one LOOP iteration of h as a CUDA graph, by what it runs
+int build_graph(mgpu_handle *h, int what) {
+    StepGraph &G = h->sg[what];
+    if (G.exec) return 0;
     CK(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
-    int rc = capture_step(h);
+    int rc = capture_step(h, what);
     cudaGraph_t g = nullptr;
     cudaError_t e = cudaStreamEndCapture(h->stream, &g);
     if (rc) {
@@ -398,9 +422,9 @@ int build_graph(mgpu_handle *h) {
         return rc;
     }
     if (e != cudaSuccess) return fail(MGPU_E_CUDA, std::string("graph capture: ") + cudaGetErrorString(e));
-    h->graph = g;
-    CK(cudaGraphGetNodes(g, nullptr, &h->graph_nodes));
-    CK(cudaGraphInstantiate(&h->gexec, g, 0));
+    G.graph = g;
+    CK(cudaGraphGetNodes(g, nullptr, &G.nodes));
+    CK(cudaGraphInstantiate(&G.exec, g, 0));
     return 0;
 }
 
@@ -429,7 +453,40 @@ void fill_monitors(const DevCtl &c, mgpu_monitors *m) {
 int read_ctl(mgpu_handle *h) {
     CK(cudaMemcpyAsync(h->h_ctl, h->d.ctl, sizeof(DevCtl), cudaMemcpyDeviceToHost, h->stream));
     CK(cudaStreamSynchronize(h->stream));
+    h->ctl_known = true;
     return 0;
+}
+
+// What the step after the mirrored control block c runs, q steps on: bit 0
+// LOSS, bit 1 the tail, by the tests of k_step_begin.  q > 0 holds only up
+// to the next tail, which rewrites what the end test reads.
+int step_what(const Dev &d, const DevCtl &c, int q, bool force_end) {
+    const int n = c.nstep + 1 + q;
+    const bool end = c.ifend || force_end || n == d.NSTEPS_MAX || (c.EAVG < d.CONLIM && c.ECONT < 0.01f) ||
+                     (fabsf(c.EMAX) < 4.0f * d.CONLIM && c.ECONT < 0.01f);
+    const bool loss = (d.ILOS == 10 || (d.ILOS >= 100 && d.ILOS < 300)) && n % d.NLOS == 0 && !d.FROZEN;
+    return (loss ? 1 : 0) | (n % 5 == 0 || end ? 2 : 0);
+}
+
+// launches the steps that follow the mirrored control block, none of them
+// past the next tail
+int launch_steps(mgpu_handle *h, int n, bool force_end) {
+    h->ctl_known = false;
+    for (int q = 0; q < n; ++q) {
+        const int what = step_what(h->d, *h->h_ctl, q, force_end);
+        int rc = build_graph(h, what);
+        if (rc) return rc;
+        CK(cudaGraphLaunch(h->sg[what].exec, h->stream));
+    }
+    return 0;
+}
+
+// the number of steps from the mirrored control block to the next tail
+int steps_to_tail(const Dev &d, const DevCtl &c) {
+    if (step_what(d, c, 0, false) & 2) return 1;
+    int n = (c.nstep / 5 + 1) * 5 - c.nstep;
+    if (d.NSTEPS_MAX > c.nstep && d.NSTEPS_MAX - c.nstep < n) n = d.NSTEPS_MAX - c.nstep;
+    return n;
 }
 
 }  // namespace
@@ -440,7 +497,7 @@ HandleView handle_view(const mgpu_handle *h) { return HandleView{&h->d, h->strea
 
 int api_fail(int code, const char *msg) { return fail(code, msg); }
 
-void enqueue_step_core(const Dev &d, Launch L) { enqueue_core(d, L); }
+void enqueue_step_core(const Dev &d, Launch L) { enqueue_core(d, L, L); }
 AdjState *&handle_adj(mgpu_handle *h) { return h->adj; }
 Dev &handle_dev(mgpu_handle *h) { return h->d; }
 int handle_sm_count(const mgpu_handle *h) { return h->sm_count; }
@@ -582,8 +639,7 @@ void mgpu_destroy(mgpu_handle *h) {
     if (h->stream) cudaStreamSynchronize(h->stream);
     if (h->adj) adj_destroy(h->adj);
     if (h->flush_buf) cudaFree(h->flush_buf);
-    if (h->gexec) cudaGraphExecDestroy(h->gexec);
-    if (h->graph) cudaGraphDestroy(h->graph);
+    for (StepGraph &G : h->sg) G.drop();
     for (void *p : h->allocs) cudaFree(p);
     if (h->h_ctl) cudaFreeHost(h->h_ctl);
     if (h->stream) cudaStreamDestroy(h->stream);
@@ -1019,6 +1075,7 @@ int32_t mgpu_stepup(mgpu_handle *h, float relax) {
 
 int32_t mgpu_loss_init(mgpu_handle *h) {
     if (!h || !h->committed) return fail(MGPU_E_STATE, "loss_init before commit");
+    h->ctl_known = false;
     Launch L{h->stream, h->sm_count};
     launch_loss(h->d, L, true);
     CK(cudaGetLastError());
@@ -1028,11 +1085,11 @@ int32_t mgpu_loss_init(mgpu_handle *h) {
 
 int32_t mgpu_step(mgpu_handle *h, int32_t force_end, mgpu_monitors *mon) {
     if (!h || !h->committed) return fail(MGPU_E_STATE, "step before commit");
-    int rc = build_graph(h);
-    if (rc) return rc;
+    int rc = 0;
+    if (!h->ctl_known && (rc = read_ctl(h))) return rc;
     int fe = force_end ? 1 : 0;
     CK(cudaMemcpyAsync(&h->d.ctl->force_end, &fe, sizeof(int), cudaMemcpyHostToDevice, h->stream));
-    CK(cudaGraphLaunch(h->gexec, h->stream));
+    if ((rc = launch_steps(h, 1, fe != 0))) return rc;
     if ((rc = read_ctl(h))) return rc;
     const DevCtl &c = *h->h_ctl;
     if (mon) fill_monitors(c, mon);
@@ -1043,8 +1100,7 @@ int32_t mgpu_step(mgpu_handle *h, int32_t force_end, mgpu_monitors *mon) {
 int32_t mgpu_run(mgpu_handle *h, int32_t nsteps, mgpu_monitors *mon) {
     if (!h || !h->committed) return fail(MGPU_E_STATE, "run before commit");
     if (nsteps < 0) return fail(MGPU_E_ARG, "negative step count");
-    int rc = build_graph(h);
-    if (rc) return rc;
+    int rc = 0;
     // The end test at the top of step n (3762-3764) reads NSTEP and the
     // monitors EMAX, EAVG and ECONT, which only a tail (every fifth step, or
     // the final one) rewrites.  So no step after a tail up to and including
@@ -1052,7 +1108,7 @@ int32_t mgpu_run(mgpu_handle *h, int32_t nsteps, mgpu_monitors *mon) {
     // NSTEPS_MAX falls among them: such a run of steps is launched back to
     // back, then the control block is read, and the run stops right after
     // the final step, where LOOP stops (5444-5451).
-    if ((rc = read_ctl(h))) return rc;
+    if (!h->ctl_known && (rc = read_ctl(h))) return rc;
     int done = 0;
     for (;;) {
         const DevCtl &c = *h->h_ctl;
@@ -1063,14 +1119,9 @@ int32_t mgpu_run(mgpu_handle *h, int32_t nsteps, mgpu_monitors *mon) {
             return fail(MGPU_E_NONFINITE, "non-finite or non-positive density in the flow field");
         if (c.ifend) return 1;
         if (done >= nsteps) return 0;
-        const int n0 = c.nstep;
-        int n = 1;                              // a met test makes the next step the final one
-        if (!c.converged) {
-            n = (n0 / 5 + 1) * 5 - n0;          // up to the next tail
-            if (h->d.NSTEPS_MAX > n0 && h->d.NSTEPS_MAX - n0 < n) n = h->d.NSTEPS_MAX - n0;
-        }
+        int n = steps_to_tail(h->d, c);
         if (n > nsteps - done) n = nsteps - done;
-        for (int s = 0; s < n; ++s) CK(cudaGraphLaunch(h->gexec, h->stream));
+        if ((rc = launch_steps(h, n, false))) return rc;
         done += n;
         if ((rc = read_ctl(h))) return rc;
     }
@@ -1313,14 +1364,7 @@ int32_t mgpu_autotune(mgpu_handle *h, int32_t *chosen, double *ms) {
     if (d.ts_bs[0] != cand[best[0]] || d.ts_bs[1] != cand[best[1]]) {
         d.ts_bs[0] = cand[best[0]];
         d.ts_bs[1] = cand[best[1]];
-        if (h->gexec) {
-            cudaGraphExecDestroy(h->gexec);
-            h->gexec = nullptr;
-        }
-        if (h->graph) {
-            cudaGraphDestroy(h->graph);
-            h->graph = nullptr;
-        }
+        for (StepGraph &G : h->sg) G.drop();
     }
     if (chosen) {
         chosen[0] = cand[best[0]];
@@ -1334,8 +1378,7 @@ int32_t mgpu_autotune(mgpu_handle *h, int32_t *chosen, double *ms) {
 
 int32_t mgpu_bench_steps(mgpu_handle *h, int32_t nsteps, int32_t flush_l2, double *total_ms) {
     if (!h || !h->committed || !total_ms || nsteps < 0) return fail(MGPU_E_ARG, "bad arguments to mgpu_bench_steps");
-    int rc = build_graph(h);
-    if (rc) return rc;
+    int rc = 0;
     if (flush_l2 && !h->flush_buf) {
         int l2 = 0;
         cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, h->device);
@@ -1344,11 +1387,21 @@ int32_t mgpu_bench_steps(mgpu_handle *h, int32_t nsteps, int32_t flush_l2, doubl
     }
     std::vector<cudaEvent_t> ev((size_t)2 * nsteps);
     for (auto &e : ev) CK(cudaEventCreate(&e));
-    for (int s = 0; s < nsteps; ++s) {
-        if (flush_l2) CK(cudaMemsetAsync(h->flush_buf, s & 0xff, h->flush_bytes, h->stream));
-        CK(cudaEventRecord(ev[2 * s], h->stream));
-        CK(cudaGraphLaunch(h->gexec, h->stream));
-        CK(cudaEventRecord(ev[2 * s + 1], h->stream));
+    // the steps up to each tail are queued together; the control block is
+    // read after each tail, outside the events
+    for (int s = 0; s < nsteps;) {
+        if (!h->ctl_known && (rc = read_ctl(h))) return rc;
+        int n = steps_to_tail(h->d, *h->h_ctl);
+        if (n > nsteps - s) n = nsteps - s;
+        h->ctl_known = false;
+        for (int q = 0; q < n; ++q, ++s) {
+            const int what = step_what(h->d, *h->h_ctl, q, false);
+            if ((rc = build_graph(h, what))) return rc;
+            if (flush_l2) CK(cudaMemsetAsync(h->flush_buf, s & 0xff, h->flush_bytes, h->stream));
+            CK(cudaEventRecord(ev[2 * s], h->stream));
+            CK(cudaGraphLaunch(h->sg[what].exec, h->stream));
+            CK(cudaEventRecord(ev[2 * s + 1], h->stream));
+        }
     }
     CK(cudaStreamSynchronize(h->stream));
     double tot = 0.0;
@@ -1367,6 +1420,7 @@ int32_t mgpu_bench_steps(mgpu_handle *h, int32_t nsteps, int32_t flush_l2, doubl
 int32_t mgpu_profile_steps(mgpu_handle *h, int32_t nsteps, mgpu_kernel_time *out, int32_t max_entries,
                            int32_t *n_out) {
     if (!h || !h->committed || !out || !n_out || nsteps < 0) return fail(MGPU_E_ARG, "bad arguments to mgpu_profile_steps");
+    h->ctl_known = false;
     std::map<std::string, std::pair<int, double>> acc;
     std::vector<std::string> order;
     for (int s = 0; s < nsteps; ++s) {
@@ -1451,7 +1505,7 @@ int32_t mgpu_batch_create(mgpu_handle *const *handles, int32_t n, mgpu_batch **o
         mgpu_handle *h = b->hs[i];
         e = cudaStreamWaitEvent(h->stream, b->fork, 0);
         if (e != cudaSuccess) break;
-        rc = capture_step(h);
+        rc = capture_step(h, -1);
         if (rc) break;
         e = cudaEventRecord(b->joins[i], h->stream);
         if (e == cudaSuccess) e = cudaStreamWaitEvent(b->stream, b->joins[i], 0);
@@ -1477,6 +1531,7 @@ int batch_read(mgpu_batch *b, mgpu_monitors *mons, int *ended) {
     for (mgpu_handle *h : b->hs)
         CK(cudaMemcpyAsync(h->h_ctl, h->d.ctl, sizeof(DevCtl), cudaMemcpyDeviceToHost, b->stream));
     CK(cudaStreamSynchronize(b->stream));
+    for (mgpu_handle *h : b->hs) h->ctl_known = true;
     int nend = 0;
     for (size_t i = 0; i < b->hs.size(); ++i) {
         const DevCtl &c = *b->hs[i]->h_ctl;
@@ -1497,6 +1552,7 @@ int32_t mgpu_batch_run(mgpu_batch *b, int32_t nsteps, mgpu_monitors *mons) {
     if (!b || nsteps < 0) return fail(MGPU_E_ARG, "bad arguments to mgpu_batch_run");
     const int chunk = 50;
     int done = 0, ended = 0, rc = 0;
+    for (mgpu_handle *h : b->hs) h->ctl_known = false;
     while (done < nsteps) {
         int m = nsteps - done < chunk ? nsteps - done : chunk;
         for (int s = 0; s < m; ++s) CK(cudaGraphLaunch(b->gexec, b->stream));
@@ -1515,6 +1571,7 @@ int32_t mgpu_batch_bench_steps(mgpu_batch *b, int32_t nsteps, int32_t flush_l2, 
         b->flush_bytes = (size_t)(l2 > 0 ? l2 : 128 << 20) * 2;
         CK(cudaMalloc(&b->flush_buf, b->flush_bytes));
     }
+    for (mgpu_handle *h : b->hs) h->ctl_known = false;
     std::vector<cudaEvent_t> ev((size_t)2 * nsteps);
     for (auto &e : ev) CK(cudaEventCreate(&e));
     for (int s = 0; s < nsteps; ++s) {
@@ -1539,12 +1596,9 @@ int32_t mgpu_batch_bench_steps(mgpu_batch *b, int32_t nsteps, int32_t flush_l2, 
 int32_t mgpu_kernels_per_step(mgpu_handle *h, int32_t which) {
     if (!h || !h->committed) return fail(MGPU_E_STATE, "kernels_per_step before commit");
     if (which < 0 || which > 3) return fail(MGPU_E_ARG, "kernels_per_step: which must be 0..3");
-    int rc = build_graph(h);
+    int rc = build_graph(h, which);
     if (rc) return rc;
-    size_t n = h->graph_nodes - 2;   // every top-level node but the two conditionals is a kernel
-    if (which & 1) n += h->loss_nodes;
-    if (which & 2) n += h->tail_nodes;
-    return (int32_t)n;
+    return (int32_t)h->sg[which].nodes;   // every node is a kernel
 }
 
 }  // extern "C"
