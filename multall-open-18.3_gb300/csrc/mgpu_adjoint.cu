@@ -2398,7 +2398,7 @@ int32_t mgpu_adjoint_prepare(mgpu_handle *h) {
     ACK(cudaMemsetAsync(s->flag, 0, sizeof(int), st));
     Launch L{st, handle_sm_count(h)};
     launch_step_begin(rec, L);
-    launch_prim(rec, L);
+    launch_prim(rec, L, -1);
     enqueue_step_core(rec, L);
     ACK(cudaGetLastError());
     ACK(cp(a.tVX, d.VX, N)); ACK(cp(a.tVR, d.VR, N)); ACK(cp(a.tVT, d.VT, N)); ACK(cp(a.tROVT, d.ROVT, N));

@@ -318,21 +318,16 @@ void enqueue_core(const Dev &d, Launch L, Launch Lf, cudaEvent_t join = nullptr,
     if (d.any_cusp2) launch_cusp(d, L);
 }
 
-void enqueue_tail(const Dev &d, Launch L) {
-    launch_tail(d, L);
-    launch_stepup(d, L, 0.25f, true);
-}
-
 // kernel by kernel, every kernel present (LOSS and tail kernels return
 // early when their flag is off); used for profiling
 int enqueue_step(mgpu_handle *h, Prof *prof = nullptr) {
     const Dev &d = h->d;
     Launch L{h->stream, h->sm_count, prof};
     launch_step_begin(d, L);
-    launch_prim(d, L);
+    launch_prim(d, L, -1);
     launch_loss(d, L, false);
     enqueue_core(d, L, L);
-    enqueue_tail(d, L);
+    launch_tail(d, L);
     CK(cudaGetLastError());
     return 0;
 }
@@ -383,9 +378,12 @@ int capture_step(mgpu_handle *h, int what) {
         dg.cond_tail = (unsigned long long)ht;
     }
     Launch L{h->stream, h->sm_count, nullptr};
-    launch_step_begin(dg, L);
-    L.pdl = true;          // kernel-to-kernel edges of the step are programmatic
-    launch_prim(dg, L);
+    if (what < 0) {
+        launch_step_begin(dg, L);
+        L.pdl = true;      // kernel-to-kernel edges of the step are programmatic
+    }
+    launch_prim(dg, L, what);
+    L.pdl = true;
     // the exit-pressure sums depend on nothing the next kernels write, so they
     // run beside LOSS, the mass/energy fluxes and TSTEP(RO, ROE)
     CK(cudaEventRecord(h->ev_fork, h->stream));
@@ -396,7 +394,7 @@ int capture_step(mgpu_handle *h, int what) {
     if (what >= 0) {
         if (what & 1) launch_loss(dg, L, false);
         enqueue_core(dg, L, L, h->ev_join, &sab);
-        if (what & 2) enqueue_tail(dg, L);
+        if (what & 2) launch_tail(dg, L);
         CK(cudaGetLastError());
         return 0;
     }
@@ -405,7 +403,7 @@ int capture_step(mgpu_handle *h, int what) {
     // an inviscid problem (ILOS = 0) has no LOSS node
     int rc = dg.ILOS == 0 ? 0 : add_conditional(h, hl, [&](Launch L2) { launch_loss(dg, L2, false); });
     if (!rc) enqueue_core(dg, L, L0, h->ev_join, &sab);
-    if (!rc) rc = add_conditional(h, ht, [&](Launch L2) { enqueue_tail(dg, L2); });
+    if (!rc) rc = add_conditional(h, ht, [&](Launch L2) { launch_tail(dg, L2); });
     return rc;
 }
 
@@ -1067,7 +1065,7 @@ int32_t mgpu_commit(mgpu_handle *h) {
 int32_t mgpu_stepup(mgpu_handle *h, float relax) {
     if (!h || !h->committed) return fail(MGPU_E_STATE, "stepup before commit");
     Launch L{h->stream, h->sm_count};
-    launch_stepup(h->d, L, relax, false);
+    launch_stepup(h->d, L, relax);
     CK(cudaGetLastError());
     CK(cudaStreamSynchronize(h->stream));
     return 0;

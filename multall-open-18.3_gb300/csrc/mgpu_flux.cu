@@ -20,8 +20,7 @@ static inline unsigned grid_for(size_t n, unsigned block) { return (unsigned)((n
 // (multall-open-18.3.f:3759-3815), and the viscosity update LOSS makes on
 // entry (8088-8112).
 // ---------------------------------------------------------------------
-__global__ void k_step_begin(Dev d) {
-    pdl_wait();
+__device__ __noinline__ void step_control(const Dev &d) {
     DevCtl *c = d.ctl;
     int n = c->nstep + 1;
     c->nstep = n;
@@ -59,13 +58,12 @@ __global__ void k_step_begin(Dev d) {
         if (d.ILOS != 0) cudaGraphSetConditional((cudaGraphConditionalHandle)d.cond_loss, c->do_loss ? 1u : 0u);
         cudaGraphSetConditional((cudaGraphConditionalHandle)d.cond_tail, c->do_tail ? 1u : 0u);
     }
-    if (c->do_tail) {
-        c->mon.vrms = 0.0;
-        c->mon.vmax_key = 0ull;
-        c->mon.eavg_sum = 0.0;
-        c->mon.emax_key = 0ull;
-        c->mon.health = 0;
-    }
+    if (c->do_loss) loss_viscosity(d, c, n);
+}
+
+__global__ void k_step_begin(const __grid_constant__ Dev d) {
+    pdl_wait();
+    step_control(d);
 }
 
 void launch_step_begin(const Dev &d, Launch L) {
@@ -77,45 +75,23 @@ void launch_step_begin(const Dev &d, Launch L) {
 // primitive variables (7450) and P, HO, T (5900); with the 5-step tail
 // also the sum and the maximum of |W|^2 (5910, uses the previous WT).
 // ---------------------------------------------------------------------
-template <int BS>
-__device__ inline void block_reduce_sum_key(int order, double s, unsigned long long key, double *out_s,
-                                            unsigned long long *out_k) {
-    __shared__ double ss[BS / 32];
-    __shared__ unsigned long long sk[BS / 32];
-    for (int o = 16; o > 0; o >>= 1) {
-        s = racc(order, s, __shfl_down_sync(0xffffffffu, s, o));
-        unsigned long long ok = __shfl_down_sync(0xffffffffu, key, o);
-        key = ok > key ? ok : key;
-    }
-    int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-    if (l == 0) {
-        ss[w] = s;
-        sk[w] = key;
-    }
-    __syncthreads();
-    if (w == 0) {
-        s = l < BS / 32 ? ss[l] : 0.0;
-        key = l < BS / 32 ? sk[l] : 0ull;
-        for (int o = 16; o > 0; o >>= 1) {
-            s = racc(order, s, __shfl_down_sync(0xffffffffu, s, o));
-            unsigned long long ok = __shfl_down_sync(0xffffffffu, key, o);
-            key = ok > key ? ok : key;
-        }
-        if (l == 0) {
-            *out_s = s;
-            *out_k = key;
-        }
-    }
-}
-
 constexpr int PRIM_BS = 256;
 
-__global__ void __launch_bounds__(PRIM_BS) k_prim(Dev d) {
+// One thread a node; the first grid_for(N) CTAs.  what >= 0: one more CTA
+// runs the step control, whose only effect on this kernel, the tail flag,
+// the host knows already.  On a step with the tail the last CTA turns the
+// partial sums into VREF and VMAX.
+__global__ void __launch_bounds__(PRIM_BS) k_prim(const __grid_constant__ Dev d, int what) {
     pdl_wait();
+    const unsigned nblk = gridDim.x - (what >= 0 ? 1 : 0);
+    if (blockIdx.x == nblk) {
+        if (threadIdx.x == 0) step_control(d);
+        return;
+    }
     size_t n = (size_t)blockIdx.x * PRIM_BS + threadIdx.x;
     size_t N = (size_t)d.IM * d.JM * d.KM;
-    int do_tail = d.ctl->do_tail;
-    double eke_s = 0.0;
+    const bool do_tail = what >= 0 ? (what & 2) != 0 : d.ctl->do_tail != 0;
+    float eke_s = 0.0f;
     unsigned long long key = 0ull;
     if (n < N) {
         int i, j, k;
@@ -138,7 +114,7 @@ __global__ void __launch_bounds__(PRIM_BS) k_prim(Dev d) {
             d.VT[n] = vt;
             if (do_tail) {
                 float EKE = vr * vr + wt * wt + vx * vx;
-                eke_s = (double)EKE;
+                eke_s = EKE;
                 key = max_key(EKE, n);
             }
             if (thermo) {
@@ -150,13 +126,39 @@ __global__ void __launch_bounds__(PRIM_BS) k_prim(Dev d) {
             }
         }
     }
-    if (do_tail)
-        block_reduce_sum_key<PRIM_BS>(d.REDUCE_ORDER, eke_s, key, &d.part_sum[blockIdx.x], &d.part_key[blockIdx.x]);
+    if (!do_tail) return;
+    df s;
+    cta_sum_key<PRIM_BS>(d.REDUCE_ORDER, df_of(eke_s), key, &s, &key);
+    if (threadIdx.x == 0) {
+        d.part_sum[blockIdx.x] = s;
+        d.part_key[blockIdx.x] = key;
+    }
+    if (!last_cta(&d.ctl->ticket, nblk)) return;
+    s = df_of(0.0f);
+    key = 0ull;
+    for (unsigned p = threadIdx.x; p < nblk; p += PRIM_BS) {
+        s = dacc(d.REDUCE_ORDER, s, d.part_sum[p]);
+        const unsigned long long k2 = d.part_key[p];
+        key = k2 > key ? k2 : key;
+    }
+    cta_sum_key<PRIM_BS>(d.REDUCE_ORDER, s, key, &s, &key);
+    if (threadIdx.x == 0) {
+        DevCtl *c = d.ctl;
+        c->VREF = sqrtf(df_val(s) * d.RIJKM);
+        c->VMAX = 0.0f;
+        if (key) {
+            const unsigned lin = 0xFFFFFFFFu - (unsigned)(key & 0xFFFFFFFFull);
+            c->VMAX = sqrtf(__uint_as_float((unsigned)(key >> 32)));
+            c->IVMAX = (int)(lin % d.IM) + 1;
+            c->JVMAX = (int)((lin / d.IM) % d.JM) + 1;
+            c->KVMAX = (int)(lin / ((unsigned)d.IM * d.JM)) + 1;
+        }
+    }
 }
 
-void launch_prim(const Dev &d, Launch L) {
+void launch_prim(const Dev &d, Launch L, int what) {
     size_t N = (size_t)d.IM * d.JM * d.KM;
-    launchk(L, k_prim, dim3(grid_for(N, PRIM_BS)), dim3(PRIM_BS), 0, d);
+    launchk(L, k_prim, dim3(grid_for(N, PRIM_BS) + (what >= 0 ? 1 : 0)), dim3(PRIM_BS), 0, d, what);
     mark(L, "k_prim");
 }
 

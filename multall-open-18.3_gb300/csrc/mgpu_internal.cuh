@@ -24,16 +24,6 @@ namespace mgpu {
 #define MGPU_T_INT32 int32_t
 #define MGPU_T_FLOAT32 float
 
-// Reduction slots written by the step and read back by the host.
-struct DevMon {
-    double vrms;            // sum of |W|^2 (VRMS)
-    unsigned long long vmax_key;
-    double eavg_sum;
-    unsigned long long emax_key;
-    int health;
-    int pad;
-};
-
 // State that changes from step to step; one per problem, in device memory.
 struct DevCtl {
     int nstep;        // NSTEP
@@ -51,7 +41,7 @@ struct DevCtl {
     int IMAXE, JMAXE, KMAXE, JCONT, IVMAX, JVMAX, KVMAX;
     int health;
     double flow_in, flow_out;
-    DevMon mon;
+    unsigned ticket;  // CTAs of the running launch that have delivered their partial sums (last_cta)
     // exit pressures that the throttle condition moves from step to step
     // (4488-4505), and CHECK_FLOW(JM) of the last tail
     float PDOWN_HUB, PDOWN_TIP, THROTTLE_PRES, CHECK_FLOW_JM;
@@ -128,7 +118,7 @@ struct Dev {
     float *ADJ_RO_MACH;    // RO as the Mach limiter finds it
     double *BLADE_FLOW;                // (JM)
     // per-block reduction partials of the 5-step tail
-    double *part_sum;
+    df *part_sum;
     unsigned long long *part_key;
     int *part_cnt;
     int nparts;
@@ -221,11 +211,82 @@ __device__ __forceinline__ df dacc(int order, df s, df x) {
     return order == 2 ? df{s.hi + x.hi, 0.0f} : df_add(s, x);
 }
 
+// Sum of one FP32 value a thread and the largest key over a CTA of BS
+// threads, for the monitors: thread 0 receives both.  REDUCE_ORDER 2 adds in
+// FP32, the other orders in double-float, which leaves the FP64 pipe alone
+// (an FP64 tree over every node made k_prim 40 us instead of 12 on the steps
+// that run the tail, 65 x 242 x 49).  The key's halves go through the warp's
+// integer maximum.
+__device__ __forceinline__ unsigned long long warp_max_key(unsigned long long key) {
+    const unsigned hi = (unsigned)(key >> 32), m = __reduce_max_sync(0xffffffffu, hi);
+    const unsigned lo = __reduce_max_sync(0xffffffffu, hi == m ? (unsigned)key : 0u);
+    return ((unsigned long long)m << 32) | lo;
+}
+template <int BS>
+__device__ __forceinline__ void cta_sum_key(int order, df s, unsigned long long key, df *out_s,
+                                            unsigned long long *out_k) {
+    __shared__ df ss[BS / 32];
+    __shared__ unsigned long long sk[BS / 32];
+    for (int o = 16; o > 0; o >>= 1) s = dacc(order, s, df_shfl_down(s, o));
+    key = warp_max_key(key);
+    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+    if (l == 0) {
+        ss[w] = s;
+        sk[w] = key;
+    }
+    __syncthreads();
+    if (w == 0) {
+        s = l < BS / 32 ? ss[l] : df{0.0f, 0.0f};
+        key = l < BS / 32 ? sk[l] : 0ull;
+        for (int o = BS / 64; o > 0; o >>= 1) s = dacc(order, s, df_shfl_down(s, o));
+        key = warp_max_key(key);
+        *out_s = s;
+        *out_k = key;
+    }
+}
+
+// True in every thread of the CTA that is the last of a launch's n CTAs to
+// get here; what the others stored before it is then visible to it.  The
+// ticket is back at zero afterwards.
+__device__ __forceinline__ bool last_cta(unsigned *ticket, unsigned n) {
+    __shared__ unsigned s_last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) s_last = atomicInc(ticket, n - 1) == n - 1;
+    __syncthreads();
+    if (!s_last) return false;
+    __threadfence();
+    return true;
+}
+
 // Order-preserving key for "largest value, earliest index wins": the value
 // must be >= 0 (squares, absolute values); NaN counts as smallest.
 __device__ inline unsigned long long max_key(float v, size_t lin) {
     if (!(v >= 0.0f)) return 0ull;
     return ((unsigned long long)__float_as_uint(v) << 32) | (unsigned long long)(0xFFFFFFFFu - (unsigned)lin);
+}
+
+// The viscosity that LOSS, NEW_LOSS and SPAL_LOSS set on entry (8088-8112,
+// 12545-12568), by one thread: nothing it reads changes between the start of
+// the step, where step_control calls it on the steps that run them, and LOSS.
+__device__ inline void loss_viscosity(const Dev &d, DevCtl *c, int nstep) {
+    float VISLAM = c->VISLAM;
+    if (nstep == 1 || nstep < d.NSTEPS_MAX / 4) {
+        if (d.REYNO > 100.0f) {
+            int J1 = A1(d.JLE, 1), J2 = A1(d.JTE, 1);
+            if (A1(d.JLE, 1) > d.JM) J1 = 1;
+            if (A1(d.JTE, 1) > d.JM) J2 = d.JM;
+            float XCHORD = A2(d.SMERID, J2, d.KMID) - A2(d.SMERID, J1, d.KMID);
+            float a = A3(d.ROVX, d.IMID, J2, d.KMID), b = A3(d.ROVR, d.IMID, J2, d.KMID), cc = A3(d.ROWT, d.IMID, J2, d.KMID);
+            float ROW2 = sqrtf(a * a + b * b + cc * cc);
+            VISLAM = XCHORD * ROW2 / d.REYNO;
+        }
+        if (d.REYNO > 0.0f && d.REYNO < 99.99f) VISLAM = d.REYNO / 100000.0f;
+        if (d.REYNO < 0.0f) VISLAM = -d.REYNO * 1.0E-5f;
+        float TCOND = d.CP * VISLAM / d.PRANDTL;
+        c->FTCOND = TCOND / VISLAM;
+        c->VISLAM = VISLAM;
+    }
 }
 
 // ---------------------------------------------------------------------
@@ -284,13 +345,15 @@ inline void mark(const Launch &L, const char *name) {
 }
 
 void launch_step_begin(const Dev &d, Launch L);
-void launch_prim(const Dev &d, Launch L);
+// what < 0: the step control has run (k_step_begin); otherwise the launch
+// runs it too, for a step of which the host knows that the tail runs (bit 1)
+void launch_prim(const Dev &d, Launch L, int what);
 void launch_loss(const Dev &d, Launch L, bool init_call);
 void launch_new_loss(const Dev &d, Launch L, bool init_call);
 // pieces NEW_LOSS and SPAL_LOSS share: the laminar viscosity for the first
 // quarter of the steps, SET_PWALLGRAD, and the wall shear stresses, face
 // stresses and force update (mgpu_loss.cu)
-void launch_loss_prologue(const Dev &d, Launch L, bool init_call);
+void launch_loss_prologue(const Dev &d, Launch L);
 void launch_pwallgrad(const Dev &d, Launch L, bool init_call);
 void launch_viscous_walls_and_forces(const Dev &d, Launch L, bool init_call);
 void launch_roavg_cell(const Dev &d, Launch L);
@@ -326,7 +389,7 @@ size_t sa_work_floats(const Dev &d);
 // viscosity), mgpu_tstep.cu
 void launch_tstep_cells_prolong(const Dev &d, Launch L, int v0, int nv);
 void launch_tail(const Dev &d, Launch L);
-void launch_stepup(const Dev &d, Launch L, float relax, bool gated);
+void launch_stepup(const Dev &d, Launch L, float relax);
 void launch_integrals(const Dev &d, Launch L, double *out8);
 
 // Raises a kernel's dynamic shared-memory limit to `bytes` (at least the

@@ -14,29 +14,10 @@ namespace mgpu {
 static inline unsigned grid_for(size_t n, unsigned block) { return (unsigned)((n + block - 1) / block); }
 
 
-// viscosity set on entry to LOSS (8088-8112); one thread
-__global__ void k_loss_prologue(Dev d, int init_call) {
+// the viscosity of SETUP's first LOSS; in a step, step_control has set it
+__global__ void k_loss_prologue(const __grid_constant__ Dev d) {
     pdl_wait();
-    DevCtl *c = d.ctl;
-    if (!init_call && !c->do_loss) return;
-    int nstep = init_call ? 1 : c->nstep;
-    float VISLAM = c->VISLAM;
-    if (nstep == 1 || nstep < d.NSTEPS_MAX / 4) {
-        if (d.REYNO > 100.0f) {
-            int J1 = A1(d.JLE, 1), J2 = A1(d.JTE, 1);
-            if (A1(d.JLE, 1) > d.JM) J1 = 1;
-            if (A1(d.JTE, 1) > d.JM) J2 = d.JM;
-            float XCHORD = A2(d.SMERID, J2, d.KMID) - A2(d.SMERID, J1, d.KMID);
-            float a = A3(d.ROVX, d.IMID, J2, d.KMID), b = A3(d.ROVR, d.IMID, J2, d.KMID), cc = A3(d.ROWT, d.IMID, J2, d.KMID);
-            float ROW2 = sqrtf(a * a + b * b + cc * cc);
-            VISLAM = XCHORD * ROW2 / d.REYNO;
-        }
-        if (d.REYNO > 0.0f && d.REYNO < 99.99f) VISLAM = d.REYNO / 100000.0f;
-        if (d.REYNO < 0.0f) VISLAM = -d.REYNO * 1.0E-5f;
-        float TCOND = d.CP * VISLAM / d.PRANDTL;
-        c->FTCOND = TCOND / VISLAM;
-        c->VISLAM = VISLAM;
-    }
+    loss_viscosity(d, d.ctl, 1);
 }
 
 // Shih et al. wall function (WALLFUN).  DPDS is the caller's DPDS_CELL
@@ -684,8 +665,7 @@ void launch_loss(const Dev &d, Launch L, bool init_call) {
         launch_new_loss(d, L, init_call);
         return;
     }
-    launchk(L, k_loss_prologue, dim3(1), dim3(1), 0, d, init_call ? 1 : 0);
-    mark(L, "k_loss_prologue");
+    if (init_call) launch_loss_prologue(d, L);
     if (d.YPLUSWALL < -10.0f) {
         int nc = d.IMM1 * d.KMM1 * (d.JM - 1);
         launchk(L, k_pwallgrad_cells, dim3((nc + 255) / 256), dim3(256), 0, d, init_call ? 1 : 0);
@@ -730,66 +710,40 @@ __global__ void __launch_bounds__(TAIL_BS) k_tail_flow(Dev d) {
     }
 }
 
-// finishes the |W|^2 reduction of k_prim: VREF and VMAX
-__global__ void k_tail_vref(Dev d, int nparts) {
+// VSOUND / (|W| + c) of node n, c and |W| limited below (STEPUP 7916-7950)
+struct StepupLimits {
+    float TLIM, VLIM;
+};
+__device__ __forceinline__ StepupLimits stepup_limits(const Dev &d) {
+    const float vm = A1(d.VM1, d.KMID);
+    return {0.1f * A1(d.TO1, d.KMID), 0.01f * vm * vm};
+}
+__device__ __forceinline__ float stepup_node(const Dev &d, StepupLimits q, float vx, float vt, float vr, float ho, float wt) {
+    float VSQ = vx * vx + vt * vt + vr * vr;
+    float HSTAT = ho - 0.5f * VSQ;
+    float TSTATIC = HSTAT * d.RCP;
+    if (TSTATIC < q.TLIM) TSTATIC = q.TLIM;
+    float WSQ = VSQ - (vt * vt - wt * wt);
+    if (WSQ < q.VLIM) WSQ = q.VLIM;
+    float V_SONIC = sqrtf(d.GA * d.RGAS * TSTATIC);
+    float VPLUSC = sqrtf(WSQ) + V_SONIC;
+    return d.VSOUND / VPLUSC;
+}
+
+// The tail's node pass: the % change of Vm with its sum and maximum, the
+// health count, and STEPUP's node values (TEMP1).  Each thread takes TAIL_NPT
+// nodes (TAIL_BS apart, so the loads stay coalesced), two at a time with all
+// loads of the two in flight, and adds their |DVMER| in FP32 before the CTA's
+// sum.  The last CTA forms EAVG, EMAX and the continuity error ECONT.
+constexpr int TAIL_NPT = 8;
+
+__global__ void __launch_bounds__(TAIL_BS) k_tail_nodes(const __grid_constant__ Dev d) {
     pdl_wait();
     DevCtl *c = d.ctl;
     if (!c->do_tail) return;
-    const int ro = d.REDUCE_ORDER;
-    double s = 0.0;
-    unsigned long long key = 0ull;
-    for (int p = threadIdx.x; p < nparts; p += blockDim.x) {
-        s = racc(ro, s, d.part_sum[p]);
-        unsigned long long k2 = d.part_key[p];
-        key = k2 > key ? k2 : key;
-    }
-    __shared__ double ss[32];
-    __shared__ unsigned long long sk[32];
-    for (int o = 16; o > 0; o >>= 1) {
-        s = racc(ro, s, __shfl_down_sync(0xffffffffu, s, o));
-        unsigned long long ok = __shfl_down_sync(0xffffffffu, key, o);
-        key = ok > key ? ok : key;
-    }
-    if ((threadIdx.x & 31) == 0) {
-        ss[threadIdx.x >> 5] = s;
-        sk[threadIdx.x >> 5] = key;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double t = 0.0;
-        unsigned long long kk = 0ull;
-        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) {
-            t = racc(ro, t, ss[w]);
-            kk = sk[w] > kk ? sk[w] : kk;
-        }
-        c->mon.vrms = t;
-        float vrms = (float)t;
-        c->VREF = sqrtf(vrms * d.RIJKM);
-        if (kk) {
-            unsigned lin = 0xFFFFFFFFu - (unsigned)(kk & 0xFFFFFFFFull);
-            float v = __uint_as_float((unsigned)(kk >> 32));
-            c->VMAX = sqrtf(v);
-            c->IVMAX = (int)(lin % d.IM) + 1;
-            c->JVMAX = (int)((lin / d.IM) % d.JM) + 1;
-            c->KVMAX = (int)(lin / ((unsigned)d.IM * d.JM)) + 1;
-        } else {
-            c->VMAX = 0.0f;
-        }
-    }
-}
-
-// Each thread of k_tail_dvm takes TAIL_NPT nodes (TAIL_BS apart, so the
-// loads stay coalesced) and adds their |DVMER| in FP32 before the FP64 tree:
-// GB300 issues few FP64 instructions per clock, and a tree per node kept
-// the kernel on the FP64 pipe.
-constexpr int TAIL_NPT = 8;
-
-__global__ void __launch_bounds__(TAIL_BS) k_tail_dvm(Dev d) {
-    pdl_wait();
-    const DevCtl *c = d.ctl;
-    if (!c->do_tail) return;
     const int N = d.IM * d.JM * d.KM;                   // below 2^31: commit limits the node count
     const float RVEF = 100.0f / c->VREF;
+    const StepupLimits lim = stepup_limits(d);
     float sf = 0.0f;
     unsigned long long key = 0ull;
     int bad = 0;
@@ -799,14 +753,15 @@ __global__ void __launch_bounds__(TAIL_BS) k_tail_dvm(Dev d) {
         if (n >= N) break;
         const int jk = n / d.IM;                         // (j-1) + JM*(k-1)
         const bool jin = jk % d.JM != 0;                 // j >= 2
-        float ro = d.RO[n];
-        if (!isfinite(ro) || !(ro > 0.0f) || !isfinite(d.ROE[n]) || !isfinite(d.ROVX[n]) || !isfinite(d.ROVR[n]) ||
-            !isfinite(d.RORVT[n]))
-            bad += 1;
+        const float ro = d.RO[n], roe = d.ROE[n], rovx = d.ROVX[n], rovr = d.ROVR[n], rorvt = d.RORVT[n];
+        const float vx = d.VX[n], vr = d.VR[n], vt = d.VT[n], ho = d.HO[n], wt = d.WT[n];
+        const float XD = d.DX[jk], RD = d.DR[jk], SD = d.DS[jk];
+        const bool fine = isfinite(ro) & (ro > 0.0f) & isfinite(roe) & isfinite(rovx) & isfinite(rovr) & isfinite(rorvt);
+        bad += fine ? 0 : 1;
+        if (!d.FROZEN) d.TEMP1[n] = stepup_node(d, lim, vx, vt, vr, ho, wt);
         if (jin) {
-            float XD = d.DX[jk], RD = d.DR[jk], SD = d.DS[jk];
-            float VM_START = (XD * d.VX[n] + RD * d.VR[n]) / SD;
-            float VM_END = (XD * d.ROVX[n] + RD * d.ROVR[n]) / SD / ro;
+            float VM_START = (XD * vx + RD * vr) / SD;
+            float VM_END = (XD * rovx + RD * rovr) / SD / ro;
             float DVMER = (VM_END - VM_START) * RVEF;
             d.STORE[n] = DVMER;
             sf += fabsf(DVMER);
@@ -814,50 +769,23 @@ __global__ void __launch_bounds__(TAIL_BS) k_tail_dvm(Dev d) {
             key = kn > key ? kn : key;
         }
     }
-    double s = (double)sf;
-    __shared__ double ss[TAIL_BS / 32];
-    __shared__ unsigned long long sk[TAIL_BS / 32];
-    __shared__ int sc[TAIL_BS / 32];
     const int ro = d.REDUCE_ORDER;
-    for (int o = 16; o > 0; o >>= 1) {
-        s = racc(ro, s, __shfl_down_sync(0xffffffffu, s, o));
-        unsigned long long ok = __shfl_down_sync(0xffffffffu, key, o);
-        key = ok > key ? ok : key;
-        bad += __shfl_down_sync(0xffffffffu, bad, o);
-    }
-    int w = threadIdx.x >> 5;
-    if ((threadIdx.x & 31) == 0) {
-        ss[w] = s;
-        sk[w] = key;
-        sc[w] = bad;
-    }
-    __syncthreads();
+    df s;
+    cta_sum_key<TAIL_BS>(ro, df_of(sf), key, &s, &key);
+    bad = __syncthreads_count(bad & 1) + 2 * __syncthreads_count(bad & 2) + 4 * __syncthreads_count(bad & 4) +
+          8 * __syncthreads_count(bad & 8);              // bad <= TAIL_NPT
     if (threadIdx.x == 0) {
-        double t = 0.0;
-        unsigned long long kk = 0ull;
-        int cnt = 0;
-        for (int q = 0; q < TAIL_BS / 32; ++q) {
-            t = racc(ro, t, ss[q]);
-            kk = sk[q] > kk ? sk[q] : kk;
-            cnt += sc[q];
-        }
-        d.part_sum[blockIdx.x] = t;
-        d.part_key[blockIdx.x] = kk;
-        d.part_cnt[blockIdx.x] = cnt;
+        d.part_sum[blockIdx.x] = s;
+        d.part_key[blockIdx.x] = key;
+        d.part_cnt[blockIdx.x] = bad;
     }
-}
-
-__global__ void k_tail_final(Dev d, int nparts) {
-    pdl_wait();
-    DevCtl *c = d.ctl;
-    if (!c->do_tail) return;
-    const int ro = d.REDUCE_ORDER;
-    double s = 0.0;
-    unsigned long long key = 0ull;
-    int bad = 0;
-    for (int p = threadIdx.x; p < nparts; p += blockDim.x) {
-        s = racc(ro, s, d.part_sum[p]);
-        unsigned long long k2 = d.part_key[p];
+    if (!last_cta(&c->ticket, gridDim.x)) return;
+    s = df_of(0.0f);
+    key = 0ull;
+    bad = 0;
+    for (unsigned p = threadIdx.x; p < gridDim.x; p += TAIL_BS) {
+        s = dacc(ro, s, d.part_sum[p]);
+        const unsigned long long k2 = d.part_key[p];
         key = k2 > key ? k2 : key;
         bad += d.part_cnt[p];
     }
@@ -865,7 +793,7 @@ __global__ void k_tail_final(Dev d, int nparts) {
     // the first J that reaches it, one J per thread as a (value, J) key
     unsigned long long ek = 0ull;
     const float cf1f = (float)d.BLADE_FLOW[0];
-    for (int j = threadIdx.x + 1; j <= d.JM; j += blockDim.x) {
+    for (int j = threadIdx.x + 1; j <= d.JM; j += TAIL_BS) {
         float RATIO = (float)d.BLADE_FLOW[j - 1] / cf1f;
         float EMASS = fabsf(1.0f - RATIO);
         if (EMASS > 0.0f) {
@@ -873,38 +801,25 @@ __global__ void k_tail_final(Dev d, int nparts) {
             ek = kj > ek ? kj : ek;
         }
     }
-    __shared__ double ss[32];
-    __shared__ unsigned long long sk[32], se[32];
-    __shared__ int sc[32];
-    for (int o = 16; o > 0; o >>= 1) {
-        s = racc(ro, s, __shfl_down_sync(0xffffffffu, s, o));
-        unsigned long long ok = __shfl_down_sync(0xffffffffu, key, o);
-        key = ok > key ? ok : key;
-        unsigned long long oe = __shfl_down_sync(0xffffffffu, ek, o);
-        ek = oe > ek ? oe : ek;
-        bad += __shfl_down_sync(0xffffffffu, bad, o);
-    }
+    __shared__ unsigned long long se[TAIL_BS / 32];
+    __shared__ int sc[TAIL_BS / 32];
+    ek = warp_max_key(ek);
+    bad = __reduce_add_sync(0xffffffffu, bad);
     if ((threadIdx.x & 31) == 0) {
-        ss[threadIdx.x >> 5] = s;
-        sk[threadIdx.x >> 5] = key;
         se[threadIdx.x >> 5] = ek;
         sc[threadIdx.x >> 5] = bad;
     }
-    __syncthreads();
+    cta_sum_key<TAIL_BS>(ro, s, key, &s, &key);
     if (threadIdx.x == 0) {
-        double t = 0.0;
-        unsigned long long kk = 0ull, ke = 0ull;
+        unsigned long long ke = 0ull;
         int cnt = 0;
-        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) {
-            t = racc(ro, t, ss[w]);
-            kk = sk[w] > kk ? sk[w] : kk;
+        for (int w = 0; w < TAIL_BS / 32; ++w) {
             ke = se[w] > ke ? se[w] : ke;
             cnt += sc[w];
         }
-        c->mon.eavg_sum = t;
-        c->EAVG = (float)t / (float)(d.IM * d.JMM1 * d.KM);
-        if (kk) {
-            unsigned lin = 0xFFFFFFFFu - (unsigned)(kk & 0xFFFFFFFFull);
+        c->EAVG = df_val(s) / (float)(d.IM * d.JMM1 * d.KM);
+        if (key) {
+            unsigned lin = 0xFFFFFFFFu - (unsigned)(key & 0xFFFFFFFFull);
             c->EMAX = d.STORE[lin];
             c->IMAXE = (int)(lin % d.IM) + 1;
             c->JMAXE = (int)((lin / d.IM) % d.JM) + 1;
@@ -931,47 +846,35 @@ __global__ void k_tail_final(Dev d, int nparts) {
     }
 }
 
-void launch_tail(const Dev &d, Launch L) {
-    launchk(L, k_tail_flow, dim3(d.JM), dim3(TAIL_BS), 0, d);
-    mark(L, "k_tail_flow");
-    size_t N = (size_t)d.IM * d.JM * d.KM;
-    int prim_parts = (int)grid_for(N, 256);
-    launchk(L, k_tail_vref, dim3(1), dim3(1024), 0, d, prim_parts);
-    mark(L, "k_tail_vref");
-    int parts = (int)grid_for(N, (size_t)TAIL_BS * TAIL_NPT);
-    launchk(L, k_tail_dvm, dim3(parts), dim3(TAIL_BS), 0, d);
-    mark(L, "k_tail_dvm");
-    launchk(L, k_tail_final, dim3(1), dim3(1024), 0, d, parts);
-    mark(L, "k_tail_final");
-}
-
 // ---------------------------------------------------------------------
 // STEPUP(RELAX) (7916-8002): local time step ~ c/(|W|+c), relaxed
 // ---------------------------------------------------------------------
-__global__ void k_stepup_node(Dev d, int gated) {
+__global__ void k_stepup_node(const __grid_constant__ Dev d) {
+    pdl_wait();
+    size_t n = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    size_t N = (size_t)d.IM * d.JM * d.KM;
+    if (n >= N) return;
+    d.TEMP1[n] = stepup_node(d, stepup_limits(d), d.VX[n], d.VT[n], d.VR[n], d.HO[n], d.WT[n]);
+}
+
+// One thread a cell.  The cell of J = JMIX+1 takes the step of JMIX+2, whose
+// thread writes both: STEP is then read only by the thread that writes it,
+// and needs no second pass.
+__global__ void k_stepup_cell(const __grid_constant__ Dev d, float RELAX, int gated) {
     pdl_wait();
     if (gated && (!d.ctl->do_tail || d.FROZEN)) return;
     size_t n = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     size_t N = (size_t)d.IM * d.JM * d.KM;
     if (n >= N) return;
-    float TLIM = 0.1f * A1(d.TO1, d.KMID);
-    float VLIM = 0.01f * A1(d.VM1, d.KMID) * A1(d.VM1, d.KMID);
-    float vx = d.VX[n], vt = d.VT[n], vr = d.VR[n];
-    float VSQ = vx * vx + vt * vt + vr * vr;
-    float HSTAT = d.HO[n] - 0.5f * VSQ;
-    float TSTATIC = HSTAT * d.RCP;
-    if (TSTATIC < TLIM) TSTATIC = TLIM;
-    float WTREL = d.WT[n];
-    float WSQ = VSQ - (vt * vt - WTREL * WTREL);
-    if (WSQ < VLIM) WSQ = VLIM;
-    float V_SONIC = sqrtf(d.GA * d.RGAS * TSTATIC);
-    float VPLUSC = sqrtf(WSQ) + V_SONIC;
-    d.TEMP1[n] = d.VSOUND / VPLUSC;
-}
-
-__device__ inline float stepup_cell(const Dev &d, int i, int j, int k, float RELAX) {
+    int i, j, k;
+    node_ijk(d, n, i, j, k);
+    if (i >= d.IM || j < 2 || k >= d.KM) return;
+    const bool mix1 = A1(d.INDMIX, j - 1) == 1 && j < d.JM;           // J = JMIX+1
+    const bool mix2 = j >= 3 && A1(d.INDMIX, j - 2) == 1;             // J = JMIX+2 (JMIX+1 < JM)
+    if (mix1) return;
     const float *T = d.TEMP1;
-    int ip1 = i + 1, kp1 = k + 1;
+    const int ip1 = i + 1, kp1 = k + 1;
+    const float bstep = d.BSTEP[n], old = d.STEP[n];
     float AMACHP;
     if (j == 2)
         AMACHP = A3(T, i, 1, k) + A3(T, ip1, 1, k) + A3(T, i, 1, kp1) + A3(T, ip1, 1, kp1);
@@ -979,55 +882,35 @@ __device__ inline float stepup_cell(const Dev &d, int i, int j, int k, float REL
         AMACHP = A3(T, i, j - 1, k) + A3(T, i, j - 1, kp1) + A3(T, ip1, j - 1, k) + A3(T, ip1, j - 1, kp1);
     float AMACHL = A3(T, i, j, k) + A3(T, i, j, kp1) + A3(T, ip1, j, k) + A3(T, ip1, j, kp1);
     float AVMACH = 0.125f * (AMACHL + AMACHP);
-    float STEPNEW = A3(d.BSTEP, i, j, k) * AVMACH;
-    return RELAX * STEPNEW + (1.0f - RELAX) * A3(d.STEP, i, j, k);
-}
-
-__global__ void k_stepup_cell(Dev d, float RELAX, int gated) {
-    pdl_wait();
-    if (gated && (!d.ctl->do_tail || d.FROZEN)) return;
-    size_t n = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    size_t N = (size_t)d.IM * d.JM * d.KM;
-    if (n >= N) return;
-    int i, j, k;
-    node_ijk(d, n, i, j, k);
-    if (i >= d.IM || j < 2 || k >= d.KM) return;
-    float step = stepup_cell(d, i, j, k, RELAX);
-    float rstep = step / d.BSTEP[n];
-    if (A1(d.INDMIX, j - 1) == 1 && j < d.JM) {     // J = JMIX+1: take the step of JMIX+2
-        step = stepup_cell(d, i, j + 1, k, RELAX);
-        rstep = 0.0f;
-    }
-    // the JMIX+2 cell reads its own old STEP in stepup_cell, so write after
-    // every reader of this cell's old value: STEP(I,J,K) is only read by
-    // this cell and by the JMIX+1 cell below it, which recomputes it.
-    d.TMP[n] = step;
-    d.STORE[n] = rstep;
-}
-
-__global__ void k_stepup_store(Dev d, int gated) {
-    pdl_wait();
-    if (gated && (!d.ctl->do_tail || d.FROZEN)) return;
-    size_t n = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    size_t N = (size_t)d.IM * d.JM * d.KM;
-    if (n >= N) return;
-    int i, j, k;
-    node_ijk(d, n, i, j, k);
-    if (i >= d.IM || j < 2 || k >= d.KM) return;
-    const float step = d.TMP[n], rstep = d.STORE[n];   // both loads before the stores
+    float STEPNEW = bstep * AVMACH;
+    const float step = RELAX * STEPNEW + (1.0f - RELAX) * old;
     d.STEP[n] = step;
-    d.RSTEP[n] = rstep;
+    d.RSTEP[n] = step / bstep;
+    if (mix2) {
+        d.STEP[n - d.IM] = step;
+        d.RSTEP[n - d.IM] = 0.0f;
+    }
 }
 
-void launch_stepup(const Dev &d, Launch L, float relax, bool gated) {
-    size_t N = (size_t)d.IM * d.JM * d.KM;
-    unsigned g = grid_for(N, 256);
-    launchk(L, k_stepup_node, dim3(g), dim3(256), 0, d, gated ? 1 : 0);
-    mark(L, "k_stepup_node");
-    launchk(L, k_stepup_cell, dim3(g), dim3(256), 0, d, relax, gated ? 1 : 0);
+static void launch_stepup_cell(const Dev &d, Launch L, float relax, bool gated) {
+    launchk(L, k_stepup_cell, dim3(grid_for((size_t)d.IM * d.JM * d.KM, 256)), dim3(256), 0, d, relax, gated ? 1 : 0);
     mark(L, "k_stepup_cell");
-    launchk(L, k_stepup_store, dim3(g), dim3(256), 0, d, gated ? 1 : 0);
-    mark(L, "k_stepup_store");
+}
+
+void launch_stepup(const Dev &d, Launch L, float relax) {
+    launchk(L, k_stepup_node, dim3(grid_for((size_t)d.IM * d.JM * d.KM, 256)), dim3(256), 0, d);
+    mark(L, "k_stepup_node");
+    launch_stepup_cell(d, L, relax, false);
+}
+
+// the tail: monitors, then STEPUP(0.25)
+void launch_tail(const Dev &d, Launch L) {
+    launchk(L, k_tail_flow, dim3(d.JM), dim3(TAIL_BS), 0, d);
+    mark(L, "k_tail_flow");
+    size_t N = (size_t)d.IM * d.JM * d.KM;
+    launchk(L, k_tail_nodes, dim3(grid_for(N, (size_t)TAIL_BS * TAIL_NPT)), dim3(TAIL_BS), 0, d);
+    mark(L, "k_tail_nodes");
+    launch_stepup_cell(d, L, 0.25f, true);
 }
 
 // ---------------------------------------------------------------------
@@ -1100,7 +983,7 @@ void launch_integrals(const Dev &d, Launch L, double *out) {
 // over the I and K faces into the body forces.  The reference scatters each
 // face's stress into its two cells; here every cell gathers its faces in
 // the order the reference adds them, so each force is the same FP32 sum.
-//   k_loss_prologue (as LOSS)            VISLAM, FTCOND (12545-12568)
+//   loss_viscosity (as LOSS)             VISLAM, FTCOND (12545-12568)
 //   k_nl_cells        one thread a cell  strain rates, VISC_RAT, VISC_LAM (DO 150)
 //   k_nl_transition   one CTA a J plane  laminar lines (DO 160)
 //   k_pwallgrad_*     YPLUSWALL < -10    DPDS_CELL
@@ -1550,8 +1433,8 @@ __global__ void __launch_bounds__(256) k_nl_forces(const __grid_constant__ Dev d
     d.QSOURCE[n] = RF_VIS1 * qs0 - RF_VIS * es;
 }
 
-void launch_loss_prologue(const Dev &d, Launch L, bool init_call) {
-    launchk(L, k_loss_prologue, dim3(1), dim3(1), 0, d, init_call ? 1 : 0);
+void launch_loss_prologue(const Dev &d, Launch L) {
+    launchk(L, k_loss_prologue, dim3(1), dim3(1), 0, d);
     mark(L, "k_loss_prologue");
 }
 
@@ -1577,7 +1460,7 @@ void launch_viscous_walls_and_forces(const Dev &d, Launch L, bool init_call) {
 
 void launch_new_loss(const Dev &d, Launch L, bool init_call) {
     const int ic = init_call ? 1 : 0;
-    launch_loss_prologue(d, L, init_call);
+    if (init_call) launch_loss_prologue(d, L);
     const int nc = d.IMM1 * d.KMM1 * (d.JM - 1);
     launchk(L, k_nl_cells, dim3((nc + 255) / 256), dim3(256), 0, d, ic);
     mark(L, "k_nl_cells");

@@ -684,7 +684,7 @@ void launch_sa_inlet(const Dev &d, Launch L) {
 void launch_spal_loss(const Dev &d, Launch L, bool init_call) {
     const int ic = init_call ? 1 : 0;
     const unsigned nc = (unsigned)((d.IMM1 * (d.JM - 1) * d.KMM1 + SA_BS - 1) / SA_BS);
-    launch_loss_prologue(d, L, init_call);
+    if (init_call) launch_loss_prologue(d, L);
     launchk(L, k_sa_cells, dim3(nc), dim3(SA_BS), 0, d, ic);
     mark(L, "k_sa_cells");
     launchk(L, k_sa_grad, dim3(nc), dim3(SA_BS), 0, d, ic);
