@@ -72,6 +72,7 @@ struct mgpu_handle {
     cudaStream_t aux = nullptr;      // a parallel branch of the step graph (k_bc_sums)
     cudaStream_t aux2 = nullptr;     // another (the Spalart-Allmaras transport)
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+    cudaEvent_t ev_dens0 = nullptr, ev_dens1 = nullptr;
     cudaEvent_t ev_sa0 = nullptr, ev_sa1 = nullptr, ev_sa2 = nullptr;
     int device = 0;
     int sm_count = 0;
@@ -275,8 +276,17 @@ struct SaBranch {
     cudaEvent_t start = nullptr, bc = nullptr, done = nullptr;
 };
 
+// A third: the density limiter reads and writes nothing that TSTEP of the
+// momenta touches, so its walks along J (58 us on 73 x 752 x 57, one block's
+// work) run beside it; the Mach limiter waits for both.
+struct DensBranch {
+    cudaStream_t s = nullptr;
+    cudaEvent_t start = nullptr, done = nullptr;
+};
+
 // Lf: how the first kernel follows what was launched before it
-void enqueue_core(const Dev &d, Launch L, Launch Lf, cudaEvent_t join = nullptr, const SaBranch *sa = nullptr) {
+void enqueue_core(const Dev &d, Launch L, Launch Lf, cudaEvent_t join = nullptr, const SaBranch *sa = nullptr,
+                  const DensBranch *dens = nullptr) {
     Launch L0 = L;        // follows a join of two branches: plain stream order
     L0.pdl = false;
     launch_flux_mass_energy(d, Lf);
@@ -307,12 +317,19 @@ void enqueue_core(const Dev &d, Launch L, Launch Lf, cudaEvent_t join = nullptr,
     }
     if (d.IN_FLOW != 0) launch_setflo(d, L);
     launch_flux_mom(d, L);          // also PEFF and the density limiter's column flags
-    launch_tstep(d, L, V_ROVX, 3);
-    if (sab) {
-        cudaStreamWaitEvent(L.s, sa->done, 0);
-        launch_limiters(d, L0);
+    if (dens) {
+        cudaEventRecord(dens->start, L.s);
+        cudaStreamWaitEvent(dens->s, dens->start, 0);
+        if (sab) cudaStreamWaitEvent(dens->s, sa->done, 0);
+        launch_density_fix(d, Launch{dens->s, L.sm_count, nullptr});
+        cudaEventRecord(dens->done, dens->s);
+        launch_tstep(d, L, V_ROVX, 3);
+        cudaStreamWaitEvent(L.s, dens->done, 0);
+        launch_mach_limiter(d, L0);
     } else {
-        launch_limiters(d, L);
+        launch_tstep(d, L, V_ROVX, 3);
+        launch_density_fix(d, L);
+        launch_mach_limiter(d, L);
     }
     launch_mixplan(d, L);
     if (d.any_cusp2) launch_cusp(d, L);
@@ -391,9 +408,10 @@ int capture_step(mgpu_handle *h, int what) {
     launch_bc_sums(dg, Launch{h->aux, h->sm_count, nullptr});
     CK(cudaEventRecord(h->ev_join, h->aux));
     SaBranch sab{h->aux2, h->ev_sa0, h->ev_sa1, h->ev_sa2};
+    DensBranch dens{h->aux, h->ev_dens0, h->ev_dens1};
     if (what >= 0) {
         if (what & 1) launch_loss(dg, L, false);
-        enqueue_core(dg, L, L, h->ev_join, &sab);
+        enqueue_core(dg, L, L, h->ev_join, &sab, &dens);
         if (what & 2) launch_tail(dg, L);
         CK(cudaGetLastError());
         return 0;
@@ -402,7 +420,7 @@ int capture_step(mgpu_handle *h, int what) {
     L0.pdl = false;
     // an inviscid problem (ILOS = 0) has no LOSS node
     int rc = dg.ILOS == 0 ? 0 : add_conditional(h, hl, [&](Launch L2) { launch_loss(dg, L2, false); });
-    if (!rc) enqueue_core(dg, L, L0, h->ev_join, &sab);
+    if (!rc) enqueue_core(dg, L, L0, h->ev_join, &sab, &dens);
     if (!rc) rc = add_conditional(h, ht, [&](Launch L2) { launch_tail(dg, L2); });
     return rc;
 }
@@ -564,6 +582,8 @@ int32_t mgpu_create(int32_t im, int32_t jm, int32_t km, int32_t nrows, mgpu_hand
     e = cudaStreamCreateWithFlags(&h->aux, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&h->ev_fork, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&h->ev_join, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&h->ev_dens0, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&h->ev_dens1, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&h->aux2, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&h->ev_sa0, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&h->ev_sa1, cudaEventDisableTiming);
@@ -646,7 +666,7 @@ void mgpu_destroy(mgpu_handle *h) {
     if (h->aux2) cudaStreamDestroy(h->aux2);
     if (h->ev_fork) cudaEventDestroy(h->ev_fork);
     if (h->ev_join) cudaEventDestroy(h->ev_join);
-    for (cudaEvent_t ev : {h->ev_sa0, h->ev_sa1, h->ev_sa2})
+    for (cudaEvent_t ev : {h->ev_sa0, h->ev_sa1, h->ev_sa2, h->ev_dens0, h->ev_dens1})
         if (ev) cudaEventDestroy(ev);
     delete h;
 }
@@ -989,6 +1009,22 @@ int32_t mgpu_commit(mgpu_handle *h) {
     if ((rc = upload(h, d.FILAM, FILAM)) || (rc = upload(h, d.FITURB, FITURB)) || (rc = upload(h, d.FIWAKE, FIWAKE)) ||
         (rc = upload(h, d.FIUP, FIUP)) || (rc = upload(h, d.FKLAM, FKLAM)) || (rc = upload(h, d.FKTURB, FKTURB)))
         return rc;
+    // the running sums of FP that NEW_MIXPLAN's periodicity correction takes
+    {
+        std::vector<float> s4(d.IM);
+        std::vector<double> s8(d.IM);
+        float f4 = 0.0f;
+        double f8 = 0.0;
+        for (int i = 0; i < d.IM; ++i) {
+            s4[i] = f4;
+            s8[i] = f8;
+            f4 = f4 + FP[i];
+            f8 += (double)FP[i];
+        }
+        if ((rc = dalloc(h, &d.FPSUM4, d.IM)) || (rc = dalloc(h, &d.FPSUM8, d.IM)) || (rc = upload(h, d.FPSUM4, s4)) ||
+            (rc = upload(h, d.FPSUM8, s8)))
+            return rc;
+    }
     // multigrid block extents
     std::vector<int> s, e;
     struct Ext {

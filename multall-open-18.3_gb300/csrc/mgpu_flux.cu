@@ -892,10 +892,13 @@ __global__ void k_mach_limiter(Dev d) {
     }
 }
 
-void launch_limiters(const Dev &d, Launch L) {
+void launch_density_fix(const Dev &d, Launch L) {
     int lines = d.IM * d.KM;
     launchk(L, k_density_fix, dim3((lines + 127) / 128), dim3(128), 0, d);
     mark(L, "k_density_fix");
+}
+
+void launch_mach_limiter(const Dev &d, Launch L) {
     size_t N = (size_t)d.IM * d.JM * d.KM;
     launchk(L, k_mach_limiter, dim3(grid_for(N, 256)), dim3(256), 0, d);
     mark(L, "k_mach_limiter");
@@ -903,18 +906,23 @@ void launch_limiters(const Dev &d, Launch L) {
 
 // ---------------------------------------------------------------------
 // NEW_MIXPLAN (14922-15251), IFGAS=0: one CTA per (row interface, K).
-// The threads fill the per-I isentropic states and angles; the outward
-// Prandtl-Meyer sweeps for a supersonic relative flow and the periodicity
-// correction run in the reference's order on one thread; the threads then
-// relax the J=JMIX+2 (or JMIX-1) plane.
+// The threads fill the per-I isentropic states and angles, and for a
+// supersonic relative flow the increments of the outward Prandtl-Meyer
+// sweeps; two threads, one per direction, only add them up in the
+// reference's order; the threads then turn back the periodicity error (with
+// the partial sums of FP that mgpu_commit tabulates) and relax the J=JMIX+2
+// (or JMIX-1) plane.  One thread forming the increments and the FP64 sums
+// along its sweep made the launch 48 us on 73 x 752 x 57.
 // ---------------------------------------------------------------------
 constexpr int MIX_MAXI = 160;
-constexpr int MIX_BS = 64;
+constexpr int MIX_BS = 96;
 
-__global__ void __launch_bounds__(MIX_BS) k_mixplan(Dev d) {
+__global__ void __launch_bounds__(MIX_BS) k_mixplan(const __grid_constant__ Dev d) {
     pdl_wait();
     __shared__ float ALPHAA[MIX_MAXI], GAMA[MIX_MAXI], WREF_JP2[MIX_MAXI], ROREF_JP2[MIX_MAXI], PISENT[MIX_MAXI];
     __shared__ float ROISENT[MIX_MAXI], WMACH_JP2[MIX_MAXI], TISENT[MIX_MAXI], WIS_JP2[MIX_MAXI];
+    __shared__ float DALPHA[MIX_MAXI];
+    __shared__ bool SWEEP[MIX_MAXI];
     const int nr = blockIdx.x / d.KM + 1, k = blockIdx.x % d.KM + 1;
     const int IM = d.IM;
     const float RFMIX1 = 1.0f - d.RFMIX;
@@ -1005,42 +1013,47 @@ __global__ void __launch_bounds__(MIX_BS) k_mixplan(Dev d) {
         GAMA[i - 1] = F_ANGLE1 * GAMAMIX + F_ANGLE * GAMAJP3;
     }
     int NMACH = __syncthreads_or(nmach);
-    if (NMACH != 0 && threadIdx.x == 0) {
-        float FROTN = 1.0f;
-        if (WTMIX < 0.0f) FROTN = -1.0f;
-        for (int i = d.IMID + 1; i <= IM; ++i) {
-            int a = i - 1, b = i - 2;   // 0-based I and I-1
-            if (WMACH_JP2[a] > 1.001f && WMACH_JP2[b] > 1.001f) {
+    if (NMACH != 0) {
+        const float FROTN = WTMIX < 0.0f ? -1.0f : 1.0f;
+        // DALPHA(I): what the sweep adds to the angle of the neighbour b
+        // towards IMID where SWEEP(I); elsewhere I keeps its own angle
+        for (int i = threadIdx.x + 1; i <= IM; i += MIX_BS) {
+            const int a = i - 1, b = i > d.IMID ? i - 2 : i;
+            const bool on = i != d.IMID && WMACH_JP2[a] > 1.001f && WMACH_JP2[b] > 1.001f;
+            float dal = 0.0f;
+            if (on) {
                 float DELP = PISENT[a] - PISENT[b];
                 float DELTAI = sqrtf(WMACH_JP2[a] * WMACH_JP2[a] - 1.0f) / (ROREF_JP2[a] * WREF_JP2[a] * WREF_JP2[a]);
-                float DELTAIM1 = sqrtf(WMACH_JP2[b] * WMACH_JP2[b] - 1.0f) / (ROREF_JP2[b] * WREF_JP2[b] * WREF_JP2[b]);
-                ALPHAA[a] = ALPHAA[b] + FROTN * DELP * 0.5f * (DELTAI + DELTAIM1);
+                float DELTAIB = sqrtf(WMACH_JP2[b] * WMACH_JP2[b] - 1.0f) / (ROREF_JP2[b] * WREF_JP2[b] * WREF_JP2[b]);
+                dal = FROTN * DELP * 0.5f * (DELTAI + DELTAIB);
+            }
+            DALPHA[a] = dal;
+            SWEEP[a] = on;
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            float al = ALPHAA[d.IMID - 1];
+#pragma unroll 4
+            for (int a = d.IMID; a < IM; ++a) {
+                al = SWEEP[a] ? al + DALPHA[a] : ALPHAA[a];
+                ALPHAA[a] = al;
+            }
+        } else if (threadIdx.x == 32) {
+            float al = ALPHAA[d.IMID - 1];
+#pragma unroll 4
+            for (int a = d.IMID - 2; a >= 0; --a) {
+                al = SWEEP[a] ? al + DALPHA[a] : ALPHAA[a];
+                ALPHAA[a] = al;
             }
         }
-        for (int i = d.IMID - 1; i >= 1; --i) {
-            int a = i - 1, b = i;       // I and I+1
-            if (WMACH_JP2[a] > 1.001f && WMACH_JP2[b] > 1.001f) {
-                float DELP = PISENT[a] - PISENT[b];
-                float DELTAI = sqrtf(WMACH_JP2[a] * WMACH_JP2[a] - 1.0f) / (ROREF_JP2[a] * WREF_JP2[a] * WREF_JP2[a]);
-                float DELTAIP1 = sqrtf(WMACH_JP2[b] * WMACH_JP2[b] - 1.0f) / (ROREF_JP2[b] * WREF_JP2[b] * WREF_JP2[b]);
-                ALPHAA[a] = ALPHAA[b] + FROTN * DELP * 0.5f * (DELTAI + DELTAIP1);
-            }
-        }
-        float ROTN = ALPHAA[IM - 1] - ALPHAA[0];
-        // periodicity correction (15177-15182); FP64 running sum in the
-        // default precision split, REAL*4 with REDUCE_ORDER 1 and 2
-        if (d.REDUCE_ORDER != 0) {
-            float SUMFP = 0.0f;
-            for (int i = 1; i <= IM; ++i) {
-                ALPHAA[i - 1] = ALPHAA[i - 1] - ROTN * (SUMFP - 0.5f);
-                SUMFP = SUMFP + A1(d.FP, i);
-            }
-        } else {
-            double SUMFP = 0.0;
-            for (int i = 1; i <= IM; ++i) {
-                ALPHAA[i - 1] = (float)((double)ALPHAA[i - 1] - (double)ROTN * (SUMFP - 0.5));
-                SUMFP += (double)A1(d.FP, i);
-            }
+        __syncthreads();
+        const float ROTN = ALPHAA[IM - 1] - ALPHAA[0];
+        __syncthreads();
+        // periodicity correction (15177-15182); the running sum of FP in FP64
+        // in the default precision split, REAL*4 with REDUCE_ORDER 1 and 2
+        for (int i = threadIdx.x + 1; i <= IM; i += MIX_BS) {
+            if (d.REDUCE_ORDER != 0) ALPHAA[i - 1] = ALPHAA[i - 1] - ROTN * (d.FPSUM4[i - 1] - 0.5f);
+            else ALPHAA[i - 1] = (float)((double)ALPHAA[i - 1] - (double)ROTN * (d.FPSUM8[i - 1] - 0.5));
         }
     }
     __syncthreads();

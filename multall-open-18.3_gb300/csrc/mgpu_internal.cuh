@@ -101,6 +101,8 @@ struct Dev {
     float *PLIM;                       // (KM)
     float *FILAM, *FITURB, *FIWAKE, *FIUP, *FKLAM, *FKTURB;   // (NROWS, IM|KM)
     float *VLIMIT, *ROLIMIT;           // (NROWS)
+    float *FPSUM4;                     // (IM) FP(1) + ... + FP(I-1), REAL*4 in order
+    double *FPSUM8;                    // (IM) the same in FP64
     int *DFLAG;                        // (IM*KM) density-limiter column flags
     float *BCBUF;                      // (4, KM) PAVG2, PAVG3, PAVGOUT, and the PD each K's exit update uses
     float *FLOWJ;                      // (JM) SETFLO's FLOW(J)
@@ -371,7 +373,8 @@ void launch_cusp(const Dev &d, Launch L);         // IF_CUSP = 2 rows
 void launch_flux_mom(const Dev &d, Launch L);
 // TSTEP for the nv variables v0 .. v0+nv-1 of d.var
 void launch_tstep(const Dev &d, Launch L, int v0, int nv);
-void launch_limiters(const Dev &d, Launch L);
+void launch_density_fix(const Dev &d, Launch L);
+void launch_mach_limiter(const Dev &d, Launch L);
 void launch_mixplan(const Dev &d, Launch L);
 // node arrays at the start of the Spalart-Allmaras work buffer (SAW); then
 // REYNOLDS(1..64) and the scalars VORTICITY_FAC, PGRAD_FAC and the inlet
