@@ -76,8 +76,7 @@ struct Adj {
     // objective seeds: node quantities (VX, VT, VR, HO, P) and cell FLOWX on
     // two J planes
     const float *seed;
-    const int *seed_on;          // 0: the plain transposed step (Krylov products)
-    int seed_j[2];
+    const int *seed_on;          // [0] 0: the plain transposed step (Krylov products); [1], [2] the planes
 };
 
 namespace {
@@ -1032,28 +1031,41 @@ __global__ void __launch_bounds__(64) rk_mixplan(const Dev d, const Adj a) {
 // RO(J+1) + RO(J+2)) / 4, J walked upwards; the coefficients come from a
 // replay of the recorded column (rk_density_prep).
 // =====================================================================
-__global__ void rk_density_prep(const Dev d, const Adj a) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+// A warp a column: the lanes test the recorded values, and only a column in
+// which one of them triggers (the first is the same in the replay) is replayed,
+// by one lane; rk_density reads the coefficients of those columns alone.
+__global__ void __launch_bounds__(256) rk_density_prep(const Dev d, const Adj a) {
+    const int t = (int)(blockIdx.x * 8 + (threadIdx.x >> 5)), lane = threadIdx.x & 31;
     if (t >= d.IM * d.KM) return;
     const int i = t % d.IM + 1, k = t / d.IM + 1;
-    float *C0 = const_cast<float *>(a.tDC0), *CA = const_cast<float *>(a.tDCA);
-    int any = 0;
     const float *RO = a.tROL;
-    float rm2 = A3(RO, i, 1, k), rm1 = A3(RO, i, 2, k), r0 = A3(RO, i, 3, k), rp1 = A3(RO, i, 4, k);
-    for (int j = 3; j <= d.JM - 3; ++j) {
-        const float rp2 = A3(RO, i, j + 2, k);
-        const float ROAVG = 0.25f * (rm2 + rm1 + rp1 + rp2);
-        float ro = r0, c0 = 1.0f, ca = 0.0f;
-        if (ro < 0.6f * ROAVG) { ro = 0.5f * (ro + 0.6f * ROAVG); c0 *= 0.5f; ca = 0.5f * ca + 0.3f; }
-        if (ro > 1.5f * ROAVG) { ro = 0.5f * (ro + 1.5f * ROAVG); c0 *= 0.5f; ca = 0.5f * ca + 0.75f; }
-        if (ro < d.ROLIM) { ro = 0.5f * (ro + d.ROLIM); c0 *= 0.5f; ca *= 0.5f; }
-        if (c0 != 1.0f) any = 1;
-        A3(C0, i, j, k) = c0;
-        A3(CA, i, j, k) = ca;
-        rm2 = rm1;
-        rm1 = ro;
-        r0 = rp1;
-        rp1 = rp2;
+    bool trig = false;
+    for (int j = 3 + lane; j <= d.JM - 3; j += 32) {
+        const float ROAVG = 0.25f * (A3(RO, i, j - 2, k) + A3(RO, i, j - 1, k) + A3(RO, i, j + 1, k) + A3(RO, i, j + 2, k));
+        const float ro = A3(RO, i, j, k);
+        trig = trig || ro < 0.6f * ROAVG || ro > 1.5f * ROAVG || ro < d.ROLIM;
+    }
+    const bool col = __any_sync(0xffffffffu, trig);
+    if (lane != 0) return;
+    int any = 0;
+    if (col) {
+        float *C0 = const_cast<float *>(a.tDC0), *CA = const_cast<float *>(a.tDCA);
+        float rm2 = A3(RO, i, 1, k), rm1 = A3(RO, i, 2, k), r0 = A3(RO, i, 3, k), rp1 = A3(RO, i, 4, k);
+        for (int j = 3; j <= d.JM - 3; ++j) {
+            const float rp2 = A3(RO, i, j + 2, k);
+            const float ROAVG = 0.25f * (rm2 + rm1 + rp1 + rp2);
+            float ro = r0, c0 = 1.0f, ca = 0.0f;
+            if (ro < 0.6f * ROAVG) { ro = 0.5f * (ro + 0.6f * ROAVG); c0 *= 0.5f; ca = 0.5f * ca + 0.3f; }
+            if (ro > 1.5f * ROAVG) { ro = 0.5f * (ro + 1.5f * ROAVG); c0 *= 0.5f; ca = 0.5f * ca + 0.75f; }
+            if (ro < d.ROLIM) { ro = 0.5f * (ro + d.ROLIM); c0 *= 0.5f; ca *= 0.5f; }
+            if (c0 != 1.0f) any = 1;
+            A3(C0, i, j, k) = c0;
+            A3(CA, i, j, k) = ca;
+            rm2 = rm1;
+            rm1 = ro;
+            r0 = rp1;
+            rp1 = rp2;
+        }
     }
     const_cast<int *>(a.tDCOL)[t] = any;
 }
@@ -1751,6 +1763,14 @@ __global__ void __launch_bounds__(RT_BS) rk_ts_cells(const __grid_constant__ Dev
     }
 }
 
+// the seeds' switch and planes: device data, so that one captured reverse step
+// serves every objective and linearisation point
+__global__ void rk_seed_set(int *seed_on, int j1, int j2) {
+    seed_on[0] = 1;
+    seed_on[1] = j1;
+    seed_on[2] = j2;
+}
+
 // objective seeds added at the start of each reverse step
 __global__ void rk_seed(const Dev d, const Adj a) {
     const int IM = d.IM, KM = d.KM;
@@ -1759,7 +1779,7 @@ __global__ void rk_seed(const Dev d, const Adj a) {
     const int per = 5 * np + nc;
     if (t >= 2 * per || !*a.seed_on) return;
     const int p = t / per, r = t % per;
-    const int j = a.seed_j[p];
+    const int j = a.seed_on[1 + p];
     const float s = a.seed[t];
     if (s == 0.0f) return;
     if (r < 5 * np) {
@@ -1854,33 +1874,27 @@ __global__ void rk_seed_plane(const Dev d, const Adj a, float *seed, int j,
         if (e_ != cudaSuccess) return api_fail(MGPU_E_CUDA, (std::string(#call) + ": " + cudaGetErrorString(e_)).c_str()); \
     } while (0)
 
-// row means of |STORE| after the row mixing, as the negative feedback of the
-// recorded step formed them (1501-1525): one CTA per variable
+// Row means of |STORE| after the row mixing, as the negative feedback of the
+// recorded step formed them (1501-1525), from its per-plane sums: one CTA per
+// variable.  (Summed again over the cells in FP64 they took 1540 us at
+// 65 x 242 x 49.)
 __global__ void rk_blk(const __grid_constant__ Dev d, const __grid_constant__ Adj a) {
-    __shared__ double sh[RT_BS / 32];
     __shared__ float chg[64];
-    const AdjVar &V = a.v[blockIdx.x];
-    float *blk = const_cast<float *>(V.tBLK);
-    const int IMM1 = d.IMM1, KMM1 = d.KMM1, NROWS = d.NROWS;
-    for (int nr = 1; nr <= NROWS; ++nr) {
-        const int JST = A1(d.JSTART, nr) + 1, JEN = A1(d.JMIX, nr) - 1;
-        const int nc = IMM1 * KMM1 * (JEN - JST + 1);
-        double s = 0.0;
-        for (int c = threadIdx.x; c < nc; c += RT_BS) {
-            const int i = c % IMM1 + 1, r = c / IMM1;
-            const int k = r % KMM1 + 1, j = JST + r / KMM1;
-            s += (double)fabsf(A3(V.tST, i, j, k));
-        }
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-        if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = s;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            double t = 0.0;
-            for (int w = 0; w < RT_BS / 32; ++w) t += sh[w];
-            chg[nr - 1] = (float)t / (float)nc;
-        }
-        __syncthreads();
+    const VarSet &V = d.var[blockIdx.x];
+    float *blk = const_cast<float *>(a.v[blockIdx.x].tBLK);
+    const int w = threadIdx.x >> 5, l = threadIdx.x & 31, NROWS = d.NROWS, ro = d.REDUCE_ORDER;
+    if (ro == 1) {
+        for (int nr = threadIdx.x; nr < NROWS; nr += RT_BS) blk[nr] = V.AVG_BLK[nr];
+        return;
     }
+    for (int nr = w + 1; nr <= NROWS; nr += RT_BS / 32) {
+        const int JST = A1(d.JSTART, nr) + 1, JEN = A1(d.JMIX, nr) - 1;
+        df s = df_of(0.0f);
+        for (int jj = JST + l; jj <= JEN; jj += 32) s = dacc(ro, s, V.pabs[jj - 1]);
+        for (int o = 16; o > 0; o >>= 1) s = dacc(ro, s, df_shfl_down(s, o));
+        if (l == 0) chg[nr - 1] = df_val(s) / (float)(d.IMM1 * d.KMM1 * (JEN - JST + 1));
+    }
+    __syncthreads();
     if (threadIdx.x == 0) {
         if (NROWS == 1) blk[0] = chg[0];
         if (NROWS == 2) {
@@ -1893,6 +1907,41 @@ __global__ void rk_blk(const __grid_constant__ Dev d, const __grid_constant__ Ad
             blk[0] = 0.5f * (chg[0] + chg[1]);
         }
     }
+}
+
+// Many whole-array copies (or, without a source, zeroings) in one launch: entry
+// blockIdx.y.  The arrays are whole allocations or multiples of four floats
+// into one, so both ends are 16-byte aligned.
+struct CopyList {
+    static constexpr int MAX = 64;
+    int n = 0;
+    struct {
+        float *dst;
+        const float *src;
+        size_t len;
+    } e[MAX];
+    void add(const void *dst, const void *src, size_t len) {
+        e[n].dst = (float *)dst;
+        e[n].src = (const float *)src;
+        e[n++].len = len;
+    }
+};
+__global__ void __launch_bounds__(RT_BS) rk_copy(const __grid_constant__ CopyList l) {
+    float *dst = l.e[blockIdx.y].dst;
+    const float *src = l.e[blockIdx.y].src;
+    const size_t len = l.e[blockIdx.y].len, n4 = len / 4, step = (size_t)gridDim.x * RT_BS;
+    const size_t t0 = (size_t)blockIdx.x * RT_BS + threadIdx.x;
+    for (size_t t = t0; t < n4; t += step)
+        reinterpret_cast<float4 *>(dst)[t] =
+            src ? reinterpret_cast<const float4 *>(src)[t] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    for (size_t t = 4 * n4 + t0; t < len; t += step) dst[t] = src ? src[t] : 0.0f;
+}
+static void run_copies(const CopyList &l, int sm_count, cudaStream_t st) {
+    size_t most = 0;
+    for (int q = 0; q < l.n; ++q) most = l.e[q].len > most ? l.e[q].len : most;
+    size_t g = (most / 4 + RT_BS - 1) / RT_BS;
+    if (g > (size_t)2 * sm_count) g = (size_t)2 * sm_count;
+    rk_copy<<<dim3(g ? (unsigned)g : 1u, (unsigned)l.n), RT_BS, 0, st>>>(l);
 }
 
 // sum of squares of the five conserved-variable adjoints and of their change
@@ -2062,6 +2111,7 @@ __global__ void rk_metrics(const Dev d, const Adj a, float *gth) {
     }
 }
 
+constexpr int NSAVE = 14;
 struct AdjState {
     mgpu_handle *h = nullptr;
     Adj a;
@@ -2071,7 +2121,11 @@ struct AdjState {
     float *seed = nullptr;
     float *prev = nullptr;       // 5 N: the conserved-variable adjoints before the last iteration
     double *norms = nullptr;
-    std::vector<double> sums;    // (4, JM) EFICOOL sums of the recorded step
+    double sums[8] = {};         // EFICOOL sums of the recorded step at the objectives' two stations
+    // NSAVE node arrays (each padded to four floats) and PD
+    float *save = nullptr;       // what the recorded step changes of the state, put back after it
+    DevCtl *savectl = nullptr;
+    float *gth = nullptr;        // dJ/dTHETA
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t gexec = nullptr;
     int objective = -1;
@@ -2229,7 +2283,14 @@ int allocate(AdjState *s, const Dev &d) {
     F(&s->seed, (size_t)2 * per);
     F(&s->prev, 5 * N);
     if (!rc) rc = aalloc(s, &s->norms, 2);
-    if (!rc) rc = aalloc(s, &s->seed_on, 1);
+    if (!rc) rc = aalloc(s, &s->seed_on, 3);
+    F(&s->save, NSAVE * ((N + 3) / 4 * 4) + (size_t)d.KM);
+    if (!rc) rc = aalloc(s, &s->savectl, 1);
+    F(&s->gth, N);
+    // the zeroing of these ran on the legacy stream, which the handle's own
+    // stream does not wait for
+    if (!rc && cudaStreamSynchronize(cudaStreamLegacy) != cudaSuccess)
+        rc = api_fail(MGPU_E_CUDA, "adjoint device allocation");
     a.seed_on = s->seed_on;
     a.tctl = s->tctl;
     a.flag = s->flag;
@@ -2321,16 +2382,20 @@ int unpack(AdjState *s, const Dev &d, const float *src, cudaStream_t st) {
 int zero_adjoints(AdjState *s, const Dev &d, cudaStream_t st) {
     const size_t N = (size_t)d.IM * d.JM * d.KM;
     Adj &a = s->a;
+    CopyList l;
     for (int v = 0; v < NVAR; ++v) {
         AdjVar &V = a.v[v];
         float *z[] = {V.D, V.DIFF, V.SR, V.ST, V.TM, V.Y, V.XF, V.TF, V.RF};
         for (float *p : z)
-            if (p) ACK(cudaMemsetAsync(p, 0, N * sizeof(float), st));
+            if (p && p != a.FLOWX && p != a.FLOWT && p != a.FLOWR) l.add(p, nullptr, N);
     }
     float *z[] = {a.P, a.HO, a.VX, a.VR, a.VT, a.ROVT, a.PEFF, a.FLOWX, a.FLOWT, a.FLOWR, a.WT};
-    for (float *p : z) ACK(cudaMemsetAsync(p, 0, N * sizeof(float), st));
+    for (float *p : z) l.add(p, nullptr, N);
     float *zk[] = {a.PD, a.PDK, a.PAVG, a.SSUM};
-    for (float *p : zk) ACK(cudaMemsetAsync(p, 0, (size_t)d.KM * sizeof(float), st));
+    for (float *p : zk) l.add(p, nullptr, (size_t)d.KM);
+    l.add(s->seed, nullptr, (size_t)2 * (5 * d.IM * d.KM + d.IMM1 * d.KMM1));
+    run_copies(l, handle_sm_count(s->h), st);
+    ACK(cudaGetLastError());
     return 0;
 }
 
@@ -2360,32 +2425,35 @@ int32_t mgpu_adjoint_prepare(mgpu_handle *h) {
     const Dev &d = dh;
     cudaStream_t st = hv.stream;
     const size_t N = (size_t)d.IM * d.JM * d.KM, np = (size_t)d.IM * d.KM;
-    const size_t fb = N * sizeof(float);
     Adj &a = s->a;
-    // the state before the recorded step
-    auto cp = [&](const float *dst, const float *src, size_t n) {
-        return cudaMemcpyAsync((void *)dst, src, n * sizeof(float), cudaMemcpyDeviceToDevice, st);
-    };
-    ACK(cp(a.tRO, d.RO, N)); ACK(cp(a.tROVX, d.ROVX, N)); ACK(cp(a.tROVR, d.ROVR, N));
-    ACK(cp(a.tRORVT, d.RORVT, N)); ACK(cp(a.tROE, d.ROE, N)); ACK(cp(a.tPEFF0, d.PEFF, N));
+    // the state before the recorded step, and everything else the step
+    // changes, which is put back afterwards
+    const size_t Np = (N + 3) / 4 * 4;
+    float *const keep[] = {d.DRO, d.DROE, d.DROVX, d.DROVR, d.DRORVT, d.P, d.HO, d.T_STATIC, d.VX, d.VR, d.VT,
+                           d.WT, d.ROWT, d.ROVT};
+    const int nkeep = (int)(sizeof(keep) / sizeof(keep[0]));
+    static_assert(sizeof(keep) / sizeof(keep[0]) == NSAVE, "AdjState::save holds NSAVE arrays");
+    float *const savepd = s->save + nkeep * Np;
+    const int sm = handle_sm_count(h);
+    {
+        CopyList l;
+        l.add(a.tRO, d.RO, N);
+        l.add(a.tROVX, d.ROVX, N);
+        l.add(a.tROVR, d.ROVR, N);
+        l.add(a.tRORVT, d.RORVT, N);
+        l.add(a.tROE, d.ROE, N);
+        l.add(a.tPEFF0, d.PEFF, N);
+        for (int q = 0; q < nkeep; ++q) l.add(s->save + q * Np, keep[q], N);
+        l.add(savepd, d.PD, (size_t)d.KM);
+        run_copies(l, sm, st);
+    }
     ACK(cudaMemcpy2DAsync((void *)a.tHOJM, (size_t)d.IM * 4, d.HO + (size_t)d.IM * (d.JM - 1), (size_t)d.IM * d.JM * 4,
                           (size_t)d.IM * 4, d.KM, cudaMemcpyDeviceToDevice, st));
     ACK(cudaMemcpy2DAsync((void *)a.tROVT1, (size_t)d.IM * 4, d.ROVT, (size_t)d.IM * d.JM * 4, (size_t)d.IM * 4, d.KM,
                           cudaMemcpyDeviceToDevice, st));
     ACK(cudaMemcpy2DAsync((void *)a.tP1, (size_t)d.IM * 4, d.P, (size_t)d.IM * d.JM * 4, (size_t)d.IM * 4, d.KM,
                           cudaMemcpyDeviceToDevice, st));
-    // everything else the step changes, restored afterwards
-    float *const keep[] = {d.DRO, d.DROE, d.DROVX, d.DROVR, d.DRORVT, d.P, d.HO, d.T_STATIC, d.VX, d.VR, d.VT,
-                           d.WT, d.ROWT, d.ROVT};
-    const int nkeep = (int)(sizeof(keep) / sizeof(keep[0]));
-    float *save = nullptr, *savepd = nullptr;
-    DevCtl *savectl = nullptr;
-    ACK(cudaMallocAsync((void **)&save, nkeep * fb, st));
-    ACK(cudaMallocAsync((void **)&savepd, (size_t)d.KM * 4, st));
-    ACK(cudaMallocAsync((void **)&savectl, sizeof(DevCtl), st));
-    for (int q = 0; q < nkeep; ++q) ACK(cudaMemcpyAsync(save + (size_t)q * N, keep[q], fb, cudaMemcpyDeviceToDevice, st));
-    ACK(cudaMemcpyAsync(savepd, d.PD, (size_t)d.KM * 4, cudaMemcpyDeviceToDevice, st));
-    ACK(cudaMemcpyAsync(savectl, d.ctl, sizeof(DevCtl), cudaMemcpyDeviceToDevice, st));
+    ACK(cudaMemcpyAsync(s->savectl, d.ctl, sizeof(DevCtl), cudaMemcpyDeviceToDevice, st));
     // the recorded step: LOSS and STEPUP held
     Dev rec = d;
     rec.use_cond = 0;
@@ -2401,61 +2469,58 @@ int32_t mgpu_adjoint_prepare(mgpu_handle *h) {
     launch_prim(rec, L, -1);
     enqueue_step_core(rec, L);
     ACK(cudaGetLastError());
-    ACK(cp(a.tVX, d.VX, N)); ACK(cp(a.tVR, d.VR, N)); ACK(cp(a.tVT, d.VT, N)); ACK(cp(a.tROVT, d.ROVT, N));
-    ACK(cp(a.tP, d.P, N)); ACK(cp(a.tHO, d.HO, N)); ACK(cp(a.tPEFF, d.PEFF, N));
-    ACK(cp(a.tFLOWX, d.FLOWX, N)); ACK(cp(a.tFLOWT, d.FLOWT, N)); ACK(cp(a.tFLOWR, d.FLOWR, N));
-    for (int v = 0; v < NVAR; ++v) ACK(cp(a.v[v].tST, d.var[v].ST, N));
-    ACK(cp(a.tBCBUF, d.BCBUF, (size_t)4 * d.KM));
-    ACK(cp(a.tWT, d.WT, N));
-    ACK(cp(a.tVLIM, d.VLIMIT, (size_t)d.NROWS));
-    ACK(cp(a.tROLIM, d.ROLIMIT, (size_t)d.NROWS));
+    {
+        CopyList l;
+        l.add(a.tVX, d.VX, N);
+        l.add(a.tVR, d.VR, N);
+        l.add(a.tVT, d.VT, N);
+        l.add(a.tROVT, d.ROVT, N);
+        l.add(a.tP, d.P, N);
+        l.add(a.tHO, d.HO, N);
+        l.add(a.tPEFF, d.PEFF, N);
+        l.add(a.tFLOWX, d.FLOWX, N);
+        l.add(a.tFLOWT, d.FLOWT, N);
+        l.add(a.tFLOWR, d.FLOWR, N);
+        for (int v = 0; v < NVAR; ++v) l.add(a.v[v].tST, d.var[v].ST, N);
+        l.add(a.tBCBUF, d.BCBUF, (size_t)4 * d.KM);
+        l.add(a.tWT, d.WT, N);
+        l.add(a.tVLIM, d.VLIMIT, (size_t)d.NROWS);
+        l.add(a.tROLIM, d.ROLIMIT, (size_t)d.NROWS);
+        run_copies(l, sm, st);
+    }
     ACK(cudaMemcpyAsync(s->tctl, d.ctl, sizeof(DevCtl), cudaMemcpyDeviceToDevice, st));
     // the EFICOOL sums of the step's arrays (the objectives' forward values)
     double *dint = handle_int_buf(h);
-    launch_integrals(rec, L, dint);
+    launch_station_sums(rec, L, d.NSTAGES == 1 ? 1 : 2, d.JM - 1, dint, IntLines{});
     rk_blk<<<NVAR, RT_BS, 0, st>>>(d, a);
-    rk_density_prep<<<gridn(np, 128), 128, 0, st>>>(d, a);
+    rk_density_prep<<<gridn(np, 8), 256, 0, st>>>(d, a);
     ACK(cudaGetLastError());
-    s->sums.assign((size_t)4 * d.JM, 0.0);
-    ACK(cudaMemcpyAsync(s->sums.data(), dint, s->sums.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
+    ACK(cudaMemcpyAsync(s->sums, dint, sizeof(s->sums), cudaMemcpyDeviceToHost, st));
     // restore the state
-    ACK(cudaMemcpyAsync(d.RO, a.tRO, fb, cudaMemcpyDeviceToDevice, st));
-    ACK(cudaMemcpyAsync(d.ROVX, a.tROVX, fb, cudaMemcpyDeviceToDevice, st));
-    ACK(cudaMemcpyAsync(d.ROVR, a.tROVR, fb, cudaMemcpyDeviceToDevice, st));
-    ACK(cudaMemcpyAsync(d.RORVT, a.tRORVT, fb, cudaMemcpyDeviceToDevice, st));
-    ACK(cudaMemcpyAsync(d.ROE, a.tROE, fb, cudaMemcpyDeviceToDevice, st));
-    ACK(cudaMemcpyAsync(d.PEFF, a.tPEFF0, fb, cudaMemcpyDeviceToDevice, st));
-    for (int q = 0; q < nkeep; ++q) ACK(cudaMemcpyAsync(keep[q], save + (size_t)q * N, fb, cudaMemcpyDeviceToDevice, st));
-    ACK(cudaMemcpyAsync(d.PD, savepd, (size_t)d.KM * 4, cudaMemcpyDeviceToDevice, st));
-    ACK(cudaMemcpyAsync(d.ctl, savectl, sizeof(DevCtl), cudaMemcpyDeviceToDevice, st));
-    ACK(cudaFreeAsync(save, st));
-    ACK(cudaFreeAsync(savepd, st));
-    ACK(cudaFreeAsync(savectl, st));
+    {
+        CopyList l;
+        l.add(d.RO, a.tRO, N);
+        l.add(d.ROVX, a.tROVX, N);
+        l.add(d.ROVR, a.tROVR, N);
+        l.add(d.RORVT, a.tRORVT, N);
+        l.add(d.ROE, a.tROE, N);
+        l.add(d.PEFF, a.tPEFF0, N);
+        for (int q = 0; q < nkeep; ++q) l.add(keep[q], s->save + q * Np, N);
+        l.add(d.PD, savepd, (size_t)d.KM);
+        run_copies(l, sm, st);
+    }
+    ACK(cudaMemcpyAsync(d.ctl, s->savectl, sizeof(DevCtl), cudaMemcpyDeviceToDevice, st));
     int flag = 0;
     ACK(cudaMemcpyAsync(&flag, s->flag, sizeof(int), cudaMemcpyDeviceToHost, st));
     ACK(cudaStreamSynchronize(st));
     s->limiters = flag & 3;
     ACK(cudaMemsetAsync(s->flag, 0, sizeof(int), st));
     if ((rc = zero_adjoints(s, d, st))) return rc;
-    ACK(cudaMemsetAsync(s->seed, 0, (size_t)2 * (5 * d.IM * d.KM + d.IMM1 * d.KMM1) * sizeof(float), st));
-    s->a.seed_j[0] = 1;
-    s->a.seed_j[1] = 2;
+    rk_seed_set<<<1, 1, 0, st>>>(s->seed_on, 1, 2);
+    ACK(cudaGetLastError());
     s->objective = -1;
     s->value = 0.0;
     s->iters = 0;
-    // the reverse step as a CUDA graph
-    if (s->gexec) {
-        cudaGraphExecDestroy(s->gexec);
-        s->gexec = nullptr;
-    }
-    if (s->graph) {
-        cudaGraphDestroy(s->graph);
-        s->graph = nullptr;
-    }
-    {
-        const int one = 1;
-        ACK(cudaMemcpyAsync(s->seed_on, &one, sizeof(int), cudaMemcpyHostToDevice, st));
-    }
     ACK(cudaStreamSynchronize(st));
     s->ready = true;
     return 0;
@@ -2488,12 +2553,11 @@ int32_t mgpu_adjoint_objective(mgpu_handle *h, int32_t which, double *value) {
     const int per = 5 * d.IM * d.KM + d.IMM1 * d.KMM1;
     ACK(cudaMemsetAsync(s->seed, 0, (size_t)2 * per * sizeof(float), st));
     const int J1 = d.NSTAGES == 1 ? 1 : 2, J2M1 = d.JM - 1;
-    s->a.seed_j[0] = J1;
-    s->a.seed_j[1] = J2M1;
-    const std::vector<double> &v = s->sums;
-    auto bf = [&](int j) { return v[(size_t)(j - 1)]; };
-    auto spo = [&](int j) { return v[(size_t)d.JM + j - 1] / bf(j); };
-    auto sto = [&](int j) { return v[(size_t)2 * d.JM + j - 1] / bf(j); };
+    rk_seed_set<<<1, 1, 0, st>>>(s->seed_on, J1, J2M1);
+    const double *v = s->sums;
+    auto bf = [&](int j) { return v[j == J1 ? 0 : 4]; };
+    auto spo = [&](int j) { return v[j == J1 ? 1 : 5] / bf(j); };
+    auto sto = [&](int j) { return v[j == J1 ? 2 : 6] / bf(j); };
     double J = 0.0, g[2][3] = {{0, 0, 0}, {0, 0, 0}};   // per plane: dJ/dspo, dJ/dsto, dJ/dbf
     if (which == 1) {
         J = bf(J1);
@@ -2530,13 +2594,6 @@ int32_t mgpu_adjoint_objective(mgpu_handle *h, int32_t which, double *value) {
                                                                   g[p][2], spo(j), sto(j), bf(j));
         }
         ACK(cudaGetLastError());
-    }
-    // the seeds are kernel parameters of the captured graph (seed_j)
-    if (s->gexec) {
-        cudaGraphExecDestroy(s->gexec);
-        s->gexec = nullptr;
-        cudaGraphDestroy(s->graph);
-        s->graph = nullptr;
     }
     ACK(cudaStreamSynchronize(st));
     s->objective = which;
@@ -2764,13 +2821,11 @@ int32_t mgpu_adjoint_gradient_theta(mgpu_handle *h, float *djdtheta, int64_t nby
     const size_t N = (size_t)d.IM * d.JM * d.KM;
     if ((int64_t)(N * sizeof(float)) != nbytes) return api_fail(MGPU_E_ARG, "THETA gradient size mismatch");
     cudaStream_t st = handle_view(h).stream;
-    float *gth = nullptr;
-    ACK(cudaMallocAsync((void **)&gth, N * sizeof(float), st));
+    float *gth = s->gth;
     ACK(cudaMemsetAsync(gth, 0, N * sizeof(float), st));
     rk_metrics<<<gridn(N, 256), 256, 0, st>>>(d, s->a, gth);
     ACK(cudaGetLastError());
     ACK(cudaMemcpyAsync(djdtheta, gth, N * sizeof(float), cudaMemcpyDeviceToHost, st));
-    ACK(cudaFreeAsync(gth, st));
     ACK(cudaStreamSynchronize(st));
     return 0;
 }

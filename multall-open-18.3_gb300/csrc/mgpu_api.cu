@@ -83,7 +83,13 @@ struct mgpu_handle {
     std::vector<void *> allocs;
     StepGraph sg[4];             // one LOOP iteration by what it runs: 1 LOSS, 2 the tail
     bool ctl_known = false;      // h_ctl mirrors the control block: nothing has run since it was read
-    double *d_int = nullptr;     // integrals output (4 x JM)
+    double *d_int = nullptr;     // launch_station_sums (INT_BUF)
+    double *h_int = nullptr;     // its result, pinned (INT_OUT)
+    // host copies of what the reports read of the bound data, which is fixed
+    // after commit
+    std::vector<int> r_nstage, r_jstart, r_jmix, r_nrow;
+    std::vector<float> r_fp;
+    float r_po1 = 0.0f;          // PO1(KMID)
     void *flush_buf = nullptr;   // > L2, rewritten between timed iterations
     size_t flush_bytes = 0;
     DevCtl *h_ctl = nullptr;     // pinned mirror of the control block
@@ -444,6 +450,16 @@ int build_graph(mgpu_handle *h, int what) {
     return 0;
 }
 
+// FP64 mass averages at stations J1 and J2 (and lines of P) into h->h_int
+int station_sums(mgpu_handle *h, int J1, int J2, const IntLines &lines) {
+    launch_station_sums(h->d, Launch{h->stream, h->sm_count}, J1, J2, h->d_int, lines);
+    CK(cudaGetLastError());
+    const size_t bytes = 8 * sizeof(double) + (size_t)lines.n * lines.n * h->d.IM * sizeof(float);
+    CK(cudaMemcpyAsync(h->h_int, h->d_int, bytes, cudaMemcpyDeviceToHost, h->stream));
+    CK(cudaStreamSynchronize(h->stream));
+    return 0;
+}
+
 void fill_monitors(const DevCtl &c, mgpu_monitors *m) {
     memset(m, 0, sizeof(*m));
     m->nstep = c.nstep;
@@ -645,8 +661,9 @@ int32_t mgpu_create(int32_t im, int32_t jm, int32_t km, int32_t nrows, mgpu_hand
     if ((rc = dalloc(h, &d.part_key, d.nparts))) return bail(rc);
     if ((rc = dalloc(h, &d.part_cnt, d.nparts))) return bail(rc);
     if ((rc = dalloc(h, &d.ctl, 1))) return bail(rc);
-    if ((rc = dalloc(h, &h->d_int, (size_t)4 * jm))) return bail(rc);
+    if ((rc = dalloc(h, &h->d_int, (size_t)INT_BUF))) return bail(rc);
     e = cudaMallocHost((void **)&h->h_ctl, sizeof(DevCtl));
+    if (e == cudaSuccess) e = cudaMallocHost((void **)&h->h_int, INT_OUT * sizeof(double));
     if (e != cudaSuccess) return bail(fail(MGPU_E_NOMEM, cudaGetErrorString(e)));
     *out = h;
     return 0;
@@ -660,6 +677,7 @@ void mgpu_destroy(mgpu_handle *h) {
     for (StepGraph &G : h->sg) G.drop();
     for (void *p : h->allocs) cudaFree(p);
     if (h->h_ctl) cudaFreeHost(h->h_ctl);
+    if (h->h_int) cudaFreeHost(h->h_int);
     if (h->stream) cudaStreamDestroy(h->stream);
     if (h->side) cudaStreamDestroy(h->side);
     if (h->aux) cudaStreamDestroy(h->aux);
@@ -977,6 +995,13 @@ int32_t mgpu_commit(mgpu_handle *h) {
             return fail(MGPU_E_ARG, "leading/trailing edge indices out of range");
     if (INDMIX[d.JM - 1] != 0) return fail(MGPU_E_ARG, "INDMIX(JM) must be 0");
 
+    // what the reports read of the bound data
+    if (h->bound[find_array("NSTAGE")] && (rc = geti("NSTAGE", h->r_nstage))) return rc;
+    h->r_jstart = JSTART;
+    h->r_jmix = JMIX;
+    h->r_nrow = NROW;
+    h->r_fp = FP;
+    h->r_po1 = PO1[d.KMID - 1];
     d.RFTHROTL1 = 1.0f - d.RFTHROTL;
     // gas constants, SETUP 6459-6468
     d.GA1 = d.GA - 1.0f;
@@ -1177,27 +1202,17 @@ int32_t mgpu_sync(mgpu_handle *h) {
 int32_t mgpu_integrals_compute(mgpu_handle *h, mgpu_integrals *out) {
     if (!h || !h->committed || !out) return fail(MGPU_E_STATE, "integrals before commit");
     const Dev &d = h->d;
-    Launch L{h->stream, h->sm_count};
-    launch_integrals(d, L, h->d_int);
-    CK(cudaGetLastError());
-    std::vector<double> v((size_t)4 * d.JM);
-    CK(cudaMemcpyAsync(v.data(), h->d_int, v.size() * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-    CK(cudaStreamSynchronize(h->stream));
     // whole-machine efficiency (11269-11394): for one stage the inlet
     // station is J=1, otherwise J=2; the exit station is JM-1
     int J1 = d.NSTAGES == 1 ? 1 : 2, J2M1 = d.JM - 1;
-    auto bf = [&](int j) { return v[(size_t)(j - 1)]; };
-    auto spo = [&](int j) { return v[(size_t)d.JM + j - 1] / bf(j); };
-    auto sto = [&](int j) { return v[(size_t)2 * d.JM + j - 1] / bf(j); };
-    auto sps = [&](int j) { return v[(size_t)3 * d.JM + j - 1] / bf(j); };
-    double PO1M = 0.0;
-    {
-        std::vector<float> po1;
-        int a = find_array("PO1");
-        int rc = download(h, po1, (const float *)h->dptr[a], d.KM);
-        if (rc) return rc;
-        PO1M = po1[d.KMID - 1];
-    }
+    int rc = station_sums(h, J1, J2M1, IntLines{});
+    if (rc) return rc;
+    const double *v = h->h_int;
+    auto bf = [&](int j) { return v[j == J1 ? 0 : 4]; };
+    auto spo = [&](int j) { return v[j == J1 ? 1 : 5] / bf(j); };
+    auto sto = [&](int j) { return v[j == J1 ? 2 : 6] / bf(j); };
+    auto sps = [&](int j) { return v[j == J1 ? 3 : 7] / bf(j); };
+    const double PO1M = h->r_po1;
     double FGA = (double)d.FGA;
     double POIN = spo(J1) * PO1M, PO2 = spo(J2M1) * PO1M, PSOUT = sps(J2M1);
     double TO_IN = sto(J1), TO_OUT = sto(J2M1);
@@ -1225,22 +1240,9 @@ int32_t mgpu_stage_performance(mgpu_handle *h, int32_t nstg, mgpu_stage *out) {
     const int NSTAGES = d.NSTAGES, NROWS = d.NROWS;
     const int NSTGP1 = NSTAGES == 1 ? 1 : NSTAGES + 1;
     if (nstg < 1 || nstg > NSTGP1) return fail(MGPU_E_ARG, "stage number out of range");
-    const int an = find_array("NSTAGE");
-    if (!h->bound[an]) return fail(MGPU_E_STATE, "bind the row array NSTAGE for the stage table");
-    std::vector<int> NSTAGE, JSTART, JMIX, NROW;
-    std::vector<float> P, FP, PO1;
-    auto geti = [&](const char *n, std::vector<int> &v) {
-        int a = find_array(n);
-        return download(h, v, (const int *)h->dptr[a], shape_count(h, kArrays[a].shape));
-    };
-    auto getf = [&](const char *n, std::vector<float> &v) {
-        int a = find_array(n);
-        return download(h, v, (const float *)h->dptr[a], shape_count(h, kArrays[a].shape));
-    };
-    int rc = 0;
-    if ((rc = geti("NSTAGE", NSTAGE)) || (rc = geti("JSTART", JSTART)) || (rc = geti("JMIX", JMIX)) ||
-        (rc = geti("NROW", NROW)) || (rc = getf("P", P)) || (rc = getf("FP", FP)) || (rc = getf("PO1", PO1)))
-        return rc;
+    if (!h->bound[find_array("NSTAGE")]) return fail(MGPU_E_STATE, "bind the row array NSTAGE for the stage table");
+    const std::vector<int> &NSTAGE = h->r_nstage, &JSTART = h->r_jstart, &JMIX = h->r_jmix, &NROW = h->r_nrow;
+    const std::vector<float> &FP = h->r_fp;
     // the stages' stations, as the reader sets them (1522-1536)
     std::vector<int> JSTG_START(NSTAGES + 2, 0), JSTG_END(NSTAGES + 2, 0);
     JSTG_START[1] = 1;
@@ -1267,38 +1269,35 @@ int32_t mgpu_stage_performance(mgpu_handle *h, int32_t nstg, mgpu_stage *out) {
         JMS = (J1 + J2) / 2;
     }
     if (J1 < 1 || J2M1 > d.JM || J1 >= J2M1) return fail(MGPU_E_ARG, "stage stations out of range");
-    Launch L{h->stream, h->sm_count};
-    launch_integrals(d, L, h->d_int);
-    CK(cudaGetLastError());
-    std::vector<double> v((size_t)4 * d.JM);
-    CK(cudaMemcpyAsync(v.data(), h->d_int, v.size() * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-    CK(cudaStreamSynchronize(h->stream));
-    auto bf = [&](int j) { return v[(size_t)(j - 1)]; };
-    auto spo = [&](int j) { return v[(size_t)d.JM + j - 1] / bf(j); };
-    auto sto = [&](int j) { return v[(size_t)2 * d.JM + j - 1] / bf(j); };
-    auto sps = [&](int j) { return v[(size_t)3 * d.JM + j - 1] / bf(j); };
-    const double PO1M = PO1[d.KMID - 1], FGA = (double)d.FGA;
+    const int KMID2 = d.KM / 2;
+    IntLines lines{};
+    if (!whole) lines = IntLines{3, {J1, JMS, J2M1}, {1, KMID2, d.KM}};
+    int rc = station_sums(h, J1, J2M1, lines);
+    if (rc) return rc;
+    const double *v = h->h_int;
+    auto bf = [&](int j) { return v[j == J1 ? 0 : 4]; };
+    auto spo = [&](int j) { return v[j == J1 ? 1 : 5] / bf(j); };
+    auto sto = [&](int j) { return v[j == J1 ? 2 : 6] / bf(j); };
+    auto sps = [&](int j) { return v[j == J1 ? 3 : 7] / bf(j); };
+    const double PO1M = h->r_po1, FGA = (double)d.FGA;
     out->j1 = J1;
     out->j2m1 = J2M1;
     out->jmix = JMS;
     out->has_reaction = !whole;
     out->reac_hub = out->reac_mid = out->reac_tip = 0.0;
     if (!whole) {
-        // pitchwise static pressures, REAL*4 in I order (11300-11349)
-        const int KMID2 = d.KM / 2;
-        auto pline = [&](int j, int k) {
+        // pitchwise static pressures, REAL*4 in I order (11300-11349), at the
+        // stations J1, JMS, J2M1 (a) and K = 1, KM/2, KM (b)
+        auto pline = [&](int a, int b) {
+            const float *P = (const float *)(h->h_int + 8) + (size_t)(3 * a + b) * d.IM;
             float s = 0.0f;
-            for (int i = 1; i <= d.IMM1; ++i) {
-                const size_t a = (size_t)(i - 1) + (size_t)d.IM * ((size_t)(j - 1) + (size_t)d.JM * (size_t)(k - 1));
-                s = s + 0.5f * (P[a] + P[a + 1]) * FP[i - 1];
-            }
+            for (int i = 0; i < d.IMM1; ++i) s = s + 0.5f * (P[i] + P[i + 1]) * FP[i];
             return s;
         };
-        const int ks[3] = {1, KMID2, d.KM};
         float rr[3];
-        const float pmid_in = pline(J1, KMID2), pmid_out = pline(J2M1, KMID2);
+        const float pmid_in = pline(0, 1), pmid_out = pline(2, 1);
         for (int q = 0; q < 3; ++q) {
-            const float pin = pline(J1, ks[q]), pm = pline(JMS, ks[q]), po = pline(J2M1, ks[q]);
+            const float pin = pline(0, q), pm = pline(1, q), po = pline(2, q);
             rr[q] = (pm - po) / (pin - po);
             if (pmid_out > pmid_in) rr[q] = 1.0f - rr[q];    // a compressor
         }

@@ -393,7 +393,16 @@ size_t sa_work_floats(const Dev &d);
 void launch_tstep_cells_prolong(const Dev &d, Launch L, int v0, int nv);
 void launch_tail(const Dev &d, Launch L);
 void launch_stepup(const Dev &d, Launch L, float relax);
-void launch_integrals(const Dev &d, Launch L, double *out8);
+// the FP64 mass averages of EFICOOL at two stations: out[4 p + q] = mass flow,
+// flow x PO/PO1, flow x TO, flow x P at station p, and behind them, with
+// lines.n = 3, P(1..IM) at (j[a], k[b]) as floats, line 3 a + b; work space in
+// out up to INT_BUF doubles
+struct IntLines {
+    int n, j[3], k[3];
+};
+constexpr int INT_OUT = 8 + 9 * 160 / 2;      // doubles of the result
+constexpr int INT_BUF = INT_OUT + 2 * 24 * 4;
+void launch_station_sums(const Dev &d, Launch L, int J1, int J2, double *out, const IntLines &lines);
 
 // Raises a kernel's dynamic shared-memory limit to `bytes` (at least the
 // 48 KB default) and never lowers it: the limit belongs to the function, not
@@ -465,7 +474,7 @@ void adj_destroy(AdjState *a);
 AdjState *&handle_adj(mgpu_handle *h);
 Dev &handle_dev(mgpu_handle *h);
 int handle_sm_count(const mgpu_handle *h);
-double *handle_int_buf(mgpu_handle *h);        // (4, JM) FP64 integrals scratch
+double *handle_int_buf(mgpu_handle *h);        // INT_BUF doubles
 const void *handle_array(const mgpu_handle *h, const char *name, size_t *bytes);
 // Records msg for mgpu_last_error() and returns code.
 int api_fail(int code, const char *msg);

@@ -916,62 +916,83 @@ void launch_tail(const Dev &d, Launch L) {
 // ---------------------------------------------------------------------
 // EFICOOL node quantities (5610) and SUMFLX mass averages per J, FP64
 // ---------------------------------------------------------------------
-__global__ void k_int_node(Dev d) {
-    pdl_wait();
-    size_t n = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    size_t N = (size_t)d.IM * d.JM * d.KM;
-    if (n >= N) return;
-    float TO1M = A1(d.TO1, d.KMID), PO1M = A1(d.PO1, d.KMID);
-    float vx = d.VX[n], vt = d.VT[n], vr = d.VR[n];
-    float EKE = 0.5f * (vx * vx + vt * vt + vr * vr);
-    float TS = (d.HO[n] - EKE) * d.RCP;
-    float TSTAG = d.HO[n] * d.RCP;
-    if (TSTAG < 0.1f * TO1M) TSTAG = 0.1f * TO1M;
-    if (TS < 0.1f * TO1M) TS = 0.1f * TO1M;
-    float PSTAT = d.P[n];
-    if (PSTAT < 0.02f * PO1M) PSTAT = 0.02f * PO1M;
-    float PSTAG = PSTAT * powf(TSTAG / TS, d.RFGA);
-    d.TEMP1[n] = TSTAG;       // TEMP1: stagnation temperature
-    d.TMP[n] = PSTAG / PO1M;  // TEMP2: stagnation pressure ratio
-}
+// One CTA per station and slice of K rows forms the stagnation temperature
+// and pressure ratio of its nodes and sums its cells in FP64; the last CTA adds
+// the slices in order.  Only the two stations that the efficiencies take are
+// summed: over all JM stations the FP64 work took 60 us at 65 x 242 x 49, and
+// at one CTA a station one SM's FP64 pipe would still take 25.  lines.n = 3:
+// the last CTA also gathers P along I at the three stations and three K of
+// the reactions.
+constexpr int INT_BS = 128;
+constexpr int INT_SPLIT = 24;
+constexpr int INT_ROWS = 159 / INT_SPLIT + 2;     // node rows of a slice: commit limits KM to 160
 
-__global__ void __launch_bounds__(TAIL_BS) k_int_sum(Dev d, double *out) {
+__global__ void __launch_bounds__(INT_BS) k_int_stations(const __grid_constant__ Dev d, int J1, int J2, double *out,
+                                                         const __grid_constant__ IntLines lines) {
     pdl_wait();
-    int j = blockIdx.x + 1;
-    int ncell = d.IMM1 * d.KMM1;
-    double bf = 0, spo = 0, sto = 0, sps = 0;
-    double nb = (double)A1(d.NBLADE, j);
-    for (int c = threadIdx.x; c < ncell; c += TAIL_BS) {
-        int i = c % d.IMM1 + 1, k = c / d.IMM1 + 1;
-        double DFLOW = -(double)A3(d.FLOWX, i, j, k) * nb;
-        double DFLOW4 = 0.25 * DFLOW;
-        bf += DFLOW;
-        spo += DFLOW4 * ((double)A3(d.TMP, i, j, k) + A3(d.TMP, i + 1, j, k) + A3(d.TMP, i + 1, j, k + 1) + A3(d.TMP, i, j, k + 1));
-        sto += DFLOW4 * ((double)A3(d.TEMP1, i, j, k) + A3(d.TEMP1, i + 1, j, k) + A3(d.TEMP1, i + 1, j, k + 1) +
-                         A3(d.TEMP1, i, j, k + 1));
-        sps += DFLOW4 * ((double)A3(d.P, i, j, k) + A3(d.P, i + 1, j, k) + A3(d.P, i + 1, j, k + 1) + A3(d.P, i, j, k + 1));
+    __shared__ float s_t[INT_ROWS * 160], s_r[INT_ROWS * 160], s_p[INT_ROWS * 160];
+    __shared__ double sh[INT_BS / 32][4];
+    const int j = blockIdx.y ? J2 : J1;
+    const int per = (d.KMM1 + INT_SPLIT - 1) / INT_SPLIT;
+    const int ka = (int)blockIdx.x * per + 1, ke = min(ka + per - 1, d.KMM1);   // cell rows
+    const int IM = d.IM, IMM1 = d.IMM1;
+    const float TO1M = A1(d.TO1, d.KMID), PO1M = A1(d.PO1, d.KMID);
+    for (int t = threadIdx.x; t < (ke >= ka ? (ke - ka + 2) * IM : 0); t += INT_BS) {
+        const int n = ix3(d, t % IM + 1, j, ka + t / IM);
+        const float vx = d.VX[n], vt = d.VT[n], vr = d.VR[n], ho = d.HO[n];
+        float PSTAT = d.P[n];
+        s_p[t] = PSTAT;
+        float EKE = 0.5f * (vx * vx + vt * vt + vr * vr);
+        float TS = (ho - EKE) * d.RCP;
+        float TSTAG = ho * d.RCP;
+        if (TSTAG < 0.1f * TO1M) TSTAG = 0.1f * TO1M;
+        if (TS < 0.1f * TO1M) TS = 0.1f * TO1M;
+        if (PSTAT < 0.02f * PO1M) PSTAT = 0.02f * PO1M;
+        s_t[t] = TSTAG;
+        s_r[t] = PSTAT * powf(TSTAG / TS, d.RFGA) / PO1M;
     }
-    __shared__ double sh[4][TAIL_BS / 32];
-    double v[4] = {bf, spo, sto, sps};
+    __syncthreads();
+    double v[4] = {0.0, 0.0, 0.0, 0.0};
+    const double nb = (double)A1(d.NBLADE, j);
+    for (int c = threadIdx.x; c < (ke >= ka ? (ke - ka + 1) * IMM1 : 0); c += INT_BS) {
+        const int il = c % IMM1, kl = c / IMM1, o = il + IM * kl;
+        const double DFLOW = -(double)A3(d.FLOWX, il + 1, j, ka + kl) * nb;
+        const double DFLOW4 = 0.25 * DFLOW;
+        auto four = [&](const float *q) { return (double)q[o] + q[o + 1] + q[o + IM + 1] + q[o + IM]; };
+        v[0] += DFLOW;
+        v[1] += DFLOW4 * four(s_r);
+        v[2] += DFLOW4 * four(s_t);
+        v[3] += DFLOW4 * four(s_p);
+    }
     for (int q = 0; q < 4; ++q) {
         double x = v[q];
         for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-        if ((threadIdx.x & 31) == 0) sh[q][threadIdx.x >> 5] = x;
+        if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5][q] = x;
     }
     __syncthreads();
+    double *part = out + INT_OUT;                 // (2, INT_SPLIT, 4)
     if (threadIdx.x < 4) {
         double t = 0.0;
-        for (int w = 0; w < TAIL_BS / 32; ++w) t += sh[threadIdx.x][w];
-        out[(size_t)threadIdx.x * d.JM + (j - 1)] = t;
+        for (int w = 0; w < INT_BS / 32; ++w) t += sh[w][threadIdx.x];
+        part[((size_t)blockIdx.y * INT_SPLIT + blockIdx.x) * 4 + threadIdx.x] = t;
+    }
+    if (!last_cta(&d.ctl->ticket, gridDim.x * gridDim.y)) return;
+    if (threadIdx.x < 8) {
+        const int p = threadIdx.x >> 2, q = threadIdx.x & 3;
+        double t = 0.0;
+        for (int w = 0; w < INT_SPLIT; ++w) t += part[((size_t)p * INT_SPLIT + w) * 4 + q];
+        out[threadIdx.x] = t;
+    }
+    float *ln = (float *)(out + 8);
+    for (int t = threadIdx.x; t < lines.n * lines.n * IM; t += INT_BS) {
+        const int l = t / IM;
+        ln[t] = A3(d.P, t % IM + 1, lines.j[l / 3], lines.k[l % 3]);
     }
 }
 
-void launch_integrals(const Dev &d, Launch L, double *out) {
-    size_t N = (size_t)d.IM * d.JM * d.KM;
-    launchk(L, k_int_node, dim3(grid_for(N, 256)), dim3(256), 0, d);
-    mark(L, "k_int_node");
-    launchk(L, k_int_sum, dim3(d.JM), dim3(TAIL_BS), 0, d, out);
-    mark(L, "k_int_sum");
+void launch_station_sums(const Dev &d, Launch L, int J1, int J2, double *out, const IntLines &lines) {
+    launchk(L, k_int_stations, dim3(INT_SPLIT, 2), dim3(INT_BS), 0, d, J1, J2, out, lines);
+    mark(L, "k_int_stations");
 }
 
 // ---------------------------------------------------------------------
