@@ -367,15 +367,37 @@ __global__ void __launch_bounds__(1024) k_bc_sums(Dev d) {
     for (int k = threadIdx.x; k < KM; k += blockDim.x) d.PD[k] = s_pd[k];
 }
 
-__global__ void k_bc_apply(Dev d) {
+// Two threads a point, in different CTAs (blockIdx.y): the inlet state and the
+// exit state, which depend on nothing of each other; each loads what it reads
+// before it stores.
+__global__ void k_bc_apply(const __grid_constant__ Dev d) {
     pdl_wait();
     int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= d.IM * d.KM) return;
     int i = t % d.IM + 1, k = t / d.IM + 1;
+    if (blockIdx.y) {
+        // exit: pitchwise pressure variation extrapolated from upstream
+        float vr = A3(d.VR, i, d.JM, k), vt = A3(d.VT, i, d.JM, k), vx = A3(d.VX, i, d.JM, k);
+        float EKE = 0.5f * (vr * vr + vt * vt + vx * vx);
+        float pe = d.BCBUF[3 * d.KM + k - 1] + d.FEXTRAP * (A3(d.P, i, d.JMM1, k) - d.BCBUF[2 * d.KM + k - 1]);
+        float hoe = 2.0f * A3(d.HO, i, d.JMM1, k) - A3(d.HO, i, d.JM - 2, k);
+        float TEXIT = (hoe - EKE) / d.CP;
+        float roe_ = pe / d.RGAS / TEXIT;
+        A3(d.P, i, d.JM, k) = pe;
+        A3(d.HO, i, d.JM, k) = hoe;
+        A3(d.RO, i, d.JM, k) = roe_;
+        A3(d.ROE, i, d.JM, k) = roe_ * (d.CV * TEXIT + EKE);
+        return;
+    }
     float PO1 = A1(d.PO1, k), TO1 = A1(d.TO1, k);
     // inlet, isentropic from the stagnation state
     float RO_STAG = PO1 / d.RGAS / TO1;
     float RO_IN = A3(d.RO, i, 1, k);
+    const float p2 = A3(d.P, i, 2, k), p3 = A3(d.P, i, 3, k);
+    float vt1 = A3(d.VT, i, 1, k), vx1 = A3(d.VX, i, 1, k), vr1 = A3(d.VR, i, 1, k);
+    const float vr2 = A3(d.VR, i, 2, k), r1 = A2(d.R, 1, k);
+    float p1 = A3(d.P, i, 1, k);
+    const float rpo1 = A1(d.RPO1, k), bscos = A1(d.BSCOS, k), bssin = A1(d.BSSIN, k), plim = A1(d.PLIM, k);
     if (d.ADJ_ROIN) d.ADJ_ROIN[t] = RO_IN;
     // the Spalart-Allmaras inlet value divides by RO(IMID,1,KMID) as the
     // reference's K, I loop finds it: the inlet points before (IMID, KMID)
@@ -383,25 +405,20 @@ __global__ void k_bc_apply(Dev d) {
     if (d.SAW && i == d.IMID && k == d.KMID) d.SAW[sa_work_node_floats(d) + 64 + 2] = RO_IN;
     if (RO_IN > 0.9999f * RO_STAG) RO_IN = 0.9999f * RO_STAG;
     float PNEW = PO1 * powf(RO_IN / RO_STAG, d.GA);
-    float p1 = A3(d.P, i, 1, k);
     int ip = d.IN_PRESS < 0 ? -d.IN_PRESS : d.IN_PRESS;
     if (d.IN_PRESS == 0) p1 = d.RFIN1 * p1 + d.RFIN * PNEW;
-    if (ip == 1) p1 = d.RFIN1 * p1 + d.RFIN2 * A3(d.P, i, 2, k) - d.RFIN * A3(d.P, i, 3, k);
+    if (ip == 1) p1 = d.RFIN1 * p1 + d.RFIN2 * p2 - d.RFIN * p3;
     if (ip == 3) p1 = d.RFIN1 * p1 + d.RFIN2 * d.BCBUF[k - 1] - d.RFIN * d.BCBUF[d.KM + k - 1];
     if (ip == 4) p1 = d.RFIN1 * p1 + d.RFIN2 * A3(d.P, d.IMID, 2, d.KMID) - d.RFIN * A3(d.P, d.IMID, 3, d.KMID);
-    float plim = A1(d.PLIM, k);
     if (p1 > plim) p1 = 0.9f * p1 + 0.1f * plim;
     if (p1 > 0.99999f * PO1) p1 = PO1 * 0.99999f;
-    A3(d.P, i, 1, k) = p1;
-    float TSTATIC = TO1 * powf(p1 * A1(d.RPO1, k), d.FGA);
+    float TSTATIC = TO1 * powf(p1 * rpo1, d.FGA);
     float VABSQ = 2.0f * d.CP * (TO1 - TSTATIC);
-    A3(d.T_STATIC, i, 1, k) = TSTATIC;
     float VABS = sqrtf(VABSQ);
     float VMER = 0.0f;
-    float vt1 = A3(d.VT, i, 1, k);
     if (d.IN_VTAN == 0) {
-        VMER = VABS * A1(d.BSCOS, k);
-        vt1 = VABS * A1(d.BSSIN, k);
+        VMER = VABS * bscos;
+        vt1 = VABS * bssin;
     }
     if (d.IN_VTAN == 1) {
         float VMERSQ = VABSQ - A1(d.VTIN, k) * A1(d.VTIN, k);
@@ -411,21 +428,21 @@ __global__ void k_bc_apply(Dev d) {
     }
     if (d.IN_VTAN == 2) {
         float WR = A2(d.UBLADE, 1, k);
-        float VRELSQ = VABSQ - WR * WR * A1(d.BSCOS, k) * A1(d.BSCOS, k);
+        float VRELSQ = VABSQ - WR * WR * bscos * bscos;
         if (VRELSQ < 0.01f) VRELSQ = 0.01f;
-        float VREL = sqrtf(VRELSQ) - WR * A1(d.BSSIN, k);
-        VMER = VREL * A1(d.BSCOS, k);
-        vt1 = VREL * A1(d.BSSIN, k) + WR;
+        float VREL = sqrtf(VRELSQ) - WR * bssin;
+        VMER = VREL * bscos;
+        vt1 = VREL * bssin + WR;
     }
-    A3(d.VT, i, 1, k) = vt1;
-    float vx1 = A3(d.VX, i, 1, k), vr1 = A3(d.VR, i, 1, k);
-    float vr2 = A3(d.VR, i, 2, k);
     if (d.IN_VR > 0) vx1 = VMER * A1(d.BRCOS, k);
     float VXSQ = VMER * VMER - vr2 * vr2;
     if (VXSQ < 0.0000001f * TO1 * d.CP) VXSQ = 0.0000001f * TO1 * d.CP;
     if (d.IN_VR <= 0) vx1 = sqrtf(VXSQ);
     if (d.IN_VR > 0) vr1 = VMER * A1(d.BRSIN, k);
     if (d.IN_VR <= 0) vr1 = vr2;
+    A3(d.P, i, 1, k) = p1;
+    A3(d.T_STATIC, i, 1, k) = TSTATIC;
+    A3(d.VT, i, 1, k) = vt1;
     A3(d.VX, i, 1, k) = vx1;
     A3(d.VR, i, 1, k) = vr1;
     float ro1 = p1 / (d.RGAS * TSTATIC);
@@ -433,21 +450,10 @@ __global__ void k_bc_apply(Dev d) {
     A3(d.RO, i, 1, k) = ro1;
     A3(d.ROVT, i, 1, k) = rovt1;
     A3(d.ROVR, i, 1, k) = ro1 * vr1;
-    A3(d.RORVT, i, 1, k) = rovt1 * A2(d.R, 1, k);
+    A3(d.RORVT, i, 1, k) = rovt1 * r1;
     A3(d.ROVX, i, 1, k) = ro1 * vx1;
     A3(d.ROE, i, 1, k) = p1 / d.GA1 + ro1 * 0.5f * VABSQ;
     A3(d.HO, i, 1, k) = d.CP * TO1;
-    // exit: pitchwise pressure variation extrapolated from upstream
-    float vr = A3(d.VR, i, d.JM, k), vt = A3(d.VT, i, d.JM, k), vx = A3(d.VX, i, d.JM, k);
-    float EKE = 0.5f * (vr * vr + vt * vt + vx * vx);
-    float pe = d.BCBUF[3 * d.KM + k - 1] + d.FEXTRAP * (A3(d.P, i, d.JMM1, k) - d.BCBUF[2 * d.KM + k - 1]);
-    float hoe = 2.0f * A3(d.HO, i, d.JMM1, k) - A3(d.HO, i, d.JM - 2, k);
-    float TEXIT = (hoe - EKE) / d.CP;
-    float roe_ = pe / d.RGAS / TEXIT;
-    A3(d.P, i, d.JM, k) = pe;
-    A3(d.HO, i, d.JM, k) = hoe;
-    A3(d.RO, i, d.JM, k) = roe_;
-    A3(d.ROE, i, d.JM, k) = roe_ * (d.CV * TEXIT + EKE);
 }
 
 static size_t bc_sums_smem(const Dev &d) { return (size_t)32 * (4 * d.IMM1 + 2 * d.IM) * sizeof(float); }
@@ -462,7 +468,7 @@ void launch_bc_sums(const Dev &d, Launch L) {
 }
 
 void launch_bc_apply(const Dev &d, Launch L) {
-    launchk(L, k_bc_apply, dim3((d.IM * d.KM + 127) / 128), dim3(128), 0, d);
+    launchk(L, k_bc_apply, dim3((d.IM * d.KM + 127) / 128, 2), dim3(128), 0, d);
     mark(L, "k_bc_apply");
 }
 
@@ -1058,6 +1064,10 @@ __global__ void __launch_bounds__(MIX_BS) k_mixplan(const __grid_constant__ Dev 
     }
     __syncthreads();
     for (int i = threadIdx.x + 1; i <= IM; i += MIX_BS) {
+        // loaded before the first store: one variable after the other would be
+        // five round trips
+        const int n = ix3(d, i, JP2, k);
+        const float ro = d.RO[n], rovx = d.ROVX[n], rovr = d.ROVR[n], rorvt = d.RORVT[n], roe = d.ROE[n];
         float RO_JP2 = ROISENT[i - 1];
         float WT_JP2 = WIS_JP2[i - 1] * sinf(ALPHAA[i - 1]);
         float VM_JP2 = WIS_JP2[i - 1] * cosf(ALPHAA[i - 1]);
@@ -1066,11 +1076,11 @@ __global__ void __launch_bounds__(MIX_BS) k_mixplan(const __grid_constant__ Dev 
         float VT_JP2 = WT_JP2 + UNOWJP2;
         float V_JP2_SQ = VM_JP2 * VM_JP2 + VT_JP2 * VT_JP2;
         float ROE_JP2 = ROISENT[i - 1] * (d.CV * TISENT[i - 1] + 0.5f * V_JP2_SQ);
-        A3(d.RO, i, JP2, k) = RFMIX1 * A3(d.RO, i, JP2, k) + d.RFMIX * RO_JP2;
-        A3(d.ROVX, i, JP2, k) = RFMIX1 * A3(d.ROVX, i, JP2, k) + d.RFMIX * RO_JP2 * VX_JP2;
-        A3(d.ROVR, i, JP2, k) = RFMIX1 * A3(d.ROVR, i, JP2, k) + d.RFMIX * RO_JP2 * VR_JP2;
-        A3(d.RORVT, i, JP2, k) = RFMIX1 * A3(d.RORVT, i, JP2, k) + d.RFMIX * RO_JP2 * VT_JP2 * RJP2;
-        A3(d.ROE, i, JP2, k) = RFMIX1 * A3(d.ROE, i, JP2, k) + d.RFMIX * ROE_JP2;
+        d.RO[n] = RFMIX1 * ro + d.RFMIX * RO_JP2;
+        d.ROVX[n] = RFMIX1 * rovx + d.RFMIX * RO_JP2 * VX_JP2;
+        d.ROVR[n] = RFMIX1 * rovr + d.RFMIX * RO_JP2 * VR_JP2;
+        d.RORVT[n] = RFMIX1 * rorvt + d.RFMIX * RO_JP2 * VT_JP2 * RJP2;
+        d.ROE[n] = RFMIX1 * roe + d.RFMIX * ROE_JP2;
     }
 }
 

@@ -331,16 +331,31 @@ __global__ void __launch_bounds__(32 * LK_W) k_loss_kfaces(const __grid_constant
     };
     if (col) {
         const float VISLAM = s_vis[tx];
-        for (int k = ty + 2; k <= KMM1; k += LK_W) {
-            // FYPLUS keeps its previous value where Y_PLUS is NaN
-            int kk = k;
-            while (kk >= 2 && isnan(A3(d.Y_PLUS, i, j, kk))) --kk;
-            float FYPLUS = kk >= 2 ? fyplus_of(A3(d.Y_PLUS, i, j, kk), d.YPLAM, d.YPTURB, 0.0f) : 0.0f;
-            float DPERP = A3(d.VOL, i, j, k) / LK(AREA, k);
-            LK(VLAM, k) = d.FKLAM[(size_t)(NRW - 1) * KM + k - 1] * VISLAM / DPERP;
-            float vt = d.FKTURB[(size_t)(NRW - 1) * KM + k - 1] * LK(ROAVG, k) * fabsf(wabs(k + 1) - wabs(k - 1)) *
-                       FMIXUP;
-            LK(VTURB, k) = vt * FYPLUS;
+        // two faces at a time, their global operands loaded together
+        for (int k0 = ty + 2; k0 <= KMM1; k0 += 2 * LK_W) {
+            float yp[2], vol[2], fl[2], ft[2];
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const int k = min(k0 + u * LK_W, KMM1);
+                yp[u] = A3(d.Y_PLUS, i, j, k);
+                vol[u] = A3(d.VOL, i, j, k);
+                fl[u] = d.FKLAM[(size_t)(NRW - 1) * KM + k - 1];
+                ft[u] = d.FKTURB[(size_t)(NRW - 1) * KM + k - 1];
+            }
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const int k = k0 + u * LK_W;
+                if (k > KMM1) continue;
+                // FYPLUS keeps its previous value where Y_PLUS is NaN
+                int kk = k;
+                float y = yp[u];
+                while (isnan(y) && --kk >= 2) y = A3(d.Y_PLUS, i, j, kk);
+                float FYPLUS = kk >= 2 ? fyplus_of(y, d.YPLAM, d.YPTURB, 0.0f) : 0.0f;
+                float DPERP = vol[u] / LK(AREA, k);
+                LK(VLAM, k) = fl[u] * VISLAM / DPERP;
+                float vt = ft[u] * LK(ROAVG, k) * fabsf(wabs(k + 1) - wabs(k - 1)) * FMIXUP;
+                LK(VTURB, k) = vt * FYPLUS;
+            }
         }
     }
     __syncthreads();
@@ -386,15 +401,34 @@ __global__ void __launch_bounds__(32 * LK_W) k_loss_kfaces(const __grid_constant
                 wv = xs * LK(VXAVG, kp) + ts * LK(VTAVG, kp) + rs * LK(VRAVG, kp);
             }
         };
-        for (int k = ty + 1; k <= KMM1; k += LK_W) {
-            float xl, rl, tl, ql, wl, xh, rh, th, qh, wh;
-            face(k, xl, rl, tl, ql, wl);
-            face(k + 1, xh, rh, th, qh, wh);
-            size_t n = ix3(d, i, j, k);
-            d.XFORCE[n] = RF_VIS1 * d.XFORCE[n] + RF_VIS * (xl - xh);
-            d.RFORCE[n] = RF_VIS1 * d.RFORCE[n] + RF_VIS * (rl - rh);
-            d.TFORCE[n] = RF_VIS1 * d.TFORCE[n] + RF_VIS * (tl * RAVGK[k - 1] - th * RAVGK[k]);
-            d.QSOURCE[n] = RF_VIS1 * d.QSOURCE[n] + RF_VIS * (ql - qh + wl - wh);
+        // two cells at a time, their old forces loaded before the first store
+        // (a store through one Dev pointer keeps later loads through another
+        // behind it: one array after the other cost four round trips a cell)
+        for (int k0 = ty + 1; k0 <= KMM1; k0 += 2 * LK_W) {
+            float f[2][4];
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const int k = k0 + u * LK_W;
+                if (k > KMM1) continue;
+                const int n = ix3(d, i, j, k);
+                f[u][0] = d.XFORCE[n];
+                f[u][1] = d.RFORCE[n];
+                f[u][2] = d.TFORCE[n];
+                f[u][3] = d.QSOURCE[n];
+            }
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const int k = k0 + u * LK_W;
+                if (k > KMM1) continue;
+                float xl, rl, tl, ql, wl, xh, rh, th, qh, wh;
+                face(k, xl, rl, tl, ql, wl);
+                face(k + 1, xh, rh, th, qh, wh);
+                const int n = ix3(d, i, j, k);
+                d.XFORCE[n] = RF_VIS1 * f[u][0] + RF_VIS * (xl - xh);
+                d.RFORCE[n] = RF_VIS1 * f[u][1] + RF_VIS * (rl - rh);
+                d.TFORCE[n] = RF_VIS1 * f[u][2] + RF_VIS * (tl * RAVGK[k - 1] - th * RAVGK[k]);
+                d.QSOURCE[n] = RF_VIS1 * f[u][3] + RF_VIS * (ql - qh + wl - wh);
+            }
         }
     }
 #undef LK
@@ -629,12 +663,29 @@ __global__ void __launch_bounds__(32 * LI_W, 8) k_loss_ifaces(const __grid_const
         }
     }
     __syncwarp();
-    for (int i = lane + 1; i <= IMM1; i += 32) {
-        size_t n = ix3(d, i, j, k);
-        d.XFORCE[n] = d.XFORCE[n] + RF_VIS * (XSTRES[i] - XSTRES[i + 1]);
-        d.RFORCE[n] = d.RFORCE[n] + RF_VIS * (RSTRES[i] - RSTRES[i + 1]);
-        d.TFORCE[n] = d.TFORCE[n] + RF_VIS * (TSTRES[i] - TSTRES[i + 1]) * RAVGK;
-        d.QSOURCE[n] = d.QSOURCE[n] + RF_VIS * (QFLOW[i] - QFLOW[i + 1] + WVISC[i] - WVISC[i + 1]);
+    // two cells a lane at a time, loads before stores as in k_loss_kfaces
+    for (int i0 = lane + 1; i0 <= IMM1; i0 += 64) {
+        float f[2][4];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const int i = i0 + 32 * u;
+            if (i > IMM1) continue;
+            const int n = ix3(d, i, j, k);
+            f[u][0] = d.XFORCE[n];
+            f[u][1] = d.RFORCE[n];
+            f[u][2] = d.TFORCE[n];
+            f[u][3] = d.QSOURCE[n];
+        }
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const int i = i0 + 32 * u;
+            if (i > IMM1) continue;
+            const int n = ix3(d, i, j, k);
+            d.XFORCE[n] = f[u][0] + RF_VIS * (XSTRES[i] - XSTRES[i + 1]);
+            d.RFORCE[n] = f[u][1] + RF_VIS * (RSTRES[i] - RSTRES[i + 1]);
+            d.TFORCE[n] = f[u][2] + RF_VIS * (TSTRES[i] - TSTRES[i + 1]) * RAVGK;
+            d.QSOURCE[n] = f[u][3] + RF_VIS * (QFLOW[i] - QFLOW[i + 1] + WVISC[i] - WVISC[i + 1]);
+        }
     }
 }
 
