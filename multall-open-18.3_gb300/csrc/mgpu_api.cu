@@ -282,9 +282,10 @@ struct SaBranch {
     cudaEvent_t start = nullptr, bc = nullptr, done = nullptr;
 };
 
-// A third: the density limiter reads and writes nothing that TSTEP of the
-// momenta touches, so its walks along J (58 us on 73 x 752 x 57, one block's
-// work) run beside it; the Mach limiter waits for both.
+// A third: the density limiter reads and writes nothing that the momentum
+// fluxes and TSTEP of the momenta touch, so its scan and its walks along J
+// (58 us on 73 x 752 x 57, a few blocks' work) run beside them; the Mach
+// limiter waits for both.
 struct DensBranch {
     cudaStream_t s = nullptr;
     cudaEvent_t start = nullptr, done = nullptr;
@@ -322,18 +323,19 @@ void enqueue_core(const Dev &d, Launch L, Launch Lf, cudaEvent_t join = nullptr,
         launch_sa_inlet(d, L);
     }
     if (d.IN_FLOW != 0) launch_setflo(d, L);
-    launch_flux_mom(d, L);          // also PEFF and the density limiter's column flags
     if (dens) {
         cudaEventRecord(dens->start, L.s);
         cudaStreamWaitEvent(dens->s, dens->start, 0);
         if (sab) cudaStreamWaitEvent(dens->s, sa->done, 0);
         launch_density_fix(d, Launch{dens->s, L.sm_count, nullptr});
         cudaEventRecord(dens->done, dens->s);
-        launch_tstep(d, L, V_ROVX, 3);
+    }
+    launch_flux_mom(d, L);          // also PEFF
+    launch_tstep(d, L, V_ROVX, 3);
+    if (dens) {
         cudaStreamWaitEvent(L.s, dens->done, 0);
         launch_mach_limiter(d, L0);
     } else {
-        launch_tstep(d, L, V_ROVX, 3);
         launch_density_fix(d, L);
         launch_mach_limiter(d, L);
     }
@@ -634,9 +636,14 @@ int32_t mgpu_create(int32_t im, int32_t jm, int32_t km, int32_t nrows, mgpu_hand
             V.RF = d.FLOWR;
             V.SR = d.ZERO;
         } else {
-            float **fl[] = {&V.XF, &V.TF, &V.RF, &V.SR};
+            float **fl[] = {&V.XF, &V.TF, &V.RF};
             for (float **w : fl)
                 if ((rc = dalloc(h, w, N))) return bail(rc);
+            // the sources of ROE, ROVX and RORVT are COMMON arrays
+            if (v == V_ROE) V.SR = d.QSOURCE;
+            else if (v == V_ROVX) V.SR = d.XFORCE;
+            else if (v == V_RORVT) V.SR = d.TFORCE;
+            else if ((rc = dalloc(h, &V.SR, N))) return bail(rc);
         }
         if ((rc = dalloc(h, &V.ST, N)) || (rc = dalloc(h, &V.TM, N)) || (rc = dalloc(h, &V.psum, jm)) ||
             (rc = dalloc(h, &V.pabs, jm)) || (rc = dalloc(h, &V.AVG_BLK, nrows)))

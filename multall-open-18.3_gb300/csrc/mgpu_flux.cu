@@ -183,85 +183,172 @@ __device__ inline float tflux_energy_at(const Dev &d, float flowt, int i, int j,
     return (flowt * AVGHO + A2(d.WRABT, j, k) * AVGPB) * 0.25f;
 }
 
-__global__ void k_flux_mass_energy(Dev d) {
-    pdl_wait();
-    const int n = blockIdx.x * blockDim.x + threadIdx.x;
-    const int N = d.IM * d.JM * d.KM;
-    if (n >= N) return;
-    int i, j, k;
-    node_ijk(d, (size_t)n, i, j, k);
+// The periodic balance of the I = 1 / IM faces of one (J, K) off the blades
+// (5020-5045, 900): both edges' mass fluxes and energy fluxes are the mean of
+// the two.  One thread each, in CTAs of their own: in the node pass every warp
+// holds an edge, and all of its lanes would wait for the edges' loads.
+__device__ inline bool edge_jk(const Dev &d, int e, int &j, int &k) {
+    j = e % d.JM + 1;
+    k = e / d.JM + 1;
+    return j >= 2 && k <= d.KMM1 && A1(d.IND, j) != 1;
+}
+static inline unsigned edge_ctas(const Dev &d) { return grid_for((size_t)d.JM * d.KMM1, 256); }
+
+__device__ __noinline__ void edges_mass_energy(const Dev &d, int e) {
+    int j, k;
+    if (!edge_jk(d, e, j, k)) return;
     const VarSet &V = d.var[V_ROE];
-    // results are kept in registers and stored at the end, so that no store
-    // orders the loads of a later section behind it
-    const bool hx = i < d.IM && k < d.KM, ht = j >= 2 && k < d.KM, hr = i < d.IM && j >= 2;
-    const bool hs = hx && j >= 2;
-    float fx = 0.0f, ft = 0.0f, fr = 0.0f;
-    float xf = 0.0f, src = 0.0f, rf = 0.0f, tf = 0.0f;
-    // mass fluxes (5020-5045)
-    if (hx) {
-        float AVGRVX = A3(d.ROVX, i, j, k) + A3(d.ROVX, i, j, k + 1) + A3(d.ROVX, i + 1, j, k) + A3(d.ROVX, i + 1, j, k + 1);
-        float AVGRVR = A3(d.ROVR, i, j, k) + A3(d.ROVR, i, j, k + 1) + A3(d.ROVR, i + 1, j, k) + A3(d.ROVR, i + 1, j, k + 1);
-        fx = 0.25f * (AVGRVX * A3(d.AQX, i, j, k) + AVGRVR * A3(d.AQR, i, j, k));
+    const float f1 = flowt_raw(d, 1, j, k), fm = flowt_raw(d, d.IM, j, k);
+    const float ft = 0.5f * (f1 + fm);
+    const float t1 = tflux_energy_at(d, ft, 1, j, k), tm = tflux_energy_at(d, ft, d.IM, j, k);
+    const float tf = 0.5f * (t1 + tm);
+    A3(d.FLOWT, 1, j, k) = ft;
+    A3(d.FLOWT, d.IM, j, k) = ft;
+    A3(V.TF, 1, j, k) = tf;
+    A3(V.TF, d.IM, j, k) = tf;
+}
+
+// A thread of the flux passes marches S nodes up K at one (I, J), lanes on
+// successive I: what it loads at level K+1 -- its own column and the ones at
+// I+1, J-1 and both -- serves the faces of K and then of K+1, so a node costs
+// 18 loads of flow quantities instead of 33 (momenta: 20 instead of 40), and
+// the index arithmetic is one addition a node.  Columns outside the grid load
+// the thread's own, for faces that are not stored.
+struct March {
+    int i, j, k, ke, n, o1, oj;       // node (i, j, k), last K, offsets to I+1 and J-1
+    bool hi, hj, on;
+    __device__ March(const Dev &d, int b, int S) {
+        const int ncol = (d.IM * d.JM + 255) / 256;
+        const int t = (b % ncol) * 256 + (int)threadIdx.x;
+        k = (b / ncol) * S + 1;
+        ke = min(k + S - 1, d.KM);
+        on = t < d.IM * d.JM;
+        j = t / d.IM + 1;
+        i = t - (j - 1) * d.IM + 1;
+        n = t + d.IM * d.JM * (k - 1);
+        hi = i < d.IM;
+        hj = j >= 2;
+        o1 = hi ? 1 : 0;
+        oj = hj ? -d.IM : 0;
     }
-    const float ro = d.RO[n];
-    const float rowt = d.ROVT[n] - A2(d.UBLADE, j, k) * ro;
-    const float wt = rowt / ro;
-    bool tbal = false;          // periodic I = 1 / IM face: FLOWT there is the balanced value ft at both
-    if (ht) {
-        ft = flowt_raw(d, i, j, k);
-        if (i == 1 || i == d.IM) {
-            if (A1(d.IND, j) != 1) {
-                float f1 = (i == 1) ? ft : flowt_raw(d, 1, j, k);
-                float fm = (i == d.IM) ? ft : flowt_raw(d, d.IM, j, k);
-                ft = 0.5f * (f1 + fm);
-                tbal = true;
-            } else {
-                int nr = A1(d.NROW, j);
-                if (k >= A1(d.KS1, nr) && k <= A1(d.KS2, nr)) ft = 0.0f;
+};
+// nodes a thread marches: as many as leave 16 warps for every SM
+static int march_length(const Dev &d, int sm_count) {
+    const long long cols = (long long)(d.IM * d.JM + 255) / 256 * 8;
+    long long s = (long long)d.KM * cols / (16LL * sm_count);
+    return (int)(s < 1 ? 1 : s > 8 ? 8 : s);
+}
+static unsigned march_ctas(const Dev &d, int S) {
+    return (unsigned)((d.IM * d.JM + 255) / 256 * ((d.KM + S - 1) / S));
+}
+
+// One K level of a quantity: at (I, J), (I+1, J), (I, J-1), (I+1, J-1)
+struct Q4 {
+    float c, r, m, q;
+    __device__ void load(const float *__restrict__ p, int n, const March &w) {
+        c = p[n];
+        r = p[n + w.o1];
+        m = p[n + w.oj];
+        q = p[n + w.oj + w.o1];
+    }
+};
+
+// mass fluxes (5020-5045), ROWT, WT, and from them the energy fluxes
+// (5501-5503), whose source QSOURCE TSTEP reads in place
+__global__ void __launch_bounds__(256, 3) k_flux_mass_energy(const __grid_constant__ Dev d, int S, int edges) {
+    pdl_wait();
+    if ((int)blockIdx.x < edges) {
+        edges_mass_energy(d, (int)(blockIdx.x * 256 + threadIdx.x));
+        return;
+    }
+    March w(d, (int)blockIdx.x - edges, S);
+    if (!w.on) return;
+    const VarSet &V = d.var[V_ROE];
+    const int sK = d.IM * d.JM, KM = d.KM;
+    const bool edge = w.i == 1 || w.i == d.IM;
+    const bool own_t = w.hj && !(edge && A1(d.IND, w.j) != 1);     // the balanced faces are edges_mass_energy's
+    int ks1 = 1, ks2 = 0;                                           // K of a blade surface: no flow through it
+    if (edge && own_t) {
+        const int nr = A1(d.NROW, w.j);
+        ks1 = A1(d.KS1, nr);
+        ks2 = A1(d.KS2, nr);
+    }
+    struct Level {
+        Q4 vx, vr, ho;
+        float ro, rowt, rowtm, pe, pem;
+        __device__ void load(const Dev &d, const March &w, int n, int k) {
+            vx.load(d.ROVX, n, w);
+            vr.load(d.ROVR, n, w);
+            ho.load(d.HO, n, w);
+            ro = d.RO[n];
+            const float rovt = d.ROVT[n], rom = d.RO[n + w.oj], rovtm = d.ROVT[n + w.oj];
+            const int jk = w.j - 1 + d.JM * (k - 1);
+            const float ub = d.UBLADE[jk], ubm = d.UBLADE[w.hj ? jk - 1 : jk];
+            pe = d.PEFF[n];
+            pem = d.PEFF[n + w.oj];
+            rowt = rovt - ub * ro;
+            rowtm = rovtm - ubm * rom;
+        }
+    };
+    Level a, b;
+    int n = w.n;
+    a.load(d, w, n, w.k);
+#pragma unroll 2
+    for (int k = w.k; k <= w.ke; ++k, n += sK) {
+        const bool hk = k < KM, hx = w.hi && hk, ht = own_t && hk, hr = w.hi && w.hj;
+        const int jk = w.j - 1 + d.JM * (k - 1);
+        float aqx = 0.0f, aqr = 0.0f, abx = 0.0f, abr = 0.0f, abt = 0.0f, wrabt = 0.0f, asx = 0.0f, asr = 0.0f;
+        if (hk) b.load(d, w, n + sK, k + 1);
+        if (hx) {
+            aqx = d.AQX[n];
+            aqr = d.AQR[n];
+        }
+        if (ht) {
+            abx = d.ABX[n];
+            abr = d.ABR[n];
+            abt = d.ABT[jk];
+            wrabt = d.WRABT[jk];
+        }
+        if (hr) {
+            asx = d.ASX[n];
+            asr = d.ASR[n];
+        }
+        if (hx) {
+            const float AVGRVX = a.vx.c + b.vx.c + a.vx.r + b.vx.r, AVGRVR = a.vr.c + b.vr.c + a.vr.r + b.vr.r;
+            const float fx = 0.25f * (AVGRVX * aqx + AVGRVR * aqr);
+            const float AVGHO = a.ho.c + b.ho.c + a.ho.r + b.ho.r;
+            d.FLOWX[n] = fx;
+            V.XF[n] = fx * AVGHO * 0.25f;
+        }
+        d.ROWT[n] = a.rowt;
+        d.WT[n] = a.rowt / a.ro;
+        if (ht) {
+            const float AVGRVX = a.vx.c + a.vx.m + b.vx.m + b.vx.c, AVGRVR = a.vr.c + a.vr.m + b.vr.m + b.vr.c;
+            const float AVGRVT = a.rowt + a.rowtm + b.rowtm + b.rowt;
+            float ft = (AVGRVX * abx + AVGRVT * abt + AVGRVR * abr) * 0.25f;
+            if (k >= ks1 && k <= ks2) ft = 0.0f;
+            const float AVGHO = a.ho.c + a.ho.m + b.ho.m + b.ho.c, AVGPB = a.pe + a.pem + b.pem + b.pe;
+            d.FLOWT[n] = ft;
+            V.TF[n] = (ft * AVGHO + wrabt * AVGPB) * 0.25f;
+        }
+        if (hr) {
+            float fr = 0.0f;
+            if (k >= 2 && hk) {
+                const float AVGRVX = a.vx.c + a.vx.m + a.vx.q + a.vx.r, AVGRVR = a.vr.c + a.vr.m + a.vr.q + a.vr.r;
+                fr = 0.25f * (AVGRVX * asx + AVGRVR * asr);
             }
+            const float AVGHO = 0.25f * (a.ho.c + a.ho.m + a.ho.q + a.ho.r);
+            d.FLOWR[n] = fr;
+            V.RF[n] = fr * AVGHO;
         }
+        a = b;
     }
-    if (hr) {
-        if (k >= 2 && k <= d.KMM1) {
-            float AVGRVX = A3(d.ROVX, i, j, k) + A3(d.ROVX, i, j - 1, k) + A3(d.ROVX, i + 1, j - 1, k) + A3(d.ROVX, i + 1, j, k);
-            float AVGRVR = A3(d.ROVR, i, j, k) + A3(d.ROVR, i, j - 1, k) + A3(d.ROVR, i + 1, j - 1, k) + A3(d.ROVR, i + 1, j, k);
-            fr = 0.25f * (AVGRVX * A3(d.ASX, i, j, k) + AVGRVR * A3(d.ASR, i, j, k));
-        }
-    }
-    // energy fluxes (5501-5503) from this node's mass fluxes, and their
-    // periodic balance (900): with IND(J) != 1 the mass flux of both edge
-    // faces is the balanced ft, so the two edge energy fluxes are formed here
-    if (hx) {
-        float AVGHO = A3(d.HO, i, j, k) + A3(d.HO, i, j, k + 1) + A3(d.HO, i + 1, j, k) + A3(d.HO, i + 1, j, k + 1);
-        xf = fx * AVGHO * 0.25f;
-        if (hs) src = d.QSOURCE[n];
-    }
-    if (hr) {
-        float AVGHO = 0.25f * (A3(d.HO, i, j, k) + A3(d.HO, i, j - 1, k) + A3(d.HO, i + 1, j - 1, k) + A3(d.HO, i + 1, j, k));
-        rf = fr * AVGHO;
-    }
-    if (ht) {
-        tf = tflux_energy_at(d, ft, i, j, k);
-        if (tbal) {
-            float t1 = (i == 1) ? tf : tflux_energy_at(d, ft, 1, j, k);
-            float tm = (i == d.IM) ? tf : tflux_energy_at(d, ft, d.IM, j, k);
-            tf = 0.5f * (t1 + tm);
-        }
-    }
-    if (hx) d.FLOWX[n] = fx;
-    d.ROWT[n] = rowt;
-    d.WT[n] = wt;
-    if (ht) d.FLOWT[n] = ft;
-    if (hr) d.FLOWR[n] = fr;
-    if (hx) V.XF[n] = xf;
-    if (hs) V.SR[n] = src;
-    if (hr) V.RF[n] = rf;
-    if (ht) V.TF[n] = tf;
 }
 
 void launch_flux_mass_energy(const Dev &d, Launch L) {
-    size_t N = (size_t)d.IM * d.JM * d.KM;
-    launchk(L, k_flux_mass_energy, dim3(grid_for(N, 256)), dim3(256), 0, d);
+    const int S = march_length(d, L.sm_count);
+    const unsigned e = edge_ctas(d);
+    launchk(L, k_flux_mass_energy, dim3(e + march_ctas(d, S)), dim3(256), 0, d, S, (int)e);
     mark(L, "k_flux_mass_energy");
 }
 
@@ -632,161 +719,149 @@ __device__ inline float tflux_rvt_raw(const Dev &d, int i, int j, int k, float A
     return (A3(d.FLOWT, i, j, k) * AVGVT + A2(d.ABT, j, k) * AVGP) * AVGR;
 }
 
-__device__ inline float tflux_rmom_raw(const Dev &d, int i, int j, int k, float *avgp4) {
+__device__ inline float tflux_rmom_raw(const Dev &d, int i, int j, int k) {
     const float *VR = d.VR;
     float AVGVR = A3(VR, i, j, k) + A3(VR, i, j - 1, k) + A3(VR, i, j - 1, k + 1) + A3(VR, i, j, k + 1);
     float AVGP = peff_at(d, i, j, k) + peff_at(d, i, j - 1, k) + peff_at(d, i, j - 1, k + 1) + peff_at(d, i, j, k + 1);
-    *avgp4 = AVGP;
     return 0.25f * (A3(d.FLOWT, i, j, k) * AVGVR + AVGP * A3(d.ABR, i, j, k));
 }
 
-// The three momentum equations' fluxes in one pass over the nodes
-// (6100-6120, 6200-6230, 6300-6330 with the cusp and periodic balances).
-// Each thread loads its node's neighbour cube of PEFF, VX, VT, VR and ROVT
-// once -- the values at (i+di, j+dj, k+dk), di, dk in {0,1}, dj in {-1,0} --
-// and forms every average from registers, each sum in the order of the
-// reference's expression.  The balances at I=1 and I=IM, which also need the
-// other end's column, keep the direct loads of the helpers above.
+// the momenta's balances at I = 1 and IM of one (J, K) off the blades (cusp:
+// 6100-6120; periodic: 6200-6230, 6300-6330)
+__device__ __noinline__ void edges_mom(const Dev &d, int e) {
+    int j, k;
+    if (!edge_jk(d, e, j, k)) return;
+    const int IM = d.IM;
+    const float *VX = d.VX;
+    const float AVGPCUSP = peff_at(d, 1, j, k) + peff_at(d, 1, j - 1, k) + peff_at(d, 1, j, k + 1) +
+                           peff_at(d, 1, j - 1, k + 1) + peff_at(d, IM, j, k) + peff_at(d, IM, j - 1, k) +
+                           peff_at(d, IM, j, k + 1) + peff_at(d, IM, j - 1, k + 1);
+    const float AVGVXCUSP = A3(VX, 1, j, k) + A3(VX, 1, j - 1, k) + A3(VX, 1, j, k + 1) + A3(VX, 1, j - 1, k + 1) +
+                            A3(VX, IM, j, k) + A3(VX, IM, j - 1, k) + A3(VX, IM, j, k + 1) + A3(VX, IM, j - 1, k + 1);
+    const float AVGR = 0.25f * A2(d.RAVG_CELL, j, k);
+    const float rvt = 0.5f * (tflux_rvt_raw(d, 1, j, k, AVGR) + tflux_rvt_raw(d, IM, j, k, AVGR));
+    const float AVGP1 = 0.25f * (peff_at(d, 1, j, k) + peff_at(d, 1, j - 1, k) + peff_at(d, 1, j, k + 1) +
+                                 peff_at(d, 1, j - 1, k + 1));
+    const float AVGPM = 0.25f * (peff_at(d, IM, j, k) + peff_at(d, IM, j - 1, k) + peff_at(d, IM, j, k + 1) +
+                                 peff_at(d, IM, j - 1, k + 1));
+    const float abr1 = A3(d.ABR, 1, j, k), abrm = A3(d.ABR, IM, j, k);
+    const float T1 = tflux_rmom_raw(d, 1, j, k) - AVGP1 * abr1;
+    const float T2 = tflux_rmom_raw(d, IM, j, k) - AVGPM * abrm;
+    const float x1 = 0.125f * (A3(d.FLOWT, 1, j, k) * AVGVXCUSP + AVGPCUSP * A3(d.ABX, 1, j, k));
+    const float xm = 0.125f * (A3(d.FLOWT, IM, j, k) * AVGVXCUSP + AVGPCUSP * A3(d.ABX, IM, j, k));
+    A3(d.var[V_ROVX].TF, 1, j, k) = x1;
+    A3(d.var[V_ROVX].TF, IM, j, k) = xm;
+    A3(d.var[V_RORVT].TF, 1, j, k) = rvt;
+    A3(d.var[V_RORVT].TF, IM, j, k) = rvt;
+    A3(d.var[V_ROVR].TF, 1, j, k) = 0.5f * ((T1 + T2) + (AVGP1 + AVGPM) * abr1);
+    A3(d.var[V_ROVR].TF, IM, j, k) = 0.5f * ((T1 + T2) + (AVGP1 + AVGPM) * abrm);
+}
 
-__global__ void __launch_bounds__(256, 3) k_flux_mom(Dev d) {
+// The three momentum equations' fluxes (6100-6120, 6200-6230, 6300-6330 with
+// the cusp and periodic balances) marching up K as k_flux_mass_energy does,
+// each sum in the order of the reference's expression; also PEFF of this step,
+// which the next step's energy fluxes read.  The axial and tangential sources
+// XFORCE and TFORCE are read in place by TSTEP.
+__global__ void __launch_bounds__(256, 2) k_flux_mom(const __grid_constant__ Dev d, int S, int edges) {
     pdl_wait();
-    const int n = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-    const int N = d.IM * d.JM * d.KM;
-    if (n >= N) return;
-    int i, j, k;
-    node_ijk(d, (size_t)n, i, j, k);
-    const int IM = d.IM, sJ = d.IM, sK = d.IM * d.JM;
-    const bool hi = i < IM, hj = j >= 2, hk = k < d.KM;
-    const float *__restrict__ PP = d.P;
-    const float *__restrict__ VX = d.VX;
-    const float *__restrict__ VT = d.VT;
-    const float *__restrict__ VR = d.VR;
-    const float *__restrict__ RV = d.ROVT;
-    // c[di][dj + 1][dk]; positions outside the grid are never used
-    float pe[2][2][2] = {}, vx[2][2][2] = {}, vt[2][2][2] = {}, vr[2][2][2] = {}, rv[2][2][2] = {};
-#pragma unroll
-    for (int di = 0; di < 2; ++di)
-#pragma unroll
-        for (int dj = -1; dj <= 0; ++dj)
-#pragma unroll
-            for (int dk = 0; dk < 2; ++dk) {
-                if ((di && !hi) || (dj && !hj) || (dk && !hk)) continue;
-                const int o = n + di + dj * sJ + dk * sK;
-                pe[di][dj + 1][dk] = peff_of(d, PP, o, j + dj);
-                vt[di][dj + 1][dk] = VT[o];
-                if (!(di && dj && dk)) {
-                    vx[di][dj + 1][dk] = VX[o];
-                    vr[di][dj + 1][dk] = VR[o];
-                }
-                if (hi && hj && hk) rv[di][dj + 1][dk] = RV[o];
-            }
-#define C(a, di, dj, dk) a[di][(dj) + 1][dk]
-    // every per-node operand is loaded before the first store, so that the
-    // loads are in flight together (the stores below may not be reordered
-    // ahead of loads through other Dev pointers)
-    const bool fK = hi && hk, fJ = hi && hj, fI = hj && hk, fS = fJ && hk;
-    const float xforce = fK ? d.XFORCE[n] : 0.0f, tforce = fK ? d.TFORCE[n] : 0.0f;
-    const float aqx = fK ? d.AQX[n] : 0.0f, aqr = fK ? d.AQR[n] : 0.0f, flowx = fK ? d.FLOWX[n] : 0.0f;
-    const float rjk = A2(d.R, j, k);
-    const float rk1 = fK ? A2(d.R, j, k + 1) : 0.0f, rj1 = fJ ? A2(d.R, j - 1, k) : 0.0f;
-    const float asx = fJ ? d.ASX[n] : 0.0f, asr = fJ ? d.ASR[n] : 0.0f, flowr = fJ ? d.FLOWR[n] : 0.0f;
-    const float rforce = fS ? d.RFORCE[n] : 0.0f, volor = fS ? d.VOLOR[n] : 0.0f;
-    const float FT = fI ? d.FLOWT[n] : 0.0f, abx = fI ? d.ABX[n] : 0.0f, abr = fI ? d.ABR[n] : 0.0f;
-    const float abt = fI ? A2(d.ABT, j, k) : 0.0f, ravg = fI ? A2(d.RAVG_CELL, j, k) : 0.0f;
-    const bool edge = (i == 1 || i == IM) && A1(d.IND, j) != 1;
-    const float *RO = d.RO;
-    const bool dens = j >= 3 && j <= d.JM - 3;
-    const float ro0 = RO[n];
-    const float rom2 = dens ? RO[n - 2 * sJ] : 0.0f, rom1 = dens ? RO[n - sJ] : 0.0f;
-    const float rop1 = dens ? RO[n + sJ] : 0.0f, rop2 = dens ? RO[n + 2 * sJ] : 0.0f;
-    d.PEFF[n] = C(pe, 0, 0, 0);    // PEFF of this step, read by the next step's energy fluxes
-    const VarSet &VXm = d.var[V_ROVX], &VTm = d.var[V_RORVT], &VRm = d.var[V_ROVR];
-    // faces K = const (XFLUX) and the axial / tangential sources
-    if (fK) {
-        VXm.SR[n] = xforce;
-        float AVGP = C(pe, 0, 0, 0) + C(pe, 0, 0, 1) + C(pe, 1, 0, 1) + C(pe, 1, 0, 0);
-        float AVGVX = C(vx, 0, 0, 0) + C(vx, 0, 0, 1) + C(vx, 1, 0, 1) + C(vx, 1, 0, 0);
-        VXm.XF[n] = 0.25f * (AVGP * aqx + flowx * AVGVX);
-        float AVGR = 0.125f * (rjk + rk1);
-        float AVGVT = C(vt, 0, 0, 0) + C(vt, 0, 0, 1) + C(vt, 1, 0, 0) + C(vt, 1, 0, 1);
-        VTm.SR[n] = tforce;
-        VTm.XF[n] = flowx * AVGR * AVGVT;
-        float AVGVR = C(vr, 0, 0, 0) + C(vr, 0, 0, 1) + C(vr, 1, 0, 0) + C(vr, 1, 0, 1);
-        VRm.XF[n] = 0.25f * (flowx * AVGVR + aqr * AVGP);
+    if ((int)blockIdx.x < edges) {
+        edges_mom(d, (int)(blockIdx.x * 256 + threadIdx.x));
+        return;
     }
-    // faces J = const (RFLUX) and the radial source
-    if (fJ) {
-        float AVGP = C(pe, 0, 0, 0) + C(pe, 0, -1, 0) + C(pe, 1, -1, 0) + C(pe, 1, 0, 0);
-        float AVGVX = C(vx, 0, 0, 0) + C(vx, 0, -1, 0) + C(vx, 1, -1, 0) + C(vx, 1, 0, 0);
-        VXm.RF[n] = 0.25f * (AVGP * asx + flowr * AVGVX);
-        float AVGR = (rjk + rj1) * 0.125f;
-        float AVGVT = C(vt, 0, 0, 0) + C(vt, 0, -1, 0) + C(vt, 1, -1, 0) + C(vt, 1, 0, 0);
-        VTm.RF[n] = flowr * AVGVT * AVGR;
-        float AVGVR = C(vr, 0, 0, 0) + C(vr, 0, -1, 0) + C(vr, 1, -1, 0) + C(vr, 1, 0, 0);
-        VRm.RF[n] = 0.25f * (flowr * AVGVR + asr * AVGP);
-        if (hk) {
-            float AVGRVT = C(rv, 0, 0, 0) + C(rv, 0, 0, 1) + C(rv, 0, -1, 0) + C(rv, 0, -1, 1) + C(rv, 1, 0, 0) +
-                           C(rv, 1, 0, 1) + C(rv, 1, -1, 0) + C(rv, 1, -1, 1);
-            float AVGVT8 = 0.125f * (C(vt, 0, 0, 0) + C(vt, 0, -1, 0) + C(vt, 0, -1, 1) + C(vt, 0, 0, 1) + C(vt, 1, 0, 0) +
-                                     C(vt, 1, -1, 0) + C(vt, 1, -1, 1) + C(vt, 1, 0, 1));
-            float AVGP8 = C(pe, 0, 0, 0) + C(pe, 0, -1, 0) + C(pe, 0, -1, 1) + C(pe, 0, 0, 1) + C(pe, 1, 0, 0) +
-                          C(pe, 1, -1, 0) + C(pe, 1, -1, 1) + C(pe, 1, 0, 1);
+    March w(d, (int)blockIdx.x - edges, S);
+    if (!w.on) return;
+    const VarSet &VXm = d.var[V_ROVX], &VTm = d.var[V_RORVT], &VRm = d.var[V_ROVR];
+    const int sK = d.IM * d.JM, KM = d.KM;
+    const bool own_t = w.hj && !((w.i == 1 || w.i == d.IM) && A1(d.IND, w.j) != 1);   // the others: edges_mom
+    struct Level {
+        Q4 pe, vx, vt, vr, rv;
+        float r;
+        __device__ void load(const Dev &d, const March &w, int n, int k) {
+            pe.c = peff_of(d, d.P, n, w.j);
+            pe.r = peff_of(d, d.P, n + w.o1, w.j);
+            pe.m = peff_of(d, d.P, n + w.oj, w.hj ? w.j - 1 : w.j);
+            pe.q = peff_of(d, d.P, n + w.oj + w.o1, w.hj ? w.j - 1 : w.j);
+            vx.load(d.VX, n, w);
+            vt.load(d.VT, n, w);
+            vr.load(d.VR, n, w);
+            rv.load(d.ROVT, n, w);
+            r = d.R[w.j - 1 + d.JM * (k - 1)];
+        }
+    };
+    Level a, b;
+    int n = w.n;
+    a.load(d, w, n, w.k);
+#pragma unroll 2
+    for (int k = w.k; k <= w.ke; ++k, n += sK) {
+        const bool hk = k < KM, fK = w.hi && hk, fJ = w.hi && w.hj, fI = own_t && hk, fS = fJ && hk;
+        const int jk = w.j - 1 + d.JM * (k - 1);
+        float aqx = 0.0f, aqr = 0.0f, flowx = 0.0f, asx = 0.0f, asr = 0.0f, flowr = 0.0f, rj1 = 0.0f;
+        float rforce = 0.0f, volor = 0.0f, FT = 0.0f, abx = 0.0f, abr = 0.0f, abt = 0.0f, ravg = 0.0f;
+        if (hk) b.load(d, w, n + sK, k + 1);
+        if (fK) {
+            aqx = d.AQX[n];
+            aqr = d.AQR[n];
+            flowx = d.FLOWX[n];
+        }
+        if (fJ) {
+            asx = d.ASX[n];
+            asr = d.ASR[n];
+            flowr = d.FLOWR[n];
+            rj1 = d.R[jk - 1];
+        }
+        if (fS) {
+            rforce = d.RFORCE[n];
+            volor = d.VOLOR[n];
+        }
+        if (fI) {
+            FT = d.FLOWT[n];
+            abx = d.ABX[n];
+            abr = d.ABR[n];
+            abt = d.ABT[jk];
+            ravg = d.RAVG_CELL[jk];
+        }
+        d.PEFF[n] = a.pe.c;
+        // faces K = const (XFLUX)
+        if (fK) {
+            const float AVGP = a.pe.c + b.pe.c + b.pe.r + a.pe.r, AVGVX = a.vx.c + b.vx.c + b.vx.r + a.vx.r;
+            VXm.XF[n] = 0.25f * (AVGP * aqx + flowx * AVGVX);
+            const float AVGR = 0.125f * (a.r + b.r), AVGVT = a.vt.c + b.vt.c + a.vt.r + b.vt.r;
+            VTm.XF[n] = flowx * AVGR * AVGVT;
+            const float AVGVR = a.vr.c + b.vr.c + a.vr.r + b.vr.r;
+            VRm.XF[n] = 0.25f * (flowx * AVGVR + aqr * AVGP);
+        }
+        // faces J = const (RFLUX) and the radial source
+        if (fJ) {
+            const float AVGP = a.pe.c + a.pe.m + a.pe.q + a.pe.r, AVGVX = a.vx.c + a.vx.m + a.vx.q + a.vx.r;
+            VXm.RF[n] = 0.25f * (AVGP * asx + flowr * AVGVX);
+            const float AVGR = (a.r + rj1) * 0.125f, AVGVT = a.vt.c + a.vt.m + a.vt.q + a.vt.r;
+            VTm.RF[n] = flowr * AVGVT * AVGR;
+            const float AVGVR = a.vr.c + a.vr.m + a.vr.q + a.vr.r;
+            VRm.RF[n] = 0.25f * (flowr * AVGVR + asr * AVGP);
+        }
+        if (fS) {
+            const float AVGRVT = a.rv.c + b.rv.c + a.rv.m + b.rv.m + a.rv.r + b.rv.r + a.rv.q + b.rv.q;
+            const float AVGVT8 = 0.125f * (a.vt.c + a.vt.m + b.vt.m + b.vt.c + a.vt.r + a.vt.q + b.vt.q + b.vt.r);
+            const float AVGP8 = a.pe.c + a.pe.m + b.pe.m + b.pe.c + a.pe.r + a.pe.q + b.pe.q + b.pe.r;
             VRm.SR[n] = rforce - (AVGRVT * AVGVT8 + AVGP8) * volor;
         }
-    }
-    // faces I = const (TFLUX)
-    if (fI) {
-        float AVGP = C(pe, 0, 0, 0) + C(pe, 0, -1, 0) + C(pe, 0, -1, 1) + C(pe, 0, 0, 1);
-        if (edge) {
-            float AVGPCUSP = peff_at(d, 1, j, k) + peff_at(d, 1, j - 1, k) + peff_at(d, 1, j, k + 1) +
-                             peff_at(d, 1, j - 1, k + 1) + peff_at(d, IM, j, k) + peff_at(d, IM, j - 1, k) +
-                             peff_at(d, IM, j, k + 1) + peff_at(d, IM, j - 1, k + 1);
-            float AVGVXCUSP = A3(VX, 1, j, k) + A3(VX, 1, j - 1, k) + A3(VX, 1, j, k + 1) + A3(VX, 1, j - 1, k + 1) +
-                              A3(VX, IM, j, k) + A3(VX, IM, j - 1, k) + A3(VX, IM, j, k + 1) + A3(VX, IM, j - 1, k + 1);
-            VXm.TF[n] = 0.125f * (FT * AVGVXCUSP + AVGPCUSP * abx);
-        } else {
-            float AVGVX = C(vx, 0, 0, 0) + C(vx, 0, -1, 0) + C(vx, 0, -1, 1) + C(vx, 0, 0, 1);
+        // faces I = const (TFLUX)
+        if (fI) {
+            const float AVGP = a.pe.c + a.pe.m + b.pe.m + b.pe.c, AVGVX = a.vx.c + a.vx.m + b.vx.m + b.vx.c;
             VXm.TF[n] = 0.25f * (FT * AVGVX + abx * AVGP);
+            const float AVGVT = a.vt.c + a.vt.m + b.vt.m + b.vt.c;
+            VTm.TF[n] = (FT * AVGVT + abt * AVGP) * (0.25f * ravg);
+            const float AVGVR = a.vr.c + a.vr.m + b.vr.m + b.vr.c;
+            VRm.TF[n] = 0.25f * (FT * AVGVR + AVGP * abr);
         }
-        const float AVGR = 0.25f * ravg;
-        float AVGVT = C(vt, 0, 0, 0) + C(vt, 0, -1, 0) + C(vt, 0, -1, 1) + C(vt, 0, 0, 1);
-        float tf = (FT * AVGVT + abt * AVGP) * AVGR;
-        if (edge) {
-            float t1 = (i == 1) ? tf : tflux_rvt_raw(d, 1, j, k, AVGR);
-            float tm = (i == IM) ? tf : tflux_rvt_raw(d, IM, j, k, AVGR);
-            tf = 0.5f * (t1 + tm);
-        }
-        VTm.TF[n] = tf;
-        float AVGVR = C(vr, 0, 0, 0) + C(vr, 0, -1, 0) + C(vr, 0, -1, 1) + C(vr, 0, 0, 1);
-        float tr = 0.25f * (FT * AVGVR + AVGP * abr);
-        if (edge) {
-            float ap1, apm;
-            float t1raw = tflux_rmom_raw(d, 1, j, k, &ap1);
-            float tmraw = tflux_rmom_raw(d, IM, j, k, &apm);
-            float AVGP1 = 0.25f * (peff_at(d, 1, j, k) + peff_at(d, 1, j - 1, k) + peff_at(d, 1, j, k + 1) +
-                                   peff_at(d, 1, j - 1, k + 1));
-            float AVGPM = 0.25f * (peff_at(d, IM, j, k) + peff_at(d, IM, j - 1, k) + peff_at(d, IM, j, k + 1) +
-                                   peff_at(d, IM, j - 1, k + 1));
-            float T1 = t1raw - AVGP1 * A3(d.ABR, 1, j, k);
-            float T2 = tmraw - AVGPM * A3(d.ABR, IM, j, k);
-            tr = 0.5f * ((T1 + T2) + (AVGP1 + AVGPM) * abr);
-        }
-        VRm.TF[n] = tr;
-    }
-#undef C
-    // the density limiter's column flags (7200): RO is final here (after
-    // TSTEP(RO) and the inlet/exit conditions) and TSTEP of the momenta
-    // does not change it
-    if (d.ADJ_RO_LIM) d.ADJ_RO_LIM[n] = ro0;
-    if (dens) {
-        const float ROAVG = 0.25f * (rom2 + rom1 + rop1 + rop2);
-        if (density_triggers(ro0, ROAVG, d.ROLIM)) d.DFLAG[(size_t)(k - 1) * d.IM + (i - 1)] = 1;
+        a = b;
     }
 }
 
 void launch_flux_mom(const Dev &d, Launch L) {
-    size_t N = (size_t)d.IM * d.JM * d.KM;
-    launchk(L, k_flux_mom, dim3(grid_for(N, 256)), dim3(256), 0, d);
+    const int S = march_length(d, L.sm_count);
+    const unsigned e = edge_ctas(d);
+    launchk(L, k_flux_mom, dim3(e + march_ctas(d, S)), dim3(256), 0, d, S, (int)e);
     mark(L, "k_flux_mom");
 }
 
@@ -794,11 +869,27 @@ void launch_flux_mom(const Dev &d, Launch L) {
 // density limiter (7200).  The reference walks J in place, so RO(J-1) and
 // RO(J-2) are already limited when RO(J) is tested.  A column's result
 // differs from its input only if some J triggers a limit on the unmodified
-// values (the first trigger is the same in both), so k_flux_mom flags those
-// columns in parallel and k_density_fix replays the sequential walk on
-// flagged columns only.  The thread owning (IMID,KMID) then sets the
+// values (the first trigger is the same in both), so k_density_scan flags
+// those columns in parallel and k_density_fix replays the sequential walk on
+// flagged columns only.  RO is final after TSTEP(RO) and the inlet/exit
+// conditions, so both run beside TSTEP of the momenta.  The thread owning (IMID,KMID) then sets the
 // per-row Mach limits VLIMIT/ROLIMIT (7250) from its final densities.
 // ---------------------------------------------------------------------
+__global__ void k_density_scan(const __grid_constant__ Dev d) {
+    pdl_wait();
+    const int n = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+    if (n >= d.IM * d.JM * d.KM) return;
+    int i, j, k;
+    node_ijk(d, (size_t)n, i, j, k);
+    const float *RO = d.RO;
+    const float ro0 = RO[n];
+    if (d.ADJ_RO_LIM) d.ADJ_RO_LIM[n] = ro0;
+    if (j < 3 || j > d.JM - 3) return;
+    const int sJ = d.IM;
+    const float ROAVG = 0.25f * (RO[n - 2 * sJ] + RO[n - sJ] + RO[n + sJ] + RO[n + 2 * sJ]);
+    if (density_triggers(ro0, ROAVG, d.ROLIM)) d.DFLAG[ixik(d, i, k)] = 1;
+}
+
 constexpr int DF_AHEAD = 64;     // J values a flagged column loads together in k_density_fix
 
 __global__ void k_density_fix(Dev d) {
@@ -899,6 +990,8 @@ __global__ void k_mach_limiter(Dev d) {
 }
 
 void launch_density_fix(const Dev &d, Launch L) {
+    launchk(L, k_density_scan, dim3(grid_for((size_t)d.IM * d.JM * d.KM, 256)), dim3(256), 0, d);
+    mark(L, "k_density_scan");
     int lines = d.IM * d.KM;
     launchk(L, k_density_fix, dim3((lines + 127) / 128), dim3(128), 0, d);
     mark(L, "k_density_fix");

@@ -368,8 +368,7 @@ void launch_bc_sums(const Dev &d, Launch L);
 void launch_bc_apply(const Dev &d, Launch L);
 void launch_setflo(const Dev &d, Launch L);       // IN_FLOW != 0
 void launch_cusp(const Dev &d, Launch L);         // IF_CUSP = 2 rows
-// XMOM, RVT and RMOM fluxes; also PEFF (4321) and the density limiter's
-// column flags
+// XMOM, RVT and RMOM fluxes; also PEFF (4321)
 void launch_flux_mom(const Dev &d, Launch L);
 // TSTEP for the nv variables v0 .. v0+nv-1 of d.var
 void launch_tstep(const Dev &d, Launch L, int v0, int nv);
