@@ -1090,6 +1090,23 @@ int32_t mgpu_commit(mgpu_handle *h) {
             return true;
         };
         d.mg_nested = nested(IB1, IB2, d.IMM1) && nested(KB1, KB2, d.KMM1) ? 1 : 0;
+        // the blocks of a plane's cells, as the prolongation reads them
+        std::vector<unsigned short> cb1((size_t)d.IMM1 * d.KMM1), cb2(cb1.size());
+        std::vector<int> mg12((size_t)d.NIB1 * d.NKB1, 0);
+        for (int k = 0; k < d.KMM1; ++k)
+            for (int i = 0; i < d.IMM1; ++i) {
+                if (IB1[i] < 1 || IB1[i] > d.NIB1 || KB1[k] < 1 || KB1[k] > d.NKB1 || IB2[i] < 1 || IB2[i] > d.NIB2 ||
+                    KB2[k] < 1 || KB2[k] > d.NKB2)
+                    return fail(MGPU_E_ARG, "multigrid I or K map out of range");
+                const int u1 = (KB1[k] - 1) * d.NIB1 + IB1[i] - 1, u2 = (KB2[k] - 1) * d.NIB2 + IB2[i] - 1;
+                cb1[(size_t)k * d.IMM1 + i] = (unsigned short)u1;
+                cb2[(size_t)k * d.IMM1 + i] = (unsigned short)u2;
+                mg12[u1] = u2;
+            }
+        if ((rc = dalloc(h, &d.CB1, cb1.size())) || (rc = dalloc(h, &d.CB2, cb2.size())) ||
+            (rc = dalloc(h, &d.MG12, mg12.size())) || (rc = upload(h, d.CB1, cb1)) || (rc = upload(h, d.CB2, cb2)) ||
+            (rc = upload(h, d.MG12, mg12)))
+            return rc;
     }
     for (int j = 2; j <= d.JM; ++j) {
         if (JB1[j - 1] < 1 || JB1[j - 1] > d.NJB1 + 1 || JB2[j - 1] < 1 || JB2[j - 1] > d.NJB2 + 1 ||

@@ -129,6 +129,8 @@ struct Dev {
     int *IB1_S, *IB1_E, *IB2_S, *IB2_E;                 // (NIBn) I extent of each block
     int *KB1_S, *KB1_E, *KB2_S, *KB2_E;                 // (NKBn) K extent of each block
     int *SB_START, *SB_END;                             // (NSBLK)
+    unsigned short *CB1, *CB2;         // (IMM1*KMM1) level-1 and level-2 block of each cell of a plane
+    int *MG12;                         // (NIB1*NKB1) level-2 block of each level-1 block, where nested
     int mg_nested;                     // every level-2 block is a union of level-1 blocks (in I and in K)
     DevCtl *ctl;
     // graph conditionals selecting the LOSS and 5-step tail bodies (set by

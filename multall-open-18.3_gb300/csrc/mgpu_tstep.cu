@@ -23,6 +23,8 @@
 // single threads in the reference's sequential REAL*4 order (parity checks);
 // with REDUCE_ORDER=2 (the plain FP32 path) they are the default path's
 // trees with FP32 adds.
+#include <type_traits>
+
 #include "mgpu_internal.cuh"
 
 namespace mgpu {
@@ -105,6 +107,28 @@ struct Walk2 {
         if (i > ni) {
             i -= ni;
             ++k;
+        }
+    }
+};
+
+// The same walk of a plane's points by their offset n in a node array, with
+// K stride ks and the plane's first point at n0
+struct WalkN {
+    int i, n, di, dn, dw, ni;
+    __device__ WalkN(int ni_, int ks, int n0, int start, int stride) : ni(ni_) {
+        const int k = start / ni_, dk = stride / ni_;
+        i = start - k * ni_;
+        n = n0 + i + ks * k;
+        di = stride - dk * ni_;
+        dn = di + ks * dk;
+        dw = ks - ni_;
+    }
+    __device__ void next() {
+        i += di;
+        n += dn;
+        if (i >= ni) {
+            i -= ni;
+            n += dw;
         }
     }
 };
@@ -344,7 +368,14 @@ __device__ __forceinline__ float plane_partials_sum(const float *__restrict__ P,
 }
 
 // ---------------------------------------------------------------------
-// prolong: 1500, with the block sums assembled from the plane partials
+// prolong: 1500, with the block sums assembled from the plane partials.
+// A block's correction, sum x block step, is one value for all of its cells,
+// so it is formed once per block, and where every level-2 block is a union of
+// level-1 blocks the three levels are added up once per level-1 block too; a
+// cell takes its block's number from a table (CB1, CB2) and one value from
+// shared memory.  Each value is the same product and sum as cell by cell,
+// where gathering four block indices and two block steps for each cell made
+// 120 instructions and six dependent loads of it.
 // ---------------------------------------------------------------------
 template <int BS>
 __global__ void __launch_bounds__(BS, 1024 / BS) k_ts_prolong(const __grid_constant__ Dev d, int v0, int want_abs) {
@@ -359,37 +390,40 @@ __global__ void __launch_bounds__(BS, 1024 / BS) k_ts_prolong(const __grid_const
     float *b1 = sm, *b2 = sm + n1;
     const int j1 = A1(d.JB1, j), j2 = A1(d.JB2, j), jsb = A1(d.JSBLK, j);
     const int nc = IMM1 * KMM1;
-    const int ks = d.IM * d.JM, pj = d.IM * (j - 1);
     const int m1 = d.NIB1 * (d.NJB1 + 1), m2 = d.NIB2 * (d.NJB2 + 1);
+    const bool nested = d.mg_nested != 0;
+    float *__restrict__ ST = V.ST;
+    const float *__restrict__ STEP = d.STEP;
+    const float *__restrict__ RSTEP = d.RSTEP;
     // operands of this thread's first TS_U cells, loaded before the block
     // sums so their latency overlaps the assembly below
-    float pst[TS_U], pstp[TS_U], prs[TS_U], ps1[TS_U], ps2[TS_U];
-    int pb1[TS_U], pb2[TS_U];
-    Walk2 w(IMM1, threadIdx.x, BS);
+    float pst[TS_U], pstp[TS_U], prs[TS_U];
+    int pb1[TS_U], pb2[TS_U], pn[TS_U];
+    WalkN w(IMM1, d.IM * d.JM, d.IM * (j - 1), threadIdx.x, BS);
+    auto load = [&](int c0) {
 #pragma unroll
-    for (int u = 0; u < TS_U; ++u) {
-        const int i = w.i, k = w.k;
-        w.next();
-        if (threadIdx.x + u * BS < nc) {
-            const int n = pj + (i - 1) + ks * (k - 1);
-            const int i1 = A1(d.IB1, i), i2 = A1(d.IB2, i), k1 = A1(d.KB1, k), k2 = A1(d.KB2, k);
-            pst[u] = V.ST[n];
-            pstp[u] = d.STEP[n];
-            prs[u] = d.RSTEP[n];
-            ps1[u] = d.STEP1[(i1 - 1) + d.NIB1 * (j1 - 1) + m1 * (k1 - 1)];
-            ps2[u] = d.STEP2[(i2 - 1) + d.NIB2 * (j2 - 1) + m2 * (k2 - 1)];
-            pb1[u] = (k1 - 1) * d.NIB1 + (i1 - 1);
-            pb2[u] = (k2 - 1) * d.NIB2 + (i2 - 1);
+        for (int u = 0; u < TS_U; ++u) {
+            const int c = c0 + u * BS;
+            pn[u] = w.n;
+            if (c < nc) {
+                pst[u] = ST[w.n];
+                pstp[u] = STEP[w.n];
+                prs[u] = RSTEP[w.n];
+                pb1[u] = d.CB1[c];
+                pb2[u] = nested ? 0 : d.CB2[c];
+            }
+            w.next();
         }
-    }
+    };
+    load(threadIdx.x);
     if (d.REDUCE_ORDER == 1) {
         for (int t = threadIdx.x; t < n1; t += BS) {
-            int ib = t % d.NIB1 + 1, kb = t / d.NIB1 + 1;
-            b1[t] = V.B1CHG[(ib - 1) + d.NIB1 * (j1 - 1) + m1 * (kb - 1)];
+            const int o = t % d.NIB1 + d.NIB1 * (j1 - 1) + m1 * (t / d.NIB1);
+            b1[t] = V.B1CHG[o] * d.STEP1[o];
         }
         for (int t = threadIdx.x; t < n2; t += BS) {
-            int ib = t % d.NIB2 + 1, kb = t / d.NIB2 + 1;
-            b2[t] = V.B2CHG[(ib - 1) + d.NIB2 * (j2 - 1) + m2 * (kb - 1)];
+            const int o = t % d.NIB2 + d.NIB2 * (j2 - 1) + m2 * (t / d.NIB2);
+            b2[t] = V.B2CHG[o] * d.STEP2[o];
         }
         if (threadIdx.x == 0) s_sb = A1(V.SBSUM, jsb);
     } else {
@@ -397,8 +431,14 @@ __global__ void __launch_bounds__(BS, 1024 / BS) k_ts_prolong(const __grid_const
         // the last block); each sum adds the planes' partials in J order
         const int a1 = j1 <= d.NJB1 ? A1(d.JB1_START, j1) : 1, e1 = j1 <= d.NJB1 ? A1(d.JB1_END, j1) : 0;
         const int a2 = j2 <= d.NJB2 ? A1(d.JB2_START, j2) : 1, e2 = j2 <= d.NJB2 ? A1(d.JB2_END, j2) : 0;
-        for (int t = threadIdx.x; t < n1; t += BS) b1[t] = plane_partials_sum(V.P1, n1, t, a1, e1);
-        for (int t = threadIdx.x; t < n2; t += BS) b2[t] = plane_partials_sum(V.P2, n2, t, a2, e2);
+        for (int t = threadIdx.x; t < n1; t += BS) {
+            const float st1 = d.STEP1[t % d.NIB1 + d.NIB1 * (j1 - 1) + m1 * (t / d.NIB1)];
+            b1[t] = plane_partials_sum(V.P1, n1, t, a1, e1) * st1;
+        }
+        for (int t = threadIdx.x; t < n2; t += BS) {
+            const float st2 = d.STEP2[t % d.NIB2 + d.NIB2 * (j2 - 1) + m2 * (t / d.NIB2)];
+            b2[t] = plane_partials_sum(V.P2, n2, t, a2, e2) * st2;
+        }
         if (threadIdx.x < 32) {
             int a = A1(d.SB_START, jsb), b = A1(d.SB_END, jsb);
             const int ro = d.REDUCE_ORDER;
@@ -416,47 +456,22 @@ __global__ void __launch_bounds__(BS, 1024 / BS) k_ts_prolong(const __grid_const
         if (threadIdx.x == 0) s_sb = 0.0f;
     }
     __syncthreads();
-    const float SBCHG = s_sb, SSB = A1(d.STEPSBK, jsb);
-    float sabs = 0.0f;            // FP32 per thread, double-float across threads (as in k_ts_cells)
-    w = Walk2(IMM1, threadIdx.x, BS);
-#pragma unroll
-    for (int u = 0; u < TS_U; ++u) {
-        const int i = w.i, k = w.k;
-        w.next();
-        if (threadIdx.x + u * BS < nc) {
-            const int n = pj + (i - 1) + ks * (k - 1);
-            float DELTA = pst[u] * pstp[u] + (b1[pb1[u]] * ps1[u] + b2[pb2[u]] * ps2[u] + SBCHG * SSB) * prs[u];
-            V.ST[n] = DELTA;
-            sabs += fabsf(DELTA);
-        }
+    const float SB = s_sb * A1(d.STEPSBK, jsb);
+    if (nested) {
+        for (int t = threadIdx.x; t < n1; t += BS) b1[t] = b1[t] + b2[d.MG12[t]] + SB;
+        __syncthreads();
     }
-    // the remaining cells, TS_U at a time: their loads are issued together,
-    // before the stores of the group (a store of ST keeps later loads behind it)
-    for (int c0 = threadIdx.x + TS_U * BS; c0 < nc; c0 += TS_U * BS) {
-        int cn[TS_U];
+    float sabs = 0.0f;            // FP32 per thread, double-float across threads (as in k_ts_cells)
+    // TS_U cells at a time: their loads are issued together, before the stores
+    // of the group (a store of ST keeps later loads behind it)
+    for (int c0 = threadIdx.x; c0 < nc; c0 += TS_U * BS) {
+        if (c0 != (int)threadIdx.x) load(c0);
 #pragma unroll
         for (int u = 0; u < TS_U; ++u) {
-            const int i = w.i, k = w.k;
-            w.next();
-            cn[u] = -1;
-            if (c0 + u * BS < nc) {
-                const int n = pj + (i - 1) + ks * (k - 1);
-                const int i1 = A1(d.IB1, i), i2 = A1(d.IB2, i), k1 = A1(d.KB1, k), k2 = A1(d.KB2, k);
-                cn[u] = n;
-                pst[u] = V.ST[n];
-                pstp[u] = d.STEP[n];
-                prs[u] = d.RSTEP[n];
-                ps1[u] = d.STEP1[(i1 - 1) + d.NIB1 * (j1 - 1) + m1 * (k1 - 1)];
-                ps2[u] = d.STEP2[(i2 - 1) + d.NIB2 * (j2 - 1) + m2 * (k2 - 1)];
-                pb1[u] = (k1 - 1) * d.NIB1 + (i1 - 1);
-                pb2[u] = (k2 - 1) * d.NIB2 + (i2 - 1);
-            }
-        }
-#pragma unroll
-        for (int u = 0; u < TS_U; ++u) {
-            if (cn[u] < 0) continue;
-            float DELTA = pst[u] * pstp[u] + (b1[pb1[u]] * ps1[u] + b2[pb2[u]] * ps2[u] + SBCHG * SSB) * prs[u];
-            V.ST[cn[u]] = DELTA;
+            if (c0 + u * BS >= nc) break;
+            const float corr = nested ? b1[pb1[u]] : b1[pb1[u]] + b2[pb2[u]] + SB;
+            const float DELTA = pst[u] * pstp[u] + corr * prs[u];
+            ST[pn[u]] = DELTA;
             sabs += fabsf(DELTA);
         }
     }
