@@ -399,6 +399,7 @@ int capture_step(mgpu_handle *h, int what) {
         if (h->d.ILOS != 0) CK(cudaGraphConditionalHandleCreate(&hl, cg, 0, cudaGraphCondAssignDefault));
         CK(cudaGraphConditionalHandleCreate(&ht, cg, 0, cudaGraphCondAssignDefault));
         dg.use_cond = 1;
+        dg.in_batch = 1;
         dg.cond_loss = (unsigned long long)hl;
         dg.cond_tail = (unsigned long long)ht;
     }

@@ -11,11 +11,11 @@
 //   prolong  block sums assembled from the plane partials (level-1 blocks
 //            span <= JR planes, level-2 <= JRBB, superblocks a row part);
 //            STORE*STEP + corrections*RSTEP; per-plane sum of |STORE|
-//   update   per-row mean |STORE| (negative feedback, 1501-1525) applied to
-//            the cell planes J and J+1, the second mixing-plane average
-//            (1850), then every node of plane J gathers its <= 8 cell
-//            changes in the order the reference's scatter loop adds them
-//            (1100) -- no atomics, result written to TMP
+//   update   per-row mean |STORE| and the negative feedback of the cell
+//            changes (1501-1525), the second mixing-plane average (1850), then
+//            every node gathers its <= 8 cell changes in the order the
+//            reference's scatter loop adds them (1100) -- no atomics, result
+//            written to TMP
 //   smooth   streamwise smoothing of plane J from TMP planes J-2..J+2, then
 //            pitchwise, spanwise, corners, exit smoothing, periodic,
 //            tip-gap and mixing-plane averaging in shared memory -> D
@@ -37,10 +37,13 @@ static inline unsigned grid_for(size_t n, unsigned block) { return (unsigned)((n
 // of 3 x 241 CTAs fills five 192-thread slots per SM in one wave, where four
 // 256-thread slots take 1.2 waves.
 constexpr int TS_U = 3;          // cells per thread whose loads are issued together
-constexpr int TS_UG = 4;         // the same for the damping and gather phases of update
 constexpr int SV_U = 3;          // points per thread whose streamwise loads are issued together
 constexpr int SM_SEG = 8;        // points per thread of one pitchwise or spanwise smoothing segment
+constexpr int TS_UG = 4;         // cells per thread whose loads the pair update issues together
 constexpr int UG_SEG = 3;        // nodes per thread of one K column in the pair update's gather
+constexpr int UP_S = 3;          // nodes along K of one thread of update
+constexpr int UP_T = 288;        // most threads of an update CTA (three CTAs at 72 registers)
+constexpr int UP_R = 16;         // most J planes of an update CTA
 
 // CTA sum of one double-float per thread (thread 0 receives it)
 template <int BS>
@@ -531,195 +534,223 @@ __global__ void k_ts_avgblk_seq(const __grid_constant__ Dev d, int v0) {
 }
 
 // ---------------------------------------------------------------------
-// update: negative feedback, second MP average, corner gather -> TMP
+// the row's mean |STORE| after the mixing with its neighbour rows (1501-1515)
 // ---------------------------------------------------------------------
-template <int BS>
-__global__ void __launch_bounds__(BS, 1024 / BS) k_ts_update(const __grid_constant__ Dev d, int v0) {
+__device__ inline float row_mean(const float *chg, int nr, int NROWS) {
+    if (NROWS == 1) return chg[0];
+    if (NROWS == 2 || nr == 1) return 0.5f * (chg[0] + chg[1]);
+    if (nr == NROWS) return 0.5f * (chg[NROWS - 2] + chg[NROWS - 1]);
+    return 0.25f * (chg[nr - 2] + chg[nr]) + 0.5f * chg[nr - 1];
+}
+
+// ---------------------------------------------------------------------
+// update: negative feedback, second MP average, corner gather -> TMP.
+//
+// A CTA owns R successive node planes and a tile of K rows, all of I: one
+// thread a column of UP_S nodes along K at one I, marching up J.  It damps the
+// cell changes of one plane ahead into shared memory (two plane tiles, one
+// barrier a plane); the corner weights, which do not depend on J, stay in
+// registers, and so do the cells beside the thread's column, which serve the
+// two node planes beside their plane.  So a cell is damped
+// (1 + 1/R)(1 + 1/rows) times, where a CTA per plane pair damped it 1.5 times
+// and read each weight and cell again for every plane, at 230 instructions a
+// node.  The next plane's cells are in flight during the current one's gather.
+// Cells outside the grid are zeros in shared memory.
+// ---------------------------------------------------------------------
+__global__ void __launch_bounds__(UP_T, 3) k_ts_update(const __grid_constant__ Dev d, int v0, int rows, int ntile, int R) {
     pdl_wait();
     extern __shared__ float sm[];
     const VarSet &V = d.var[v0 + blockIdx.y];
     const float *__restrict__ D = V.D;
-    __shared__ float s_blk[64];
-    __shared__ float chg[64];
-    const int j = blockIdx.x + 1;
-    const int IM = d.IM, IMM1 = d.IMM1, KM = d.KM, KMM1 = d.KMM1;
-    const int nc = IMM1 * KMM1;
-    float *cA = sm, *cB = sm + nc;            // cell planes j and j+1
-    const DevCtl *ctl = d.ctl;
-    const int damp_on = ctl->damp_on;
-    const float DAMP = ctl->DAMP;
-    if (damp_on) {
-        if (d.REDUCE_ORDER == 1) {
-            for (int r = threadIdx.x; r < d.NROWS; r += BS) s_blk[r] = V.AVG_BLK[r];
-        } else {
-            int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-            for (int nr = w + 1; nr <= d.NROWS; nr += BS / 32) {
-                int JST = A1(d.JSTART, nr) + 1, JEN = A1(d.JMIX, nr) - 1;
-                const int ro = d.REDUCE_ORDER;
-                df s = df_of(0.0f);
-                for (int jj = JST + l; jj <= JEN; jj += 32) s = dacc(ro, s, V.pabs[jj - 1]);
-                for (int o = 16; o > 0; o >>= 1) s = dacc(ro, s, df_shfl_down(s, o));
-                if (l == 0) chg[nr - 1] = df_val(s) / (float)(IMM1 * KMM1 * (JEN - JST + 1));
-            }
-            __syncthreads();
-            if (threadIdx.x == 0) {
-                int NROWS = d.NROWS;
-                if (NROWS == 1) s_blk[0] = chg[0];
-                if (NROWS == 2) {
-                    s_blk[1] = 0.5f * (chg[0] + chg[1]);
-                    s_blk[0] = s_blk[1];
-                }
-                if (NROWS > 2) {
-                    for (int nr = 2; nr <= NROWS - 1; ++nr)
-                        s_blk[nr - 1] = 0.25f * (chg[nr - 2] + chg[nr]) + 0.5f * chg[nr - 1];
-                    s_blk[NROWS - 1] = 0.5f * (chg[NROWS - 2] + chg[NROWS - 1]);
-                    s_blk[0] = 0.5f * (chg[0] + chg[1]);
-                }
+    const float *__restrict__ ST = V.ST;
+    float *__restrict__ TM = V.TM;
+    __shared__ float s_blk[UP_R + 1], s_fd[UP_R + 1], s_fu[UP_R + 1], s_chg[64];
+    __shared__ int s_role[UP_R + 1], s_jmx[UP_R + 1];
+    const int IM = d.IM, JM = d.JM, IMM1 = d.IMM1, KM = d.KM, KMM1 = d.KMM1;
+    const int tile = blockIdx.x % ntile, ja = (int)(blockIdx.x / ntile) * R + 1;
+    const int jb = min(ja + R - 1, JM), k0 = 1 + tile * rows;
+    const int tid = threadIdx.x, seg = tid / IM, il = tid - seg * IM;     // I = il + 1
+    const int PW = IM + 1, buf = (rows + 1) * PW;     // cell (i, k) at i + PW * (k - k0 + 1), i = 0 .. IM
+    const bool act = seg * UP_S < rows;
+    const int damp_on = d.ctl->damp_on;
+    const float DAMP = d.ctl->DAMP;
+    for (int t = tid; t < 2 * buf; t += blockDim.x) sm[t] = 0.0f;
+    const int ks = IM * JM, kb = k0 + seg * UP_S;       // this thread's nodes: K = kb .. kb + UP_S - 1
+    const int nn = il + IM * (ja - 1) + ks * (kb - 1);  // node (il + 1, ja, kb)
+    int kn = act ? min(UP_S, min(k0 + rows, KM + 1) - kb) : 0;
+    if (kn < 0) kn = 0;
+    const bool ci = act && il < IMM1;                    // this thread has cells
+    const bool c0 = ci && seg == 0 && k0 >= 2;           // and the row below the tile
+    float wtr[UP_S], wtl[UP_S], wbr[UP_S], wbl[UP_S];
+#pragma unroll
+    for (int q = 0; q < UP_S; ++q) {
+        const int k = kb + q, o = il + IM * (k - 1);
+        const bool on = q < kn, hL = il >= 1, hR = il < IMM1, hD = k >= 2, hU = k <= KMM1;
+        wtr[q] = on && hL && hD ? d.FTR[o - 1 - IM] : 0.0f;
+        wtl[q] = on && hR && hD ? d.FTL[o - IM] : 0.0f;
+        wbr[q] = on && hL && hU ? d.FBR[o - 1] : 0.0f;
+        wbl[q] = on && hR && hU ? d.FBL[o] : 0.0f;
+    }
+    // cell changes of plane jc into this thread's registers
+    float st[UP_S + 1], dv[UP_S];
+    auto load_cells = [&](int jc) {
+        const int n = nn + IM * (jc - ja);
+        const bool pl = jc >= 2 && jc <= JM;
+#pragma unroll
+        for (int q = 0; q < UP_S; ++q)
+            if (pl && ci && q < kn && kb + q <= KMM1) st[q] = ST[n + ks * q];
+        if (pl && c0) st[UP_S] = ST[n - ks];
+    };
+    auto load_nodes = [&](int j) {
+#pragma unroll
+        for (int q = 0; q < UP_S; ++q)
+            if (q < kn) dv[q] = D[nn + IM * (j - ja) + ks * q];
+    };
+    // damped cells of plane jc = ja + p into its tile
+    auto damp_cells = [&](int p) {
+        const int jc = ja + p;
+        float *c = sm + (p & 1) * buf + il + 1;
+        const bool pl = jc >= 2 && jc <= JM;
+        const float blk = s_blk[p];
+        auto damped = [&](float v) {
+            if (!damp_on) return v;
+            const float FDAMP = fabsf(v) / blk;
+            return v / (1.0f + FDAMP / DAMP);
+        };
+#pragma unroll
+        for (int q = 0; q < UP_S; ++q)
+            if (ci && q < kn && kb + q <= KMM1) c[PW * (seg * UP_S + q + 1)] = pl ? damped(st[q]) : 0.0f;
+        if (c0) c[0] = pl ? damped(st[UP_S]) : 0.0f;
+        __syncthreads();
+        const int role = s_role[p];
+        if (role != 1 && role != 3) return;
+        // second pitchwise average on the mixing-plane cells (1850)
+        const bool lowx = d.FEXTRAP < 0.001f;
+        float *row0 = sm + (p & 1) * buf + 1;
+        const bool lane_par = d.REDUCE_ORDER == 0;
+        const int r0 = lane_par ? tid >> 5 : tid, rstep = lane_par ? (int)blockDim.x >> 5 : (int)blockDim.x;
+        for (int r = r0; r <= rows; r += rstep) {
+            const int k = k0 - 1 + r;
+            if (k < 1 || k > KMM1) continue;
+            const float FLOWDIRN = -A3(d.FLOWX, d.IMID, s_jmx[p], k);
+            if (!(role == 3 ? (FLOWDIRN > 0.0f || lowx) : (FLOWDIRN < 0.0f || lowx))) continue;
+            float *row = row0 + r * PW;
+            if (lane_par) {
+                const float m = warp_sum64(IMM1, [&](int i) { return row[i]; }) / (float)IMM1;
+                __syncwarp();
+                for (int i = tid & 31; i < IMM1; i += 32) row[i] = m;
+            } else {
+                const float m = mp_line_sum(row, IMM1) / (float)IMM1;
+                for (int i = 0; i < IMM1; ++i) row[i] = m;
             }
         }
         __syncthreads();
-    }
-    // damped cell changes of the two planes this node plane touches
-    for (int h = 0; h < 2; ++h) {
-        int jc = j + h;
-        if (jc < 2 || jc > d.JM) continue;
-        float *c = h ? cB : cA;
-        const float blk = damp_on ? s_blk[A1(d.NROW, jc) - 1] : 1.0f;
-        const float *__restrict__ stp = V.ST + (size_t)IM * (jc - 1);     // plane jc, (i, k) at i-1 + IM*JM*(k-1)
-        const size_t kstride = (size_t)IM * d.JM;
-        Walk2 w(IMM1, threadIdx.x, BS);
-        for (int t0 = threadIdx.x; t0 < nc; t0 += TS_UG * BS) {
-            float sv[TS_UG];
+    };
+    // the cells beside this thread's nodes, column I-1 and I, from the row
+    // below its first node to the row above its last
+    float ca[UP_S + 1][2], cb[UP_S + 1][2];
+    auto read_cells = [&](int p, float (*o)[2]) {
+        const float *c = sm + (p & 1) * buf + il + PW * (seg * UP_S);
 #pragma unroll
-            for (int u = 0; u < TS_UG; ++u) {
-                if (t0 + u * BS < nc) sv[u] = stp[(size_t)(w.i - 1) + kstride * (w.k - 1)];
-                w.next();
-            }
-#pragma unroll
-            for (int u = 0; u < TS_UG; ++u) {
-                const int t = t0 + u * BS;
-                if (t >= nc) break;
-                float v = sv[u];
-                if (damp_on) {
-                    float FDAMP = fabsf(v) / blk;
-                    v = v / (1.0f + FDAMP / DAMP);
-                }
-                c[t] = v;
-            }
+        for (int q = 0; q <= UP_S; ++q) {
+            o[q][0] = c[PW * q];
+            o[q][1] = c[PW * q + 1];
         }
+    };
+    load_cells(ja);
+    // the row means of |STORE| (1501-1515) that this CTA's cell planes take,
+    // from the planes' sums: a warp a row and its neighbour rows
+    if (damp_on && d.REDUCE_ORDER != 1) {
+        const int w = tid >> 5, l = tid & 31, nw = (int)blockDim.x >> 5, ro = d.REDUCE_ORDER;
+        const int r0 = max(A1(d.NROW, ja) - 1, 1), r1 = min(A1(d.NROW, min(jb + 1, JM)) + 1, d.NROWS);
+        for (int nr = r0 + w; nr <= r1; nr += nw) {
+            const int JST = A1(d.JSTART, nr) + 1, JEN = A1(d.JMIX, nr) - 1;
+            df s = df_of(0.0f);
+            for (int jj = JST + l; jj <= JEN; jj += 32) s = dacc(ro, s, V.pabs[jj - 1]);
+            for (int o = 16; o > 0; o >>= 1) s = dacc(ro, s, df_shfl_down(s, o));
+            if (l == 0) s_chg[nr - 1] = df_val(s) / (float)(IMM1 * KMM1 * (JEN - JST + 1));
+        }
+    }
+    __syncthreads();                       // the zeroed tiles and the rows' sums
+    // per cell plane jc = ja + q: the row mean, the mixing-plane role and the
+    // streamwise weights it has in the node planes before and after it
+    for (int q = tid; q <= jb - ja + 1; q += blockDim.x) {
+        const int jc = ja + q;
+        int nr = 0, role = 0;
+        if (jc >= 2 && jc <= JM) {
+            role = mp_role(d, jc, &nr);
+            s_blk[q] = !damp_on ? 1.0f : d.REDUCE_ORDER == 1 ? V.AVG_BLK[A1(d.NROW, jc) - 1]
+                                                             : row_mean(s_chg, A1(d.NROW, jc), d.NROWS);
+            s_fu[q] = A1(d.FACUP, jc);
+        } else {
+            s_blk[q] = 1.0f;
+            s_fu[q] = 0.0f;
+        }
+        s_fd[q] = jc <= JM ? A1(d.FACDWN, jc) : 0.0f;
+        s_role[q] = role;
+        s_jmx[q] = role == 1 || role == 3 ? A1(d.JMIX, nr) : 0;
     }
     __syncthreads();
-    // second pitchwise average on the mixing-plane cells (1850)
-    const bool lowx = d.FEXTRAP < 0.001f;
-    bool any = false;
-    for (int h = 0; h < 2; ++h) {
-        int jc = j + h;
-        if (jc < 2 || jc > d.JM) continue;
-        int mnr;
-        int role = mp_role(d, jc, &mnr);
-        if (role != 1 && role != 3) continue;
-        any = true;
-        float *c = h ? cB : cA;
-        int jmx = A1(d.JMIX, mnr);
-        const bool lane_par = d.REDUCE_ORDER == 0;
-        const int k0 = lane_par ? (int)(threadIdx.x >> 5) + 1 : (int)threadIdx.x + 1;
-        const int kstep = lane_par ? BS / 32 : BS;
-        for (int k = k0; k <= KMM1; k += kstep) {
-            float FLOWDIRN = -A3(d.FLOWX, d.IMID, jmx, k);
-            bool on = role == 3 ? (FLOWDIRN > 0.0f || lowx) : (FLOWDIRN < 0.0f || lowx);
-            if (!on) continue;
-            float *row = c + (size_t)(k - 1) * IMM1;
-            if (lane_par) {
-                float s = warp_sum64(IMM1, [&](int i) { return row[i]; }) / (float)IMM1;
-                __syncwarp();
-                for (int i = (int)(threadIdx.x & 31); i < IMM1; i += 32) row[i] = s;
-            } else {
-                float s = mp_line_sum(row, IMM1) / (float)IMM1;
-                for (int i = 0; i < IMM1; ++i) row[i] = s;
+    damp_cells(0);
+    load_cells(ja + 1);
+    load_nodes(ja);
+    if (act) read_cells(0, ca);
+#pragma unroll 2
+    for (int j = ja; j <= jb; ++j) {
+        const int p = j - ja;
+        damp_cells(p + 1);
+        if (j < jb) load_cells(j + 2);
+        if (!act) continue;
+        read_cells(p + 1, cb);
+        const float fd = s_fd[p], fu = s_fu[p + 1];
+        float *tm = TM + nn + IM * p;
+        if (fd == 1.0f && fu == 1.0f) {            // all planes but the first and the last two
+#pragma unroll
+            for (int q = 0; q < UP_S; ++q) {
+                float v = dv[q];
+                v = v + ca[q][0] * wtr[q];
+                v = v + ca[q][1] * wtl[q];
+                v = v + cb[q][0] * wtr[q];
+                v = v + cb[q][1] * wtl[q];
+                v = v + ca[q + 1][0] * wbr[q];
+                v = v + ca[q + 1][1] * wbl[q];
+                v = v + cb[q + 1][0] * wbr[q];
+                v = v + cb[q + 1][1] * wbl[q];
+                if (q < kn) tm[ks * q] = v;
+            }
+        } else {
+#pragma unroll
+            for (int q = 0; q < UP_S; ++q) {
+                float v = dv[q];
+                v = v + ca[q][0] * wtr[q] * fd;
+                v = v + ca[q][1] * wtl[q] * fd;
+                v = v + cb[q][0] * wtr[q] * fu;
+                v = v + cb[q][1] * wtl[q] * fu;
+                v = v + ca[q + 1][0] * wbr[q] * fd;
+                v = v + ca[q + 1][1] * wbl[q] * fd;
+                v = v + cb[q + 1][0] * wbr[q] * fu;
+                v = v + cb[q + 1][1] * wbl[q] * fu;
+                if (q < kn) tm[ks * q] = v;
             }
         }
-    }
-    if (any) __syncthreads();
-    // gather (1100): cells (kc, jc, ic) in the reference's loop order
-    const int np = IM * KM;
-    const float fdn = A1(d.FACDWN, j);
-    const float fup = j + 1 <= d.JM ? A1(d.FACUP, j + 1) : 0.0f;
-    const bool hA = j >= 2, hB = j + 1 <= d.JM;
-    const float *__restrict__ FBL = d.FBL;
-    const float *__restrict__ FBR = d.FBR;
-    const float *__restrict__ FTL = d.FTL;
-    const float *__restrict__ FTR = d.FTR;
-    const size_t nbase = (size_t)IM * (j - 1), kstride = (size_t)IM * d.JM;
-    Walk2 w(IM, threadIdx.x, BS);
-    for (int t0 = threadIdx.x; t0 < np; t0 += TS_UG * BS) {
-        // loads of TS_UG nodes first: the node value and, for interior nodes,
-        // the four corner weights
-        float dv[TS_UG], wtr[TS_UG], wtl[TS_UG], wbr[TS_UG], wbl[TS_UG];
-        int ni[TS_UG], nk[TS_UG];
+        if (j < jb) load_nodes(j + 1);
 #pragma unroll
-        for (int u = 0; u < TS_UG; ++u) {
-            const int i = w.i, k = w.k;
-            ni[u] = i;
-            nk[u] = k;
-            w.next();
-            if (t0 + u * BS < np) {
-                dv[u] = D[nbase + (size_t)(i - 1) + kstride * (k - 1)];
-                if (hA && hB && i >= 2 && i <= IMM1 && k >= 2 && k <= KMM1) {
-                    wtr[u] = FTR[(i - 2) + IM * (k - 2)];
-                    wtl[u] = FTL[(i - 1) + IM * (k - 2)];
-                    wbr[u] = FBR[(i - 2) + IM * (k - 1)];
-                    wbl[u] = FBL[(i - 1) + IM * (k - 1)];
-                }
-            }
-        }
-#pragma unroll
-        for (int u = 0; u < TS_UG; ++u) {
-            if (t0 + u * BS >= np) break;
-            const int i = ni[u], k = nk[u];
-            const size_t n = nbase + (size_t)(i - 1) + kstride * (k - 1);
-            float v = dv[u];
-            if (hA && hB && i >= 2 && i <= IMM1 && k >= 2 && k <= KMM1) {
-                // interior node: all eight cells, weights FTR/FTL of row k-1 and FBR/FBL of row k
-                const int lo = (i - 2) + IMM1 * (k - 2), hi = lo + IMM1;   // cells (i-1, k-1), (i-1, k)
-                v = v + cA[lo] * wtr[u] * fdn;
-                v = v + cA[lo + 1] * wtl[u] * fdn;
-                v = v + cB[lo] * wtr[u] * fup;
-                v = v + cB[lo + 1] * wtl[u] * fup;
-                v = v + cA[hi] * wbr[u] * fdn;
-                v = v + cA[hi + 1] * wbl[u] * fdn;
-                v = v + cB[hi] * wbr[u] * fup;
-                v = v + cB[hi + 1] * wbl[u] * fup;
-            } else {
-                for (int kc = k - 1; kc <= k; ++kc) {
-                    if (kc < 1 || kc > KMM1) continue;
-                    for (int h = 0; h < 2; ++h) {
-                        if (!(h ? hB : hA)) continue;
-                        const float *c = h ? cB : cA;
-                        float fac = h ? fup : fdn;
-                        for (int ic = i - 1; ic <= i; ++ic) {
-                            if (ic < 1 || ic > IMM1) continue;
-                            float wt;
-                            if (ic == i) wt = (kc == k) ? AIK(FBL, ic, kc) : AIK(FTL, ic, kc);
-                            else wt = (kc == k) ? AIK(FBR, ic, kc) : AIK(FTR, ic, kc);
-                            v = v + c[(kc - 1) * IMM1 + (ic - 1)] * wt * fac;
-                        }
-                    }
-                }
-            }
-            V.TM[n] = v;
+        for (int q = 0; q <= UP_S; ++q) {
+            ca[q][0] = cb[q][0];
+            ca[q][1] = cb[q][1];
         }
     }
 }
 
 // ---------------------------------------------------------------------
 // update over a pair of node planes: the same result as k_ts_update for
-// node planes j0 and j0+1, from one CTA of PBS threads.  The CTA damps the
-// three cell planes j0, j0+1, j0+2 once each (k_ts_update damps every cell
-// plane in the two CTAs that read it: 2 dampings per cell plane, here 1.5),
-// and each thread gathers the same (i, k) on both node planes, so the four
-// corner weights, the index arithmetic and the reads of the middle cell
-// plane serve both planes.  Every value is formed by the same expressions
-// in the same order as in k_ts_update.
+// node planes j0 and j0+1, from one CTA of PBS threads, for planes so small
+// that a CTA's threads cover the three cell planes at once: on 9 x 7 points
+// 10.4 us a launch against 14.3 for k_ts_update, whose march damps one plane
+// after the other; on 37 x 33 points k_ts_update is the faster one.  The CTA
+// damps the cell planes j0, j0+1, j0+2 once each, and each thread gathers the
+// same (i, k) on both node planes.  Every value is formed by the same
+// expressions in the same order as in k_ts_update.
 // ---------------------------------------------------------------------
 template <int PBS>
 __global__ void __launch_bounds__(PBS, 1024 / PBS) k_ts_update_pair(const __grid_constant__ Dev d, int v0) {
@@ -751,20 +782,7 @@ __global__ void __launch_bounds__(PBS, 1024 / PBS) k_ts_update_pair(const __grid
                 if (l == 0) chg[nr - 1] = df_val(s) / (float)(IMM1 * KMM1 * (JEN - JST + 1));
             }
             __syncthreads();
-            if (threadIdx.x == 0) {
-                int NROWS = d.NROWS;
-                if (NROWS == 1) s_blk[0] = chg[0];
-                if (NROWS == 2) {
-                    s_blk[1] = 0.5f * (chg[0] + chg[1]);
-                    s_blk[0] = s_blk[1];
-                }
-                if (NROWS > 2) {
-                    for (int nr = 2; nr <= NROWS - 1; ++nr)
-                        s_blk[nr - 1] = 0.25f * (chg[nr - 2] + chg[nr]) + 0.5f * chg[nr - 1];
-                    s_blk[NROWS - 1] = 0.5f * (chg[NROWS - 2] + chg[NROWS - 1]);
-                    s_blk[0] = 0.5f * (chg[0] + chg[1]);
-                }
-            }
+            for (int r = threadIdx.x; r < d.NROWS; r += PBS) s_blk[r] = row_mean(chg, r + 1, d.NROWS);
         }
         __syncthreads();
     }
@@ -936,6 +954,46 @@ __global__ void __launch_bounds__(PBS, 1024 / PBS) k_ts_update_pair(const __grid
             dn0l = up0l; dn0r = up0r; dn1l = up1l; dn1r = up1r; dn2l = up2l; dn2r = up2r;
         }
     }
+}
+
+// How update is cut: segments of UP_S rows per CTA (its threads are IM a
+// segment, at most UP_T), the number of K tiles and the planes per CTA.  The
+// segments minimise the lanes and rows that a cut leaves idle or damps twice.
+// The planes minimise the launch's length, waves of CTAs times a march of R
+// planes and about one and a half more for its start: the smallest grids take
+// one plane a CTA (one load, one barrier, one store), a grid that fills the
+// GPU as many as make whole waves; in a batch, where the other problems fill
+// it, eight.
+struct UpdateCut {
+    int rows, ntile, R, threads;
+    size_t smem;
+};
+static UpdateCut update_cut(const Dev &d, int sm_count, int nv) {
+    UpdateCut c{};
+    double best = 1e30;
+    for (int ns = 1; ns * d.IM <= UP_T && (ns == 1 || (ns - 1) * UP_S < d.KM); ++ns) {
+        const int rows = ns * UP_S, nt = (d.KM + rows - 1) / rows, th = (ns * d.IM + 31) / 32 * 32;
+        const double cost = (double)nt * (rows + 1) * th / (ns * d.IM);
+        if (cost < best) {
+            best = cost;
+            c.rows = rows;
+            c.ntile = nt;
+            c.threads = th;
+        }
+    }
+    const long long slots = (long long)sm_count * (65536 / (72 * c.threads));
+    best = 1e30;
+    for (int R = 1; R <= UP_R; ++R) {
+        const long long ctas = (long long)((d.JM + R - 1) / R) * c.ntile * nv;
+        const double cost = (double)((ctas + slots - 1) / slots) * (R + 1.5);
+        if (cost < best) {
+            best = cost;
+            c.R = R;
+        }
+    }
+    if (d.in_batch) c.R = 8;
+    c.smem = (size_t)2 * (c.rows + 1) * (d.IM + 1) * sizeof(float);
+    return c;
 }
 
 // ---------------------------------------------------------------------
@@ -1286,11 +1344,15 @@ __global__ void k_copy_tm_st(const __grid_constant__ Dev d, int v0, size_t n) {
     if (t < n) V.ST[t] = V.TM[t];
 }
 
+// k_ts_update_pair where a 512-thread CTA covers a plane's points (TS_PAIR = 0:
+// never); the crossover lies between 63 points, where it is 4 us faster a
+// launch, and 1221, where it is 1 us slower
+static bool pair_update(const Dev &d) { return d.TS_PAIR && d.IM * d.KM <= 512; }
+
 static size_t cells_smem(const Dev &d) {
     return ((size_t)d.IMM1 * d.KMM1 + d.KMM1 + (size_t)d.NIB1 * d.NKB1) * sizeof(float);
 }
 static size_t prolong_smem(const Dev &d) { return ((size_t)d.NIB1 * d.NKB1 + (size_t)d.NIB2 * d.NKB2) * sizeof(float); }
-static size_t update_smem(const Dev &d) { return (size_t)2 * d.IMM1 * d.KMM1 * sizeof(float); }
 static size_t update_pair_smem(const Dev &d) { return (size_t)3 * d.IMM1 * d.KMM1 * sizeof(float); }
 static size_t smooth_smem(const Dev &d) { return ((size_t)2 * (d.IM | 1) * d.KM + 2 * d.IM + 2 * d.KM) * sizeof(float); }
 
@@ -1301,8 +1363,7 @@ static cudaError_t configure_bs(const Dev &d) {
         size_t bytes;
     } k[] = {{(const void *)k_ts_cells<BS>, cells_smem(d)},
              {(const void *)k_ts_prolong<BS>, prolong_smem(d)},
-             {(const void *)k_ts_update<BS>, update_smem(d)},
-             {(const void *)k_ts_update_pair<2 * BS>, update_pair_smem(d)},
+             {(const void *)k_ts_update_pair<2 * BS>, pair_update(d) ? update_pair_smem(d) : 0},
              {(const void *)k_ts_smooth<BS>, smooth_smem(d)}};
     for (auto &x : k) {
         if (x.bytes > 200 * 1024) return cudaErrorInvalidValue;
@@ -1366,11 +1427,13 @@ template <int BS>
 static void launch_tstep_bs(const Dev &d, Launch L, int v0, int nv) {
     launch_tstep_front<BS>(d, L, v0, nv);
     const unsigned ja = (unsigned)d.JM, vy = (unsigned)nv;
-    if (d.TS_PAIR) {
+    if (pair_update(d)) {
         launchk(L, k_ts_update_pair<2 * BS>, dim3((ja + 1) / 2, vy), dim3(2 * BS), update_pair_smem(d), d, v0);
         mark(L, "k_ts_update_pair");
     } else {
-        launchk(L, k_ts_update<BS>, dim3(ja, vy), dim3(BS), update_smem(d), d, v0);
+        const UpdateCut u = update_cut(d, L.sm_count, nv);
+        launchk(L, k_ts_update, dim3((ja + u.R - 1) / u.R * u.ntile, vy), dim3(u.threads), u.smem, d, v0, u.rows, u.ntile,
+                u.R);
         mark(L, "k_ts_update");
     }
     launchk(L, k_ts_smooth<BS>, dim3(ja, vy), dim3(BS), smooth_smem(d), d, v0);
