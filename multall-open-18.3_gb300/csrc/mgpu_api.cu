@@ -1114,6 +1114,96 @@ int32_t mgpu_commit(mgpu_handle *h) {
             JSBLK[j - 1] < 1 || JSBLK[j - 1] > d.NSBLK)
             return fail(MGPU_E_ARG, "multigrid J map out of range");
     }
+    // the J planes' table
+    {
+        std::vector<int> IND, INDLE, KTIPS, KTIPE;
+        std::vector<float> FACUP, FACDWN, STEPSBK;
+        if ((rc = geti("IND", IND)) || (rc = geti("INDLE", INDLE)) || (rc = geti("KTIPS", KTIPS)) ||
+            (rc = geti("KTIPE", KTIPE)) || (rc = getf("FACUP", FACUP)) || (rc = getf("FACDWN", FACDWN)) ||
+            (rc = getf("STEPSBK", STEPSBK)))
+            return rc;
+        std::vector<int> b1s, b1e, b2s, b2e, sbs, sbe;
+        if ((rc = extents(JB1, 2, d.JM, d.NJB1, b1s, b1e, "JB1")) || (rc = extents(JB2, 2, d.JM, d.NJB2, b2s, b2e, "JB2")) ||
+            (rc = extents(JSBLK, 2, d.JM, d.NSBLK, sbs, sbe, "JSBLK")))
+            return rc;
+        std::vector<PlaneInfo> tab(d.JM);
+        for (int j = 1; j <= d.JM; ++j) {
+            PlaneInfo &p = tab[j - 1];
+            memset(&p, 0, sizeof(p));
+            const int nr = NROW[j - 1];
+            p.nrow = nr;
+            p.J1 = JSTART[nr - 1];
+            p.J2 = JMIX[nr - 1];
+            for (int r = 0; r < d.NRWSM1; ++r) {
+                const int q = j - JMIX[r];
+                if (!p.role && q >= 0 && q <= 2) {
+                    p.role = q + 1;
+                    p.jmx = JMIX[r];
+                }
+                if (d.IFMIX != 0 && (q == 0 || q == 1)) p.mix = 1;
+            }
+            p.kts = KTIPS[nr - 1];
+            p.kte = KTIPE[nr - 1];
+            // the reference tests these cases in this order and the last one
+            // that holds wins
+            if (j >= p.J1 + 3 && j <= p.J2 - 3) p.sc = 1;
+            if (j == p.J2 || j == p.J1) p.sc = 0;
+            if (j == p.J1 + 2) p.sc = 2;
+            if (j == p.J1 + 1) p.sc = 3;
+            if (j == p.J2 - 2) p.sc = 4;
+            if (j == p.J2 - 1) p.sc = 5;
+            for (int r = 0; r < d.NROWS; ++r) {
+                if (j == JLED[r] - 2 || j == JLED[r] - 1) p.lc = 1;
+                if (j == JLED[r]) p.lc = 2;
+            }
+            p.periodic = !(IND[j - 1] == 1 || INDLE[j - 1] == 1);
+            p.tip1 = p.kts;
+            p.tip2 = p.kte;
+            if (p.kts > 0) {
+                if (p.tip1 == 1) p.tip2 = p.tip2 - 1;
+                if (p.tip2 == d.KM) p.tip1 = p.tip1 + 1;
+            } else {
+                p.tip1 = 1;
+                p.tip2 = 0;
+            }
+            if (j >= 2) {
+                p.jb1 = JB1[j - 1];
+                p.jb2 = JB2[j - 1];
+                p.jsb = JSBLK[j - 1];
+                p.a1 = p.jb1 <= d.NJB1 ? b1s[p.jb1 - 1] : 1;
+                p.e1 = p.jb1 <= d.NJB1 ? b1e[p.jb1 - 1] : 0;
+                p.a2 = p.jb2 <= d.NJB2 ? b2s[p.jb2 - 1] : 1;
+                p.e2 = p.jb2 <= d.NJB2 ? b2e[p.jb2 - 1] : 0;
+                p.sa = sbs[p.jsb - 1];
+                p.se = sbe[p.jsb - 1];
+                p.stepsbk = STEPSBK[p.jsb - 1];
+                p.ratpitch = (float)NBLADE[j - 2] / (float)NBLADE[j - 1];
+            }
+            p.facdwn = FACDWN[j - 1];
+            p.facup = FACUP[j - 1];
+        }
+        if ((rc = dalloc(h, &d.PLANE, tab.size())) || (rc = upload(h, d.PLANE, tab))) return rc;
+        // the blocks' cells in I and K
+        std::vector<int> i1s, i1e, k1s, k1e, i2s, i2e, k2s, k2e;
+        if ((rc = extents(IB1, 1, d.IMM1, d.NIB1, i1s, i1e, "IB1")) || (rc = extents(KB1, 1, d.KMM1, d.NKB1, k1s, k1e, "KB1")) ||
+            (rc = extents(IB2, 1, d.IMM1, d.NIB2, i2s, i2e, "IB2")) || (rc = extents(KB2, 1, d.KMM1, d.NKB2, k2s, k2e, "KB2")))
+            return rc;
+        std::vector<int4> x1, x2;
+        for (int k = 0; k < d.NKB1; ++k)
+            for (int i = 0; i < d.NIB1; ++i) x1.push_back(make_int4(i1s[i], i1e[i], k1s[k], k1e[k]));
+        for (int k = 0; k < d.NKB2; ++k)
+            for (int i = 0; i < d.NIB2; ++i) {
+                int4 x = make_int4(i2s[i], i2e[i], k2s[k], k2e[k]);
+                if (d.mg_nested)
+                    x = x.y < x.x || x.w < x.z
+                            ? make_int4(1, 0, 1, 0)
+                            : make_int4(IB1[x.x - 1], IB1[x.y - 1], KB1[x.z - 1], KB1[x.w - 1]);
+                x2.push_back(x);
+            }
+        if ((rc = dalloc(h, &d.MG1X, x1.size())) || (rc = upload(h, d.MG1X, x1)) || (rc = dalloc(h, &d.MG2X, x2.size())) ||
+            (rc = upload(h, d.MG2X, x2)))
+            return rc;
+    }
     for (int v = 0; v < (sa ? NVAR + 1 : NVAR); ++v) {
         VarSet &V = d.var[v];
         if ((rc = dalloc(h, &V.B1CHG, shape_count(h, SH_MG1))) || (rc = dalloc(h, &V.B2CHG, shape_count(h, SH_MG2))) ||

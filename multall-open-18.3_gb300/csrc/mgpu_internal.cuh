@@ -74,6 +74,26 @@ enum { V_RO = 0, V_ROE = 1, V_ROVX = 2, V_RORVT = 3, V_ROVR = 4 };
 // variable, cell-centred, after the five conserved ones
 constexpr int V_SA = 5;
 
+// What TSTEP's kernels need to know of a J plane, as mgpu_commit derives it
+// from the row cards: one 128-byte line in place of chains of table loads
+// (NROW -> JMIX -> plane), which were a third of a small launch's time.
+struct alignas(16) PlaneInfo {
+    int nrow, J1, J2;          // NROW(J), its JSTART and JMIX
+    int role, jmx;             // place at a mixing plane: 1 JMIX, 2 JMIX+1, 3 JMIX+2 (else 0), and that JMIX
+    int kts, kte;              // KTIPS, KTIPE of the row
+    int sc, lc;                // SMOOTH_VAR's streamwise case (15375-15406) and leading-edge case (15417-15434)
+    int periodic, mix;         // I = 1 / IM are averaged; the plane is averaged over the pitch (100)
+    int tip1, tip2;            // tip-gap average over K = tip1..tip2 (510; empty without a gap)
+    int jb1, jb2, jsb;         // multigrid blocks
+    int a1, e1, a2, e2;        // J planes of the level-1 and level-2 block (empty past the last)
+    int sa, se;                // J planes of the superblock
+    float ratpitch;            // NBLADE(J-1) / NBLADE(J)
+    float facdwn, facup;
+    float stepsbk;
+    int pad[6];
+};
+static_assert(sizeof(PlaneInfo) == 128, "one line a plane");
+
 struct Dev {
     // dimensions
     int IM, JM, KM, NROWS;
@@ -129,6 +149,9 @@ struct Dev {
     int *IB1_S, *IB1_E, *IB2_S, *IB2_E;                 // (NIBn) I extent of each block
     int *KB1_S, *KB1_E, *KB2_S, *KB2_E;                 // (NKBn) K extent of each block
     int *SB_START, *SB_END;                             // (NSBLK)
+    PlaneInfo *PLANE;                  // (JM)
+    int4 *MG1X, *MG2X;                 // cells I0, I1, K0, K1 of each level-1 block of a plane; of each level-2
+                                       // block, or, nested, its level-1 blocks
     unsigned short *CB1, *CB2;         // (IMM1*KMM1) level-1 and level-2 block of each cell of a plane
     int *MG12;                         // (NIB1*NKB1) level-2 block of each level-1 block, where nested
     int mg_nested;                     // every level-2 block is a union of level-1 blocks (in I and in K)

@@ -55,23 +55,10 @@ __device__ inline df block_sum(int order, df v, df *sh) {
     df r = df_of(0.0f);
     if (w == 0) {
         r = l < BS / 32 ? sh[l] : df_of(0.0f);
-        for (int o = 16; o > 0; o >>= 1) r = dacc(order, r, df_shfl_down(r, o));
+        for (int o = BS > 256 ? 8 : BS > 128 ? 4 : 2; o > 0; o >>= 1) r = dacc(order, r, df_shfl_down(r, o));
     }
     __syncthreads();
     return r;
-}
-
-// position of plane j relative to the mixing planes: 1 = JMIX, 2 = JMIX+1,
-// 3 = JMIX+2 (0 otherwise); *nr receives the row interface
-__device__ inline int mp_role(const Dev &d, int j, int *nr) {
-    for (int r = 1; r <= d.NRWSM1; ++r) {
-        int jx = A1(d.JMIX, r);
-        if (j == jx) { *nr = r; return 1; }
-        if (j == jx + 1) { *nr = r; return 2; }
-        if (j == jx + 2) { *nr = r; return 3; }
-    }
-    *nr = 0;
-    return 0;
 }
 
 // Pitchwise sum of a mixing-plane line in I order, REAL*4 as the reference
@@ -152,10 +139,13 @@ __global__ void __launch_bounds__(BS, 1024 / BS) k_ts_cells(const __grid_constan
     const int nc = IMM1 * KMM1;
     float *st = sm;              // STORE of this plane, [k-1][i-1]
     float *lsum = sm + nc;       // per-K line sums
-    int mnr;
-    const int role = mp_role(d, j, &mnr);
+    const PlaneInfo &pl = d.PLANE[j - 1];
+    const int role = pl.role, jmx = pl.jmx, kts = pl.kts, kte = pl.kte;
+    const float RATPITCH = pl.ratpitch;
     const bool lowx = d.FEXTRAP < 0.001f;
-    const int jmx = role ? A1(d.JMIX, mnr) : 0;
+    // the cells of this thread's first level-1 block, for the partial sums below
+    const int n1 = d.NIB1 * d.NKB1, n2 = d.NIB2 * d.NKB2;
+    const int4 blk1 = d.MG1X[min((int)threadIdx.x, n1 - 1)], blk2 = d.MG2X[min((int)threadIdx.x, n2 - 1)];
     if ((role == 1 || role == 3) && !lowx) {
         // stage the XFLUX plane in shared memory (coalesced), then add each
         // I-line in the reference's order
@@ -177,9 +167,6 @@ __global__ void __launch_bounds__(BS, 1024 / BS) k_ts_cells(const __grid_constan
         }
     }
     __syncthreads();
-    const float RATPITCH = (float)A1(d.NBLADE, j - 1) / (float)A1(d.NBLADE, j);
-    const int nr = A1(d.NROW, j);
-    const int kts = A1(d.KTIPS, nr), kte = A1(d.KTIPE, nr);
     const float F1 = d.F1, F2 = d.F2, F3 = d.F3;
     const float *__restrict__ XF = V.XF;
     const float *__restrict__ RF = V.RF;
@@ -272,7 +259,14 @@ __global__ void __launch_bounds__(BS, 1024 / BS) k_ts_cells(const __grid_constan
     const df ps = block_sum<BS>(d.REDUCE_ORDER, df_of(psf), shd);
     if (threadIdx.x == 0) V.psum[j - 1] = ps;
     // level-1 and level-2 partial sums of this plane
-    const int n1 = d.NIB1 * d.NKB1, n2 = d.NIB2 * d.NKB2;
+    auto block_cells = [&](int4 x) {
+        float s = 0.0f;
+        for (int k = x.z; k <= x.w; ++k)
+            for (int i = x.x; i <= x.y; ++i) s = s + st[(k - 1) * IMM1 + (i - 1)];
+        return s;
+    };
+    float *__restrict__ P1 = V.P1 + (size_t)(j - 1) * n1;
+    float *__restrict__ P2 = V.P2 + (size_t)(j - 1) * n2;
     if (d.mg_nested) {
         // every level-2 block is a union of level-1 blocks: the level-1
         // partials first (in shared memory), then each level-2 partial as the
@@ -280,39 +274,22 @@ __global__ void __launch_bounds__(BS, 1024 / BS) k_ts_cells(const __grid_constan
         // 3 x 3 cells, where the direct sum is an 81-term chain)
         float *p1 = lsum + KMM1;
         for (int u = threadIdx.x; u < n1; u += BS) {
-            const int ib = u % d.NIB1 + 1, kb = u / d.NIB1 + 1;
-            const int i0 = A1(d.IB1_S, ib), i1 = A1(d.IB1_E, ib), k0 = A1(d.KB1_S, kb), k1 = A1(d.KB1_E, kb);
-            float s = 0.0f;
-            for (int k = k0; k <= k1; ++k)
-                for (int i = i0; i <= i1; ++i) s = s + st[(k - 1) * IMM1 + (i - 1)];
+            const float s = block_cells(u < BS ? blk1 : d.MG1X[u]);
             p1[u] = s;
-            V.P1[(size_t)(j - 1) * n1 + u] = s;
+            P1[u] = s;
         }
         __syncthreads();
         for (int u = threadIdx.x; u < n2; u += BS) {
-            const int ib = u % d.NIB2 + 1, kb = u / d.NIB2 + 1;
-            const int a0 = A1(d.IB1, A1(d.IB2_S, ib)), a1 = A1(d.IB1, A1(d.IB2_E, ib));
-            const int c0 = A1(d.KB1, A1(d.KB2_S, kb)), c1 = A1(d.KB1, A1(d.KB2_E, kb));
+            const int4 x = u < BS ? blk2 : d.MG2X[u];
             float s = 0.0f;
-            for (int kb1 = c0; kb1 <= c1; ++kb1)
-                for (int ib1 = a0; ib1 <= a1; ++ib1) s = s + p1[(kb1 - 1) * d.NIB1 + (ib1 - 1)];
-            V.P2[(size_t)(j - 1) * n2 + u] = s;
+            for (int kb1 = x.z; kb1 <= x.w; ++kb1)
+                for (int ib1 = x.x; ib1 <= x.y; ++ib1) s = s + p1[(kb1 - 1) * d.NIB1 + (ib1 - 1)];
+            P2[u] = s;
         }
         return;
     }
-    for (int t = threadIdx.x; t < n1 + n2; t += BS) {
-        const bool lv1 = t < n1;
-        int u = lv1 ? t : t - n1;
-        int nib = lv1 ? d.NIB1 : d.NIB2;
-        int ib = u % nib + 1, kb = u / nib + 1;
-        int i0 = lv1 ? A1(d.IB1_S, ib) : A1(d.IB2_S, ib), i1 = lv1 ? A1(d.IB1_E, ib) : A1(d.IB2_E, ib);
-        int k0 = lv1 ? A1(d.KB1_S, kb) : A1(d.KB2_S, kb), k1 = lv1 ? A1(d.KB1_E, kb) : A1(d.KB2_E, kb);
-        float s = 0.0f;
-        for (int k = k0; k <= k1; ++k)
-            for (int i = i0; i <= i1; ++i) s = s + st[(k - 1) * IMM1 + (i - 1)];
-        if (lv1) V.P1[(size_t)(j - 1) * n1 + u] = s;
-        else V.P2[(size_t)(j - 1) * n2 + u] = s;
-    }
+    for (int u = threadIdx.x; u < n1; u += BS) P1[u] = block_cells(u < BS ? blk1 : d.MG1X[u]);
+    for (int u = threadIdx.x; u < n2; u += BS) P2[u] = block_cells(u < BS ? blk2 : d.MG2X[u]);
 }
 
 // ---------------------------------------------------------------------
@@ -391,7 +368,8 @@ __global__ void __launch_bounds__(BS, 1024 / BS) k_ts_prolong(const __grid_const
     const int IMM1 = d.IMM1, KMM1 = d.KMM1;
     const int n1 = d.NIB1 * d.NKB1, n2 = d.NIB2 * d.NKB2;
     float *b1 = sm, *b2 = sm + n1;
-    const int j1 = A1(d.JB1, j), j2 = A1(d.JB2, j), jsb = A1(d.JSBLK, j);
+    const PlaneInfo &pl = d.PLANE[j - 1];
+    const int j1 = pl.jb1, j2 = pl.jb2, jsb = pl.jsb;
     const int nc = IMM1 * KMM1;
     const int m1 = d.NIB1 * (d.NJB1 + 1), m2 = d.NIB2 * (d.NJB2 + 1);
     const bool nested = d.mg_nested != 0;
@@ -432,8 +410,7 @@ __global__ void __launch_bounds__(BS, 1024 / BS) k_ts_prolong(const __grid_const
     } else {
         // the J planes of this plane's level-1 and level-2 blocks (empty past
         // the last block); each sum adds the planes' partials in J order
-        const int a1 = j1 <= d.NJB1 ? A1(d.JB1_START, j1) : 1, e1 = j1 <= d.NJB1 ? A1(d.JB1_END, j1) : 0;
-        const int a2 = j2 <= d.NJB2 ? A1(d.JB2_START, j2) : 1, e2 = j2 <= d.NJB2 ? A1(d.JB2_END, j2) : 0;
+        const int a1 = pl.a1, e1 = pl.e1, a2 = pl.a2, e2 = pl.e2;
         for (int t = threadIdx.x; t < n1; t += BS) {
             const float st1 = d.STEP1[t % d.NIB1 + d.NIB1 * (j1 - 1) + m1 * (t / d.NIB1)];
             b1[t] = plane_partials_sum(V.P1, n1, t, a1, e1) * st1;
@@ -443,10 +420,9 @@ __global__ void __launch_bounds__(BS, 1024 / BS) k_ts_prolong(const __grid_const
             b2[t] = plane_partials_sum(V.P2, n2, t, a2, e2) * st2;
         }
         if (threadIdx.x < 32) {
-            int a = A1(d.SB_START, jsb), b = A1(d.SB_END, jsb);
             const int ro = d.REDUCE_ORDER;
             df s = df_of(0.0f);
-            for (int jj = a + (int)threadIdx.x; jj <= b; jj += 32) s = dacc(ro, s, V.psum[jj - 1]);
+            for (int jj = pl.sa + (int)threadIdx.x; jj <= pl.se; jj += 32) s = dacc(ro, s, V.psum[jj - 1]);
             for (int o = 16; o > 0; o >>= 1) s = dacc(ro, s, df_shfl_down(s, o));
             if (threadIdx.x == 0) s_sb = df_val(s);
         }
@@ -459,7 +435,7 @@ __global__ void __launch_bounds__(BS, 1024 / BS) k_ts_prolong(const __grid_const
         if (threadIdx.x == 0) s_sb = 0.0f;
     }
     __syncthreads();
-    const float SB = s_sb * A1(d.STEPSBK, jsb);
+    const float SB = s_sb * pl.stepsbk;
     if (nested) {
         for (int t = threadIdx.x; t < n1; t += BS) b1[t] = b1[t] + b2[d.MG12[t]] + SB;
         __syncthreads();
@@ -662,7 +638,7 @@ __global__ void __launch_bounds__(UP_T, 3) k_ts_update(const __grid_constant__ D
     // from the planes' sums: a warp a row and its neighbour rows
     if (damp_on && d.REDUCE_ORDER != 1) {
         const int w = tid >> 5, l = tid & 31, nw = (int)blockDim.x >> 5, ro = d.REDUCE_ORDER;
-        const int r0 = max(A1(d.NROW, ja) - 1, 1), r1 = min(A1(d.NROW, min(jb + 1, JM)) + 1, d.NROWS);
+        const int r0 = max(d.PLANE[ja - 1].nrow - 1, 1), r1 = min(d.PLANE[min(jb + 1, JM) - 1].nrow + 1, d.NROWS);
         for (int nr = r0 + w; nr <= r1; nr += nw) {
             const int JST = A1(d.JSTART, nr) + 1, JEN = A1(d.JMIX, nr) - 1;
             df s = df_of(0.0f);
@@ -676,19 +652,19 @@ __global__ void __launch_bounds__(UP_T, 3) k_ts_update(const __grid_constant__ D
     // streamwise weights it has in the node planes before and after it
     for (int q = tid; q <= jb - ja + 1; q += blockDim.x) {
         const int jc = ja + q;
-        int nr = 0, role = 0;
+        const PlaneInfo &pl = d.PLANE[min(jc, JM) - 1];
         if (jc >= 2 && jc <= JM) {
-            role = mp_role(d, jc, &nr);
-            s_blk[q] = !damp_on ? 1.0f : d.REDUCE_ORDER == 1 ? V.AVG_BLK[A1(d.NROW, jc) - 1]
-                                                             : row_mean(s_chg, A1(d.NROW, jc), d.NROWS);
-            s_fu[q] = A1(d.FACUP, jc);
+            s_blk[q] = !damp_on ? 1.0f : d.REDUCE_ORDER == 1 ? V.AVG_BLK[pl.nrow - 1]
+                                                             : row_mean(s_chg, pl.nrow, d.NROWS);
+            s_fu[q] = pl.facup;
+            s_role[q] = pl.role;
         } else {
             s_blk[q] = 1.0f;
             s_fu[q] = 0.0f;
+            s_role[q] = 0;
         }
-        s_fd[q] = jc <= JM ? A1(d.FACDWN, jc) : 0.0f;
-        s_role[q] = role;
-        s_jmx[q] = role == 1 || role == 3 ? A1(d.JMIX, nr) : 0;
+        s_fd[q] = jc <= JM ? pl.facdwn : 0.0f;
+        s_jmx[q] = pl.jmx;
     }
     __syncthreads();
     damp_cells(0);
@@ -792,7 +768,7 @@ __global__ void __launch_bounds__(PBS, 1024 / PBS) k_ts_update_pair(const __grid
         const int jc = j0 + h;
         if (jc < 2 || jc > JM) continue;
         float *c = sm + h * nc;
-        const float blk = damp_on ? s_blk[A1(d.NROW, jc) - 1] : 1.0f;
+        const float blk = damp_on ? s_blk[d.PLANE[jc - 1].nrow - 1] : 1.0f;
         const float *__restrict__ stp = V.ST + IM * (jc - 1);
         Walk2 w(IMM1, threadIdx.x, PBS);
         for (int t0 = threadIdx.x; t0 < nc; t0 += TS_UG * PBS) {
@@ -822,12 +798,10 @@ __global__ void __launch_bounds__(PBS, 1024 / PBS) k_ts_update_pair(const __grid
     for (int h = 0; h < 3; ++h) {
         const int jc = j0 + h;
         if (jc < 2 || jc > JM) continue;
-        int mnr;
-        const int role = mp_role(d, jc, &mnr);
+        const int role = d.PLANE[jc - 1].role, jmx = d.PLANE[jc - 1].jmx;
         if (role != 1 && role != 3) continue;
         any = true;
         float *c = sm + h * nc;
-        const int jmx = A1(d.JMIX, mnr);
         const bool lane_par = d.REDUCE_ORDER == 0;
         const int k0 = lane_par ? (int)(threadIdx.x >> 5) + 1 : (int)threadIdx.x + 1;
         const int kstep = lane_par ? PBS / 32 : PBS;
@@ -1000,35 +974,6 @@ static UpdateCut update_cut(const Dev &d, int sm_count, int nv) {
 // smooth: SMOOTH_VAR (3900-9000, 8502) + periodic (8000), tip gap (510),
 // mixing-plane average (100): TMP -> D, one CTA per J-plane
 // ---------------------------------------------------------------------
-// Streamwise smoothing case of plane j (SMOOTH_VAR 15375-15406): the
-// reference tests the cases in this order and the last one that holds wins.
-__device__ inline int stream_case(const Dev &d, int j) {
-    int nr = A1(d.NROW, j);
-    int J1 = A1(d.JSTART, nr), J2 = A1(d.JMIX, nr);
-    int sc = 0;                                   // 0: unchanged
-    if (j >= J1 + 3 && j <= J2 - 3) sc = 1;       // 2nd + 4th order interior
-    if (j == J2) sc = 0;
-    if (j == J1) sc = 0;
-    if (j == J1 + 2) sc = 2;
-    if (j == J1 + 1) sc = 3;
-    if (j == J2 - 2) sc = 4;
-    if (j == J2 - 1) sc = 5;
-    return sc;
-}
-
-// Leading-edge periodic smoothing case of plane j (15417-15434): 1 on the
-// two planes before a row's JLED, 2 on JLED itself; the last row that
-// matches wins.
-__device__ inline int le_case(const Dev &d, int j) {
-    int lc = 0;
-    for (int r = 1; r <= d.NROWS; ++r) {
-        int JL = A1(d.JLED, r);
-        if (j == JL - 2 || j == JL - 1) lc = 1;
-        if (j == JL) lc = 2;
-    }
-    return lc;
-}
-
 template <int BS>
 __global__ void __launch_bounds__(BS, 1024 / BS) k_ts_smooth(const __grid_constant__ Dev d, int v0) {
     pdl_wait();
@@ -1045,6 +990,7 @@ __global__ void __launch_bounds__(BS, 1024 / BS) k_ts_smooth(const __grid_consta
     float *a = sm, *b = sm + IMP * KM;
     float *cFD = b + IMP * KM, *cFU = cFD + IM, *cFKD = cFU + IM, *cFKU = cFKD + KM;   // FD, FU, FKD, FKU
     const int j = blockIdx.x + 1;
+    const PlaneInfo &pl = d.PLANE[j - 1];
     const DevCtl *c = d.ctl;
     const bool stream = !(c->SFX < 0.0001f);
     for (int t = threadIdx.x; t < IM; t += BS) {
@@ -1058,10 +1004,8 @@ __global__ void __launch_bounds__(BS, 1024 / BS) k_ts_smooth(const __grid_consta
     const int ks = IM * d.JM;                        // K stride of a node array
     const float *__restrict__ Sj = S + IM * (j - 1);  // plane j: (i, k) at i-1 + ks*(k-1)
     {
-        const int sc = stream ? stream_case(d, j) : 0;
-        const int lc = stream ? le_case(d, j) : 0;
-        const int nr = A1(d.NROW, j);
-        const int J1 = A1(d.JSTART, nr), J2 = A1(d.JMIX, nr);
+        const int sc = stream ? pl.sc : 0, lc = stream ? pl.lc : 0;
+        const int J1 = pl.J1, J2 = pl.J2;
         const float SFX = c->SFX, SFX1 = c->SFX1, SFXB = c->SFXB, SFXB1 = c->SFXB1, SFXBH = c->SFXBH;
         const float SFXHM1 = c->SFXHM1, SFX14 = c->SFX14, F4 = d.FAC_4TH;
         // the J planes each case reads, as node offsets from plane j
@@ -1120,7 +1064,7 @@ __global__ void __launch_bounds__(BS, 1024 / BS) k_ts_smooth(const __grid_consta
     }
     __syncthreads();
 #define P(buf, i, k) buf[((i) - 1) + IMP * ((k) - 1)]
-    const bool periodic_j = !(A1(d.IND, j) == 1 || A1(d.INDLE, j) == 1);
+    const bool periodic_j = pl.periodic != 0;
     if (j >= 2 && !(c->SFT < 0.0001f)) {
         const float SFT = c->SFT, SFT1 = c->SFT1, F4 = d.FAC_4TH;
         // the points I = 2..IMM1 first, in segments of SM_SEG points of one K
@@ -1245,31 +1189,20 @@ __global__ void __launch_bounds__(BS, 1024 / BS) k_ts_smooth(const __grid_consta
         }
         __syncthreads();
     }
-    int nr = A1(d.NROW, j);
-    int K1 = A1(d.KTIPS, nr), K2 = A1(d.KTIPE, nr);
-    bool tip = K1 > 0;
-    if (tip) {
-        if (K1 == 1) K2 = K2 - 1;
-        if (K2 == KM) K1 = K1 + 1;
-    }
     for (int k = threadIdx.x + 1; k <= KM; k += BS) {
         if (periodic_j) {
             float v = 0.5f * (P(a, 1, k) + P(a, IM, k));
             P(a, 1, k) = v;
             P(a, IM, k) = v;
         }
-        if (tip && k >= K1 && k <= K2) {
+        if (k >= pl.tip1 && k <= pl.tip2) {
             float v = 0.5f * (P(a, 1, k) + P(a, IM, k));
             P(a, 1, k) = v;
             P(a, IM, k) = v;
         }
     }
     __syncthreads();
-    bool mp = false;
-    if (d.IFMIX != 0)
-        for (int r = 1; r <= d.NRWSM1; ++r)
-            if (j == A1(d.JMIX, r) || j == A1(d.JMIX, r) + 1) mp = true;
-    if (mp) {
+    if (pl.mix) {
         if (d.REDUCE_ORDER != 0) {
             for (int k = threadIdx.x + 1; k <= KM; k += BS) {
                 float s = 0.0f;
