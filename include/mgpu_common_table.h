@@ -77,8 +77,8 @@
     /* or 512 (0: 256 until mgpu_autotune chooses)                        */ \
     M_(TS_THREADS, 0)                                                     \
     /* not a COMMON variable: 1 (default) runs TSTEP's damping and corner */ \
-    /* gather over pairs of J-planes (one CTA of twice the threads per    */ \
-    /* pair), 0 one CTA per J-plane; the results are bitwise the same     */ \
+    /* gather of planes of at most 512 points over pairs of J-planes, 0   */ \
+    /* always marching along J; the results are bitwise the same          */ \
     M_(TS_PAIR, 1)
 
 /* ----- REAL scalars: /BKGAS/, /BKCNTL/, /BKSMTH/, /BKLOSS/, /BKINPT/ ---- */
