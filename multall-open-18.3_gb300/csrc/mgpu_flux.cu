@@ -762,7 +762,9 @@ __device__ __noinline__ void edges_mom(const Dev &d, int e) {
 // each sum in the order of the reference's expression; also PEFF of this step,
 // which the next step's energy fluxes read.  The axial and tangential sources
 // XFORCE and TFORCE are read in place by TSTEP.
-__global__ void __launch_bounds__(256, 2) k_flux_mom(const __grid_constant__ Dev d, int S, int edges) {
+// Three CTAs an SM at 80 registers (32 bytes spilled): 27 us at 65 x 242 x 49;
+// two at 128 registers 36 us.
+__global__ void __launch_bounds__(256, 3) k_flux_mom(const __grid_constant__ Dev d, int S, int edges) {
     pdl_wait();
     if ((int)blockIdx.x < edges) {
         edges_mom(d, (int)(blockIdx.x * 256 + threadIdx.x));

@@ -39,6 +39,8 @@ static inline unsigned grid_for(size_t n, unsigned block) { return (unsigned)((n
 constexpr int TS_U = 3;          // cells per thread whose loads are issued together
 constexpr int SV_U = 3;          // points per thread whose streamwise loads are issued together
 constexpr int SM_SEG = 8;        // points per thread of one pitchwise or spanwise smoothing segment
+constexpr int PR_U = 2;          // the same in prolong, whose 40 registers leave 1536 threads an SM (three cells
+                                 // and 1280 threads: 18 us a launch against 16 at 65 x 242 x 49)
 constexpr int TS_UG = 4;         // cells per thread whose loads the pair update issues together
 constexpr int UG_SEG = 3;        // nodes per thread of one K column in the pair update's gather
 constexpr int UP_S = 3;          // nodes along K of one thread of update
@@ -358,7 +360,7 @@ __device__ __forceinline__ float plane_partials_sum(const float *__restrict__ P,
 // 120 instructions and six dependent loads of it.
 // ---------------------------------------------------------------------
 template <int BS>
-__global__ void __launch_bounds__(BS, 1024 / BS) k_ts_prolong(const __grid_constant__ Dev d, int v0, int want_abs) {
+__global__ void __launch_bounds__(BS, 1536 / BS) k_ts_prolong(const __grid_constant__ Dev d, int v0, int want_abs) {
     pdl_wait();
     extern __shared__ float sm[];
     const VarSet &V = d.var[v0 + blockIdx.y];
@@ -376,14 +378,14 @@ __global__ void __launch_bounds__(BS, 1024 / BS) k_ts_prolong(const __grid_const
     float *__restrict__ ST = V.ST;
     const float *__restrict__ STEP = d.STEP;
     const float *__restrict__ RSTEP = d.RSTEP;
-    // operands of this thread's first TS_U cells, loaded before the block
+    // operands of this thread's first PR_U cells, loaded before the block
     // sums so their latency overlaps the assembly below
-    float pst[TS_U], pstp[TS_U], prs[TS_U];
-    int pb1[TS_U], pb2[TS_U], pn[TS_U];
+    float pst[PR_U], pstp[PR_U], prs[PR_U];
+    int pb1[PR_U], pb2[PR_U], pn[PR_U];
     WalkN w(IMM1, d.IM * d.JM, d.IM * (j - 1), threadIdx.x, BS);
     auto load = [&](int c0) {
 #pragma unroll
-        for (int u = 0; u < TS_U; ++u) {
+        for (int u = 0; u < PR_U; ++u) {
             const int c = c0 + u * BS;
             pn[u] = w.n;
             if (c < nc) {
@@ -441,12 +443,12 @@ __global__ void __launch_bounds__(BS, 1024 / BS) k_ts_prolong(const __grid_const
         __syncthreads();
     }
     float sabs = 0.0f;            // FP32 per thread, double-float across threads (as in k_ts_cells)
-    // TS_U cells at a time: their loads are issued together, before the stores
+    // PR_U cells at a time: their loads are issued together, before the stores
     // of the group (a store of ST keeps later loads behind it)
-    for (int c0 = threadIdx.x; c0 < nc; c0 += TS_U * BS) {
+    for (int c0 = threadIdx.x; c0 < nc; c0 += PR_U * BS) {
         if (c0 != (int)threadIdx.x) load(c0);
 #pragma unroll
-        for (int u = 0; u < TS_U; ++u) {
+        for (int u = 0; u < PR_U; ++u) {
             if (c0 + u * BS >= nc) break;
             const float corr = nested ? b1[pb1[u]] : b1[pb1[u]] + b2[pb2[u]] + SB;
             const float DELTA = pst[u] * pstp[u] + corr * prs[u];
@@ -936,8 +938,7 @@ __global__ void __launch_bounds__(PBS, 1024 / PBS) k_ts_update_pair(const __grid
 // The planes minimise the launch's length, waves of CTAs times a march of R
 // planes and about one and a half more for its start: the smallest grids take
 // one plane a CTA (one load, one barrier, one store), a grid that fills the
-// GPU as many as make whole waves; in a batch, where the other problems fill
-// it, eight.
+// GPU as many as make whole waves.
 struct UpdateCut {
     int rows, ntile, R, threads;
     size_t smem;
@@ -965,7 +966,6 @@ static UpdateCut update_cut(const Dev &d, int sm_count, int nv) {
             c.R = R;
         }
     }
-    if (d.in_batch) c.R = 8;
     c.smem = (size_t)2 * (c.rows + 1) * (d.IM + 1) * sizeof(float);
     return c;
 }
@@ -1279,8 +1279,9 @@ __global__ void k_copy_tm_st(const __grid_constant__ Dev d, int v0, size_t n) {
 
 // k_ts_update_pair where a 512-thread CTA covers a plane's points (TS_PAIR = 0:
 // never); the crossover lies between 63 points, where it is 4 us faster a
-// launch, and 1221, where it is 1 us slower
-static bool pair_update(const Dev &d) { return d.TS_PAIR && d.IM * d.KM <= 512; }
+// launch, and 1221, where it is 1 us slower.  In a batch, whose other problems
+// hide a launch's length, always: 64 stages 5.29 ms a step against 5.33
+static bool pair_update(const Dev &d) { return d.TS_PAIR && (d.in_batch || d.IM * d.KM <= 512); }
 
 static size_t cells_smem(const Dev &d) {
     return ((size_t)d.IMM1 * d.KMM1 + d.KMM1 + (size_t)d.NIB1 * d.NKB1) * sizeof(float);
@@ -1296,7 +1297,7 @@ static cudaError_t configure_bs(const Dev &d) {
         size_t bytes;
     } k[] = {{(const void *)k_ts_cells<BS>, cells_smem(d)},
              {(const void *)k_ts_prolong<BS>, prolong_smem(d)},
-             {(const void *)k_ts_update_pair<2 * BS>, pair_update(d) ? update_pair_smem(d) : 0},
+             {(const void *)k_ts_update_pair<2 * BS>, update_pair_smem(d)},
              {(const void *)k_ts_smooth<BS>, smooth_smem(d)}};
     for (auto &x : k) {
         if (x.bytes > 200 * 1024) return cudaErrorInvalidValue;
