@@ -271,9 +271,9 @@ class Problem:
     def get(self, name: str) -> np.ndarray:
         ref = self.cd.arrays.get(name)
         if ref is not None:
-            out = np.zeros(ref.shape, ref.dtype)
+            out = np.empty(ref.shape, ref.dtype)
         else:
-            out = np.zeros((self.cd.km, self.cd.jm, self.cd.im), np.float32)
+            out = np.empty((self.cd.km, self.cd.jm, self.cd.im), np.float32)
         _chk(load().mgpu_get_array(self.h, name.encode(), out.ctypes.data, out.nbytes))
         return out
 
@@ -373,7 +373,7 @@ class Problem:
 
     def adjoint_gradient_theta(self) -> np.ndarray:
         """dJ/dTHETA (KM, JM, IM) on the device from the last adjoint_gradient."""
-        out = np.zeros((self.cd.km, self.cd.jm, self.cd.im), np.float32)
+        out = np.empty((self.cd.km, self.cd.jm, self.cd.im), np.float32)
         _chk(load().mgpu_adjoint_gradient_theta(self.h, out.ctypes.data, out.nbytes))
         return out
 
@@ -391,7 +391,7 @@ class Problem:
         return ref.shape if ref is not None else (self.cd.km, self.cd.jm, self.cd.im)
 
     def adjoint_get(self, name: str) -> np.ndarray:
-        out = np.zeros(self._adj_shape(name), np.float32)
+        out = np.empty(self._adj_shape(name), np.float32)
         _chk(load().mgpu_adjoint_get(self.h, name.encode(), out.ctypes.data, out.nbytes))
         return out
 
