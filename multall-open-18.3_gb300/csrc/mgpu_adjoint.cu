@@ -43,8 +43,8 @@ struct AdjVar {
     float *XF, *TF, *RF, *SR;    // face fluxes and source
     float *ST;                   // cell changes after prolongation
     float *TM;                   // node values before SMOOTH_VAR
-    float *Y;                    // ST * RSTEP: the restriction operand of the transposed prolongation
-    float *P1, *P2;              // per-plane block partials of Y
+    float *P1, *P2;              // per-plane block partials of Y = ST * RSTEP, the restriction operand of the
+                                 // transposed prolongation
     df *psum;                    // (JM) per-plane sums of Y (double-float)
     double *pblk;                // (JM) per-plane sums of dJ/d(row mean |STORE|)
     const float *tST;            // recorded STORE after prolongation
@@ -1128,42 +1128,10 @@ __global__ void rk_mach(const Dev d, const Adj a) {
 // redistribution, SCREE, flux sum)
 // =====================================================================
 
-__device__ inline int mp_role_r(const Dev &d, int j, int *nr) {
-    for (int r = 1; r <= d.NRWSM1; ++r) {
-        int jx = A1(d.JMIX, r);
-        if (j == jx) { *nr = r; return 1; }
-        if (j == jx + 1) { *nr = r; return 2; }
-        if (j == jx + 2) { *nr = r; return 3; }
-    }
-    *nr = 0;
-    return 0;
-}
-__device__ inline int stream_case_r(const Dev &d, int j) {
-    int nr = A1(d.NROW, j);
-    int J1 = A1(d.JSTART, nr), J2 = A1(d.JMIX, nr);
-    int sc = 0;
-    if (j >= J1 + 3 && j <= J2 - 3) sc = 1;
-    if (j == J2) sc = 0;
-    if (j == J1) sc = 0;
-    if (j == J1 + 2) sc = 2;
-    if (j == J1 + 1) sc = 3;
-    if (j == J2 - 2) sc = 4;
-    if (j == J2 - 1) sc = 5;
-    return sc;
-}
-__device__ inline int le_case_r(const Dev &d, int j) {
-    int lc = 0;
-    for (int r = 1; r <= d.NROWS; ++r) {
-        int JL = A1(d.JLED, r);
-        if (j == JL - 2 || j == JL - 1) lc = 1;
-        if (j == JL) lc = 2;
-    }
-    return lc;
-}
 // the mixing-plane row of cell plane jc at K is averaged (1750, 1850)
-__device__ inline bool mp_row_on(const Dev &d, const Adj &a, int role, int mnr, int k) {
+__device__ inline bool mp_row_on(const Dev &d, const Adj &a, int role, int jmx, int k) {
     const bool lowx = d.FEXTRAP < 0.001f;
-    const float FLOWDIRN = -A3(a.tFLOWX, d.IMID, A1(d.JMIX, mnr), k);
+    const float FLOWDIRN = -A3(a.tFLOWX, d.IMID, jmx, k);
     return role == 3 ? (FLOWDIRN > 0.0f || lowx) : (FLOWDIRN < 0.0f || lowx);
 }
 
@@ -1173,20 +1141,27 @@ __global__ void __launch_bounds__(RT_BS) rk_ts_smooth(const __grid_constant__ De
     const int IM = d.IM, KM = d.KM, IMM1 = d.IMM1, KMM1 = d.KMM1;
     const int np = IM * KM;
     float *A_ = sm, *B_ = sm + np, *C_ = sm + 2 * np;
+    float *cFD = sm + 3 * np, *cFU = cFD + IM, *cFKD = cFU + IM, *cFKU = cFKD + KM;   // FD, FU, FKD, FKU
     const int j = blockIdx.x + 1;
+    const PlaneInfo &pl = d.PLANE[j - 1];
+    for (int t = threadIdx.x; t < IM; t += RT_BS) {
+        cFD[t] = d.FD[t];
+        cFU[t] = d.FU[t];
+    }
+    for (int t = threadIdx.x; t < KM; t += RT_BS) {
+        cFKD[t] = d.FKD[t];
+        cFKU[t] = d.FKU[t];
+    }
     const DevCtl *c = a.tctl;
     const size_t ks = (size_t)IM * d.JM;
 #define P(buf, i, k) buf[((i) - 1) + IM * ((k) - 1)]
-    for (int t = threadIdx.x; t < np; t += RT_BS) {
-        const int i = t % IM + 1, k = t / IM + 1;
+    for (Walk2 w(IM, threadIdx.x, RT_BS); w.t() < np; w.next()) {
+        const int i = w.i, k = w.k, t = w.t();
         A_[t] = A3(V.D, i, j, k);
     }
     __syncthreads();
     // mixing-plane average of the variable (100)
-    bool mp = false;
-    if (d.IFMIX != 0)
-        for (int r = 1; r <= d.NRWSM1; ++r)
-            if (j == A1(d.JMIX, r) || j == A1(d.JMIX, r) + 1) mp = true;
+    const bool mp = pl.mix != 0;
     if (mp) {
         for (int k = threadIdx.x + 1; k <= KM; k += RT_BS) {
             float s = 0.0f;
@@ -1194,24 +1169,17 @@ __global__ void __launch_bounds__(RT_BS) rk_ts_smooth(const __grid_constant__ De
             B_[k - 1] = s;
         }
         __syncthreads();
-        for (int t = threadIdx.x; t < np; t += RT_BS) {
-            const int i = t % IM + 1, k = t / IM + 1;
+        for (Walk2 w(IM, threadIdx.x, RT_BS); w.t() < np; w.next()) {
+            const int i = w.i, k = w.k, t = w.t();
             A_[t] = 0.5f * B_[k - 1] * ((i <= IMM1 ? A1(d.FP, i) : 0.0f) + (i >= 2 ? A1(d.FP, i - 1) : 0.0f));
         }
         __syncthreads();
     }
     // tip-gap and periodic averaging of I=1 and I=IM (510, 8000)
-    const bool periodic_j = !(A1(d.IND, j) == 1 || A1(d.INDLE, j) == 1);
+    const bool periodic_j = pl.periodic != 0;
     {
-        int nr = A1(d.NROW, j);
-        int K1 = A1(d.KTIPS, nr), K2 = A1(d.KTIPE, nr);
-        const bool tip = K1 > 0;
-        if (tip) {
-            if (K1 == 1) K2 = K2 - 1;
-            if (K2 == KM) K1 = K1 + 1;
-        }
         for (int k = threadIdx.x + 1; k <= KM; k += RT_BS) {
-            if (tip && k >= K1 && k <= K2) {
+            if (k >= pl.tip1 && k <= pl.tip2) {
                 float v = 0.5f * (P(A_, 1, k) + P(A_, IM, k));
                 P(A_, 1, k) = v;
                 P(A_, IM, k) = v;
@@ -1251,44 +1219,44 @@ __global__ void __launch_bounds__(RT_BS) rk_ts_smooth(const __grid_constant__ De
         // interior m, read by the smoothed values at m-1 and m+1.
         const float h = SFT * F4;
         // spanwise: A_ = adjoint of its output; B_ = curvature adjoints
-        for (int t = threadIdx.x; t < np; t += RT_BS) {
-            const int i = t % IM + 1, k = t / IM + 1;
+        for (Walk2 w(IM, threadIdx.x, RT_BS); w.t() < np; w.next()) {
+            const int i = w.i, k = w.k, t = w.t();
             float cb = 0.0f;
             if (k >= 2 && k <= KMM1) {
-                if (k + 1 <= KMM1) cb += A1(d.FKU, k + 1) * P(A_, i, k + 1);
-                if (k - 1 >= 2) cb += A1(d.FKD, k - 1) * P(A_, i, k - 1);
+                if (k + 1 <= KMM1) cb += cFKU[k + 1 - 1] * P(A_, i, k + 1);
+                if (k - 1 >= 2) cb += cFKD[k - 1 - 1] * P(A_, i, k - 1);
             }
             B_[t] = h * cb;
         }
         __syncthreads();
         // C_ = adjoint of the pitchwise output
-        for (int t = threadIdx.x; t < np; t += RT_BS) {
-            const int i = t % IM + 1, k = t / IM + 1;
+        for (Walk2 w(IM, threadIdx.x, RT_BS); w.t() < np; w.next()) {
+            const int i = w.i, k = w.k, t = w.t();
             float g = SFT1 * P(A_, i, k);
-            if (k - 1 >= 2 && k - 1 <= KMM1) g += SFT * A1(d.FKD, k - 1) * P(A_, i, k - 1);
-            if (k + 1 >= 2 && k + 1 <= KMM1) g += SFT * A1(d.FKU, k + 1) * P(A_, i, k + 1);
-            if (k == 2) g += SFT * P(A_, i, 1) * (1.0f + 0.5f * A1(d.FKU, 1));
-            if (k == 3) g -= SFT * P(A_, i, 1) * 0.5f * A1(d.FKU, 1);
-            if (k == KMM1) g += SFT * P(A_, i, KM) * (1.0f + 0.5f * A1(d.FKU, KM));
-            if (k == d.KMM2) g -= SFT * P(A_, i, KM) * 0.5f * A1(d.FKU, KM);
+            if (k - 1 >= 2 && k - 1 <= KMM1) g += SFT * cFKD[k - 1 - 1] * P(A_, i, k - 1);
+            if (k + 1 >= 2 && k + 1 <= KMM1) g += SFT * cFKU[k + 1 - 1] * P(A_, i, k + 1);
+            if (k == 2) g += SFT * P(A_, i, 1) * (1.0f + 0.5f * cFKU[1 - 1]);
+            if (k == 3) g -= SFT * P(A_, i, 1) * 0.5f * cFKU[1 - 1];
+            if (k == KMM1) g += SFT * P(A_, i, KM) * (1.0f + 0.5f * cFKU[KM - 1]);
+            if (k == d.KMM2) g -= SFT * P(A_, i, KM) * 0.5f * cFKU[KM - 1];
             if (k >= 2 && k <= KMM1) g += P(B_, i, k);
-            if (k - 1 >= 2 && k - 1 <= KMM1) g -= A1(d.FKD, k - 1) * P(B_, i, k - 1);
-            if (k + 1 >= 2 && k + 1 <= KMM1) g -= A1(d.FKU, k + 1) * P(B_, i, k + 1);
+            if (k - 1 >= 2 && k - 1 <= KMM1) g -= cFKD[k - 1 - 1] * P(B_, i, k - 1);
+            if (k + 1 >= 2 && k + 1 <= KMM1) g -= cFKU[k + 1 - 1] * P(B_, i, k + 1);
             C_[t] = g;
         }
         __syncthreads();
         // pitchwise: C_ = adjoint of its output; B_ = curvature adjoints, the
         // end curvature c(1) = c(IM) = a(1) - (a(2) + a(IMM1))/2 of a periodic
         // plane at I = 1 and IM
-        for (int t = threadIdx.x; t < np; t += RT_BS) {
-            const int i = t % IM + 1, k = t / IM + 1;
+        for (Walk2 w(IM, threadIdx.x, RT_BS); w.t() < np; w.next()) {
+            const int i = w.i, k = w.k, t = w.t();
             float cb = 0.0f;
             if (i >= 2 && i <= IMM1) {
-                if (i + 1 <= IMM1) cb += A1(d.FU, i + 1) * P(C_, i + 1, k);
-                if (i - 1 >= 2) cb += A1(d.FD, i - 1) * P(C_, i - 1, k);
+                if (i + 1 <= IMM1) cb += cFU[i + 1 - 1] * P(C_, i + 1, k);
+                if (i - 1 >= 2) cb += cFD[i - 1 - 1] * P(C_, i - 1, k);
             } else if (periodic_j) {
-                if (i == 1 && IMM1 >= 2) cb += A1(d.FU, 2) * P(C_, 2, k);
-                if (i == IM && IMM1 >= 2) cb += A1(d.FD, IMM1) * P(C_, IMM1, k);
+                if (i == 1 && IMM1 >= 2) cb += cFU[2 - 1] * P(C_, 2, k);
+                if (i == IM && IMM1 >= 2) cb += cFD[IMM1 - 1] * P(C_, IMM1, k);
             }
             if (periodic_j) {
                 const float e = 0.5f * (P(C_, 1, k) + P(C_, IM, k));
@@ -1298,24 +1266,24 @@ __global__ void __launch_bounds__(RT_BS) rk_ts_smooth(const __grid_constant__ De
             B_[t] = h * cb;
         }
         __syncthreads();
-        for (int t = threadIdx.x; t < np; t += RT_BS) {
-            const int i = t % IM + 1, k = t / IM + 1;
+        for (Walk2 w(IM, threadIdx.x, RT_BS); w.t() < np; w.next()) {
+            const int i = w.i, k = w.k, t = w.t();
             float g = SFT1 * P(C_, i, k);
-            if (i - 1 >= 2 && i - 1 <= IMM1) g += SFT * A1(d.FD, i - 1) * P(C_, i - 1, k);
-            if (i + 1 >= 2 && i + 1 <= IMM1) g += SFT * A1(d.FU, i + 1) * P(C_, i + 1, k);
+            if (i - 1 >= 2 && i - 1 <= IMM1) g += SFT * cFD[i - 1 - 1] * P(C_, i - 1, k);
+            if (i + 1 >= 2 && i + 1 <= IMM1) g += SFT * cFU[i + 1 - 1] * P(C_, i + 1, k);
             if (periodic_j) {
                 const float e = 0.5f * SFT * (P(C_, 1, k) + P(C_, IM, k));
                 if (i == 2) g += e;
                 if (i == IMM1) g += e;
             } else {
-                if (i == 2) g += SFT * P(C_, 1, k) * (1.0f + A1(d.FU, 1));
-                if (i == 3) g -= SFT * P(C_, 1, k) * A1(d.FU, 1);
-                if (i == IMM1) g += SFT * P(C_, IM, k) * (1.0f + A1(d.FU, IM));
-                if (i == d.IMM2) g -= SFT * P(C_, IM, k) * A1(d.FU, IM);
+                if (i == 2) g += SFT * P(C_, 1, k) * (1.0f + cFU[1 - 1]);
+                if (i == 3) g -= SFT * P(C_, 1, k) * cFU[1 - 1];
+                if (i == IMM1) g += SFT * P(C_, IM, k) * (1.0f + cFU[IM - 1]);
+                if (i == d.IMM2) g -= SFT * P(C_, IM, k) * cFU[IM - 1];
             }
             if (i >= 2 && i <= IMM1) g += P(B_, i, k);
-            if (i - 1 >= 2 && i - 1 <= IMM1) g -= A1(d.FD, i - 1) * P(B_, i - 1, k);
-            if (i + 1 >= 2 && i + 1 <= IMM1) g -= A1(d.FU, i + 1) * P(B_, i + 1, k);
+            if (i - 1 >= 2 && i - 1 <= IMM1) g -= cFD[i - 1 - 1] * P(B_, i - 1, k);
+            if (i + 1 >= 2 && i + 1 <= IMM1) g -= cFU[i + 1 - 1] * P(B_, i + 1, k);
             if (periodic_j) {
                 const float e = P(B_, 1, k) + P(B_, IM, k);
                 if (i == 1) g += e;
@@ -1328,10 +1296,8 @@ __global__ void __launch_bounds__(RT_BS) rk_ts_smooth(const __grid_constant__ De
     }
     // streamwise and leading-edge smoothing: scatter into TMP's adjoint
     const bool stream = !(c->SFX < 0.0001f);
-    const int sc = stream ? stream_case_r(d, j) : 0;
-    const int lc = stream ? le_case_r(d, j) : 0;
-    const int nr = A1(d.NROW, j);
-    const int J1 = A1(d.JSTART, nr), J2 = A1(d.JMIX, nr);
+    const int sc = stream ? pl.sc : 0, lc = stream ? pl.lc : 0;
+    const int J1 = pl.J1, J2 = pl.J2;
     const float SFX = c->SFX, SFX1 = c->SFX1, SFXB = c->SFXB, SFXB1 = c->SFXB1, SFXBH = c->SFXBH;
     const float SFXHM1 = c->SFXHM1, SFX14 = c->SFX14, F4 = d.FAC_4TH;
     int nq = 0, jq[4] = {0, 0, 0, 0};
@@ -1349,8 +1315,8 @@ __global__ void __launch_bounds__(RT_BS) rk_ts_smooth(const __grid_constant__ De
     case 5: c0 = SFXB1; addq(J2 - 2, 1.25f * SFXB); addq(J2 - 3, 0.5f * SFXB); addq(J2 - 4, -0.75f * SFXB); break;
     default: break;
     }
-    for (int t = threadIdx.x; t < np; t += RT_BS) {
-        const int i = t % IM + 1, k = t / IM + 1;
+    for (Walk2 w(IM, threadIdx.x, RT_BS); w.t() < np; w.next()) {
+        const int i = w.i, k = w.k, t = w.t();
         const float g = A_[t];
         if (g == 0.0f) continue;
         float *tm = V.TM + (size_t)(i - 1) + ks * (k - 1);     // tm[IM*(jj-1)] = TMP(i, jj, k)
@@ -1384,6 +1350,7 @@ __global__ void __launch_bounds__(RT_BS) rk_ts_gather(const __grid_constant__ De
     // the variable's own adjoint: D = TMP + gather, so dJ/dD(old) = dJ/dTMP
     {
         const int np = IM * d.KM;
+        WalkN w(IM, IM * d.JM, IM * (j - 1), threadIdx.x, RT_BS);
         for (int t0 = threadIdx.x; t0 < np; t0 += RT_U * RT_BS) {
             float v[RT_U];
             int o[RT_U];
@@ -1392,9 +1359,10 @@ __global__ void __launch_bounds__(RT_BS) rk_ts_gather(const __grid_constant__ De
                 const int t = t0 + u * RT_BS;
                 o[u] = -1;
                 if (t < np) {
-                    o[u] = ix3(d, t % IM + 1, j, t / IM + 1);
-                    v[u] = V.TM[o[u]];
+                    o[u] = w.n;
+                    v[u] = V.TM[w.n];
                 }
+                w.next();
             }
 #pragma unroll
             for (int u = 0; u < RT_U; ++u)
@@ -1405,25 +1373,30 @@ __global__ void __launch_bounds__(RT_BS) rk_ts_gather(const __grid_constant__ De
     const int jc = j;
     const int nc = IMM1 * KMM1;
     float *av = sm;
-    const float fdn = A1(d.FACDWN, jc), fup = A1(d.FACUP, jc);
+    const PlaneInfo &pl = d.PLANE[jc - 1];
+    const float fdn = pl.facdwn, fup = pl.facup;
+    const int ks = IM * d.JM;
+    const float *__restrict__ TMA = V.TM, *__restrict__ TMB = V.TM - IM;    // planes jc and jc - 1
     // RT_U cells at a time, their loads issued together
+    WalkN wn(IMM1, ks, IM * (jc - 1), threadIdx.x, RT_BS), ww(IMM1, IM, 0, threadIdx.x, RT_BS);
     for (int c0 = threadIdx.x; c0 < nc; c0 += RT_U * RT_BS) {
         float tA[RT_U][4], tB[RT_U][4], wt[RT_U][4];
 #pragma unroll
         for (int u = 0; u < RT_U; ++u) {
             const int c = c0 + u * RT_BS;
             if (c >= nc) continue;
-            const int i = c % IMM1 + 1, k = c / IMM1 + 1;
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
-                const int ii = i + (q & 1), kk = k + (q >> 1);   // (i,k) (i+1,k) (i,k+1) (i+1,k+1)
-                tA[u][q] = A3(V.TM, ii, jc, kk);
-                tB[u][q] = A3(V.TM, ii, jc - 1, kk);
+                const int n = wn.n + (q & 1) + ks * (q >> 1);        // (i,k) (i+1,k) (i,k+1) (i+1,k+1)
+                tA[u][q] = TMA[n];
+                tB[u][q] = TMB[n];
             }
-            wt[u][0] = AIK(d.FBL, i, k);
-            wt[u][1] = AIK(d.FBR, i, k);
-            wt[u][2] = AIK(d.FTL, i, k);
-            wt[u][3] = AIK(d.FTR, i, k);
+            wt[u][0] = d.FBL[ww.n];
+            wt[u][1] = d.FBR[ww.n];
+            wt[u][2] = d.FTL[ww.n];
+            wt[u][3] = d.FTR[ww.n];
+            wn.next();
+            ww.next();
         }
 #pragma unroll
         for (int u = 0; u < RT_U; ++u) {
@@ -1438,11 +1411,10 @@ __global__ void __launch_bounds__(RT_BS) rk_ts_gather(const __grid_constant__ De
     }
     __syncthreads();
     // second mixing-plane average (1850): a row set to its mean
-    int mnr;
-    const int role = mp_role_r(d, jc, &mnr);
+    const int role = pl.role;
     if (role == 1 || role == 3) {
         for (int k = threadIdx.x + 1; k <= KMM1; k += RT_BS) {
-            if (!mp_row_on(d, a, role, mnr, k)) continue;
+            if (!mp_row_on(d, a, role, pl.jmx, k)) continue;
             float *row = av + (size_t)(k - 1) * IMM1;
             float s = 0.0f;
             for (int i = 0; i < IMM1; ++i) s += row[i];
@@ -1456,8 +1428,9 @@ __global__ void __launch_bounds__(RT_BS) rk_ts_gather(const __grid_constant__ De
     const DevCtl *ctl = a.tctl;
     const int damp_on = ctl->damp_on;
     const float DAMP = ctl->DAMP;
-    const float blk = damp_on ? V.tBLK[A1(d.NROW, jc) - 1] : 1.0f;
+    const float blk = damp_on ? V.tBLK[pl.nrow - 1] : 1.0f;
     float pbf = 0.0f;             // FP32 per thread, FP64 across threads
+    wn = WalkN(IMM1, ks, IM * (jc - 1), threadIdx.x, RT_BS);
     for (int c0 = threadIdx.x; c0 < nc; c0 += RT_U * RT_BS) {
         float S[RT_U];
         int o[RT_U];
@@ -1467,9 +1440,10 @@ __global__ void __launch_bounds__(RT_BS) rk_ts_gather(const __grid_constant__ De
             o[u] = -1;
             S[u] = 0.0f;
             if (c < nc) {
-                o[u] = ix3(d, c % IMM1 + 1, jc, c / IMM1 + 1);
-                if (damp_on) S[u] = V.tST[o[u]];
+                o[u] = wn.n;
+                if (damp_on) S[u] = V.tST[wn.n];
             }
+            wn.next();
         }
 #pragma unroll
         for (int u = 0; u < RT_U; ++u) {
@@ -1497,12 +1471,15 @@ __global__ void __launch_bounds__(RT_BS) rk_ts_gather(const __grid_constant__ De
 }
 
 __global__ void __launch_bounds__(RT_BS) rk_ts_damp(const __grid_constant__ Dev d, const __grid_constant__ Adj a, int v0) {
-    __shared__ double shd[RT_BS / 32];
+    extern __shared__ float sm[];
     __shared__ float gchg[64], gblk[64];
     const AdjVar &V = a.v[v0 + blockIdx.y];
     const int IMM1 = d.IMM1, KMM1 = d.KMM1;
     const int j = blockIdx.x + 2;
     const int nc = IMM1 * KMM1;
+    float *sy = sm, *p1 = sm + nc;        // Y of this plane; its level-1 partial sums
+    const int n1 = d.NIB1 * d.NKB1, n2 = d.NIB2 * d.NKB2;
+    const int4 blk1 = d.MG1X[min((int)threadIdx.x, n1 - 1)], blk2 = d.MG2X[min((int)threadIdx.x, n2 - 1)];
     const DevCtl *ctl = a.tctl;
     const int NROWS = d.NROWS;
     float add = 0.0f;
@@ -1514,8 +1491,7 @@ __global__ void __launch_bounds__(RT_BS) rk_ts_damp(const __grid_constant__ Dev 
             const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
             for (int nr = w + 1; nr <= NROWS; nr += RT_BS / 32) {
                 double s = 0.0;
-                for (int jj = 2 + l; jj <= d.JM; jj += 32)
-                    if (A1(d.NROW, jj) == nr) s += V.pblk[jj - 1];
+                for (int jj = max(A1(d.JSTART, nr), 2) + l; jj <= A1(d.JMIX, nr); jj += 32) s += V.pblk[jj - 1];
                 for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
                 if (l == 0) {
                     gblk[nr - 1] = (float)s;
@@ -1545,12 +1521,11 @@ __global__ void __launch_bounds__(RT_BS) rk_ts_damp(const __grid_constant__ Dev 
             }
         }
         __syncthreads();
-        for (int nr = 1; nr <= NROWS; ++nr) {
-            const int JST = A1(d.JSTART, nr) + 1, JEN = A1(d.JMIX, nr) - 1;
-            if (j >= JST && j <= JEN) add = gchg[nr - 1] / (float)(IMM1 * KMM1 * (JEN - JST + 1));
-        }
+        const PlaneInfo &pl = d.PLANE[j - 1];
+        if (j > pl.J1 && j < pl.J2) add = gchg[pl.nrow - 1] / (float)(IMM1 * KMM1 * (pl.J2 - pl.J1 - 1));
     }
     float psf = 0.0f;             // FP32 per thread, FP64 across threads
+    WalkN w(IMM1, d.IM * d.JM, d.IM * (j - 1), threadIdx.x, RT_BS);
     for (int c0 = threadIdx.x; c0 < nc; c0 += RT_U * RT_BS) {
         float g[RT_U], ts[RT_U], rsp[RT_U];
         int o[RT_U];
@@ -1559,12 +1534,13 @@ __global__ void __launch_bounds__(RT_BS) rk_ts_damp(const __grid_constant__ Dev 
             const int c = c0 + u * RT_BS;
             o[u] = -1;
             if (c < nc) {
-                const int n = ix3(d, c % IMM1 + 1, j, c / IMM1 + 1);
+                const int n = w.n;
                 o[u] = n;
                 g[u] = V.ST[n];
                 ts[u] = add != 0.0f ? V.tST[n] : 0.0f;
                 rsp[u] = d.RSTEP[n];
             }
+            w.next();
         }
 #pragma unroll
         for (int u = 0; u < RT_U; ++u) {
@@ -1573,7 +1549,7 @@ __global__ void __launch_bounds__(RT_BS) rk_ts_damp(const __grid_constant__ Dev 
             if (add != 0.0f) gg += (ts[u] < 0.0f ? -add : add);
             V.ST[o[u]] = gg;
             const float y = gg * rsp[u];
-            V.Y[o[u]] = y;
+            sy[c0 + u * RT_BS] = y;
             psf += y;
         }
     }
@@ -1587,20 +1563,31 @@ __global__ void __launch_bounds__(RT_BS) rk_ts_damp(const __grid_constant__ Dev 
         for (int w = 0; w < RT_BS / 32; ++w) s = df_add(s, shdf[w]);
         V.psum[j - 1] = s;
     }
-    // level-1 and level-2 partial sums of Y over this plane
-    const int n1 = d.NIB1 * d.NKB1, n2 = d.NIB2 * d.NKB2;
-    for (int t = threadIdx.x; t < n1 + n2; t += RT_BS) {
-        const bool lv1 = t < n1;
-        const int u = lv1 ? t : t - n1;
-        const int nib = lv1 ? d.NIB1 : d.NIB2;
-        const int ib = u % nib + 1, kb = u / nib + 1;
-        const int i0 = lv1 ? A1(d.IB1_S, ib) : A1(d.IB2_S, ib), i1 = lv1 ? A1(d.IB1_E, ib) : A1(d.IB2_E, ib);
-        const int k0 = lv1 ? A1(d.KB1_S, kb) : A1(d.KB2_S, kb), k1 = lv1 ? A1(d.KB1_E, kb) : A1(d.KB2_E, kb);
+    // level-1 and level-2 partial sums of Y over this plane (behind the
+    // barrier above), the level-2 ones of the level-1 ones where they nest
+    auto block_cells = [&](int4 x) {
         float s = 0.0f;
-        for (int k = k0; k <= k1; ++k)
-            for (int i = i0; i <= i1; ++i) s += A3(V.Y, i, j, k);
-        if (lv1) V.P1[(size_t)(j - 1) * n1 + u] = s;
-        else V.P2[(size_t)(j - 1) * n2 + u] = s;
+        for (int k = x.z; k <= x.w; ++k)
+            for (int i = x.x; i <= x.y; ++i) s += sy[(k - 1) * IMM1 + (i - 1)];
+        return s;
+    };
+    float *P1 = V.P1 + (size_t)(j - 1) * n1, *P2 = V.P2 + (size_t)(j - 1) * n2;
+    for (int u = threadIdx.x; u < n1; u += RT_BS) {
+        const float s = block_cells(u < RT_BS ? blk1 : d.MG1X[u]);
+        p1[u] = s;
+        P1[u] = s;
+    }
+    __syncthreads();
+    for (int u = threadIdx.x; u < n2; u += RT_BS) {
+        const int4 x = u < RT_BS ? blk2 : d.MG2X[u];
+        float s = 0.0f;
+        if (d.mg_nested) {
+            for (int kb = x.z; kb <= x.w; ++kb)
+                for (int ib = x.x; ib <= x.y; ++ib) s += p1[(kb - 1) * d.NIB1 + (ib - 1)];
+        } else {
+            s = block_cells(x);
+        }
+        P2[u] = s;
     }
 }
 
@@ -1613,68 +1600,64 @@ __global__ void __launch_bounds__(RT_BS) rk_ts_cells(const __grid_constant__ Dev
     const int nc = IMM1 * KMM1;
     const int n1 = d.NIB1 * d.NKB1, n2 = d.NIB2 * d.NKB2;
     float *b1 = sm, *b2 = sm + n1, *st = sm + n1 + n2, *rs = st + nc;
-    const int j1 = A1(d.JB1, j), j2 = A1(d.JB2, j), jsb = A1(d.JSBLK, j);
-    const size_t m1 = (size_t)d.NIB1 * (d.NJB1 + 1), m2 = (size_t)d.NIB2 * (d.NJB2 + 1);
+    const PlaneInfo &pl = d.PLANE[j - 1];
+    const int m1 = d.NIB1 * (d.NJB1 + 1), m2 = d.NIB2 * (d.NJB2 + 1);
+    const bool nested = d.mg_nested != 0;
+    const int ks = IM * d.JM, n0 = IM * (j - 1);
+    // each block's sum by its step, once per block, and the levels added up
+    // once per level-1 block where they nest, as in k_ts_prolong
     for (int t = threadIdx.x; t < n1; t += RT_BS) {
+        const float st1 = d.STEP1[t % d.NIB1 + d.NIB1 * (pl.jb1 - 1) + m1 * (t / d.NIB1)];
         float s = 0.0f;
-        if (j1 <= d.NJB1)
-            for (int jj = A1(d.JB1_START, j1); jj <= A1(d.JB1_END, j1); ++jj) s += V.P1[(size_t)(jj - 1) * n1 + t];
-        b1[t] = s;
+        for (int jj = pl.a1; jj <= pl.e1; ++jj) s += V.P1[(size_t)(jj - 1) * n1 + t];
+        b1[t] = s * st1;
     }
     for (int t = threadIdx.x; t < n2; t += RT_BS) {
+        const float st2 = d.STEP2[t % d.NIB2 + d.NIB2 * (pl.jb2 - 1) + m2 * (t / d.NIB2)];
         float s = 0.0f;
-        if (j2 <= d.NJB2)
-            for (int jj = A1(d.JB2_START, j2); jj <= A1(d.JB2_END, j2); ++jj) s += V.P2[(size_t)(jj - 1) * n2 + t];
-        b2[t] = s;
+        for (int jj = pl.a2; jj <= pl.e2; ++jj) s += V.P2[(size_t)(jj - 1) * n2 + t];
+        b2[t] = s * st2;
     }
     if (threadIdx.x < 32) {
-        const int a0 = A1(d.SB_START, jsb), b0 = A1(d.SB_END, jsb);
         df s = df_of(0.0f);
-        for (int jj = a0 + (int)threadIdx.x; jj <= b0; jj += 32) s = df_add(s, V.psum[jj - 1]);
+        for (int jj = pl.sa + (int)threadIdx.x; jj <= pl.se; jj += 32) s = df_add(s, V.psum[jj - 1]);
         for (int o = 16; o > 0; o >>= 1) s = df_add(s, df_shfl_down(s, o));
         if (threadIdx.x == 0) s_sb = df_val(s);
     }
     __syncthreads();
-    const float SB = s_sb, SSB = A1(d.STEPSBK, jsb);
-    // RT_U cells at a time: their block indices, then their operands, are
-    // loaded together
+    const float SB = s_sb * pl.stepsbk;
+    if (nested) {
+        for (int t = threadIdx.x; t < n1; t += RT_BS) b1[t] = b1[t] + b2[d.MG12[t]] + SB;
+        __syncthreads();
+    }
+    // RT_U cells at a time, their operands loaded together
+    WalkN w(IMM1, ks, n0, threadIdx.x, RT_BS);
     for (int c0 = threadIdx.x; c0 < nc; c0 += RT_U * RT_BS) {
-        int i1[RT_U], i2[RT_U], k1[RT_U], k2[RT_U], nn[RT_U];
-        float vs[RT_U], vp[RT_U], v1[RT_U], v2[RT_U];
+        float vs[RT_U], vp[RT_U];
+        int u1[RT_U], u2[RT_U];
 #pragma unroll
         for (int u = 0; u < RT_U; ++u) {
             const int c = c0 + u * RT_BS;
-            if (c >= nc) continue;
-            const int i = c % IMM1 + 1, k = c / IMM1 + 1;
-            nn[u] = ix3(d, i, j, k);
-            i1[u] = A1(d.IB1, i); i2[u] = A1(d.IB2, i); k1[u] = A1(d.KB1, k); k2[u] = A1(d.KB2, k);
+            if (c < nc) {
+                vs[u] = V.ST[w.n];
+                vp[u] = d.STEP[w.n];
+                u1[u] = d.CB1[c];
+                u2[u] = nested ? 0 : d.CB2[c];
+            }
+            w.next();
         }
 #pragma unroll
         for (int u = 0; u < RT_U; ++u) {
             const int c = c0 + u * RT_BS;
-            if (c >= nc) continue;
-            const size_t s1 = (size_t)(i1[u] - 1) + (size_t)d.NIB1 * (j1 - 1) + m1 * (k1[u] - 1);
-            const size_t s2 = (size_t)(i2[u] - 1) + (size_t)d.NIB2 * (j2 - 1) + m2 * (k2[u] - 1);
-            vs[u] = V.ST[nn[u]];
-            vp[u] = d.STEP[nn[u]];
-            v1[u] = d.STEP1[s1];
-            v2[u] = d.STEP2[s2];
-        }
-#pragma unroll
-        for (int u = 0; u < RT_U; ++u) {
-            const int c = c0 + u * RT_BS;
-            if (c >= nc) continue;
-            st[c] = vs[u] * vp[u] + b1[(k1[u] - 1) * d.NIB1 + (i1[u] - 1)] * v1[u] +
-                    b2[(k2[u] - 1) * d.NIB2 + (i2[u] - 1)] * v2[u] + SB * SSB;
+            if (c < nc) st[c] = vs[u] * vp[u] + (nested ? b1[u1[u]] : b1[u1[u]] + b2[u2[u]] + SB);
         }
     }
     __syncthreads();
     // mixing-plane pitchwise redistribution (1750): row <- (sum of row) FP(I)
-    int mnr;
-    const int role = mp_role_r(d, j, &mnr);
+    const int role = pl.role;
     if (role == 1 || role == 3) {
         for (int k = threadIdx.x + 1; k <= KMM1; k += RT_BS) {
-            if (!mp_row_on(d, a, role, mnr, k)) continue;
+            if (!mp_row_on(d, a, role, pl.jmx, k)) continue;
             float *row = st + (size_t)(k - 1) * IMM1;
             float s = 0.0f;
             for (int i = 1; i <= IMM1; ++i) s += row[i - 1] * A1(d.FP, i);
@@ -1683,11 +1666,10 @@ __global__ void __launch_bounds__(RT_BS) rk_ts_cells(const __grid_constant__ Dev
         __syncthreads();
     }
     // SCREE: STORE = F1 DELTA + F2 DIFF, DIFF = DELTA + F3 DIFF; then the flux sum
-    const float RATPITCH = (float)A1(d.NBLADE, j - 1) / (float)A1(d.NBLADE, j);
-    const int nr = A1(d.NROW, j);
-    const int kts = A1(d.KTIPS, nr), kte = A1(d.KTIPE, nr);
+    const float RATPITCH = pl.ratpitch;
+    const int kts = pl.kts, kte = pl.kte;
     const bool lowx = d.FEXTRAP < 0.001f;
-    const int jmx = role ? A1(d.JMIX, mnr) : 0;
+    const int jmx = pl.jmx;
     const float F1 = d.F1, F2 = d.F2, F3 = d.F3;
     for (int k = threadIdx.x; k < KMM1; k += RT_BS) rs[k] = 0.0f;
     __syncthreads();
@@ -1735,22 +1717,25 @@ __global__ void __launch_bounds__(RT_BS) rk_ts_cells(const __grid_constant__ Dev
         }
         if (plain) aadd(&V.SR[n], gsrc);
     };
+    w = WalkN(IMM1, ks, n0, threadIdx.x, RT_BS);
     for (int c0 = threadIdx.x; c0 < nc; c0 += RT_U * RT_BS) {
         float gd[RT_U];
-        int o[RT_U];
+        int o[RT_U], ci[RT_U];
 #pragma unroll
         for (int u = 0; u < RT_U; ++u) {
             const int c = c0 + u * RT_BS;
             o[u] = -1;
             if (c < nc) {
-                o[u] = ix3(d, c % IMM1 + 1, j, c / IMM1 + 1);
-                gd[u] = V.DIFF[o[u]];
+                o[u] = w.n;
+                ci[u] = w.i;
+                gd[u] = V.DIFF[w.n];
             }
+            w.next();
         }
 #pragma unroll
         for (int u = 0; u < RT_U; ++u) {
             const int c = c0 + u * RT_BS;
-            if (o[u] >= 0) cell(c, c % IMM1 + 1, c / IMM1 + 1, o[u], gd[u]);
+            if (o[u] >= 0) cell(c, ci[u] + 1, (o[u] - n0 - ci[u]) / ks + 1, o[u], gd[u]);
         }
     }
     __syncthreads();
@@ -2167,18 +2152,19 @@ int aalloc(AdjState *s, T **p, size_t count) {
     return 0;
 }
 
-size_t smooth_bytes(const Dev &d) { return (size_t)3 * d.IM * d.KM * sizeof(float); }
+size_t smooth_bytes(const Dev &d) { return ((size_t)3 * d.IM * d.KM + 2 * (d.IM + d.KM)) * sizeof(float); }
 size_t gather_bytes(const Dev &d) { return (size_t)d.IMM1 * d.KMM1 * sizeof(float); }
 size_t cells_bytes(const Dev &d) {
     return ((size_t)d.NIB1 * d.NKB1 + (size_t)d.NIB2 * d.NKB2 + (size_t)d.IMM1 * d.KMM1 + d.KMM1) * sizeof(float);
 }
 
+size_t damp_bytes(const Dev &d) { return ((size_t)d.IMM1 * d.KMM1 + (size_t)d.NIB1 * d.NKB1) * sizeof(float); }
 int configure(const Dev &d) {
     struct {
         const void *f;
         size_t b;
     } k[] = {{(const void *)rk_ts_smooth, smooth_bytes(d)}, {(const void *)rk_ts_gather, gather_bytes(d)},
-             {(const void *)rk_ts_cells, cells_bytes(d)}};
+             {(const void *)rk_ts_damp, damp_bytes(d)}, {(const void *)rk_ts_cells, cells_bytes(d)}};
     for (auto &x : k) {
         if (x.b > 200 * 1024) return api_fail(MGPU_E_UNSUPPORTED, "J-plane too large for the adjoint kernels");
         ACK(raise_smem(x.f, x.b));
@@ -2192,7 +2178,7 @@ void launch_tstep_rev(const Dev &d, const Adj &a, cudaStream_t s, int v0, int nv
     const unsigned ja = (unsigned)d.JM, jp = (unsigned)(d.JM - 1);
     rk_ts_smooth<<<dim3(ja, nv), RT_BS, smooth_bytes(d), s>>>(d, a, v0);
     rk_ts_gather<<<dim3(ja, nv), RT_BS, gather_bytes(d), s>>>(d, a, v0);
-    rk_ts_damp<<<dim3(jp, nv), RT_BS, 0, s>>>(d, a, v0);
+    rk_ts_damp<<<dim3(jp, nv), RT_BS, damp_bytes(d), s>>>(d, a, v0);
     rk_ts_cells<<<dim3(jp, nv), RT_BS, cells_bytes(d), s>>>(d, a, v0);
 }
 
@@ -2247,7 +2233,7 @@ int allocate(AdjState *s, const Dev &d) {
     };
     for (int v = 0; v < NVAR; ++v) {
         AdjVar &V = a.v[v];
-        F(&V.D, N); F(&V.DIFF, N); F(&V.SR, N); F(&V.ST, N); F(&V.TM, N); F(&V.Y, N);
+        F(&V.D, N); F(&V.DIFF, N); F(&V.SR, N); F(&V.ST, N); F(&V.TM, N);
         if (v != V_RO) { F(&V.XF, N); F(&V.TF, N); F(&V.RF, N); }
         F(&V.P1, (size_t)d.JM * d.NIB1 * d.NKB1);
         F(&V.P2, (size_t)d.JM * d.NIB2 * d.NKB2);
@@ -2385,7 +2371,7 @@ int zero_adjoints(AdjState *s, const Dev &d, cudaStream_t st) {
     CopyList l;
     for (int v = 0; v < NVAR; ++v) {
         AdjVar &V = a.v[v];
-        float *z[] = {V.D, V.DIFF, V.SR, V.ST, V.TM, V.Y, V.XF, V.TF, V.RF};
+        float *z[] = {V.D, V.DIFF, V.SR, V.ST, V.TM, V.XF, V.TF, V.RF};
         for (float *p : z)
             if (p && p != a.FLOWX && p != a.FLOWT && p != a.FLOWR) l.add(p, nullptr, N);
     }

@@ -287,6 +287,49 @@ __device__ __forceinline__ bool last_cta(unsigned *ticket, unsigned n) {
     return true;
 }
 
+// (i, k) of the points t = start, start + stride, ... of an ni-wide plane,
+// 1-based, advanced without a division per point
+struct Walk2 {
+    int i, k, di, dk, ni;
+    __device__ int t() const { return i - 1 + ni * (k - 1); }
+    __device__ Walk2(int ni_, int start, int stride) : ni(ni_) {
+        i = start % ni_ + 1;
+        k = start / ni_ + 1;
+        di = stride % ni_;
+        dk = stride / ni_;
+    }
+    __device__ void next() {
+        i += di;
+        k += dk;
+        if (i > ni) {
+            i -= ni;
+            ++k;
+        }
+    }
+};
+
+// The same walk of a plane's points by their offset n in a node array, with
+// K stride ks and the plane's first point at n0
+struct WalkN {
+    int i, n, di, dn, dw, ni;
+    __device__ WalkN(int ni_, int ks, int n0, int start, int stride) : ni(ni_) {
+        const int k = start / ni_, dk = stride / ni_;
+        i = start - k * ni_;
+        n = n0 + i + ks * k;
+        di = stride - dk * ni_;
+        dn = di + ks * dk;
+        dw = ks - ni_;
+    }
+    __device__ void next() {
+        i += di;
+        n += dn;
+        if (i >= ni) {
+            i -= ni;
+            n += dw;
+        }
+    }
+};
+
 // Order-preserving key for "largest value, earliest index wins": the value
 // must be >= 0 (squares, absolute values); NaN counts as smallest.
 __device__ inline unsigned long long max_key(float v, size_t lin) {

@@ -83,48 +83,6 @@ __device__ inline float warp_sum64(int n, F term) {
     return df_val(s);
 }
 
-// (i, k) of the points t = start, start + stride, ... of an ni-wide plane,
-// 1-based, advanced without a division per point
-struct Walk2 {
-    int i, k, di, dk, ni;
-    __device__ Walk2(int ni_, int start, int stride) : ni(ni_) {
-        i = start % ni_ + 1;
-        k = start / ni_ + 1;
-        di = stride % ni_;
-        dk = stride / ni_;
-    }
-    __device__ void next() {
-        i += di;
-        k += dk;
-        if (i > ni) {
-            i -= ni;
-            ++k;
-        }
-    }
-};
-
-// The same walk of a plane's points by their offset n in a node array, with
-// K stride ks and the plane's first point at n0
-struct WalkN {
-    int i, n, di, dn, dw, ni;
-    __device__ WalkN(int ni_, int ks, int n0, int start, int stride) : ni(ni_) {
-        const int k = start / ni_, dk = stride / ni_;
-        i = start - k * ni_;
-        n = n0 + i + ks * k;
-        di = stride - dk * ni_;
-        dn = di + ks * dk;
-        dw = ks - ni_;
-    }
-    __device__ void next() {
-        i += di;
-        n += dn;
-        if (i >= ni) {
-            i -= ni;
-            n += dw;
-        }
-    }
-};
-
 // ---------------------------------------------------------------------
 // cells: 5503-5510 (tip gap), 5516-5555 (MP extrapolation), 1000 (flux
 // sum), 1750 (MP redistribution) and the multigrid partial sums
@@ -835,7 +793,6 @@ __global__ void __launch_bounds__(PBS, 1024 / PBS) k_ts_update_pair(const __grid
     const float *__restrict__ FTL = d.FTL;
     const float *__restrict__ FTR = d.FTR;
     const int nb0 = IM * (j0 - 1);
-    const int np = IM * KM;
     // one node of a node plane from its <= 8 cells (kc, h, ic), cA the cell
     // plane before it and cB the one after, added in the reference's order
     // (kc outer, then the plane, then ic); a cell outside the grid is
