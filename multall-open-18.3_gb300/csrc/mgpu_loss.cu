@@ -203,9 +203,9 @@ __global__ void __launch_bounds__(32) k_pwallgrad_smooth(const __grid_constant__
 // transition scans run one thread per column in the reference's order.
 // ---------------------------------------------------------------------
 constexpr int LK_W = 8;            // warps per CTA (K stride)
-constexpr int LK_NARR = 8;         // [K][32] arrays in shared memory (+ RAVG per K): 4 CTAs per SM at KM = 49
+constexpr int LK_NARR = 7;         // [K][32] arrays in shared memory (+ RAVG per K): 5 CTAs per SM at KM = 49
 
-__global__ void __launch_bounds__(32 * LK_W) k_loss_kfaces(const __grid_constant__ Dev d, int init_call) {
+__global__ void __launch_bounds__(32 * LK_W, 5) k_loss_kfaces(const __grid_constant__ Dev d, int init_call) {
     pdl_wait();
     const DevCtl *c = d.ctl;
     if (!init_call && !c->do_loss) return;
@@ -217,8 +217,8 @@ __global__ void __launch_bounds__(32 * LK_W) k_loss_kfaces(const __grid_constant
     const bool col = i <= d.IMM1;
     // [K][32] arrays, row k-1
     float *AREA = lsm, *VXAVG = AREA + KM * 32, *VRAVG = VXAVG + KM * 32, *VTAVG = VRAVG + KM * 32;
-    float *ROAVG = VTAVG + KM * 32, *TAVG = ROAVG + KM * 32;
-    float *VLAM = TAVG + KM * 32, *VTURB = VLAM + KM * 32, *RAVGK = VTURB + KM * 32;   // RAVGK: [K] only
+    float *TAVG = VTAVG + KM * 32, *VLAM = TAVG + KM * 32, *VTURB = VLAM + KM * 32, *RAVGK = VTURB + KM * 32;
+    float *ROAVG = VTURB;        // until step 4 turns each face's density into its viscosity; RAVGK: [K] only
     __shared__ float s_vis[32], s_ftc[32], s_tw1[32], s_twm[32];
     __shared__ float s_w1[32][4], s_wm[32][4];     // wall-face xs, rs, ts, wv at K=1 and K=KM
 #define LK(a, k) a[((k) - 1) * 32 + tx]
@@ -227,6 +227,7 @@ __global__ void __launch_bounds__(32 * LK_W) k_loss_kfaces(const __grid_constant
     const int NRW = A1(d.NROW, j);
     const float WREL = A1(d.WRAD, j), WHUB = A1(d.WHUB, j), WTIP = A1(d.WTIP, j);
     // 1. face averages
+#pragma unroll 2
     for (int k = ty + 1; k <= KM; k += LK_W) {
         float RAVG = 0.5f * (A2(d.R, j, k) + A2(d.R, j - 1, k));
         if (tx == 0) RAVGK[k - 1] = RAVG;
@@ -323,8 +324,7 @@ __global__ void __launch_bounds__(32 * LK_W) k_loss_kfaces(const __grid_constant
     // 4. laminar and mixing-length viscosities of the interior faces.  The
     //    relative speed of the faces is formed again here, and Y_PLUS is read
     //    back from this CTA's own stores of step 3 (visible after the
-    //    barrier): two K-arrays fewer in shared memory lets four CTAs share
-    //    an SM
+    //    barrier): K-arrays fewer in shared memory let five CTAs share an SM
     auto wabs = [&](int kq) {
         float WTAVG = LK(VTAVG, kq) - WREL * RAVGK[kq - 1];
         return sqrtf(LK(VXAVG, kq) * LK(VXAVG, kq) + LK(VRAVG, kq) * LK(VRAVG, kq) + WTAVG * WTAVG);
