@@ -96,17 +96,19 @@ struct mgpu_handle {
     AdjState *adj = nullptr;     // discrete adjoint, after mgpu_adjoint_prepare
 };
 
-// A batch: one CUDA graph whose branches are the step graphs of several
-// handles, forked from and joined back to the batch's own stream.
+// A batch: CUDA graphs whose branches are the step graphs of several handles,
+// forked from and joined back to the batch's own stream.
 struct mgpu_batch {
     std::vector<mgpu_handle *> hs;
     int device = 0;
     cudaStream_t stream = nullptr;
     cudaEvent_t fork = nullptr;
     std::vector<cudaEvent_t> joins;
-    cudaGraph_t graph = nullptr;
-    cudaGraphExec_t gexec = nullptr;
-    size_t graph_nodes = 0;
+    // a step that is of one kind for every member (as mgpu_handle::sg), and
+    // one in which each member's own flags decide
+    StepGraph sg[4], mixed;
+    DevCtl **d_list = nullptr;   // the members' control blocks, their copies and the host's
+    DevCtl *d_ctl = nullptr, *h_ctl = nullptr;
     void *flush_buf = nullptr;
     size_t flush_bytes = 0;
 };
@@ -387,19 +389,19 @@ int add_conditional(mgpu_handle *h, cudaGraphConditionalHandle hnd, F fn) {
 // the control block; their kernels still test the device's own flags.
 // what < 0: the LOSS and tail kernels sit in conditional bodies that the
 // step-control kernel switches on only on the steps that need them.
-int capture_step(mgpu_handle *h, int what) {
+int capture_step(mgpu_handle *h, int what, bool in_batch) {
     cudaStreamCaptureStatus st;
     cudaGraph_t cg = nullptr;
     CK(cudaStreamGetCaptureInfo(h->stream, &st, nullptr, &cg, nullptr, nullptr, nullptr));
     cudaGraphConditionalHandle hl = 0, ht = 0;
     Dev dg = h->d;
+    dg.in_batch = in_batch ? 1 : 0;
     if (what < 0) {
         // every handle of a graph belongs to one conditional node: an inviscid
         // problem (ILOS = 0), which has no LOSS node, creates no LOSS handle
         if (h->d.ILOS != 0) CK(cudaGraphConditionalHandleCreate(&hl, cg, 0, cudaGraphCondAssignDefault));
         CK(cudaGraphConditionalHandleCreate(&ht, cg, 0, cudaGraphCondAssignDefault));
         dg.use_cond = 1;
-        dg.in_batch = 1;
         dg.cond_loss = (unsigned long long)hl;
         dg.cond_tail = (unsigned long long)ht;
     }
@@ -439,7 +441,7 @@ int build_graph(mgpu_handle *h, int what) {
     StepGraph &G = h->sg[what];
     if (G.exec) return 0;
     CK(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
-    int rc = capture_step(h, what);
+    int rc = capture_step(h, what, false);
     cudaGraph_t g = nullptr;
     cudaError_t e = cudaStreamEndCapture(h->stream, &g);
     if (rc) {
@@ -1607,12 +1609,55 @@ int32_t mgpu_profile_steps(mgpu_handle *h, int32_t nsteps, mgpu_kernel_time *out
     return 0;
 }
 
+namespace {
+
+// the batch's graph of a step of kind `what` (-1: mixed)
+int batch_graph(mgpu_batch *b, int what) {
+    StepGraph &G = what < 0 ? b->mixed : b->sg[what];
+    if (G.exec) return 0;
+    CK(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
+    int rc = 0;
+    cudaError_t e = cudaEventRecord(b->fork, b->stream);
+    for (size_t i = 0; i < b->hs.size() && !rc && e == cudaSuccess; ++i) {
+        mgpu_handle *h = b->hs[i];
+        e = cudaStreamWaitEvent(h->stream, b->fork, 0);
+        if (e != cudaSuccess) break;
+        rc = capture_step(h, what, true);
+        if (rc) break;
+        e = cudaEventRecord(b->joins[i], h->stream);
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(b->stream, b->joins[i], 0);
+    }
+    cudaGraph_t g = nullptr;
+    cudaError_t e2 = cudaStreamEndCapture(b->stream, &g);
+    if (rc || e != cudaSuccess || e2 != cudaSuccess) {
+        if (g) cudaGraphDestroy(g);
+        if (rc) return rc;
+        return fail(MGPU_E_CUDA, std::string("batch capture: ") + cudaGetErrorString(e != cudaSuccess ? e : e2));
+    }
+    G.graph = g;
+    CK(cudaGraphInstantiate(&G.exec, g, 0));
+    return 0;
+}
+
+// the control blocks of a batch side by side, for one copy to the host
+__global__ void k_gather_ctl(DevCtl *const *list, DevCtl *out) {
+    static_assert(sizeof(DevCtl) % sizeof(int) == 0, "copied by words");
+    const int *src = (const int *)list[blockIdx.x];
+    int *dst = (int *)(out + blockIdx.x);
+    for (int t = threadIdx.x; t < (int)(sizeof(DevCtl) / sizeof(int)); t += blockDim.x) dst[t] = src[t];
+}
+
+}  // namespace
+
 void mgpu_batch_destroy(mgpu_batch *b) {
     if (!b) return;
     if (b->stream) cudaStreamSynchronize(b->stream);
     if (b->flush_buf) cudaFree(b->flush_buf);
-    if (b->gexec) cudaGraphExecDestroy(b->gexec);
-    if (b->graph) cudaGraphDestroy(b->graph);
+    for (StepGraph &G : b->sg) G.drop();
+    b->mixed.drop();
+    if (b->d_list) cudaFree(b->d_list);
+    if (b->d_ctl) cudaFree(b->d_ctl);
+    if (b->h_ctl) cudaFreeHost(b->h_ctl);
     for (cudaEvent_t e : b->joins)
         if (e) cudaEventDestroy(e);
     if (b->fork) cudaEventDestroy(b->fork);
@@ -1645,41 +1690,39 @@ int32_t mgpu_batch_create(mgpu_handle *const *handles, int32_t n, mgpu_batch **o
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming);
     for (int i = 0; i < n && e == cudaSuccess; ++i) e = cudaEventCreateWithFlags(&b->joins[i], cudaEventDisableTiming);
     if (e != cudaSuccess) return bail(fail(MGPU_E_CUDA, std::string("mgpu_batch_create: ") + cudaGetErrorString(e)));
-    e = cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal);
-    if (e != cudaSuccess) return bail(fail(MGPU_E_CUDA, std::string("batch capture: ") + cudaGetErrorString(e)));
-    int rc = 0;
-    e = cudaEventRecord(b->fork, b->stream);
-    for (int i = 0; i < n && !rc && e == cudaSuccess; ++i) {
-        mgpu_handle *h = b->hs[i];
-        e = cudaStreamWaitEvent(h->stream, b->fork, 0);
-        if (e != cudaSuccess) break;
-        rc = capture_step(h, -1);
-        if (rc) break;
-        e = cudaEventRecord(b->joins[i], h->stream);
-        if (e == cudaSuccess) e = cudaStreamWaitEvent(b->stream, b->joins[i], 0);
-    }
-    cudaGraph_t g = nullptr;
-    cudaError_t e2 = cudaStreamEndCapture(b->stream, &g);
-    if (rc || e != cudaSuccess || e2 != cudaSuccess) {
-        if (g) cudaGraphDestroy(g);
-        if (rc) return bail(rc);
-        return bail(fail(MGPU_E_CUDA, std::string("batch capture: ") + cudaGetErrorString(e != cudaSuccess ? e : e2)));
-    }
-    b->graph = g;
-    e = cudaGraphGetNodes(g, nullptr, &b->graph_nodes);
-    if (e == cudaSuccess) e = cudaGraphInstantiate(&b->gexec, g, 0);
-    if (e != cudaSuccess) return bail(fail(MGPU_E_CUDA, std::string("batch graph: ") + cudaGetErrorString(e)));
+    std::vector<DevCtl *> list;
+    for (mgpu_handle *h : b->hs) list.push_back(h->d.ctl);
+    e = cudaMalloc(&b->d_list, n * sizeof(DevCtl *));
+    if (e == cudaSuccess) e = cudaMalloc(&b->d_ctl, n * sizeof(DevCtl));
+    if (e == cudaSuccess) e = cudaMallocHost((void **)&b->h_ctl, n * sizeof(DevCtl));
+    if (e == cudaSuccess) e = cudaMemcpy(b->d_list, list.data(), n * sizeof(DevCtl *), cudaMemcpyHostToDevice);
+    if (e != cudaSuccess) return bail(fail(MGPU_E_NOMEM, std::string("mgpu_batch_create: ") + cudaGetErrorString(e)));
+    int rc = batch_graph(b, 0);
+    if (!rc) rc = batch_graph(b, 3);
+    if (rc) return bail(rc);
     *out = b;
     return 0;
 }
 
 namespace {
-// the control blocks of every instance, read back on the batch stream
-int batch_read(mgpu_batch *b, mgpu_monitors *mons, int *ended) {
-    for (mgpu_handle *h : b->hs)
-        CK(cudaMemcpyAsync(h->h_ctl, h->d.ctl, sizeof(DevCtl), cudaMemcpyDeviceToHost, b->stream));
+// mirrors every member's control block
+int batch_fetch(mgpu_batch *b) {
+    const size_t n = b->hs.size();
+    k_gather_ctl<<<(unsigned)n, 64, 0, b->stream>>>(b->d_list, b->d_ctl);
+    CK(cudaGetLastError());
+    CK(cudaMemcpyAsync(b->h_ctl, b->d_ctl, n * sizeof(DevCtl), cudaMemcpyDeviceToHost, b->stream));
     CK(cudaStreamSynchronize(b->stream));
-    for (mgpu_handle *h : b->hs) h->ctl_known = true;
+    for (size_t i = 0; i < n; ++i) {
+        *b->hs[i]->h_ctl = b->h_ctl[i];
+        b->hs[i]->ctl_known = true;
+    }
+    return 0;
+}
+
+// the same, with the monitors, the health test and the number that met their end
+int batch_read(mgpu_batch *b, mgpu_monitors *mons, int *ended) {
+    int rc = batch_fetch(b);
+    if (rc) return rc;
     int nend = 0;
     for (size_t i = 0; i < b->hs.size(); ++i) {
         const DevCtl &c = *b->hs[i]->h_ctl;
@@ -1694,17 +1737,47 @@ int batch_read(mgpu_batch *b, mgpu_monitors *mons, int *ended) {
     *ended = nend;
     return 0;
 }
+// every member's control block is mirrored
+int batch_known(mgpu_batch *b) {
+    bool all = true;
+    for (mgpu_handle *h : b->hs) all = all && h->ctl_known;
+    return all ? 0 : batch_fetch(b);
+}
+
+// The steps to launch before the control blocks are read again, at most
+// `most`: up to the first tail while each step is of one kind for every
+// member; otherwise (members at different steps, or past their end) a stretch
+// of mixed ones.  Leaves the mirrors invalid.
+int batch_plan(mgpu_batch *b, int most, std::vector<int> &plan) {
+    int n = most, rc = 0;
+    for (mgpu_handle *h : b->hs) {
+        const int k = steps_to_tail(h->d, *h->h_ctl);
+        n = k < n ? k : n;
+        h->ctl_known = false;
+    }
+    for (int q = 0; q < n; ++q) {
+        const int what = step_what(b->hs[0]->d, *b->hs[0]->h_ctl, q, false);
+        for (mgpu_handle *h : b->hs)
+            if (step_what(h->d, *h->h_ctl, q, false) != what) {
+                plan.assign(most < 50 ? most : 50, -1);
+                return batch_graph(b, -1);
+            }
+        if ((rc = batch_graph(b, what))) return rc;
+        plan.push_back(what);
+    }
+    return 0;
+}
 }  // namespace
 
 int32_t mgpu_batch_run(mgpu_batch *b, int32_t nsteps, mgpu_monitors *mons) {
     if (!b || nsteps < 0) return fail(MGPU_E_ARG, "bad arguments to mgpu_batch_run");
-    const int chunk = 50;
     int done = 0, ended = 0, rc = 0;
-    for (mgpu_handle *h : b->hs) h->ctl_known = false;
+    if ((rc = batch_known(b))) return rc;
     while (done < nsteps) {
-        int m = nsteps - done < chunk ? nsteps - done : chunk;
-        for (int s = 0; s < m; ++s) CK(cudaGraphLaunch(b->gexec, b->stream));
-        done += m;
+        std::vector<int> plan;
+        if ((rc = batch_plan(b, nsteps - done, plan))) return rc;
+        for (int what : plan) CK(cudaGraphLaunch((what < 0 ? b->mixed : b->sg[what]).exec, b->stream));
+        done += (int)plan.size();
         if ((rc = batch_read(b, mons, &ended))) return rc;
     }
     if (nsteps == 0 && (rc = batch_read(b, mons, &ended))) return rc;
@@ -1719,14 +1792,21 @@ int32_t mgpu_batch_bench_steps(mgpu_batch *b, int32_t nsteps, int32_t flush_l2, 
         b->flush_bytes = (size_t)(l2 > 0 ? l2 : 128 << 20) * 2;
         CK(cudaMalloc(&b->flush_buf, b->flush_bytes));
     }
-    for (mgpu_handle *h : b->hs) h->ctl_known = false;
+    int ended = 0, rc = 0;
+    if ((rc = batch_known(b))) return rc;
     std::vector<cudaEvent_t> ev((size_t)2 * nsteps);
     for (auto &e : ev) CK(cudaEventCreate(&e));
-    for (int s = 0; s < nsteps; ++s) {
-        if (flush_l2) CK(cudaMemsetAsync(b->flush_buf, s & 0xff, b->flush_bytes, b->stream));
-        CK(cudaEventRecord(ev[2 * s], b->stream));
-        CK(cudaGraphLaunch(b->gexec, b->stream));
-        CK(cudaEventRecord(ev[2 * s + 1], b->stream));
+    for (int s = 0; s < nsteps;) {
+        std::vector<int> plan;
+        if ((rc = batch_plan(b, nsteps - s, plan))) return rc;
+        for (int what : plan) {
+            if (flush_l2) CK(cudaMemsetAsync(b->flush_buf, s & 0xff, b->flush_bytes, b->stream));
+            CK(cudaEventRecord(ev[2 * s], b->stream));
+            CK(cudaGraphLaunch((what < 0 ? b->mixed : b->sg[what]).exec, b->stream));
+            CK(cudaEventRecord(ev[2 * s + 1], b->stream));
+            ++s;
+        }
+        if (s < nsteps && (rc = batch_read(b, nullptr, &ended))) return rc;
     }
     CK(cudaStreamSynchronize(b->stream));
     double tot = 0.0;
@@ -1737,7 +1817,6 @@ int32_t mgpu_batch_bench_steps(mgpu_batch *b, int32_t nsteps, int32_t flush_l2, 
     }
     for (auto &e : ev) cudaEventDestroy(e);
     *total_ms = tot;
-    int ended = 0;
     return batch_read(b, nullptr, &ended);
 }
 
