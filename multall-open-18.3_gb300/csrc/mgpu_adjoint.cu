@@ -99,6 +99,7 @@ __device__ __forceinline__ void aadd(float *p, float v) {
 // R1: primitive variables (k_prim)
 // =====================================================================
 __global__ void rk_prim(const Dev d, const Adj a) {
+    pdl_wait();
     const int n = blockIdx.x * blockDim.x + threadIdx.x;
     const int N = d.IM * d.JM * d.KM;
     if (n >= N) return;
@@ -181,6 +182,7 @@ __device__ __forceinline__ void rev_flowt_raw(const Dev &d, const Adj &a, int i,
 // -U RO from ABT; ROVR on its I-face nodes), FLOWR q = 5, 6 (ROVX, ROVR on
 // its J-face nodes).  The periodic edge faces scatter with atomics.
 __global__ void rk_flux_mass_coef(const Dev d, const Adj a) {
+    pdl_wait();
     const int n = blockIdx.x * blockDim.x + threadIdx.x;
     const int N = d.IM * d.JM * d.KM;
     if (n >= N) return;
@@ -251,6 +253,7 @@ __global__ void rk_flux_mass_coef(const Dev d, const Adj a) {
 }
 
 __global__ void rk_flux_mass_gather(const Dev d, const Adj a) {
+    pdl_wait();
     const int n = blockIdx.x * blockDim.x + threadIdx.x;
     const int N = d.IM * d.JM * d.KM;
     if (n >= N) return;
@@ -308,6 +311,7 @@ __global__ void rk_flux_mass_gather(const Dev d, const Adj a) {
 // read-modify-writes.
 constexpr int RBC_BS = 1024;
 __global__ void __launch_bounds__(RBC_BS) rk_bc_sums(const Dev d, const Adj a) {
+    pdl_wait();
     __shared__ float gss[512], sr[512], gpd[512];
     const int KM = d.KM, IM = d.IM, IMM1 = d.IMM1;
     for (int k = threadIdx.x; k < KM; k += blockDim.x) {
@@ -394,6 +398,7 @@ __device__ __forceinline__ void rev_tflux_energy_raw(const Dev &d, const Adj &a,
 // nodes), RFLUX q = 1 (HO on the J-face nodes), TFLUX q = 2, 3 (HO, PEFF on the
 // I-face nodes); the periodic edge faces scatter with atomics.
 __global__ void rk_flux_energy_coef(const Dev d, const Adj a) {
+    pdl_wait();
     const int n = blockIdx.x * blockDim.x + threadIdx.x;
     const int N = d.IM * d.JM * d.KM;
     if (n >= N) return;
@@ -431,6 +436,7 @@ __global__ void rk_flux_energy_coef(const Dev d, const Adj a) {
 }
 
 __global__ void rk_flux_energy_gather(const Dev d, const Adj a) {
+    pdl_wait();
     const int n = blockIdx.x * blockDim.x + threadIdx.x;
     const int N = d.IM * d.JM * d.KM;
     if (n >= N) return;
@@ -471,6 +477,7 @@ __global__ void rk_flux_energy_gather(const Dev d, const Adj a) {
 // IN_VR <= 0
 // =====================================================================
 __global__ void rk_bc_apply(const Dev d, const Adj a) {
+    pdl_wait();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= d.IM * d.KM) return;
     const int i = t % d.IM + 1, k = t / d.IM + 1;
@@ -570,6 +577,7 @@ __global__ void rk_bc_apply(const Dev d, const Adj a) {
 // that use g, so it never meets the load of the same address in flight.
 // =====================================================================
 __global__ void rk_peff(const Dev d, const Adj a) {
+    pdl_wait();
     const int n = blockIdx.x * blockDim.x + threadIdx.x;
     const int N = d.IM * d.JM * d.KM;
     if (n >= N) return;
@@ -671,6 +679,7 @@ __device__ __forceinline__ void rev_mom_iface_edge(const Dev &d, const Adj &a, i
 constexpr int MOM_NCOEF = 15;
 
 __global__ void rk_flux_mom_coef(const Dev d, const Adj a) {
+    pdl_wait();
     const int n = blockIdx.x * blockDim.x + threadIdx.x;
     const int N = d.IM * d.JM * d.KM;
     if (n >= N) return;
@@ -798,6 +807,7 @@ __global__ void rk_flux_mom_coef(const Dev d, const Adj a) {
 }
 
 __global__ void rk_flux_mom_gather(const Dev d, const Adj a) {
+    pdl_wait();
     const int n = blockIdx.x * blockDim.x + threadIdx.x;
     const int N = d.IM * d.JM * d.KM;
     if (n >= N) return;
@@ -911,6 +921,7 @@ template <int N> __device__ inline Dual<N> dcos(const Dual<N> &x) { return lin(c
 constexpr int MIXN = 14;
 
 __global__ void __launch_bounds__(64) rk_mixplan(const Dev d, const Adj a) {
+    pdl_wait();
     typedef Dual<MIXN> D;
     __shared__ float red[5][64];
     const int nr = blockIdx.x / d.KM + 1, k = blockIdx.x % d.KM + 1;
@@ -1071,6 +1082,7 @@ __global__ void __launch_bounds__(256) rk_density_prep(const Dev d, const Adj a)
 }
 
 __global__ void rk_density(const Dev d, const Adj a) {
+    pdl_wait();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= d.IM * d.KM || !a.tDCOL[t]) return;
     const int i = t % d.IM + 1, k = t / d.IM + 1;
@@ -1088,6 +1100,7 @@ __global__ void rk_density(const Dev d, const Adj a) {
 }
 
 __global__ void rk_mach(const Dev d, const Adj a) {
+    pdl_wait();
     const int n = blockIdx.x * blockDim.x + threadIdx.x;
     const int N = d.IM * d.JM * d.KM;
     if (n >= N) return;
@@ -1136,6 +1149,7 @@ __device__ inline bool mp_row_on(const Dev &d, const Adj &a, int role, int jmx, 
 }
 
 __global__ void __launch_bounds__(RT_BS) rk_ts_smooth(const __grid_constant__ Dev d, const __grid_constant__ Adj a, int v0) {
+    pdl_wait();
     extern __shared__ float sm[];
     const AdjVar &V = a.v[v0 + blockIdx.y];
     const int IM = d.IM, KM = d.KM, IMM1 = d.IMM1, KMM1 = d.KMM1;
@@ -1342,6 +1356,7 @@ __global__ void __launch_bounds__(RT_BS) rk_ts_smooth(const __grid_constant__ De
 }
 
 __global__ void __launch_bounds__(RT_BS) rk_ts_gather(const __grid_constant__ Dev d, const __grid_constant__ Adj a, int v0) {
+    pdl_wait();
     extern __shared__ float sm[];
     __shared__ double shd[RT_BS / 32];
     const AdjVar &V = a.v[v0 + blockIdx.y];
@@ -1471,6 +1486,7 @@ __global__ void __launch_bounds__(RT_BS) rk_ts_gather(const __grid_constant__ De
 }
 
 __global__ void __launch_bounds__(RT_BS) rk_ts_damp(const __grid_constant__ Dev d, const __grid_constant__ Adj a, int v0) {
+    pdl_wait();
     extern __shared__ float sm[];
     __shared__ float gchg[64], gblk[64];
     const AdjVar &V = a.v[v0 + blockIdx.y];
@@ -1523,6 +1539,16 @@ __global__ void __launch_bounds__(RT_BS) rk_ts_damp(const __grid_constant__ Dev 
         __syncthreads();
         const PlaneInfo &pl = d.PLANE[j - 1];
         if (j > pl.J1 && j < pl.J2) add = gchg[pl.nrow - 1] / (float)(IMM1 * KMM1 * (pl.J2 - pl.J1 - 1));
+    }
+    // TMP's adjoint has been read (rk_ts_gather): left at zero for the next
+    // step's scatter, plane 1 by the CTA of plane 2
+    {
+        const int IM = d.IM, np = IM * d.KM;
+        WalkN wz(IM, IM * d.JM, IM * (j - 1), threadIdx.x, RT_BS);
+        for (int t = threadIdx.x; t < np; t += RT_BS, wz.next()) {
+            V.TM[wz.n] = 0.0f;
+            if (j == 2) V.TM[wz.n - IM] = 0.0f;
+        }
     }
     float psf = 0.0f;             // FP32 per thread, FP64 across threads
     WalkN w(IMM1, d.IM * d.JM, d.IM * (j - 1), threadIdx.x, RT_BS);
@@ -1592,6 +1618,7 @@ __global__ void __launch_bounds__(RT_BS) rk_ts_damp(const __grid_constant__ Dev 
 }
 
 __global__ void __launch_bounds__(RT_BS) rk_ts_cells(const __grid_constant__ Dev d, const __grid_constant__ Adj a, int v0) {
+    pdl_wait();
     extern __shared__ float sm[];
     __shared__ float s_sb;
     const AdjVar &V = a.v[v0 + blockIdx.y];
@@ -1758,6 +1785,7 @@ __global__ void rk_seed_set(int *seed_on, int j1, int j2) {
 
 // objective seeds added at the start of each reverse step
 __global__ void rk_seed(const Dev d, const Adj a) {
+    pdl_wait();
     const int IM = d.IM, KM = d.KM;
     const int np = IM * KM, nc = d.IMM1 * d.KMM1;
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -2173,13 +2201,12 @@ int configure(const Dev &d) {
 }
 
 void launch_tstep_rev(const Dev &d, const Adj &a, cudaStream_t s, int v0, int nv) {
-    const size_t N = (size_t)d.IM * d.JM * d.KM;
-    for (int v = v0; v < v0 + nv; ++v) cudaMemsetAsync(a.v[v].TM, 0, N * sizeof(float), s);
+    const Launch L{s, 0, nullptr, true};
     const unsigned ja = (unsigned)d.JM, jp = (unsigned)(d.JM - 1);
-    rk_ts_smooth<<<dim3(ja, nv), RT_BS, smooth_bytes(d), s>>>(d, a, v0);
-    rk_ts_gather<<<dim3(ja, nv), RT_BS, gather_bytes(d), s>>>(d, a, v0);
-    rk_ts_damp<<<dim3(jp, nv), RT_BS, damp_bytes(d), s>>>(d, a, v0);
-    rk_ts_cells<<<dim3(jp, nv), RT_BS, cells_bytes(d), s>>>(d, a, v0);
+    launchk(L, rk_ts_smooth, dim3(ja, nv), dim3(RT_BS), smooth_bytes(d), d, a, v0);
+    launchk(L, rk_ts_gather, dim3(ja, nv), dim3(RT_BS), gather_bytes(d), d, a, v0);
+    launchk(L, rk_ts_damp, dim3(jp, nv), dim3(RT_BS), damp_bytes(d), d, a, v0);
+    launchk(L, rk_ts_cells, dim3(jp, nv), dim3(RT_BS), cells_bytes(d), d, a, v0);
 }
 
 // one reverse step: the adjoints of the state after a step (plus the
@@ -2188,22 +2215,25 @@ void enqueue_reverse(const Dev &d, const Adj &a, cudaStream_t s) {
     const size_t N = (size_t)d.IM * d.JM * d.KM;
     const unsigned gN = gridn(N, 256);
     const int per = 5 * d.IM * d.KM + d.IMM1 * d.KMM1;
-    rk_seed<<<gridn((size_t)2 * per, 256), 256, 0, s>>>(d, a);
-    if (d.IFMIX > 0 && d.RFMIX > 1.0e-3f && d.NRWSM1 > 0) rk_mixplan<<<d.NRWSM1 * d.KM, 64, 0, s>>>(d, a);
-    rk_mach<<<gN, 256, 0, s>>>(d, a);
-    rk_density<<<gridn((size_t)d.IM * d.KM, 128), 128, 0, s>>>(d, a);
+    // kernel-to-kernel edges are programmatic, as in the forward step
+    Launch L{s, 0, nullptr, false};
+    launchk(L, rk_seed, dim3(gridn((size_t)2 * per, 256)), dim3(256), 0, d, a);
+    L.pdl = true;
+    if (d.IFMIX > 0 && d.RFMIX > 1.0e-3f && d.NRWSM1 > 0) launchk(L, rk_mixplan, dim3(d.NRWSM1 * d.KM), dim3(64), 0, d, a);
+    launchk(L, rk_mach, dim3(gN), dim3(256), 0, d, a);
+    launchk(L, rk_density, dim3(gridn((size_t)d.IM * d.KM, 128)), dim3(128), 0, d, a);
     launch_tstep_rev(d, a, s, V_ROVX, 3);
-    rk_flux_mom_coef<<<gN, 256, 0, s>>>(d, a);
-    rk_flux_mom_gather<<<gN, 256, 0, s>>>(d, a);
-    if (d.F_PDOWN != 0.0f) rk_peff<<<gN, 256, 0, s>>>(d, a);
-    rk_bc_apply<<<gridn((size_t)d.IM * d.KM, 128), 128, 0, s>>>(d, a);
+    launchk(L, rk_flux_mom_coef, dim3(gN), dim3(256), 0, d, a);
+    launchk(L, rk_flux_mom_gather, dim3(gN), dim3(256), 0, d, a);
+    if (d.F_PDOWN != 0.0f) launchk(L, rk_peff, dim3(gN), dim3(256), 0, d, a);
+    launchk(L, rk_bc_apply, dim3(gridn((size_t)d.IM * d.KM, 128)), dim3(128), 0, d, a);
     launch_tstep_rev(d, a, s, V_RO, 2);
-    rk_flux_energy_coef<<<gN, 256, 0, s>>>(d, a);
-    rk_flux_energy_gather<<<gN, 256, 0, s>>>(d, a);
-    rk_bc_sums<<<1, RBC_BS, 0, s>>>(d, a);
-    rk_flux_mass_coef<<<gN, 256, 0, s>>>(d, a);
-    rk_flux_mass_gather<<<gN, 256, 0, s>>>(d, a);
-    rk_prim<<<gN, 256, 0, s>>>(d, a);
+    launchk(L, rk_flux_energy_coef, dim3(gN), dim3(256), 0, d, a);
+    launchk(L, rk_flux_energy_gather, dim3(gN), dim3(256), 0, d, a);
+    launchk(L, rk_bc_sums, dim3(1), dim3(RBC_BS), 0, d, a);
+    launchk(L, rk_flux_mass_coef, dim3(gN), dim3(256), 0, d, a);
+    launchk(L, rk_flux_mass_gather, dim3(gN), dim3(256), 0, d, a);
+    launchk(L, rk_prim, dim3(gN), dim3(256), 0, d, a);
 }
 
 int unsupported(const Dev &d) {
