@@ -72,15 +72,28 @@ __device__ inline float mp_line_sum(const float *row, int n) {
 }
 
 // The default precision split's form of the same sum: accumulated in
-// double-float and rounded once, by one warp (every lane calls it, with the
-// same n).  Each lane adds every 32nd term, then a shuffle tree; every lane
-// gets the total.
+// double-float and rounded once.  Eight lanes a row, so a warp forms four
+// rows' sums at a time: each lane adds every eighth term, then three shuffle
+// steps; the row's eight lanes get the total.  Every lane of the warp calls
+// it (a row that is not wanted with n = 0).  A whole warp a row spent two
+// thirds of its instructions in five-step trees over two terms a lane, and
+// the CTAs of the mixing planes were the longest of their launch.
+constexpr int ROW_LANES = 8;
 template <class F>
-__device__ inline float warp_sum64(int n, F term) {
+__device__ inline float row_sum64(int n, F term) {
     df s = df_of(0.0f);
-    for (int i = (int)(threadIdx.x & 31); i < n; i += 32) s = df_add(s, df_of(term(i)));
-    for (int o = 16; o > 0; o >>= 1) s = df_add(s, df_shfl_xor(s, o));
+    for (int i = (int)threadIdx.x % ROW_LANES; i < n; i += ROW_LANES) s = df_add(s, df_of(term(i)));
+    for (int o = ROW_LANES / 2; o > 0; o >>= 1) s = df_add(s, df_shfl_xor(s, o));
     return df_val(s);
+}
+// Calls row(r, l, on) for the rows r of [0, nrow) with the eight lanes
+// l = 0..7 of each; on is false for the lanes past the last row, which take
+// part in the warp's shuffles only.
+template <class F>
+__device__ inline void for_rows(int nrow, F row) {
+    const int step = (int)blockDim.x / ROW_LANES, warp0 = (int)(threadIdx.x & ~31u) / ROW_LANES;
+    int r = (int)threadIdx.x / ROW_LANES;
+    for (int r0 = warp0; r0 < nrow; r0 += step, r += step) row(r, (int)threadIdx.x % ROW_LANES, r < nrow);
 }
 
 // ---------------------------------------------------------------------
@@ -99,6 +112,7 @@ __global__ void __launch_bounds__(BS, 1024 / BS) k_ts_cells(const __grid_constan
     const int nc = IMM1 * KMM1;
     float *st = sm;              // STORE of this plane, [k-1][i-1]
     float *lsum = sm + nc;       // per-K line sums
+    float *fdir = lsum + KMM1 + d.NIB1 * d.NKB1;     // and, at a mixing plane, the flow's direction
     const PlaneInfo &pl = d.PLANE[j - 1];
     const int role = pl.role, jmx = pl.jmx, kts = pl.kts, kte = pl.kte;
     const float RATPITCH = pl.ratpitch;
@@ -106,27 +120,33 @@ __global__ void __launch_bounds__(BS, 1024 / BS) k_ts_cells(const __grid_constan
     // the cells of this thread's first level-1 block, for the partial sums below
     const int n1 = d.NIB1 * d.NKB1, n2 = d.NIB2 * d.NKB2;
     const int4 blk1 = d.MG1X[min((int)threadIdx.x, n1 - 1)], blk2 = d.MG2X[min((int)threadIdx.x, n2 - 1)];
-    if ((role == 1 || role == 3) && !lowx) {
+    if (role) {
+        // the flow direction on each line of the mixing plane
+        for (int k = threadIdx.x + 1; k <= KMM1; k += BS) fdir[k - 1] = -A3(d.FLOWX, d.IMID, jmx, k);
         // stage the XFLUX plane in shared memory (coalesced), then add each
-        // I-line in the reference's order
-        int jj = role == 1 ? j - 1 : j;
-        Walk2 wx(IMM1, threadIdx.x, BS);
-        for (int c = threadIdx.x; c < nc; c += BS, wx.next()) st[c] = A3(V.XF, wx.i, jj, wx.k);
-        __syncthreads();
-        if (d.REDUCE_ORDER != 0) {
-            for (int k = threadIdx.x + 1; k <= KMM1; k += BS) {
-                const float *row = st + (size_t)(k - 1) * IMM1;
-                lsum[k - 1] = mp_line_sum(row, IMM1);
-            }
-        } else {
-            for (int k = (int)(threadIdx.x >> 5) + 1; k <= KMM1; k += BS / 32) {
-                const float *row = st + (size_t)(k - 1) * IMM1;
-                float s = warp_sum64(IMM1, [&](int i) { return row[i]; });
-                if ((threadIdx.x & 31) == 0) lsum[k - 1] = s;
-            }
+        // I-line that is extrapolated
+        const bool sums = role != 2 && !lowx;
+        if (sums) {
+            int jj = role == 1 ? j - 1 : j;
+            Walk2 wx(IMM1, threadIdx.x, BS);
+            for (int c = threadIdx.x; c < nc; c += BS, wx.next()) st[c] = A3(V.XF, wx.i, jj, wx.k);
         }
+        __syncthreads();
+        auto wanted = [&](int k) { return (role == 1) == (fdir[k - 1] > 0.0f); };
+        if (sums && d.REDUCE_ORDER != 0) {
+            for (int k = threadIdx.x + 1; k <= KMM1; k += BS)
+                if (wanted(k)) lsum[k - 1] = mp_line_sum(st + (k - 1) * IMM1, IMM1);
+        } else if (sums) {
+            for_rows(KMM1, [&](int r, int l, bool on) {
+                on = on && wanted(r + 1);
+                if (!__any_sync(0xffffffffu, on)) return;
+                const float *row = st + r * IMM1;
+                const float s = row_sum64(on ? IMM1 : 0, [&](int i) { return row[i]; });
+                if (on && l == 0) lsum[r] = s;
+            });
+        }
+        __syncthreads();
     }
-    __syncthreads();
     const float F1 = d.F1, F2 = d.F2, F3 = d.F3;
     const float *__restrict__ XF = V.XF;
     const float *__restrict__ RF = V.RF;
@@ -173,7 +193,7 @@ __global__ void __launch_bounds__(BS, 1024 / BS) k_ts_cells(const __grid_constan
             }
             float src = sr[u];
             if (role && !lowx) {
-                float FLOWDIRN = -A3(d.FLOWX, d.IMID, jmx, k);
+                const float FLOWDIRN = fdir[k - 1];
                 if (role == 1 && FLOWDIRN > 0.0f) src = src - (xm[u] - lsum[k - 1] * A1(d.FP, i)) * d.FEXTRAP;
                 if (role == 2) src = 0.0f;
                 if (role == 3 && !(FLOWDIRN > 0.0f)) src = src + (xf[u] - lsum[k - 1] * A1(d.FP, i)) * d.FEXTRAP;
@@ -185,22 +205,26 @@ __global__ void __launch_bounds__(BS, 1024 / BS) k_ts_cells(const __grid_constan
     }
     __syncthreads();
     if (role == 1 || role == 3) {
-        const bool lane_par = d.REDUCE_ORDER == 0;
-        const int k0 = lane_par ? (int)(threadIdx.x >> 5) + 1 : (int)threadIdx.x + 1;
-        const int kstep = lane_par ? BS / 32 : BS;
-        for (int k = k0; k <= KMM1; k += kstep) {
-            float FLOWDIRN = -A3(d.FLOWX, d.IMID, jmx, k);
-            bool on = role == 3 ? (FLOWDIRN > 0.0f || lowx) : (FLOWDIRN < 0.0f || lowx);
-            if (!on) continue;
-            float *row = st + (size_t)(k - 1) * IMM1;
-            if (lane_par) {
-                float s = warp_sum64(IMM1, [&](int i) { return row[i]; });
-                __syncwarp();
-                for (int i = (int)(threadIdx.x & 31); i < IMM1; i += 32) row[i] = s * A1(d.FP, i + 1);
-            } else {
-                float s = mp_line_sum(row, IMM1);
+        auto averaged = [&](int k) {
+            const float FLOWDIRN = fdir[k - 1];
+            return role == 3 ? (FLOWDIRN > 0.0f || lowx) : (FLOWDIRN < 0.0f || lowx);
+        };
+        if (d.REDUCE_ORDER != 0) {
+            for (int k = threadIdx.x + 1; k <= KMM1; k += BS) {
+                if (!averaged(k)) continue;
+                float *row = st + (k - 1) * IMM1;
+                const float s = mp_line_sum(row, IMM1);
                 for (int i = 0; i < IMM1; ++i) row[i] = s * A1(d.FP, i + 1);
             }
+        } else {
+            for_rows(KMM1, [&](int r, int l, bool on) {
+                on = on && averaged(r + 1);
+                if (!__any_sync(0xffffffffu, on)) return;
+                float *row = st + r * IMM1;
+                const int n = on ? IMM1 : 0;
+                const float s = row_sum64(n, [&](int i) { return row[i]; });
+                for (int i = l; i < n; i += ROW_LANES) row[i] = s * A1(d.FP, i + 1);
+            });
         }
         __syncthreads();
     }
@@ -216,8 +240,20 @@ __global__ void __launch_bounds__(BS, 1024 / BS) k_ts_cells(const __grid_constan
             psf += v;
         }
     }
-    const df ps = block_sum<BS>(d.REDUCE_ORDER, df_of(psf), shd);
-    if (threadIdx.x == 0) V.psum[j - 1] = ps;
+    // (each warp's part here; the last warp adds the parts below, beside the
+    // block sums)
+    const int ro = d.REDUCE_ORDER, lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+    {
+        df v = df_of(psf);
+        for (int o = 16; o > 0; o >>= 1) v = dacc(ro, v, df_shfl_down(v, o));
+        if (lane == 0) shd[wp] = v;
+    }
+    auto plane_sum = [&]() {
+        if (wp != BS / 32 - 1) return;
+        df r = lane < BS / 32 ? shd[lane] : df_of(0.0f);
+        for (int o = BS > 256 ? 8 : BS > 128 ? 4 : 2; o > 0; o >>= 1) r = dacc(ro, r, df_shfl_down(r, o));
+        if (lane == 0) V.psum[j - 1] = r;
+    };
     // level-1 and level-2 partial sums of this plane
     auto block_cells = [&](int4 x) {
         float s = 0.0f;
@@ -239,6 +275,7 @@ __global__ void __launch_bounds__(BS, 1024 / BS) k_ts_cells(const __grid_constan
             P1[u] = s;
         }
         __syncthreads();
+        plane_sum();
         for (int u = threadIdx.x; u < n2; u += BS) {
             const int4 x = u < BS ? blk2 : d.MG2X[u];
             float s = 0.0f;
@@ -250,6 +287,8 @@ __global__ void __launch_bounds__(BS, 1024 / BS) k_ts_cells(const __grid_constan
     }
     for (int u = threadIdx.x; u < n1; u += BS) P1[u] = block_cells(u < BS ? blk1 : d.MG1X[u]);
     for (int u = threadIdx.x; u < n2; u += BS) P2[u] = block_cells(u < BS ? blk2 : d.MG2X[u]);
+    __syncthreads();
+    plane_sum();
 }
 
 // ---------------------------------------------------------------------
@@ -548,6 +587,14 @@ __global__ void __launch_bounds__(UP_T, 3) k_ts_update(const __grid_constant__ D
         float *c = sm + (p & 1) * buf + il + 1;
         const bool pl = jc >= 2 && jc <= JM;
         const float blk = s_blk[p];
+        const int role = s_role[p], nrow = rows + 1;
+        const bool mp = role == 1 || role == 3;
+        // the flow's direction on a mixing plane's row r of the tile (0 off the grid)
+        auto flow = [&](int r) {
+            const int k = k0 - 1 + r;
+            return mp && r < nrow && k >= 1 && k <= KMM1 ? -A3(d.FLOWX, d.IMID, s_jmx[p], k) : 0.0f;
+        };
+        const float fdir = flow(tid / ROW_LANES);         // of this thread's first row, ahead of its use
         auto damped = [&](float v) {
             if (!damp_on) return v;
             const float FDAMP = fabsf(v) / blk;
@@ -558,27 +605,31 @@ __global__ void __launch_bounds__(UP_T, 3) k_ts_update(const __grid_constant__ D
             if (ci && q < kn && kb + q <= KMM1) c[PW * (seg * UP_S + q + 1)] = pl ? damped(st[q]) : 0.0f;
         if (c0) c[0] = pl ? damped(st[UP_S]) : 0.0f;
         __syncthreads();
-        const int role = s_role[p];
-        if (role != 1 && role != 3) return;
+        if (!mp) return;
         // second pitchwise average on the mixing-plane cells (1850)
         const bool lowx = d.FEXTRAP < 0.001f;
         float *row0 = sm + (p & 1) * buf + 1;
-        const bool lane_par = d.REDUCE_ORDER == 0;
-        const int r0 = lane_par ? tid >> 5 : tid, rstep = lane_par ? (int)blockDim.x >> 5 : (int)blockDim.x;
-        for (int r = r0; r <= rows; r += rstep) {
+        auto averaged = [&](int r, float FLOWDIRN) {
             const int k = k0 - 1 + r;
-            if (k < 1 || k > KMM1) continue;
-            const float FLOWDIRN = -A3(d.FLOWX, d.IMID, s_jmx[p], k);
-            if (!(role == 3 ? (FLOWDIRN > 0.0f || lowx) : (FLOWDIRN < 0.0f || lowx))) continue;
-            float *row = row0 + r * PW;
-            if (lane_par) {
-                const float m = warp_sum64(IMM1, [&](int i) { return row[i]; }) / (float)IMM1;
-                __syncwarp();
-                for (int i = tid & 31; i < IMM1; i += 32) row[i] = m;
-            } else {
+            return k >= 1 && k <= KMM1 &&
+                   (role == 3 ? (FLOWDIRN > 0.0f || lowx) : (FLOWDIRN < 0.0f || lowx));
+        };
+        if (d.REDUCE_ORDER != 0) {
+            for (int r = tid; r < nrow; r += (int)blockDim.x) {
+                if (!averaged(r, flow(r))) continue;
+                float *row = row0 + r * PW;
                 const float m = mp_line_sum(row, IMM1) / (float)IMM1;
                 for (int i = 0; i < IMM1; ++i) row[i] = m;
             }
+        } else {
+            for_rows(nrow, [&](int r, int l, bool on) {
+                on = on && averaged(r, r == tid / ROW_LANES ? fdir : flow(r));
+                if (!__any_sync(0xffffffffu, on)) return;
+                float *row = row0 + r * PW;
+                const int n = on ? IMM1 : 0;
+                const float m = row_sum64(n, [&](int i) { return row[i]; }) / (float)IMM1;
+                for (int i = l; i < n; i += ROW_LANES) row[i] = m;
+            });
         }
         __syncthreads();
     };
@@ -762,22 +813,26 @@ __global__ void __launch_bounds__(PBS, 1024 / PBS) k_ts_update_pair(const __grid
         if (role != 1 && role != 3) continue;
         any = true;
         float *c = sm + h * nc;
-        const bool lane_par = d.REDUCE_ORDER == 0;
-        const int k0 = lane_par ? (int)(threadIdx.x >> 5) + 1 : (int)threadIdx.x + 1;
-        const int kstep = lane_par ? PBS / 32 : PBS;
-        for (int k = k0; k <= KMM1; k += kstep) {
-            float FLOWDIRN = -A3(d.FLOWX, d.IMID, jmx, k);
-            bool on = role == 3 ? (FLOWDIRN > 0.0f || lowx) : (FLOWDIRN < 0.0f || lowx);
-            if (!on) continue;
-            float *row = c + (k - 1) * IMM1;
-            if (lane_par) {
-                float s = warp_sum64(IMM1, [&](int i) { return row[i]; }) / (float)IMM1;
-                __syncwarp();
-                for (int i = (int)(threadIdx.x & 31); i < IMM1; i += 32) row[i] = s;
-            } else {
-                float s = mp_line_sum(row, IMM1) / (float)IMM1;
+        auto averaged = [&](int k) {
+            const float FLOWDIRN = -A3(d.FLOWX, d.IMID, jmx, k);
+            return role == 3 ? (FLOWDIRN > 0.0f || lowx) : (FLOWDIRN < 0.0f || lowx);
+        };
+        if (d.REDUCE_ORDER != 0) {
+            for (int k = threadIdx.x + 1; k <= KMM1; k += PBS) {
+                if (!averaged(k)) continue;
+                float *row = c + (k - 1) * IMM1;
+                const float s = mp_line_sum(row, IMM1) / (float)IMM1;
                 for (int i = 0; i < IMM1; ++i) row[i] = s;
             }
+        } else {
+            for_rows(KMM1, [&](int r, int l, bool on) {
+                on = on && averaged(r + 1);
+                if (!__any_sync(0xffffffffu, on)) return;
+                float *row = c + r * IMM1;
+                const int n = on ? IMM1 : 0;
+                const float s = row_sum64(n, [&](int i) { return row[i]; }) / (float)IMM1;
+                for (int i = l; i < n; i += ROW_LANES) row[i] = s;
+            });
         }
     }
     if (any) __syncthreads();
@@ -1167,10 +1222,11 @@ __global__ void __launch_bounds__(BS, 1024 / BS) k_ts_smooth(const __grid_consta
                 b[k - 1] = 0.5f * s;
             }
         } else {
-            for (int k = (int)(threadIdx.x >> 5) + 1; k <= KM; k += BS / 32) {
-                float s = warp_sum64(IMM1, [&](int i) { return A1(d.FP, i + 1) * (P(a, i + 1, k) + P(a, i + 2, k)); });
-                if ((threadIdx.x & 31) == 0) b[k - 1] = 0.5f * s;
-            }
+            for_rows(KM, [&](int r, int l, bool on) {
+                const int k = r + 1;
+                const float s = row_sum64(on ? IMM1 : 0, [&](int i) { return A1(d.FP, i + 1) * (P(a, i + 1, k) + P(a, i + 2, k)); });
+                if (on && l == 0) b[r] = 0.5f * s;
+            });
         }
         __syncthreads();
         Walk2 w(IM, threadIdx.x, BS);
@@ -1241,7 +1297,7 @@ __global__ void k_copy_tm_st(const __grid_constant__ Dev d, int v0, size_t n) {
 static bool pair_update(const Dev &d) { return d.TS_PAIR && (d.in_batch || d.IM * d.KM <= 512); }
 
 static size_t cells_smem(const Dev &d) {
-    return ((size_t)d.IMM1 * d.KMM1 + d.KMM1 + (size_t)d.NIB1 * d.NKB1) * sizeof(float);
+    return ((size_t)d.IMM1 * d.KMM1 + 2 * d.KMM1 + (size_t)d.NIB1 * d.NKB1) * sizeof(float);
 }
 static size_t prolong_smem(const Dev &d) { return ((size_t)d.NIB1 * d.NKB1 + (size_t)d.NIB2 * d.NKB2) * sizeof(float); }
 static size_t update_pair_smem(const Dev &d) { return (size_t)3 * d.IMM1 * d.KMM1 * sizeof(float); }
