@@ -782,13 +782,16 @@ __device__ __forceinline__ float stepup_node(const Dev &d, StepupLimits q, float
 }
 
 // The tail's node pass: the % change of Vm with its sum and maximum, the
-// health count, and STEPUP's node values (TEMP1).  Each thread takes TAIL_NPT
-// nodes (TAIL_BS apart, so the loads stay coalesced), two at a time with all
-// loads of the two in flight, and adds their |DVMER| in FP32 before the CTA's
-// sum.  The last CTA forms EAVG, EMAX and the continuity error ECONT.
+// health count, and STEPUP's node values (TEMP1).  Each thread takes npt <=
+// TAIL_NPT nodes (TAIL_BS apart, so the loads stay coalesced), two at a time
+// with all loads of the two in flight, and adds their |DVMER| in FP32 before
+// the CTA's sum.  npt is what leaves four CTAs an SM: a grid that cannot fill
+// the GPU takes one node a thread (TAIL_NPT on every grid made the node pass
+// of 3150 nodes, on two CTAs, four latencies long).  The last CTA forms EAVG,
+// EMAX and the continuity error ECONT.
 constexpr int TAIL_NPT = 8;
 
-__global__ void __launch_bounds__(TAIL_BS) k_tail_nodes(const __grid_constant__ Dev d) {
+__global__ void __launch_bounds__(TAIL_BS) k_tail_nodes(const __grid_constant__ Dev d, int npt) {
     pdl_wait();
     DevCtl *c = d.ctl;
     if (!c->do_tail) return;
@@ -799,8 +802,8 @@ __global__ void __launch_bounds__(TAIL_BS) k_tail_nodes(const __grid_constant__ 
     unsigned long long key = 0ull;
     int bad = 0;
 #pragma unroll 2
-    for (int u = 0; u < TAIL_NPT; ++u) {
-        const int n = ((int)blockIdx.x * TAIL_NPT + u) * TAIL_BS + (int)threadIdx.x;
+    for (int u = 0; u < npt; ++u) {
+        const int n = ((int)blockIdx.x * npt + u) * TAIL_BS + (int)threadIdx.x;
         if (n >= N) break;
         const int jk = n / d.IM;                         // (j-1) + JM*(k-1)
         const bool jin = jk % d.JM != 0;                 // j >= 2
@@ -843,7 +846,9 @@ __global__ void __launch_bounds__(TAIL_BS) k_tail_nodes(const __grid_constant__ 
     // the continuity error ECONT = max over J of |1 - FLOW(J)/FLOW(1)| and
     // the first J that reaches it, one J per thread as a (value, J) key
     unsigned long long ek = 0ull;
-    const float cf1f = (float)d.BLADE_FLOW[0];
+    const double flow1 = d.BLADE_FLOW[0], flowj = d.BLADE_FLOW[d.JM - 1];
+    const int jcont = c->JCONT;
+    const float cf1f = (float)flow1;
     for (int j = threadIdx.x + 1; j <= d.JM; j += TAIL_BS) {
         float RATIO = (float)d.BLADE_FLOW[j - 1] / cf1f;
         float EMASS = fabsf(1.0f - RATIO);
@@ -868,31 +873,33 @@ __global__ void __launch_bounds__(TAIL_BS) k_tail_nodes(const __grid_constant__ 
             ke = se[w] > ke ? se[w] : ke;
             cnt += sc[w];
         }
-        c->EAVG = df_val(s) / (float)(d.IM * d.JMM1 * d.KM);
+        const float eavg = df_val(s) / (float)(d.IM * d.JMM1 * d.KM);
+        float emax = 0.0f;
         if (key) {
             unsigned lin = 0xFFFFFFFFu - (unsigned)(key & 0xFFFFFFFFull);
-            c->EMAX = d.STORE[lin];
-            c->IMAXE = (int)(lin % d.IM) + 1;
-            c->JMAXE = (int)((lin / d.IM) % d.JM) + 1;
-            c->KMAXE = (int)(lin / ((unsigned)d.IM * d.JM)) + 1;
-        } else {
-            c->EMAX = 0.0f;
+            emax = d.STORE[lin];
+            const unsigned jk = lin / (unsigned)d.IM, k = jk / (unsigned)d.JM;
+            c->IMAXE = (int)(lin - jk * (unsigned)d.IM) + 1;
+            c->JMAXE = (int)(jk - k * (unsigned)d.JM) + 1;
+            c->KMAXE = (int)k + 1;
         }
-        c->health = cnt;
         // continuity error ECONT and its station (the reference's J loop
         // keeps the first J of the largest value; none above 0 keeps JCONT)
         float econt = 0.0f;
-        int jc = c->JCONT;
+        int jc = jcont;
         if (ke) {
             econt = __uint_as_float((unsigned)(ke >> 32));
             jc = (int)(0xFFFFFFFFu - (unsigned)(ke & 0xFFFFFFFFull)) + 1;
         }
+        c->EAVG = eavg;
+        c->EMAX = emax;
+        c->health = cnt;
         c->ECONT = econt;
-        c->CHECK_FLOW_JM = (float)d.BLADE_FLOW[d.JM - 1];   // CHECK_FLOW(JM) for the throttle
+        c->CHECK_FLOW_JM = (float)flowj;   // CHECK_FLOW(JM) for the throttle
         c->JCONT = jc;
-        c->flow_in = d.BLADE_FLOW[0];
-        c->flow_out = d.BLADE_FLOW[d.JM - 1];
-        if ((c->EAVG < d.CONLIM && c->ECONT < 0.01f) || (fabsf(c->EMAX) < 4.0f * d.CONLIM && c->ECONT < 0.01f))
+        c->flow_in = flow1;
+        c->flow_out = flowj;
+        if ((eavg < d.CONLIM && econt < 0.01f) || (fabsf(emax) < 4.0f * d.CONLIM && econt < 0.01f))
             c->converged = 1;
     }
 }
@@ -959,7 +966,8 @@ void launch_tail(const Dev &d, Launch L) {
     launchk(L, k_tail_flow, dim3(d.JM), dim3(TAIL_BS), 0, d);
     mark(L, "k_tail_flow");
     size_t N = (size_t)d.IM * d.JM * d.KM;
-    launchk(L, k_tail_nodes, dim3(grid_for(N, (size_t)TAIL_BS * TAIL_NPT)), dim3(TAIL_BS), 0, d);
+    const int npt = (int)std::min<size_t>(TAIL_NPT, std::max<size_t>(1, N / ((size_t)TAIL_BS * 4 * L.sm_count)));
+    launchk(L, k_tail_nodes, dim3(grid_for(N, (size_t)TAIL_BS * npt)), dim3(TAIL_BS), 0, d, npt);
     mark(L, "k_tail_nodes");
     launch_stepup_cell(d, L, 0.25f, true);
 }

@@ -78,22 +78,43 @@ __device__ inline float mp_line_sum(const float *row, int n) {
 // it (a row that is not wanted with n = 0).  A whole warp a row spent two
 // thirds of its instructions in five-step trees over two terms a lane, and
 // the CTAs of the mixing planes were the longest of their launch.
+//
+// U terms a lane are read together before they are added, so that terms in
+// global memory cost one latency.  An added term has no low part: of the
+// double-float addition, the steps that add it are left out (same result).
 constexpr int ROW_LANES = 8;
-template <class F>
-__device__ inline float row_sum64(int n, F term) {
+__device__ __forceinline__ df df_add_f(df a, float x) {
+    const float s = a.hi + x;
+    const float bv = s - a.hi;
+    float e = (a.hi - (s - bv)) + (x - bv);
+    e = e + a.lo;
+    const float s2 = s + e;
+    return df{s2, e - (s2 - s)};
+}
+template <int LANES = ROW_LANES, int U = 4, class F>
+__device__ __forceinline__ float row_sum64(int n, F term) {
     df s = df_of(0.0f);
-    for (int i = (int)threadIdx.x % ROW_LANES; i < n; i += ROW_LANES) s = df_add(s, df_of(term(i)));
-    for (int o = ROW_LANES / 2; o > 0; o >>= 1) s = df_add(s, df_shfl_xor(s, o));
+#pragma unroll 1
+    for (int i0 = (int)threadIdx.x % LANES; i0 < n; i0 += LANES * U) {
+        float v[U];
+#pragma unroll
+        for (int q = 0; q < U; ++q) v[q] = i0 + LANES * q < n ? term(i0 + LANES * q) : 0.0f;
+#pragma unroll
+        for (int q = 0; q < U; ++q) s = df_add_f(s, v[q]);
+    }
+#pragma unroll
+    for (int o = LANES / 2; o > 0; o >>= 1) s = df_add(s, df_shfl_xor(s, o));
     return df_val(s);
 }
-// Calls row(r, l, on) for the rows r of [0, nrow) with the eight lanes
-// l = 0..7 of each; on is false for the lanes past the last row, which take
-// part in the warp's shuffles only.
-template <class F>
-__device__ inline void for_rows(int nrow, F row) {
-    const int step = (int)blockDim.x / ROW_LANES, warp0 = (int)(threadIdx.x & ~31u) / ROW_LANES;
-    int r = (int)threadIdx.x / ROW_LANES;
-    for (int r0 = warp0; r0 < nrow; r0 += step, r += step) row(r, (int)threadIdx.x % ROW_LANES, r < nrow);
+// Calls row(r, l, on) for the rows r of [0, nrow) with the lanes l of each;
+// on is false for the lanes past the last row, which take part in the warp's
+// shuffles only.
+template <int LANES = ROW_LANES, class F>
+__device__ __forceinline__ void for_rows(int nrow, F row) {
+    const int step = (int)blockDim.x / LANES, warp0 = (int)(threadIdx.x & ~31u) / LANES;
+    int r = (int)threadIdx.x / LANES;
+#pragma unroll 1
+    for (int r0 = warp0; r0 < nrow; r0 += step, r += step) row(r, (int)threadIdx.x % LANES, r < nrow);
 }
 
 // ---------------------------------------------------------------------
@@ -112,7 +133,8 @@ __global__ void __launch_bounds__(BS, 1024 / BS) k_ts_cells(const __grid_constan
     const int nc = IMM1 * KMM1;
     float *st = sm;              // STORE of this plane, [k-1][i-1]
     float *lsum = sm + nc;       // per-K line sums
-    float *fdir = lsum + KMM1 + d.NIB1 * d.NKB1;     // and, at a mixing plane, the flow's direction
+    // at a mixing plane: the flow's direction on each line, the pitchwise weights
+    float *fdir = lsum + KMM1 + d.NIB1 * d.NKB1, *fp = fdir + KMM1;
     const PlaneInfo &pl = d.PLANE[j - 1];
     const int role = pl.role, jmx = pl.jmx, kts = pl.kts, kte = pl.kte;
     const float RATPITCH = pl.ratpitch;
@@ -121,29 +143,32 @@ __global__ void __launch_bounds__(BS, 1024 / BS) k_ts_cells(const __grid_constan
     const int n1 = d.NIB1 * d.NKB1, n2 = d.NIB2 * d.NKB2;
     const int4 blk1 = d.MG1X[min((int)threadIdx.x, n1 - 1)], blk2 = d.MG2X[min((int)threadIdx.x, n2 - 1)];
     if (role) {
-        // the flow direction on each line of the mixing plane
-        for (int k = threadIdx.x + 1; k <= KMM1; k += BS) fdir[k - 1] = -A3(d.FLOWX, d.IMID, jmx, k);
-        // stage the XFLUX plane in shared memory (coalesced), then add each
-        // I-line that is extrapolated
-        const bool sums = role != 2 && !lowx;
-        if (sums) {
-            int jj = role == 1 ? j - 1 : j;
-            Walk2 wx(IMM1, threadIdx.x, BS);
-            for (int c = threadIdx.x; c < nc; c += BS, wx.next()) st[c] = A3(V.XF, wx.i, jj, wx.k);
-        }
-        __syncthreads();
-        auto wanted = [&](int k) { return (role == 1) == (fdir[k - 1] > 0.0f); };
-        if (sums && d.REDUCE_ORDER != 0) {
-            for (int k = threadIdx.x + 1; k <= KMM1; k += BS)
-                if (wanted(k)) lsum[k - 1] = mp_line_sum(st + (k - 1) * IMM1, IMM1);
-        } else if (sums) {
-            for_rows(KMM1, [&](int r, int l, bool on) {
-                on = on && wanted(r + 1);
-                if (!__any_sync(0xffffffffu, on)) return;
-                const float *row = st + r * IMM1;
-                const float s = row_sum64(on ? IMM1 : 0, [&](int i) { return row[i]; });
-                if (on && l == 0) lsum[r] = s;
-            });
+        auto flow = [&](int k) { return -A3(d.FLOWX, d.IMID, jmx, k); };
+        for (int k = threadIdx.x + 1; k <= KMM1; k += BS) fdir[k - 1] = flow(k);
+        for (int i = threadIdx.x + 1; i <= IMM1; i += BS) fp[i - 1] = A1(d.FP, i);
+        // each I-line's XFLUX is added where it is extrapolated: read
+        // straight from memory, four lanes a row so that a round takes 64
+        // rows, the terms of a row in one latency
+        if (role != 2 && !lowx) {
+            const float *xj = V.XF + IM * (role == 1 ? j - 2 : j - 1);
+            const int kx = IM * d.JM;
+            if (d.REDUCE_ORDER == 0) {
+                for_rows<4>(KMM1, [&](int r, int l, bool on) {
+                    // after the plane (role 3) only against the flow, which is rare
+                    if (role == 3 && !__any_sync(0xffffffffu, on && !(flow(r + 1) > 0.0f))) return;
+                    const float *row = xj + kx * r;
+                    const float s = row_sum64<4, 16>(on ? IMM1 : 0, [&](int i) { return row[i]; });
+                    if (on && l == 0) lsum[r] = s;
+                });
+            } else {
+                // stage the XFLUX plane in shared memory (coalesced), then
+                // add each I-line in the reference's order
+                Walk2 wx(IMM1, threadIdx.x, BS);
+                for (int c = threadIdx.x; c < nc; c += BS, wx.next()) st[c] = xj[(wx.i - 1) + kx * (wx.k - 1)];
+                __syncthreads();
+                for (int k = threadIdx.x + 1; k <= KMM1; k += BS)
+                    if ((role == 1) == (fdir[k - 1] > 0.0f)) lsum[k - 1] = mp_line_sum(st + (k - 1) * IMM1, IMM1);
+            }
         }
         __syncthreads();
     }
@@ -194,9 +219,9 @@ __global__ void __launch_bounds__(BS, 1024 / BS) k_ts_cells(const __grid_constan
             float src = sr[u];
             if (role && !lowx) {
                 const float FLOWDIRN = fdir[k - 1];
-                if (role == 1 && FLOWDIRN > 0.0f) src = src - (xm[u] - lsum[k - 1] * A1(d.FP, i)) * d.FEXTRAP;
+                if (role == 1 && FLOWDIRN > 0.0f) src = src - (xm[u] - lsum[k - 1] * fp[i - 1]) * d.FEXTRAP;
                 if (role == 2) src = 0.0f;
-                if (role == 3 && !(FLOWDIRN > 0.0f)) src = src + (xf[u] - lsum[k - 1] * A1(d.FP, i)) * d.FEXTRAP;
+                if (role == 3 && !(FLOWDIRN > 0.0f)) src = src + (xf[u] - lsum[k - 1] * fp[i - 1]) * d.FEXTRAP;
             }
             float DELTA = xf[u] - xm[u] * RATPITCH + rf[u] - rk[u] + t0 - t1 - src;
             st[c] = F1 * DELTA + F2 * df[u];
@@ -214,7 +239,7 @@ __global__ void __launch_bounds__(BS, 1024 / BS) k_ts_cells(const __grid_constan
                 if (!averaged(k)) continue;
                 float *row = st + (k - 1) * IMM1;
                 const float s = mp_line_sum(row, IMM1);
-                for (int i = 0; i < IMM1; ++i) row[i] = s * A1(d.FP, i + 1);
+                for (int i = 0; i < IMM1; ++i) row[i] = s * fp[i];
             }
         } else {
             for_rows(KMM1, [&](int r, int l, bool on) {
@@ -223,7 +248,7 @@ __global__ void __launch_bounds__(BS, 1024 / BS) k_ts_cells(const __grid_constan
                 float *row = st + r * IMM1;
                 const int n = on ? IMM1 : 0;
                 const float s = row_sum64(n, [&](int i) { return row[i]; });
-                for (int i = l; i < n; i += ROW_LANES) row[i] = s * A1(d.FP, i + 1);
+                for (int i = l; i < n; i += ROW_LANES) row[i] = s * fp[i];
             });
         }
         __syncthreads();
@@ -581,20 +606,21 @@ __global__ void __launch_bounds__(UP_T, 3) k_ts_update(const __grid_constant__ D
         for (int q = 0; q < UP_S; ++q)
             if (q < kn) dv[q] = D[nn + IM * (j - ja) + ks * q];
     };
-    // damped cells of plane jc = ja + p into its tile
-    auto damp_cells = [&](int p) {
+    // the flow's direction on row r of the tile, in a plane at a mixing plane
+    auto flow = [&](int p, int r) {
+        const int k = k0 - 1 + r;
+        const bool mp = s_role[p] == 1 || s_role[p] == 3;
+        return mp && r <= rows && k >= 1 && k <= KMM1 ? -A3(d.FLOWX, d.IMID, s_jmx[p], k) : 0.0f;
+    };
+    // damped cells of plane jc = ja + p into its tile; fdir: the direction on
+    // this thread's first row
+    auto damp_cells = [&](int p, float fdir) {
         const int jc = ja + p;
         float *c = sm + (p & 1) * buf + il + 1;
         const bool pl = jc >= 2 && jc <= JM;
         const float blk = s_blk[p];
         const int role = s_role[p], nrow = rows + 1;
         const bool mp = role == 1 || role == 3;
-        // the flow's direction on a mixing plane's row r of the tile (0 off the grid)
-        auto flow = [&](int r) {
-            const int k = k0 - 1 + r;
-            return mp && r < nrow && k >= 1 && k <= KMM1 ? -A3(d.FLOWX, d.IMID, s_jmx[p], k) : 0.0f;
-        };
-        const float fdir = flow(tid / ROW_LANES);         // of this thread's first row, ahead of its use
         auto damped = [&](float v) {
             if (!damp_on) return v;
             const float FDAMP = fabsf(v) / blk;
@@ -616,14 +642,14 @@ __global__ void __launch_bounds__(UP_T, 3) k_ts_update(const __grid_constant__ D
         };
         if (d.REDUCE_ORDER != 0) {
             for (int r = tid; r < nrow; r += (int)blockDim.x) {
-                if (!averaged(r, flow(r))) continue;
+                if (!averaged(r, flow(p, r))) continue;
                 float *row = row0 + r * PW;
                 const float m = mp_line_sum(row, IMM1) / (float)IMM1;
                 for (int i = 0; i < IMM1; ++i) row[i] = m;
             }
         } else {
             for_rows(nrow, [&](int r, int l, bool on) {
-                on = on && averaged(r, r == tid / ROW_LANES ? fdir : flow(r));
+                on = on && averaged(r, r == tid / ROW_LANES ? fdir : flow(p, r));
                 if (!__any_sync(0xffffffffu, on)) return;
                 float *row = row0 + r * PW;
                 const int n = on ? IMM1 : 0;
@@ -678,15 +704,19 @@ __global__ void __launch_bounds__(UP_T, 3) k_ts_update(const __grid_constant__ D
         s_jmx[q] = pl.jmx;
     }
     __syncthreads();
-    damp_cells(0);
+    damp_cells(0, flow(0, tid / ROW_LANES));
     load_cells(ja + 1);
+    float fdir = flow(1, tid / ROW_LANES);
     load_nodes(ja);
     if (act) read_cells(0, ca);
 #pragma unroll 2
     for (int j = ja; j <= jb; ++j) {
         const int p = j - ja;
-        damp_cells(p + 1);
-        if (j < jb) load_cells(j + 2);
+        damp_cells(p + 1, fdir);
+        if (j < jb) {
+            load_cells(j + 2);
+            fdir = flow(p + 2, tid / ROW_LANES);
+        }
         if (!act) continue;
         read_cells(p + 1, cb);
         const float fd = s_fd[p], fu = s_fu[p + 1];
@@ -755,6 +785,24 @@ __global__ void __launch_bounds__(PBS, 1024 / PBS) k_ts_update_pair(const __grid
     const DevCtl *ctl = d.ctl;
     const int damp_on = ctl->damp_on;
     const float DAMP = ctl->DAMP;
+    const int ks = IM * JM;
+    // this thread's first cell of each cell plane, and what the planes are,
+    // before the row means below: the loads' latency overlaps theirs
+    float pre[3];
+    int prow[3], role[3], jmx[3];
+    {
+        const int k = (int)threadIdx.x / IMM1, n = (int)threadIdx.x - k * IMM1 + ks * k;
+#pragma unroll
+        for (int h = 0; h < 3; ++h) {
+            const int jc = j0 + h;
+            const bool in = jc >= 2 && jc <= JM;
+            const PlaneInfo &pl = d.PLANE[min(jc, JM) - 1];
+            prow[h] = pl.nrow;
+            role[h] = in ? pl.role : 0;
+            jmx[h] = pl.jmx;
+            pre[h] = in && (int)threadIdx.x < nc ? V.ST[n + IM * (jc - 1)] : 0.0f;
+        }
+    }
     if (damp_on) {
         if (d.REDUCE_ORDER == 1) {
             for (int r = threadIdx.x; r < d.NROWS; r += PBS) s_blk[r] = V.AVG_BLK[r];
@@ -773,16 +821,27 @@ __global__ void __launch_bounds__(PBS, 1024 / PBS) k_ts_update_pair(const __grid
         }
         __syncthreads();
     }
-    // damped cell changes of the cell planes j0, j0+1, j0+2 (those in 2..JM)
-    const int ks = IM * JM;
+    // damped cell changes of the cell planes j0, j0+1, j0+2 (those in 2..JM),
+    // and the flow's direction on this thread's first row of a mixing plane
+    float fdir[3];
+#pragma unroll
     for (int h = 0; h < 3; ++h) {
         const int jc = j0 + h;
+        const int k = (int)threadIdx.x / ROW_LANES + 1;
+        fdir[h] = (role[h] == 1 || role[h] == 3) && k <= KMM1 ? -A3(d.FLOWX, d.IMID, jmx[h], k) : 0.0f;
         if (jc < 2 || jc > JM) continue;
         float *c = sm + h * nc;
-        const float blk = damp_on ? s_blk[d.PLANE[jc - 1].nrow - 1] : 1.0f;
+        const float blk = damp_on ? s_blk[prow[h] - 1] : 1.0f;
+        auto damped = [&](float v) {
+            if (!damp_on) return v;
+            const float FDAMP = fabsf(v) / blk;
+            return v / (1.0f + FDAMP / DAMP);
+        };
+        if ((int)threadIdx.x < nc) c[threadIdx.x] = damped(pre[h]);
+        if (nc <= PBS) continue;
         const float *__restrict__ stp = V.ST + IM * (jc - 1);
-        Walk2 w(IMM1, threadIdx.x, PBS);
-        for (int t0 = threadIdx.x; t0 < nc; t0 += TS_UG * PBS) {
+        Walk2 w(IMM1, threadIdx.x + PBS, PBS);
+        for (int t0 = threadIdx.x + PBS; t0 < nc; t0 += TS_UG * PBS) {
             float sv[TS_UG];
 #pragma unroll
             for (int u = 0; u < TS_UG; ++u) {
@@ -793,12 +852,7 @@ __global__ void __launch_bounds__(PBS, 1024 / PBS) k_ts_update_pair(const __grid
             for (int u = 0; u < TS_UG; ++u) {
                 const int t = t0 + u * PBS;
                 if (t >= nc) break;
-                float v = sv[u];
-                if (damp_on) {
-                    float FDAMP = fabsf(v) / blk;
-                    v = v / (1.0f + FDAMP / DAMP);
-                }
-                c[t] = v;
+                c[t] = damped(sv[u]);
             }
         }
     }
@@ -806,16 +860,17 @@ __global__ void __launch_bounds__(PBS, 1024 / PBS) k_ts_update_pair(const __grid
     // second pitchwise average on the mixing-plane cells (1850)
     const bool lowx = d.FEXTRAP < 0.001f;
     bool any = false;
+#pragma unroll 1
     for (int h = 0; h < 3; ++h) {
-        const int jc = j0 + h;
-        if (jc < 2 || jc > JM) continue;
-        const int role = d.PLANE[jc - 1].role, jmx = d.PLANE[jc - 1].jmx;
-        if (role != 1 && role != 3) continue;
+        const int rl = h == 0 ? role[0] : h == 1 ? role[1] : role[2], jm = h == 0 ? jmx[0] : h == 1 ? jmx[1] : jmx[2];
+        if (rl != 1 && rl != 3) continue;
         any = true;
         float *c = sm + h * nc;
+        const float f0 = h == 0 ? fdir[0] : h == 1 ? fdir[1] : fdir[2];
         auto averaged = [&](int k) {
-            const float FLOWDIRN = -A3(d.FLOWX, d.IMID, jmx, k);
-            return role == 3 ? (FLOWDIRN > 0.0f || lowx) : (FLOWDIRN < 0.0f || lowx);
+            const float FLOWDIRN =
+                k == (int)threadIdx.x / ROW_LANES + 1 ? f0 : -A3(d.FLOWX, d.IMID, jm, k);
+            return rl == 3 ? (FLOWDIRN > 0.0f || lowx) : (FLOWDIRN < 0.0f || lowx);
         };
         if (d.REDUCE_ORDER != 0) {
             for (int k = threadIdx.x + 1; k <= KMM1; k += PBS) {
@@ -1004,7 +1059,10 @@ __global__ void __launch_bounds__(BS, 1024 / BS) k_ts_smooth(const __grid_consta
     const int j = blockIdx.x + 1;
     const PlaneInfo &pl = d.PLANE[j - 1];
     const DevCtl *c = d.ctl;
-    const bool stream = !(c->SFX < 0.0001f);
+    const bool stream = !(c->SFX < 0.0001f), mix = pl.mix != 0;
+    // the pitchwise weight that this thread puts into shared memory for a
+    // mixing plane's average, ahead of its use
+    const float fpw = mix && (int)threadIdx.x < IMM1 ? d.FP[threadIdx.x] : 0.0f;
     for (int t = threadIdx.x; t < IM; t += BS) {
         cFD[t] = d.FD[t];
         cFU[t] = d.FU[t];
@@ -1213,28 +1271,30 @@ __global__ void __launch_bounds__(BS, 1024 / BS) k_ts_smooth(const __grid_consta
             P(a, IM, k) = v;
         }
     }
+    if (mix)                       // the smoothing is done with cFU
+        for (int i = threadIdx.x; i < IMM1; i += BS) cFU[i] = i < BS ? fpw : d.FP[i];
     __syncthreads();
-    if (pl.mix) {
+    float *Dj = D + IM * (j - 1);
+    if (mix) {
         if (d.REDUCE_ORDER != 0) {
             for (int k = threadIdx.x + 1; k <= KM; k += BS) {
                 float s = 0.0f;
-                for (int i = 1; i <= IMM1; ++i) s = s + A1(d.FP, i) * (P(a, i, k) + P(a, i + 1, k));
+                for (int i = 1; i <= IMM1; ++i) s = s + cFU[i - 1] * (P(a, i, k) + P(a, i + 1, k));
                 b[k - 1] = 0.5f * s;
             }
         } else {
             for_rows(KM, [&](int r, int l, bool on) {
-                const int k = r + 1;
-                const float s = row_sum64(on ? IMM1 : 0, [&](int i) { return A1(d.FP, i + 1) * (P(a, i + 1, k) + P(a, i + 2, k)); });
+                const float *row = a + IMP * r;
+                const float s = row_sum64(on ? IMM1 : 0, [&](int i) { return cFU[i] * (row[i] + row[i + 1]); });
                 if (on && l == 0) b[r] = 0.5f * s;
             });
         }
         __syncthreads();
         Walk2 w(IM, threadIdx.x, BS);
-        for (int t = threadIdx.x; t < np; t += BS, w.next()) P(a, w.i, w.k) = b[w.k - 1];
-        __syncthreads();
+        for (int t = threadIdx.x; t < np; t += BS, w.next()) Dj[(w.i - 1) + ks * (w.k - 1)] = b[w.k - 1];
+        return;
     }
 #undef P
-    float *Dj = D + IM * (j - 1);
     Walk2 w(IM, threadIdx.x, BS);
     for (int t = threadIdx.x; t < np; t += BS, w.next()) Dj[(w.i - 1) + ks * (w.k - 1)] = a[(w.i - 1) + IMP * (w.k - 1)];
 }
@@ -1297,7 +1357,7 @@ __global__ void k_copy_tm_st(const __grid_constant__ Dev d, int v0, size_t n) {
 static bool pair_update(const Dev &d) { return d.TS_PAIR && (d.in_batch || d.IM * d.KM <= 512); }
 
 static size_t cells_smem(const Dev &d) {
-    return ((size_t)d.IMM1 * d.KMM1 + 2 * d.KMM1 + (size_t)d.NIB1 * d.NKB1) * sizeof(float);
+    return ((size_t)d.IMM1 * d.KMM1 + 2 * d.KMM1 + d.IMM1 + (size_t)d.NIB1 * d.NKB1) * sizeof(float);
 }
 static size_t prolong_smem(const Dev &d) { return ((size_t)d.NIB1 * d.NKB1 + (size_t)d.NIB2 * d.NKB2) * sizeof(float); }
 static size_t update_pair_smem(const Dev &d) { return (size_t)3 * d.IMM1 * d.KMM1 * sizeof(float); }
