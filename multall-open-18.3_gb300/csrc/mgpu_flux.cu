@@ -77,18 +77,18 @@ void launch_step_begin(const Dev &d, Launch L) {
 // ---------------------------------------------------------------------
 constexpr int PRIM_BS = 256;
 
-// One thread a node; the first grid_for(N) CTAs.  what >= 0: one more CTA
-// runs the step control, whose only effect on this kernel, the tail flag,
-// the host knows already.  On a step with the tail the last CTA turns the
-// partial sums into VREF and VMAX.
+// One thread a node.  what >= 0: one more CTA, the first, runs the step
+// control, whose only effect on this kernel, the tail flag, the host knows
+// already.  On a step with the tail the CTAs leave their sums
+// and maxima of |W|^2, which a CTA of k_tail_flow turns into VREF and VMAX.
 __global__ void __launch_bounds__(PRIM_BS) k_prim(const __grid_constant__ Dev d, int what) {
     pdl_wait();
-    const unsigned nblk = gridDim.x - (what >= 0 ? 1 : 0);
-    if (blockIdx.x == nblk) {
+    const unsigned ctl = what >= 0 ? 1 : 0, blk = blockIdx.x - ctl;
+    if (blockIdx.x < ctl) {
         if (threadIdx.x == 0) step_control(d);
         return;
     }
-    size_t n = (size_t)blockIdx.x * PRIM_BS + threadIdx.x;
+    size_t n = (size_t)blk * PRIM_BS + threadIdx.x;
     size_t N = (size_t)d.IM * d.JM * d.KM;
     const bool do_tail = what >= 0 ? (what & 2) != 0 : d.ctl->do_tail != 0;
     float eke_s = 0.0f;
@@ -130,29 +130,8 @@ __global__ void __launch_bounds__(PRIM_BS) k_prim(const __grid_constant__ Dev d,
     df s;
     cta_sum_key<PRIM_BS>(d.REDUCE_ORDER, df_of(eke_s), key, &s, &key);
     if (threadIdx.x == 0) {
-        d.part_sum[blockIdx.x] = s;
-        d.part_key[blockIdx.x] = key;
-    }
-    if (!last_cta(&d.ctl->ticket, nblk)) return;
-    s = df_of(0.0f);
-    key = 0ull;
-    for (unsigned p = threadIdx.x; p < nblk; p += PRIM_BS) {
-        s = dacc(d.REDUCE_ORDER, s, d.part_sum[p]);
-        const unsigned long long k2 = d.part_key[p];
-        key = k2 > key ? k2 : key;
-    }
-    cta_sum_key<PRIM_BS>(d.REDUCE_ORDER, s, key, &s, &key);
-    if (threadIdx.x == 0) {
-        DevCtl *c = d.ctl;
-        c->VREF = sqrtf(df_val(s) * d.RIJKM);
-        c->VMAX = 0.0f;
-        if (key) {
-            const unsigned lin = 0xFFFFFFFFu - (unsigned)(key & 0xFFFFFFFFull);
-            c->VMAX = sqrtf(__uint_as_float((unsigned)(key >> 32)));
-            c->IVMAX = (int)(lin % d.IM) + 1;
-            c->JVMAX = (int)((lin / d.IM) % d.JM) + 1;
-            c->KVMAX = (int)(lin / ((unsigned)d.IM * d.JM)) + 1;
-        }
+        d.part_sum[blk] = s;
+        d.part_key[blk] = key;
     }
 }
 

@@ -739,10 +739,51 @@ void launch_loss(const Dev &d, Launch L, bool init_call) {
 // ---------------------------------------------------------------------
 constexpr int TAIL_BS = 256;
 
-__global__ void __launch_bounds__(TAIL_BS) k_tail_flow(Dev d) {
+// Sum and largest key of the partial sums and keys that an earlier launch's n
+// CTAs left, in warp 0.  The sums of a launch are finished by one CTA of the
+// next launch that has room for it: the last CTA of the launch itself would
+// be found by a ticket (a fence and an atomic each, 3000 CTAs on the stage)
+// and would run alone, 8 us at the end of k_prim and 3 us after the node pass.
+__device__ __forceinline__ void finish_parts(const Dev &d, int n, df *s, unsigned long long *key) {
+    df t = df_of(0.0f);
+    unsigned long long m = 0ull;
+#pragma unroll 4
+    for (int p = threadIdx.x; p < n; p += TAIL_BS) {
+        t = dacc(d.REDUCE_ORDER, t, d.part_sum[p]);
+        const unsigned long long k2 = d.part_key[p];
+        m = k2 > m ? k2 : m;
+    }
+    cta_sum_key<TAIL_BS>(d.REDUCE_ORDER, t, m, s, key);
+}
+
+// VREF and VMAX from k_prim's n partial sums of |W|^2
+__device__ void finish_vref(const Dev &d, int n) {
+    df s;
+    unsigned long long key;
+    finish_parts(d, n, &s, &key);
+    if (threadIdx.x == 0) {
+        DevCtl *c = d.ctl;
+        c->VREF = sqrtf(df_val(s) * d.RIJKM);
+        c->VMAX = 0.0f;
+        if (key) {
+            const unsigned lin = 0xFFFFFFFFu - (unsigned)(key & 0xFFFFFFFFull);
+            c->VMAX = sqrtf(__uint_as_float((unsigned)(key >> 32)));
+            c->IVMAX = (int)(lin % d.IM) + 1;
+            c->JVMAX = (int)((lin / d.IM) % d.JM) + 1;
+            c->KVMAX = (int)(lin / ((unsigned)d.IM * d.JM)) + 1;
+        }
+    }
+}
+
+// FLOW(J), a CTA a plane; one more CTA, the first, forms VREF and VMAX
+__global__ void __launch_bounds__(TAIL_BS) k_tail_flow(const __grid_constant__ Dev d, int nprim) {
     pdl_wait();
     if (!d.ctl->do_tail) return;
-    int j = blockIdx.x + 1;
+    if (blockIdx.x == 0) {
+        finish_vref(d, nprim);
+        return;
+    }
+    int j = blockIdx.x;
     int ncell = d.IMM1 * d.KMM1;
     const int ro = d.REDUCE_ORDER;
     double s = 0.0;
@@ -785,10 +826,9 @@ __device__ __forceinline__ float stepup_node(const Dev &d, StepupLimits q, float
 // health count, and STEPUP's node values (TEMP1).  Each thread takes npt <=
 // TAIL_NPT nodes (TAIL_BS apart, so the loads stay coalesced), two at a time
 // with all loads of the two in flight, and adds their |DVMER| in FP32 before
-// the CTA's sum.  npt is what leaves four CTAs an SM: a grid that cannot fill
+// the CTA's sum (k_stepup_cell finishes the sums).  npt is what leaves four CTAs an SM: a grid that cannot fill
 // the GPU takes one node a thread (TAIL_NPT on every grid made the node pass
-// of 3150 nodes, on two CTAs, four latencies long).  The last CTA forms EAVG,
-// EMAX and the continuity error ECONT.
+// of 3150 nodes, on two CTAs, four latencies long).
 constexpr int TAIL_NPT = 8;
 
 __global__ void __launch_bounds__(TAIL_BS) k_tail_nodes(const __grid_constant__ Dev d, int npt) {
@@ -833,16 +873,14 @@ __global__ void __launch_bounds__(TAIL_BS) k_tail_nodes(const __grid_constant__ 
         d.part_key[blockIdx.x] = key;
         d.part_cnt[blockIdx.x] = bad;
     }
-    if (!last_cta(&c->ticket, gridDim.x)) return;
-    s = df_of(0.0f);
-    key = 0ull;
-    bad = 0;
-    for (unsigned p = threadIdx.x; p < gridDim.x; p += TAIL_BS) {
-        s = dacc(ro, s, d.part_sum[p]);
-        const unsigned long long k2 = d.part_key[p];
-        key = k2 > key ? k2 : key;
-        bad += d.part_cnt[p];
-    }
+}
+
+// EAVG, EMAX, the health count and the continuity error ECONT from the node
+// pass's n partial sums and FLOW(J)
+__device__ void finish_tail(const Dev &d, int n) {
+    DevCtl *c = d.ctl;
+    int bad = 0;
+    for (int p = threadIdx.x; p < n; p += TAIL_BS) bad += d.part_cnt[p];
     // the continuity error ECONT = max over J of |1 - FLOW(J)/FLOW(1)| and
     // the first J that reaches it, one J per thread as a (value, J) key
     unsigned long long ek = 0ull;
@@ -865,7 +903,9 @@ __global__ void __launch_bounds__(TAIL_BS) k_tail_nodes(const __grid_constant__ 
         se[threadIdx.x >> 5] = ek;
         sc[threadIdx.x >> 5] = bad;
     }
-    cta_sum_key<TAIL_BS>(ro, s, key, &s, &key);
+    df s;
+    unsigned long long key;
+    finish_parts(d, n, &s, &key);
     if (threadIdx.x == 0) {
         unsigned long long ke = 0ull;
         int cnt = 0;
@@ -918,10 +958,19 @@ __global__ void k_stepup_node(const __grid_constant__ Dev d) {
 // One thread a cell.  The cell of J = JMIX+1 takes the step of JMIX+2, whose
 // thread writes both: STEP is then read only by the thread that writes it,
 // and needs no second pass.
-__global__ void k_stepup_cell(const __grid_constant__ Dev d, float RELAX, int gated) {
+// ntail > 0, in the tail: the node pass left ntail partial sums; one more CTA
+// (of TAIL_BS threads), the first, finishes them.
+__global__ void __launch_bounds__(TAIL_BS) k_stepup_cell(const __grid_constant__ Dev d, float RELAX, int ntail) {
     pdl_wait();
-    if (gated && (!d.ctl->do_tail || d.FROZEN)) return;
-    size_t n = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (ntail > 0) {
+        if (!d.ctl->do_tail) return;
+        if (blockIdx.x == 0) {
+            finish_tail(d, ntail);
+            return;
+        }
+        if (d.FROZEN) return;
+    }
+    size_t n = (size_t)(blockIdx.x - (ntail > 0 ? 1 : 0)) * blockDim.x + threadIdx.x;
     size_t N = (size_t)d.IM * d.JM * d.KM;
     if (n >= N) return;
     int i, j, k;
@@ -950,26 +999,28 @@ __global__ void k_stepup_cell(const __grid_constant__ Dev d, float RELAX, int ga
     }
 }
 
-static void launch_stepup_cell(const Dev &d, Launch L, float relax, bool gated) {
-    launchk(L, k_stepup_cell, dim3(grid_for((size_t)d.IM * d.JM * d.KM, 256)), dim3(256), 0, d, relax, gated ? 1 : 0);
+static void launch_stepup_cell(const Dev &d, Launch L, float relax, int ntail) {
+    const unsigned g = grid_for((size_t)d.IM * d.JM * d.KM, TAIL_BS) + (ntail > 0 ? 1 : 0);
+    launchk(L, k_stepup_cell, dim3(g), dim3(TAIL_BS), 0, d, relax, ntail);
     mark(L, "k_stepup_cell");
 }
 
 void launch_stepup(const Dev &d, Launch L, float relax) {
     launchk(L, k_stepup_node, dim3(grid_for((size_t)d.IM * d.JM * d.KM, 256)), dim3(256), 0, d);
     mark(L, "k_stepup_node");
-    launch_stepup_cell(d, L, relax, false);
+    launch_stepup_cell(d, L, relax, 0);
 }
 
 // the tail: monitors, then STEPUP(0.25)
 void launch_tail(const Dev &d, Launch L) {
-    launchk(L, k_tail_flow, dim3(d.JM), dim3(TAIL_BS), 0, d);
-    mark(L, "k_tail_flow");
     size_t N = (size_t)d.IM * d.JM * d.KM;
+    launchk(L, k_tail_flow, dim3(d.JM + 1), dim3(TAIL_BS), 0, d, (int)grid_for(N, 256));
+    mark(L, "k_tail_flow");
     const int npt = (int)std::min<size_t>(TAIL_NPT, std::max<size_t>(1, N / ((size_t)TAIL_BS * 4 * L.sm_count)));
-    launchk(L, k_tail_nodes, dim3(grid_for(N, (size_t)TAIL_BS * npt)), dim3(TAIL_BS), 0, d, npt);
+    const int ntail = (int)grid_for(N, (size_t)TAIL_BS * npt);
+    launchk(L, k_tail_nodes, dim3(ntail), dim3(TAIL_BS), 0, d, npt);
     mark(L, "k_tail_nodes");
-    launch_stepup_cell(d, L, 0.25f, true);
+    launch_stepup_cell(d, L, 0.25f, ntail);
 }
 
 // ---------------------------------------------------------------------
