@@ -330,6 +330,36 @@ struct WalkN {
     }
 };
 
+// The same walk by 32-bit byte offsets, for arrays of 4-byte elements
+// (mgpu_create keeps a node array within 2^32 bytes).  at() adds such an
+// offset to the array's base: with a base that all threads share, the
+// address is one uniform and one 32-bit register, where an element index is
+// widened and scaled for each access.
+struct WalkB {
+    int i, di, ni;
+    unsigned b, db, dw;
+    __device__ WalkB(int ni_, int ks, int n0, int start, int stride) : ni(ni_) {
+        const int k = start / ni_, dk = stride / ni_;
+        i = start - k * ni_;
+        b = 4u * (unsigned)(n0 + i + ks * k);
+        di = stride - dk * ni_;
+        db = 4u * (unsigned)(di + ks * dk);
+        dw = 4u * (unsigned)(ks - ni_);
+    }
+    __device__ void next() {
+        i += di;
+        b += db;
+        if (i >= ni) {
+            i -= ni;
+            b += dw;
+        }
+    }
+};
+template <class T>
+__device__ __forceinline__ T *at(T *p, unsigned b) {
+    return reinterpret_cast<T *>(reinterpret_cast<uintptr_t>(p) + b);
+}
+
 // Order-preserving key for "largest value, earliest index wins": the value
 // must be >= 0 (squares, absolute values); NaN counts as smallest.
 __device__ inline unsigned long long max_key(float v, size_t lin) {

@@ -39,8 +39,8 @@ static inline unsigned grid_for(size_t n, unsigned block) { return (unsigned)((n
 constexpr int TS_U = 3;          // cells per thread whose loads are issued together
 constexpr int SV_U = 3;          // points per thread whose streamwise loads are issued together
 constexpr int SM_SEG = 8;        // points per thread of one pitchwise or spanwise smoothing segment
-constexpr int PR_U = 2;          // the same in prolong, whose 40 registers leave 1536 threads an SM (three cells
-                                 // and 1280 threads: 18 us a launch against 16 at 65 x 242 x 49)
+constexpr int PR_U = 3;          // the same in prolong: five CTAs an SM at 48 registers (two cells and six CTAs: 38.9 us
+                                 // a launch against 37.6 on the 33 x 752 x 66 compressor, 16.5 against 15.8 at 65 x 242 x 49)
 constexpr int TS_UG = 4;         // cells per thread whose loads the pair update issues together
 constexpr int UG_SEG = 3;        // nodes per thread of one K column in the pair update's gather
 constexpr int UP_S = 3;          // nodes along K of one thread of update
@@ -382,7 +382,7 @@ __device__ __forceinline__ float plane_partials_sum(const float *__restrict__ P,
 // 120 instructions and six dependent loads of it.
 // ---------------------------------------------------------------------
 template <int BS>
-__global__ void __launch_bounds__(BS, 1536 / BS) k_ts_prolong(const __grid_constant__ Dev d, int v0, int want_abs) {
+__global__ void __launch_bounds__(BS, 1280 / BS) k_ts_prolong(const __grid_constant__ Dev d, int v0, int want_abs) {
     pdl_wait();
     extern __shared__ float sm[];
     const VarSet &V = d.var[v0 + blockIdx.y];
@@ -403,19 +403,20 @@ __global__ void __launch_bounds__(BS, 1536 / BS) k_ts_prolong(const __grid_const
     // operands of this thread's first PR_U cells, loaded before the block
     // sums so their latency overlaps the assembly below
     float pst[PR_U], pstp[PR_U], prs[PR_U];
-    int pb1[PR_U], pb2[PR_U], pn[PR_U];
-    WalkN w(IMM1, d.IM * d.JM, d.IM * (j - 1), threadIdx.x, BS);
+    int pb1[PR_U], pb2[PR_U];
+    unsigned pn[PR_U];
+    WalkB w(IMM1, d.IM * d.JM, d.IM * (j - 1), threadIdx.x, BS);
     auto load = [&](int c0) {
 #pragma unroll
         for (int u = 0; u < PR_U; ++u) {
             const int c = c0 + u * BS;
-            pn[u] = w.n;
+            pn[u] = w.b;
             if (c < nc) {
-                pst[u] = ST[w.n];
-                pstp[u] = STEP[w.n];
-                prs[u] = RSTEP[w.n];
-                pb1[u] = d.CB1[c];
-                pb2[u] = nested ? 0 : d.CB2[c];
+                pst[u] = *at(ST, w.b);
+                pstp[u] = *at(STEP, w.b);
+                prs[u] = *at(RSTEP, w.b);
+                pb1[u] = *at(d.CB1, 2u * (unsigned)c);
+                pb2[u] = nested ? 0 : *at(d.CB2, 2u * (unsigned)c);
             }
             w.next();
         }
@@ -474,7 +475,7 @@ __global__ void __launch_bounds__(BS, 1536 / BS) k_ts_prolong(const __grid_const
             if (c0 + u * BS >= nc) break;
             const float corr = nested ? b1[pb1[u]] : b1[pb1[u]] + b2[pb2[u]] + SB;
             const float DELTA = pst[u] * pstp[u] + corr * prs[u];
-            ST[pn[u]] = DELTA;
+            *at(ST, pn[u]) = DELTA;
             sabs += fabsf(DELTA);
         }
     }
