@@ -203,6 +203,7 @@ __global__ void __launch_bounds__(32) k_pwallgrad_smooth(const __grid_constant__
 // transition scans run one thread per column in the reference's order.
 // ---------------------------------------------------------------------
 constexpr int LK_W = 8;            // warps per CTA (K stride)
+constexpr int LK_U = 3;            // faces per thread whose loads are issued together
 constexpr int LK_NARR = 7;         // [K][32] arrays in shared memory (+ RAVG per K): 5 CTAs per SM at KM = 49
 
 __global__ void __launch_bounds__(32 * LK_W, 5) k_loss_kfaces(const __grid_constant__ Dev d, int init_call) {
@@ -218,9 +219,11 @@ __global__ void __launch_bounds__(32 * LK_W, 5) k_loss_kfaces(const __grid_const
     // [K][32] arrays, row k-1
     float *AREA = lsm, *VXAVG = AREA + KM * 32, *VRAVG = VXAVG + KM * 32, *VTAVG = VRAVG + KM * 32;
     float *TAVG = VTAVG + KM * 32, *VLAM = TAVG + KM * 32, *VTURB = VLAM + KM * 32, *RAVGK = VTURB + KM * 32;
-    float *ROAVG = VTURB;        // until step 4 turns each face's density into its viscosity; RAVGK: [K] only
-    __shared__ float s_vis[32], s_ftc[32], s_tw1[32], s_twm[32];
+    float *ROAVG = VTURB;        // until step 3 turns each face's density into its viscosity; RAVGK: [K] only
+    __shared__ float s_vis[32], s_tw1[32], s_twm[32];
     __shared__ float s_w1[32][4], s_wm[32][4];     // wall-face xs, rs, ts, wv at K=1 and K=KM
+    __shared__ unsigned s_tr[32];                  // where a column's viscosity ratio exceeds FTRANS
+    if (ty == 0) s_tr[tx] = 0u;
 #define LK(a, k) a[((k) - 1) * 32 + tx]
     const float RF_VIS = init_call ? 1.0f : d.RF_VIS;
     const float FMIXUP = init_call ? 1.0f : c->FMIXUP;
@@ -251,12 +254,8 @@ __global__ void __launch_bounds__(32 * LK_W, 5) k_loss_kfaces(const __grid_const
         return sqrtf(LK(VXAVG, k) * LK(VXAVG, k) + LK(VRAVG, k) * LK(VRAVG, k) + WTB * WTB);
     };
     if (ty == 0 && col) {
-        float VISLAM = c->VISLAM, FTCOND = c->FTCOND;
-        if (d.REYNO < 0.0001f) {
-            VISLAM = (fabsf(d.REYNO) / 100000.0f) * powf(LK(TAVG, KMID) / 288.0f, 0.62f);
-            float TCOND = d.CP * VISLAM / d.PRANDTL;
-            FTCOND = TCOND / VISLAM;
-        }
+        float VISLAM = c->VISLAM;
+        if (d.REYNO < 0.0001f) VISLAM = (fabsf(d.REYNO) / 100000.0f) * powf(LK(TAVG, KMID) / 288.0f, 0.62f);
         float TWALLK1, TWALLKM;
         if (d.YPLUSWALL < -0.001f) {
             float PERPK1 = A3(d.VOL, i, j, 1) / LK(AREA, 1);
@@ -287,7 +286,6 @@ __global__ void __launch_bounds__(32 * LK_W, 5) k_loss_kfaces(const __grid_const
             TWALLKM = d.CFWALL * LK(ROAVG, KM) * wb * wb;
         }
         s_vis[tx] = VISLAM;
-        s_ftc[tx] = FTCOND;
         s_tw1[tx] = TWALLK1;
         s_twm[tx] = TWALLKM;
         // the two wall faces (K=1 hub, K=KM casing)
@@ -309,81 +307,105 @@ __global__ void __launch_bounds__(32 * LK_W, 5) k_loss_kfaces(const __grid_const
         s_wm[tx][3] = tsm * WTIP * RAVGK[KM - 1];
     }
     __syncthreads();
-    // 3. Y_PLUS from the wall nearer in K
-    if (col) {
-        const float VISLAM = s_vis[tx];
-        const float VS1 = sqrtf(s_tw1[tx] / LK(ROAVG, 1)), VSM = sqrtf(s_twm[tx] / LK(ROAVG, KM));
-        for (int k = ty + 1; k <= KMM1; k += LK_W) {
-            float PERP = sqrtf(A3(d.DWALLSQ, i, j, k));
-            float y = k <= KMID ? VS1 * PERP * LK(ROAVG, 1) / VISLAM : VSM * PERP * LK(ROAVG, KM) / VISLAM;
-            y = fminf(y, 1000.0f);
-            A3(d.Y_PLUS, i, j, k) = y;
-        }
-    }
-    __syncthreads();
-    // 4. laminar and mixing-length viscosities of the interior faces.  The
-    //    relative speed of the faces is formed again here, and Y_PLUS is read
-    //    back from this CTA's own stores of step 3 (visible after the
-    //    barrier): K-arrays fewer in shared memory let five CTAs share an SM
+    // 3. Y_PLUS from the wall nearer in K, the laminar and mixing-length
+    //    viscosities of the interior faces, and each face's side of the
+    //    transition test.  LK_U faces at a time, their global operands loaded
+    //    together and before the stores of Y_PLUS: with Y_PLUS a pass of its
+    //    own, read back by this one, and the test a walk of one warp along
+    //    each column, a third of the kernel was waiting
     auto wabs = [&](int kq) {
         float WTAVG = LK(VTAVG, kq) - WREL * RAVGK[kq - 1];
         return sqrtf(LK(VXAVG, kq) * LK(VXAVG, kq) + LK(VRAVG, kq) * LK(VRAVG, kq) + WTAVG * WTAVG);
     };
+    bool walk = KMID < 2;          // a ratio that the test below does not cover
     if (col) {
         const float VISLAM = s_vis[tx];
-        // two faces at a time, their global operands loaded together
-        for (int k0 = ty + 2; k0 <= KMM1; k0 += 2 * LK_W) {
-            float yp[2], vol[2], fl[2], ft[2];
+        const float ro1 = LK(ROAVG, 1), rom = LK(ROAVG, KM);
+        const float VS1 = sqrtf(s_tw1[tx] / ro1), VSM = sqrtf(s_twm[tx] / rom);
+        auto yplus = [&](int k, float dwallsq) {
+            float PERP = sqrtf(dwallsq);
+            float y = k <= KMID ? VS1 * PERP * ro1 / VISLAM : VSM * PERP * rom / VISLAM;
+            return fminf(y, 1000.0f);
+        };
+        unsigned tr = 0;
+        for (int k0 = ty + 1; k0 <= KMM1; k0 += LK_U * LK_W) {
+            float dw[LK_U], vol[LK_U], fl[LK_U], ft[LK_U];
 #pragma unroll
-            for (int u = 0; u < 2; ++u) {
+            for (int u = 0; u < LK_U; ++u) {
                 const int k = min(k0 + u * LK_W, KMM1);
-                yp[u] = A3(d.Y_PLUS, i, j, k);
+                dw[u] = A3(d.DWALLSQ, i, j, k);
                 vol[u] = A3(d.VOL, i, j, k);
                 fl[u] = d.FKLAM[(size_t)(NRW - 1) * KM + k - 1];
                 ft[u] = d.FKTURB[(size_t)(NRW - 1) * KM + k - 1];
             }
 #pragma unroll
-            for (int u = 0; u < 2; ++u) {
+            for (int u = 0; u < LK_U; ++u) {
                 const int k = k0 + u * LK_W;
                 if (k > KMM1) continue;
+                float y = yplus(k, dw[u]);
+                A3(d.Y_PLUS, i, j, k) = y;
+                if (k < 2) continue;
                 // FYPLUS keeps its previous value where Y_PLUS is NaN
                 int kk = k;
-                float y = yp[u];
-                while (isnan(y) && --kk >= 2) y = A3(d.Y_PLUS, i, j, kk);
+                while (isnan(y) && --kk >= 2) y = yplus(kk, A3(d.DWALLSQ, i, j, kk));
                 float FYPLUS = kk >= 2 ? fyplus_of(y, d.YPLAM, d.YPTURB, 0.0f) : 0.0f;
                 float DPERP = vol[u] / LK(AREA, k);
-                LK(VLAM, k) = fl[u] * VISLAM / DPERP;
+                const float vl = fl[u] * VISLAM / DPERP;
                 float vt = ft[u] * LK(ROAVG, k) * fabsf(wabs(k + 1) - wabs(k - 1)) * FMIXUP;
-                LK(VTURB, k) = vt * FYPLUS;
+                vt = vt * FYPLUS;
+                LK(VLAM, k) = vl;
+                LK(VTURB, k) = vt;
+                const float RATVIS = vt / vl;
+                if (RATVIS > d.FTRANS) tr |= k < KMID ? 1u : k == KMID ? 2u : 4u;
+                walk = walk || isnan(RATVIS) || vl == 0.0f;
             }
         }
+        if (tr) atomicOr(&s_tr[tx], tr);
     }
-    __syncthreads();
-    // 5. transition, hub half then casing half (the casing scan sees the
-    //    hub half's result at KMID)
-    if (ty == 0 && col) {
-        const int JROW = j - A1(d.JSTART, NRW) + 1;
-        float *vt = VTURB + tx, *vl = VLAM + tx;   // column view, stride 32
-        auto scan = [&](int a, int b) {
-            float RMAX = 0.0f;
-            for (int q = a; q <= b; ++q) {
-                float RATVIS = vt[(q - 1) * 32] / vl[(q - 1) * 32];
-                if (RATVIS < RMAX) continue;
-                RMAX = RATVIS;
-            }
-            return RMAX > d.FTRANS;
-        };
-        bool turb = !(JROW < A1(d.JTRAN_K1, NRW)) && scan(2, KMID);
-        if (!turb)
-            for (int q = 2; q <= KMID; ++q) vt[(q - 1) * 32] = 0.0f;
-        turb = !(JROW < A1(d.JTRAN_KM, NRW)) && scan(KMID, KMM1);
-        if (!turb)
-            for (int q = KMID; q <= KMM1; ++q) vt[(q - 1) * 32] = 0.0f;
+    // 4. transition, hub half (K = 2..KMID) then casing half (KMID..KMM1; its
+    //    test sees the hub half's result at KMID): a half whose largest ratio
+    //    does not exceed FTRANS has no turbulent viscosity
+    bool hub = false, cas = false;
+    if (!__syncthreads_or(walk)) {
+        if (col) {
+            const int JROW = j - A1(d.JSTART, NRW) + 1;
+            const unsigned tr = s_tr[tx];
+            const bool neg = 0.0f > d.FTRANS;
+            hub = !(JROW < A1(d.JTRAN_K1, NRW)) && (neg || (tr & 3u));
+            cas = !(JROW < A1(d.JTRAN_KM, NRW)) && (neg || (tr & 4u) || (hub && (tr & 2u)));
+        }
+    } else {
+        // in the reference's order, where a NaN ratio starts the maximum anew
+        if (ty == 0 && col) {
+            const int JROW = j - A1(d.JSTART, NRW) + 1;
+            float *vt = VTURB + tx, *vl = VLAM + tx;   // column view, stride 32
+            auto scan = [&](int a, int b) {
+                float RMAX = 0.0f;
+                for (int q = a; q <= b; ++q) {
+                    float RATVIS = vt[(q - 1) * 32] / vl[(q - 1) * 32];
+                    if (RATVIS < RMAX) continue;
+                    RMAX = RATVIS;
+                }
+                return RMAX > d.FTRANS;
+            };
+            bool turb = !(JROW < A1(d.JTRAN_K1, NRW)) && scan(2, KMID);
+            if (!turb)
+                for (int q = 2; q <= KMID; ++q) vt[(q - 1) * 32] = 0.0f;
+            turb = !(JROW < A1(d.JTRAN_KM, NRW)) && scan(KMID, KMM1);
+            if (!turb)
+                for (int q = KMID; q <= KMM1; ++q) vt[(q - 1) * 32] = 0.0f;
+        }
+        hub = cas = true;          // VTURB is as it is to be
+        __syncthreads();
     }
-    __syncthreads();
-    // 6. stresses on faces K and K+1 of each cell, body forces relaxed by RF_VIS
+    // 5. stresses on faces K and K+1 of each cell, body forces relaxed by RF_VIS
     if (col) {
-        const float VISLAM = s_vis[tx], FTCOND = s_ftc[tx];
+        const float VISLAM = s_vis[tx];
+        float FTCOND = c->FTCOND;
+        if (d.REYNO < 0.0001f) {
+            float TCOND = d.CP * VISLAM / d.PRANDTL;
+            FTCOND = TCOND / VISLAM;
+        }
         const float RF_VIS1 = 1.0f - RF_VIS;
         auto face = [&](int kp, float &xs, float &rs, float &ts, float &qf, float &wv) {
             if (kp == 1) {
@@ -391,7 +413,9 @@ __global__ void __launch_bounds__(32 * LK_W, 5) k_loss_kfaces(const __grid_const
             } else if (kp == KM) {
                 xs = s_wm[tx][0]; rs = s_wm[tx][1]; ts = s_wm[tx][2]; qf = 0.0f; wv = s_wm[tx][3];
             } else {
-                float vl = LK(VLAM, kp), vtu = LK(VTURB, kp), ar = LK(AREA, kp);
+                float vl = LK(VLAM, kp), ar = LK(AREA, kp);
+                const bool on = (kp > KMID || hub) && (kp < KMID || cas);
+                const float vtu = on ? LK(VTURB, kp) : 0.0f;
                 float FM = ar * (vl + vtu);
                 xs = FM * (LK(VXAVG, kp + 1) - LK(VXAVG, kp - 1));
                 rs = FM * (LK(VRAVG, kp + 1) - LK(VRAVG, kp - 1));
