@@ -550,6 +550,7 @@ __global__ void __launch_bounds__(32 * LI_W, 8) k_loss_ifaces(const __grid_const
     const bool in_blade = !(j <= JLEDGE || j > JTEDGE);
     const bool in_gap = (A1(d.KTIPS, NRW) > 0) && (k >= A1(d.KTIPS, NRW)) && (k < A1(d.KTIPE, NRW));
     if (in_blade) {
+        float VS1 = 0.0f, VSM = 0.0f;
         if (!in_gap) {
             // wall shear on the two blade surfaces: lane 0 the I=1 side, lane 1 the I=IM side
             float TW = 0.0f;
@@ -571,15 +572,8 @@ __global__ void __launch_bounds__(32 * LI_W, 8) k_loss_ifaces(const __grid_const
                 }
             }
             const float TWALLI1 = __shfl_sync(0xffffffffu, TW, 0), TWALLIM = __shfl_sync(0xffffffffu, TW, 1);
-            const float VS1 = sqrtf(TWALLI1 / ROAVG[1]), VSM = sqrtf(TWALLIM / ROAVG[IM]);
-            for (int i = lane + 1; i <= IMM1; i += 32) {
-                float YPLS = i <= IMID ? VS1 * sqrtf(A3(d.DWALLSQ, i, j, k)) * ROAVG[1] / VISLAM
-                                       : VSM * sqrtf(A3(d.DWALLSQ, i, j, k)) * ROAVG[IM] / VISLAM;
-                float YPLSP = A3(d.Y_PLUS, i, j, k);
-                float y = fminf(YPLS, YPLSP);
-                A3(d.Y_PLUS, i, j, k) = y;
-                YP[i] = y;
-            }
+            VS1 = sqrtf(TWALLI1 / ROAVG[1]);
+            VSM = sqrtf(TWALLIM / ROAVG[IM]);
             if (lane == 0) {
                 float FMULT = TWALLI1 * AREA[1] / WABS[1];
                 XSTRES[1] = FMULT * VXAVG[1];
@@ -594,20 +588,57 @@ __global__ void __launch_bounds__(32 * LI_W, 8) k_loss_ifaces(const __grid_const
                 QFLOW[IM] = 0.0f;
                 WVISC[IM] = TSTRES[IM] * WREL * RAVGK;
             }
-        } else {
-            for (int i = lane + 2; i <= IMM1; i += 32) YP[i] = A3(d.Y_PLUS, i, j, k);
+        }
+        // Y_PLUS of the nearer wall and the viscosities, two points a lane at
+        // a time: their operands are loaded together, before the stores of
+        // Y_PLUS, and Y_PLUS stays in a register
+        auto vturb = [&](int i, float fit, float y) {
+            const float vt = fit * ROAVG[i] * fabsf(WABS[i + 1] - WABS[i - 1]) * FMIXUP;
+            return vt * fyplus_of(y, d.YPLAM, d.YPTURB, 0.0f);
+        };
+        bool nan = false;
+        for (int i0 = lane + 1; i0 <= IMM1; i0 += 64) {
+            float dw[2], yp[2], vol[2], fl[2], ft[2];
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const int i = min(i0 + 32 * u, IMM1), n = ix3(d, i, j, k);
+                dw[u] = in_gap ? 0.0f : d.DWALLSQ[n];
+                yp[u] = d.Y_PLUS[n];
+                vol[u] = d.VOL[n];
+                fl[u] = FIL[i - 1];
+                ft[u] = FIT[i - 1];
+            }
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const int i = i0 + 32 * u;
+                if (i > IMM1) continue;
+                float y = yp[u];
+                if (!in_gap) {
+                    float YPLS = i <= IMID ? VS1 * sqrtf(dw[u]) * ROAVG[1] / VISLAM
+                                           : VSM * sqrtf(dw[u]) * ROAVG[IM] / VISLAM;
+                    y = fminf(YPLS, y);
+                    A3(d.Y_PLUS, i, j, k) = y;
+                }
+                YP[i] = y;
+                if (i < 2) continue;
+                nan = nan || isnan(y);
+                float DPERP = vol[u] / AREA[i];
+                VLAM[i] = fl[u] * VISLAM / DPERP;
+                VTURB[i] = vturb(i, ft[u], y);
+            }
         }
         __syncwarp();
-        for (int i = lane + 2; i <= IMM1; i += 32) {
-            int ii = i;     // FYPLUS keeps its previous value where Y_PLUS is NaN
-            while (ii >= 2 && isnan(YP[ii])) --ii;
-            float FYPLUS = ii >= 2 ? fyplus_of(YP[ii], d.YPLAM, d.YPTURB, 0.0f) : 0.0f;
-            float DPERP = A3(d.VOL, i, j, k) / AREA[i];
-            VLAM[i] = FIL[i - 1] * VISLAM / DPERP;
-            float vt = FIT[i - 1] * ROAVG[i] * fabsf(WABS[i + 1] - WABS[i - 1]) * FMIXUP;
-            VTURB[i] = vt * FYPLUS;
+        if (__any_sync(0xffffffffu, nan)) {
+            // FYPLUS keeps its previous value where Y_PLUS is NaN
+            for (int i = lane + 2; i <= IMM1; i += 32) {
+                int ii = i;
+                while (ii >= 2 && isnan(YP[ii])) --ii;
+                if (ii == i) continue;
+                const float vt = FIT[i - 1] * ROAVG[i] * fabsf(WABS[i + 1] - WABS[i - 1]) * FMIXUP;
+                VTURB[i] = vt * (ii >= 2 ? fyplus_of(YP[ii], d.YPLAM, d.YPTURB, 0.0f) : 0.0f);
+            }
+            __syncwarp();
         }
-        __syncwarp();
         bool turb = !(JROW < A1(d.JTRAN_I1, NRW)) && transition_warp(VTURB, VLAM, 2, IMID, d.FTRANS);
         if (!turb)
             for (int i = lane + 2; i <= IMID; i += 32) VTURB[i] = 0.0f;
