@@ -38,7 +38,8 @@ static inline unsigned grid_for(size_t n, unsigned block) { return (unsigned)((n
 // 256-thread slots take 1.2 waves.
 constexpr int TS_U = 3;          // cells per thread whose loads are issued together
 constexpr int SV_U = 3;          // points per thread whose streamwise loads are issued together
-constexpr int SM_SEG = 8;        // points per thread of one pitchwise or spanwise smoothing segment
+constexpr int SM_SEG = 4;        // points per thread of one pitchwise or spanwise smoothing segment
+constexpr int SM_PAD = 2;        // floats before the plane buffers (a segment reads one before its line)
 constexpr int PR_U = 3;          // the same in prolong: five CTAs an SM at 48 registers (two cells and six CTAs: 38.9 us
                                  // a launch against 37.6 on the 33 x 752 x 66 compressor, 16.5 against 15.8 at 65 x 242 x 49)
 constexpr int TS_UG = 4;         // cells per thread whose loads the pair update issues together
@@ -1041,6 +1042,28 @@ static UpdateCut update_cut(const Dev &d, int sm_count, int nv) {
     return c;
 }
 
+// Two FP32 values in one instruction (PTX .f32x2), each rounded as the scalar
+// operation is.  A product is a*b + nz with nz = -0, which is a*b to the bit: a
+// mul.f32x2 whose result only an add.f32x2 takes comes out as one fused
+// operation, with one rounding less than the reference has, and so does a
+// product with a -0 that the assembler can see.
+#define MGPU_BITS(v) reinterpret_cast<unsigned long long &>(v)
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+    unsigned long long r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(MGPU_BITS(a)), "l"(MGPU_BITS(b)));
+    return reinterpret_cast<float2 &>(r);
+}
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) {
+    unsigned long long r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(MGPU_BITS(a)), "l"(MGPU_BITS(b)));
+    return reinterpret_cast<float2 &>(r);
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b, float2 nz) {
+    unsigned long long r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(MGPU_BITS(a)), "l"(MGPU_BITS(b)), "l"(MGPU_BITS(nz)));
+    return reinterpret_cast<float2 &>(r);
+}
+
 // ---------------------------------------------------------------------
 // smooth: SMOOTH_VAR (3900-9000, 8502) + periodic (8000), tip gap (510),
 // mixing-plane average (100): TMP -> D, one CTA per J-plane
@@ -1058,8 +1081,9 @@ __global__ void __launch_bounds__(BS, 1024 / BS) k_ts_smooth(const __grid_consta
     // keeps the pitchwise pass, whose lanes step from one K line to the
     // next, free of bank conflicts
     const int IMP = IM | 1;
-    float *a = sm, *b = sm + IMP * KM;
-    float *cFD = b + IMP * KM, *cFU = cFD + IM, *cFKD = cFU + IM, *cFKU = cFKD + KM;   // FD, FU, FKD, FKU
+    float *a = sm + SM_PAD, *b = a + IMP * KM;
+    // FD, FU, FKD, FKU, each twice: the operand of two lanes of arithmetic
+    float2 *cFD = reinterpret_cast<float2 *>(sm + SM_PAD + 2 * IMP * KM), *cFU = cFD + IM, *cFKD = cFU + IM, *cFKU = cFKD + KM;
     const int j = blockIdx.x + 1;
     const PlaneInfo &pl = d.PLANE[j - 1];
     const DevCtl *c = d.ctl;
@@ -1068,12 +1092,14 @@ __global__ void __launch_bounds__(BS, 1024 / BS) k_ts_smooth(const __grid_consta
     // mixing plane's average, ahead of its use
     const float fpw = mix && (int)threadIdx.x < IMM1 ? d.FP[threadIdx.x] : 0.0f;
     for (int t = threadIdx.x; t < IM; t += BS) {
-        cFD[t] = d.FD[t];
-        cFU[t] = d.FU[t];
+        const float fd = d.FD[t], fu = d.FU[t];
+        cFD[t] = make_float2(fd, fd);
+        cFU[t] = make_float2(fu, fu);
     }
     for (int t = threadIdx.x; t < KM; t += BS) {
-        cFKD[t] = d.FKD[t];
-        cFKU[t] = d.FKU[t];
+        const float fd = d.FKD[t], fu = d.FKU[t];
+        cFKD[t] = make_float2(fd, fd);
+        cFKU[t] = make_float2(fu, fu);
     }
     const int ks = IM * d.JM;                        // K stride of a node array
     const float *__restrict__ Sj = S + IM * (j - 1);  // plane j: (i, k) at i-1 + ks*(k-1)
@@ -1141,40 +1167,66 @@ __global__ void __launch_bounds__(BS, 1024 / BS) k_ts_smooth(const __grid_consta
     const bool periodic_j = pl.periodic != 0;
     if (j >= 2 && !(c->SFT < 0.0001f)) {
         const float SFT = c->SFT, SFT1 = c->SFT1, F4 = d.FAC_4TH;
-        // the points I = 2..IMM1 first, in segments of SM_SEG points of one K
-        // line per thread, the lanes on successive K lines: each point's
-        // curvature is formed once and the segment's values stay in
-        // registers.  The curvature at I = 1 and IM, which the points I = 2
-        // and IMM1 take, is one value per line (the reference's CURVE there
-        // is the I = 1 value, or 0 off the periodic planes)
-        const int nsi = (IM - 2 + SM_SEG - 1) / SM_SEG;
-        Walk2 w(KM, threadIdx.x, BS);
-        for (int t = threadIdx.x; t < nsi * KM; t += BS, w.next()) {
-            const int k = w.i, i0 = 2 + SM_SEG * (w.k - 1);
-            const int len = min(SM_SEG, IMM1 - i0 + 1);
-            const float *ak = a + IMP * (k - 1) - 1;     // ak[i] = P(a, i, k)
-            float x[SM_SEG + 4];                          // x[q] = P(a, i0 - 2 + q, k)
+        const float2 SFT2 = make_float2(SFT, SFT), SFT12 = make_float2(SFT1, SFT1), F42 = make_float2(F4, F4);
+        // Two lines a thread, in the two halves of f32x2 operations: the pass
+        // is bound by its instructions on a large grid (218 a node with one
+        // line a thread), and the weights, the tests for a line's ends and the
+        // arithmetic are shared.  59.9 -> 57.3 us a launch on the 73 x 712 x 57
+        // compressor, 11.0 -> 10.5 on the 33 x 97 x 37 row, the same at
+        // 65 x 242 x 49 (segments of 6 points 61.1, of 8 points 72.5: spills).
+        // one segment of SM_SEG points of two lines: x(q) gives points
+        // first - 2 + q of both, FD and FU the weights of point first - 1 + q,
+        // e the curvature at a line's two ends; out(q, v) takes the new points
+        // -0, as the launch's (one-dimensional) block hides it
+        const float nz1 = __uint_as_float(0x80000000u + (blockDim.y - 1u));
+        const float2 nz = make_float2(nz1, nz1);
+        auto mul = [&](float2 u, float2 v) { return mul2(u, v, nz); };
+        auto segment = [&](auto x_of, const float2 *FD, const float2 *FU, float2 e, bool begins, int last, auto out) {
+            float2 x[SM_SEG + 4], g[SM_SEG + 2];
 #pragma unroll
-            for (int q = 0; q < SM_SEG + 4; ++q) {
-                const int ii = i0 - 2 + q;
-                x[q] = (q < len + 4 && ii >= 1 && ii <= IM) ? ak[ii] : 0.0f;
-            }
-            const float cper = periodic_j ? ak[1] - 0.5f * (ak[2] + ak[IMM1]) : 0.0f;
-            float g[SM_SEG + 2];                          // g[q]: the curvature at I = i0 - 1 + q
+            for (int q = 0; q < SM_SEG + 4; ++q) x[q] = x_of(q);
 #pragma unroll
-            for (int q = 0; q < SM_SEG + 2; ++q) {
-                const int ii = i0 - 1 + q;
-                g[q] = (ii == 1 || ii >= IM) ? cper : x[q + 1] - (cFD[ii - 1] * x[q + 2] + cFU[ii - 1] * x[q]);
-            }
-            float *bk = b + IMP * (k - 1) - 1;
+            for (int q = 0; q < SM_SEG + 2; ++q)
+                g[q] = sub2(x[q + 1], add2(mul(FD[q], x[q + 2]), mul(FU[q], x[q])));
+            if (begins) g[0] = e;
+            if (last <= SM_SEG + 1)
+#pragma unroll
+                for (int q = 2; q < SM_SEG + 2; ++q)
+                    if (q == last) g[q] = e;
 #pragma unroll
             for (int q = 0; q < SM_SEG; ++q) {
-                if (q >= len) break;
-                const int ii = i0 + q;
-                const float AVG = cFD[ii - 1] * x[q + 3] + cFU[ii - 1] * x[q + 1];
-                const float SC = cFU[ii - 1] * g[q] + cFD[ii - 1] * g[q + 2];
-                bk[ii] = SFT1 * x[q + 2] + SFT * (AVG + F4 * SC);
+                const float2 fd = FD[q + 1], fu = FU[q + 1];
+                const float2 AVG = add2(mul(fd, x[q + 3]), mul(fu, x[q + 1]));
+                const float2 SC = add2(mul(fu, g[q]), mul(fd, g[q + 2]));
+                out(q, add2(mul(SFT12, x[q + 2]), mul(SFT2, add2(AVG, mul(F42, SC)))));
             }
+        };
+        // the points I = 2..IMM1 first, in segments of SM_SEG points of two K
+        // lines half the plane apart per thread, the lanes on successive K
+        // lines (an odd last line is done twice, with one result): each
+        // point's curvature is formed once and the segment's values stay in
+        // registers.  The curvature at I = 1 and IM, which the points I = 2
+        // and IMM1 take, is one value per line (the reference's CURVE there
+        // is the I = 1 value, or 0 off the periodic planes).  What a segment
+        // reads past its line's end lies in the plane buffers and is not used
+        const int KH = (KM + 1) / 2, nsi = (IM - 2 + SM_SEG - 1) / SM_SEG;
+        Walk2 w(KH, threadIdx.x, BS);
+        for (int t = threadIdx.x; t < nsi * KH; t += BS, w.next()) {
+            const int k = w.i, k2 = min(k + KH, KM), i0 = 2 + SM_SEG * (w.k - 1);
+            const int len = min(SM_SEG, IMM1 - i0 + 1);
+            const float *a1 = a + IMP * (k - 1), *a2 = a + IMP * (k2 - 1);
+            float2 cper = make_float2(0.0f, 0.0f);
+            if (periodic_j)
+                cper = make_float2(a1[0] - 0.5f * (a1[1] + a1[IMM1 - 1]), a2[0] - 0.5f * (a2[1] + a2[IMM1 - 1]));
+            float *b1 = b + IMP * (k - 1) + i0 - 1, *b2 = b + IMP * (k2 - 1) + i0 - 1;
+            const float *p1 = a1 + i0 - 3, *p2 = a2 + i0 - 3;
+            segment([&](int q) { return make_float2(p1[q], p2[q]); }, cFD + i0 - 2, cFU + i0 - 2, cper, i0 == 2,
+                    IM - (i0 - 1), [&](int q, float2 v) {
+                        if (q < len) {
+                            b1[q] = v.x;
+                            b2[q] = v.y;
+                        }
+                    });
         }
         // then the points I = 1 and IM of every line
         for (int t = threadIdx.x; t < 2 * KM; t += BS) {
@@ -1183,54 +1235,45 @@ __global__ void __launch_bounds__(BS, 1024 / BS) k_ts_smooth(const __grid_consta
             float AVG, SC;
             if (periodic_j) {
                 AVG = 0.5f * (ak[2] + ak[IMM1]);
-                const float c2 = ak[2] - (cFD[1] * ak[3] + cFU[1] * ak[1]);
-                const float cm1 = ak[IMM1] - (cFD[IMM1 - 1] * ak[IM] + cFU[IMM1 - 1] * ak[d.IMM2]);
+                const float c2 = ak[2] - (cFD[1].x * ak[3] + cFU[1].x * ak[1]);
+                const float cm1 = ak[IMM1] - (cFD[IMM1 - 1].x * ak[IM] + cFU[IMM1 - 1].x * ak[d.IMM2]);
                 SC = 0.5f * (c2 + cm1);
             } else {
-                if (i == 1) AVG = ak[2] + cFU[0] * (ak[2] - ak[3]);
-                else AVG = ak[IMM1] + cFU[IM - 1] * (ak[IMM1] - ak[d.IMM2]);
+                if (i == 1) AVG = ak[2] + cFU[0].x * (ak[2] - ak[3]);
+                else AVG = ak[IMM1] + cFU[IM - 1].x * (ak[IMM1] - ak[d.IMM2]);
                 SC = 0.0f;
             }
             P(b, i, k) = SFT1 * ak[i] + SFT * (AVG + F4 * SC);
         }
         __syncthreads();
-        // spanwise: segments of SM_SEG points of one I line per thread, the
-        // lanes on successive I lines
-        const int nsk = (KM + SM_SEG - 1) / SM_SEG;
-        w = Walk2(IM, threadIdx.x, BS);
-        for (int t = threadIdx.x; t < nsk * IM; t += BS, w.next()) {
-            const int i = w.i, k0 = 1 + SM_SEG * (w.k - 1);
-            const int len = min(SM_SEG, KM - k0 + 1);
-            const float *bi = b + (i - 1) - IMP;          // bi[IMP * kk] = P(b, i, kk)
-            float y[SM_SEG + 4];                          // y[q] = P(b, i, k0 - 2 + q)
-#pragma unroll
-            for (int q = 0; q < SM_SEG + 4; ++q) {
-                const int kk = k0 - 2 + q;
-                y[q] = (q < len + 4 && kk >= 1 && kk <= KM) ? bi[IMP * kk] : 0.0f;
-            }
-            float h[SM_SEG + 2];                          // h[q]: the curvature at K = k0 - 1 + q
-#pragma unroll
-            for (int q = 0; q < SM_SEG + 2; ++q) {
-                const int kk = k0 - 1 + q;
-                h[q] = (kk <= 1 || kk >= KM) ? 0.0f : y[q + 1] - (cFKD[kk - 1] * y[q + 2] + cFKU[kk - 1] * y[q]);
-            }
-#pragma unroll
-            for (int q = 0; q < SM_SEG; ++q) {
-                if (q >= len) break;
-                const int kk = k0 + q;
-                float AVG, SC;
-                if (kk == 1) {
-                    AVG = y[q + 3] + 0.5f * cFKU[0] * (y[q + 3] - y[q + 4]);
-                    SC = 0.0f;
-                } else if (kk == KM) {
-                    AVG = y[q + 1] + 0.5f * cFKU[KM - 1] * (y[q + 1] - y[q]);
-                    SC = 0.0f;
-                } else {
-                    AVG = cFKD[kk - 1] * y[q + 3] + cFKU[kk - 1] * y[q + 1];
-                    SC = cFKU[kk - 1] * h[q] + cFKD[kk - 1] * h[q + 2];
-                }
-                P(a, i, kk) = SFT1 * y[q + 2] + SFT * (AVG + F4 * SC);
-            }
+        // spanwise: the points K = 2..KMM1 in segments of two I lines half the
+        // plane apart, the lanes on successive I lines; the curvature at K = 1
+        // and KM is zero
+        const int IH = (IM + 1) / 2, nsk = (KM - 2 + SM_SEG - 1) / SM_SEG;
+        w = Walk2(IH, threadIdx.x, BS);
+        for (int t = threadIdx.x; t < nsk * IH; t += BS, w.next()) {
+            const int i = w.i, i2 = min(i + IH, IM), k0 = 2 + SM_SEG * (w.k - 1);
+            const int len = min(SM_SEG, KMM1 - k0 + 1);
+            const float *p1 = b + (i - 1) + IMP * (k0 - 3), *p2 = p1 + (i2 - i);
+            float *a1 = a + (i - 1) + IMP * (k0 - 1), *a2 = a1 + (i2 - i);
+            segment(
+                [&](int q) {
+                    const bool in = q < 4 || k0 - 2 + q <= KM;
+                    return make_float2(in ? p1[IMP * q] : 0.0f, in ? p2[IMP * q] : 0.0f);
+                },
+                cFKD + k0 - 2, cFKU + k0 - 2, make_float2(0.0f, 0.0f), k0 == 2, KM - (k0 - 1), [&](int q, float2 v) {
+                    if (q < len) {
+                        a1[IMP * q] = v.x;
+                        a2[IMP * q] = v.y;
+                    }
+                });
+        }
+        // then the points K = 1 and KM of every line
+        for (int t = threadIdx.x; t < 2 * IM; t += BS) {
+            const int i = (t >> 1) + 1, k = (t & 1) ? KM : 1, k1 = (t & 1) ? KMM1 : 2, k2 = (t & 1) ? d.KMM2 : 3;
+            const float y1 = k1 >= 1 ? P(b, i, k1) : 0.0f, y2 = k2 >= 1 && k2 <= KM ? P(b, i, k2) : 0.0f;
+            const float AVG = y1 + 0.5f * cFKU[k - 1].x * (y1 - y2), SC = 0.0f;
+            P(a, i, k) = SFT1 * P(b, i, k) + SFT * (AVG + F4 * SC);
         }
         __syncthreads();
         float cv = 0.0f;
@@ -1275,21 +1318,22 @@ __global__ void __launch_bounds__(BS, 1024 / BS) k_ts_smooth(const __grid_consta
             P(a, IM, k) = v;
         }
     }
-    if (mix)                       // the smoothing is done with cFU
-        for (int i = threadIdx.x; i < IMM1; i += BS) cFU[i] = i < BS ? fpw : d.FP[i];
+    float *fp = reinterpret_cast<float *>(cFU);       // the smoothing is done with it
+    if (mix)
+        for (int i = threadIdx.x; i < IMM1; i += BS) fp[i] = i < BS ? fpw : d.FP[i];
     __syncthreads();
     float *Dj = D + IM * (j - 1);
     if (mix) {
         if (d.REDUCE_ORDER != 0) {
             for (int k = threadIdx.x + 1; k <= KM; k += BS) {
                 float s = 0.0f;
-                for (int i = 1; i <= IMM1; ++i) s = s + cFU[i - 1] * (P(a, i, k) + P(a, i + 1, k));
+                for (int i = 1; i <= IMM1; ++i) s = s + fp[i - 1] * (P(a, i, k) + P(a, i + 1, k));
                 b[k - 1] = 0.5f * s;
             }
         } else {
             for_rows(KM, [&](int r, int l, bool on) {
                 const float *row = a + IMP * r;
-                const float s = row_sum64(on ? IMM1 : 0, [&](int i) { return cFU[i] * (row[i] + row[i + 1]); });
+                const float s = row_sum64(on ? IMM1 : 0, [&](int i) { return fp[i] * (row[i] + row[i + 1]); });
                 if (on && l == 0) b[r] = 0.5f * s;
             });
         }
@@ -1365,7 +1409,9 @@ static size_t cells_smem(const Dev &d) {
 }
 static size_t prolong_smem(const Dev &d) { return ((size_t)d.NIB1 * d.NKB1 + (size_t)d.NIB2 * d.NKB2) * sizeof(float); }
 static size_t update_pair_smem(const Dev &d) { return (size_t)3 * d.IMM1 * d.KMM1 * sizeof(float); }
-static size_t smooth_smem(const Dev &d) { return ((size_t)2 * (d.IM | 1) * d.KM + 2 * d.IM + 2 * d.KM) * sizeof(float); }
+static size_t smooth_smem(const Dev &d) {
+    return ((size_t)2 * (d.IM | 1) * d.KM + 4 * (d.IM + d.KM) + SM_PAD + 4 * SM_SEG) * sizeof(float);
+}
 
 template <int BS>
 static cudaError_t configure_bs(const Dev &d) {
@@ -1376,8 +1422,12 @@ static cudaError_t configure_bs(const Dev &d) {
              {(const void *)k_ts_prolong<BS>, prolong_smem(d)},
              {(const void *)k_ts_update_pair<2 * BS>, update_pair_smem(d)},
              {(const void *)k_ts_smooth<BS>, smooth_smem(d)}};
+    // the limit is on what a plane takes: the smoothing weights' second copies
+    // and the paddings (9 KB at the largest IM and KM that LOSS's line arrays
+    // let through) come on top
+    const size_t extra = (2 * (size_t)(d.IM + d.KM) + SM_PAD + 4 * SM_SEG) * sizeof(float);
     for (auto &x : k) {
-        if (x.bytes > 200 * 1024) return cudaErrorInvalidValue;
+        if (x.bytes - (x.f == (const void *)k_ts_smooth<BS> ? extra : 0) > 200 * 1024) return cudaErrorInvalidValue;
         cudaError_t e = raise_smem(x.f, x.bytes);
         if (e != cudaSuccess) return e;
     }
