@@ -193,6 +193,12 @@ __device__ __noinline__ void edges_mass_energy(const Dev &d, int e) {
 // 18 loads of flow quantities instead of 33 (momenta: 20 instead of 40), and
 // the index arithmetic is one addition a node.  Columns outside the grid load
 // the thread's own, for faces that are not stored.
+// What bounds the passes on a large grid is memory latency: 24 warps an SM each
+// wait for a level's loads before they can ask for the next one's.  Each level
+// therefore asks for the next one's lines in L2, which takes no registers:
+// momenta 92.5 -> 79.7 us and mass + energy 74.8 -> 66.4 on the 73 x 712 x 57
+// compressor (4.0 TB/s of the momenta's 27 arrays, 3.5 before), 27.6 -> 25.7 and
+// 22.7 -> 21.5 at 65 x 242 x 49, one row the same.
 struct March {
     int i, j, k, ke, n, o1, oj;       // node (i, j, k), last K, offsets to I+1 and J-1
     bool hi, hj, on;
@@ -278,6 +284,23 @@ __global__ void __launch_bounds__(256, 3) k_flux_mass_energy(const __grid_consta
         const int jk = w.j - 1 + d.JM * (k - 1);
         float aqx = 0.0f, aqr = 0.0f, abx = 0.0f, abr = 0.0f, abt = 0.0f, wrabt = 0.0f, asx = 0.0f, asr = 0.0f;
         if (hk) b.load(d, w, n + sK, k + 1);
+        // the next level's operands on their way into L2 (see March)
+        if (k + 1 <= w.ke && k + 2 <= KM) {
+            prefetch_l2(d.ROVX + n + 2 * sK);
+            prefetch_l2(d.ROVR + n + 2 * sK);
+            prefetch_l2(d.HO + n + 2 * sK);
+            prefetch_l2(d.RO + n + 2 * sK);
+            prefetch_l2(d.ROVT + n + 2 * sK);
+            prefetch_l2(d.PEFF + n + 2 * sK);
+        }
+        if (k + 1 <= w.ke && k + 1 < KM) {
+            prefetch_l2(d.AQX + n + sK);
+            prefetch_l2(d.AQR + n + sK);
+            prefetch_l2(d.ABX + n + sK);
+            prefetch_l2(d.ABR + n + sK);
+            prefetch_l2(d.ASX + n + sK);
+            prefetch_l2(d.ASR + n + sK);
+        }
         if (hx) {
             aqx = d.AQX[n];
             aqr = d.AQR[n];
@@ -779,6 +802,27 @@ __global__ void __launch_bounds__(256, 3) k_flux_mom(const __grid_constant__ Dev
         float aqx = 0.0f, aqr = 0.0f, flowx = 0.0f, asx = 0.0f, asr = 0.0f, flowr = 0.0f, rj1 = 0.0f;
         float rforce = 0.0f, volor = 0.0f, FT = 0.0f, abx = 0.0f, abr = 0.0f, abt = 0.0f, ravg = 0.0f;
         if (hk) b.load(d, w, n + sK, k + 1);
+        // the next level's operands on their way into L2 (see March)
+        if (k + 1 <= w.ke && k + 2 <= KM) {
+            prefetch_l2(d.P + n + 2 * sK);
+            prefetch_l2(d.VX + n + 2 * sK);
+            prefetch_l2(d.VT + n + 2 * sK);
+            prefetch_l2(d.VR + n + 2 * sK);
+            prefetch_l2(d.ROVT + n + 2 * sK);
+        }
+        if (k + 1 <= w.ke && k + 1 < KM) {
+            prefetch_l2(d.AQX + n + sK);
+            prefetch_l2(d.AQR + n + sK);
+            prefetch_l2(d.FLOWX + n + sK);
+            prefetch_l2(d.ASX + n + sK);
+            prefetch_l2(d.ASR + n + sK);
+            prefetch_l2(d.FLOWR + n + sK);
+            prefetch_l2(d.RFORCE + n + sK);
+            prefetch_l2(d.VOLOR + n + sK);
+            prefetch_l2(d.FLOWT + n + sK);
+            prefetch_l2(d.ABX + n + sK);
+            prefetch_l2(d.ABR + n + sK);
+        }
         if (fK) {
             aqx = d.AQX[n];
             aqr = d.AQR[n];

@@ -330,6 +330,8 @@ struct WalkN {
     }
 };
 
+__device__ __forceinline__ void prefetch_l2(const float *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
 // The same walk by 32-bit byte offsets, for arrays of 4-byte elements
 // (mgpu_create keeps a node array within 2^32 bytes).  at() adds such an
 // offset to the array's base: with a base that all threads share, the
