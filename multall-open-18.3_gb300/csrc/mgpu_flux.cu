@@ -196,9 +196,12 @@ __device__ __noinline__ void edges_mass_energy(const Dev &d, int e) {
 // What bounds the passes on a large grid is memory latency: 24 warps an SM each
 // wait for a level's loads before they can ask for the next one's.  Each level
 // therefore asks for the next one's lines in L2, which takes no registers:
-// momenta 92.5 -> 79.7 us and mass + energy 74.8 -> 66.4 on the 73 x 712 x 57
-// compressor (4.0 TB/s of the momenta's 27 arrays, 3.5 before), 27.6 -> 25.7 and
+// momenta 92.5 -> 79.7 us and mass + energy 74.8 -> 66.4 on the 73 x 752 x 57
+// compressor (4.2 TB/s of the momenta's 27 arrays, 3.7 before), 27.6 -> 25.7 and
 // 22.7 -> 21.5 at 65 x 242 x 49, one row the same.
+// The loops are not unrolled and mass + energy runs at four CTAs an SM (two
+// levels an iteration and three CTAs: 66.6 us against 60.3, momenta 80.0
+// against 78.6; at 65 x 242 x 49 the same).
 struct March {
     int i, j, k, ke, n, o1, oj;       // node (i, j, k), last K, offsets to I+1 and J-1
     bool hi, hj, on;
@@ -240,7 +243,7 @@ struct Q4 {
 
 // mass fluxes (5020-5045), ROWT, WT, and from them the energy fluxes
 // (5501-5503), whose source QSOURCE TSTEP reads in place
-__global__ void __launch_bounds__(256, 3) k_flux_mass_energy(const __grid_constant__ Dev d, int S, int edges) {
+__global__ void __launch_bounds__(256, 4) k_flux_mass_energy(const __grid_constant__ Dev d, int S, int edges) {
     pdl_wait();
     if ((int)blockIdx.x < edges) {
         edges_mass_energy(d, (int)(blockIdx.x * 256 + threadIdx.x));
@@ -278,7 +281,7 @@ __global__ void __launch_bounds__(256, 3) k_flux_mass_energy(const __grid_consta
     Level a, b;
     int n = w.n;
     a.load(d, w, n, w.k);
-#pragma unroll 2
+#pragma unroll 1
     for (int k = w.k; k <= w.ke; ++k, n += sK) {
         const bool hk = k < KM, hx = w.hi && hk, ht = own_t && hk, hr = w.hi && w.hj;
         const int jk = w.j - 1 + d.JM * (k - 1);
@@ -795,7 +798,7 @@ __global__ void __launch_bounds__(256, 3) k_flux_mom(const __grid_constant__ Dev
     Level a, b;
     int n = w.n;
     a.load(d, w, n, w.k);
-#pragma unroll 2
+#pragma unroll 1
     for (int k = w.k; k <= w.ke; ++k, n += sK) {
         const bool hk = k < KM, fK = w.hi && hk, fJ = w.hi && w.hj, fI = own_t && hk, fS = fJ && hk;
         const int jk = w.j - 1 + d.JM * (k - 1);
