@@ -7,6 +7,7 @@
 // include/mgpu_common_table.h).  No exception crosses the ABI: every entry
 // point catches, records the message for mgpu_last_error() and returns a
 // negative status.
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -96,10 +97,12 @@ struct mgpu_handle {
     AdjState *adj = nullptr;     // discrete adjoint, after mgpu_adjoint_prepare
 };
 
-// A batch: CUDA graphs whose branches are the step graphs of several handles,
-// forked from and joined back to the batch's own stream.
+// A batch: CUDA graphs of the step graphs of several handles, forked from and
+// joined back to the batch's own stream.  The members lie on a few chains side
+// by side, a chain's members one after the other (batch_chains).
 struct mgpu_batch {
     std::vector<mgpu_handle *> hs;
+    std::vector<int> after;      // the member that a member follows on its chain, -1 for the first
     int device = 0;
     cudaStream_t stream = nullptr;
     cudaEvent_t fork = nullptr;
@@ -389,13 +392,12 @@ int add_conditional(mgpu_handle *h, cudaGraphConditionalHandle hnd, F fn) {
 // the control block; their kernels still test the device's own flags.
 // what < 0: the LOSS and tail kernels sit in conditional bodies that the
 // step-control kernel switches on only on the steps that need them.
-int capture_step(mgpu_handle *h, int what, bool in_batch) {
+int capture_step(mgpu_handle *h, int what) {
     cudaStreamCaptureStatus st;
     cudaGraph_t cg = nullptr;
     CK(cudaStreamGetCaptureInfo(h->stream, &st, nullptr, &cg, nullptr, nullptr, nullptr));
     cudaGraphConditionalHandle hl = 0, ht = 0;
     Dev dg = h->d;
-    dg.in_batch = in_batch ? 1 : 0;
     if (what < 0) {
         // every handle of a graph belongs to one conditional node: an inviscid
         // problem (ILOS = 0), which has no LOSS node, creates no LOSS handle
@@ -441,7 +443,7 @@ int build_graph(mgpu_handle *h, int what) {
     StepGraph &G = h->sg[what];
     if (G.exec) return 0;
     CK(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
-    int rc = capture_step(h, what, false);
+    int rc = capture_step(h, what);
     cudaGraph_t g = nullptr;
     cudaError_t e = cudaStreamEndCapture(h->stream, &g);
     if (rc) {
@@ -495,7 +497,7 @@ int read_ctl(mgpu_handle *h) {
 }
 
 // What the step after the mirrored control block c runs, q steps on: bit 0
-// LOSS, bit 1 the tail, by the tests of k_step_begin.  q > 0 holds only up
+// LOSS, bit 1 the tail, by the tests of step_control.  q > 0 holds only up
 // to the next tail, which rewrites what the end test reads.
 int step_what(const Dev &d, const DevCtl &c, int q, bool force_end) {
     const int n = c.nstep + 1 + q;
@@ -1611,6 +1613,31 @@ int32_t mgpu_profile_steps(mgpu_handle *h, int32_t nsteps, mgpu_kernel_time *out
 
 namespace {
 
+// Puts the members on chains: as many side by side as hold 1.6 million nodes,
+// at least four, each member on the chain with the fewest nodes so far.  That
+// is enough to fill the GPU, and what one kernel of a member writes is still in
+// L2 when the next one reads it; with all members side by side each array went
+// through memory between two kernels.  64 stages of 258 thousand nodes, with
+// the read-out of their states: 51.0 ms for 10 steps on 64 chains, 48.2 on 16,
+// 47.6, 47.4 and 47.5 on 8, 6 and 4, 49.4 on 3 and 57.8 on 2.
+void batch_chains(mgpu_batch *b) {
+    const size_t n = b->hs.size();
+    double nodes = 0.0;
+    for (mgpu_handle *h : b->hs) nodes += (double)h->d.IM * h->d.JM * h->d.KM;
+    const double want = std::ceil(1.6e6 * (double)n / nodes);
+    const size_t chains = want < 4.0 ? std::min<size_t>(4, n) : want < (double)n ? (size_t)want : n;
+    std::vector<double> load(chains, 0.0);
+    std::vector<int> last(chains, -1);
+    b->after.assign(n, -1);
+    for (size_t i = 0; i < n; ++i) {
+        const size_t c = (size_t)(std::min_element(load.begin(), load.end()) - load.begin());
+        const mgpu_handle *h = b->hs[i];
+        load[c] += (double)h->d.IM * h->d.JM * h->d.KM;
+        b->after[i] = last[c];
+        last[c] = (int)i;
+    }
+}
+
 // the batch's graph of a step of kind `what` (-1: mixed)
 int batch_graph(mgpu_batch *b, int what) {
     StepGraph &G = what < 0 ? b->mixed : b->sg[what];
@@ -1620,9 +1647,9 @@ int batch_graph(mgpu_batch *b, int what) {
     cudaError_t e = cudaEventRecord(b->fork, b->stream);
     for (size_t i = 0; i < b->hs.size() && !rc && e == cudaSuccess; ++i) {
         mgpu_handle *h = b->hs[i];
-        e = cudaStreamWaitEvent(h->stream, b->fork, 0);
+        e = cudaStreamWaitEvent(h->stream, b->after[i] < 0 ? b->fork : b->joins[b->after[i]], 0);
         if (e != cudaSuccess) break;
-        rc = capture_step(h, what, true);
+        rc = capture_step(h, what);
         if (rc) break;
         e = cudaEventRecord(b->joins[i], h->stream);
         if (e == cudaSuccess) e = cudaStreamWaitEvent(b->stream, b->joins[i], 0);
@@ -1697,6 +1724,7 @@ int32_t mgpu_batch_create(mgpu_handle *const *handles, int32_t n, mgpu_batch **o
     if (e == cudaSuccess) e = cudaMallocHost((void **)&b->h_ctl, n * sizeof(DevCtl));
     if (e == cudaSuccess) e = cudaMemcpy(b->d_list, list.data(), n * sizeof(DevCtl *), cudaMemcpyHostToDevice);
     if (e != cudaSuccess) return bail(fail(MGPU_E_NOMEM, std::string("mgpu_batch_create: ") + cudaGetErrorString(e)));
+    batch_chains(b);
     int rc = batch_graph(b, 0);
     if (!rc) rc = batch_graph(b, 3);
     if (rc) return bail(rc);

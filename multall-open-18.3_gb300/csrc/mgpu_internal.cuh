@@ -159,7 +159,6 @@ struct Dev {
     // graph conditionals selecting the LOSS and 5-step tail bodies (set by
     // the step-control kernel when the step runs from the CUDA graph)
     int use_cond;
-    int in_batch;                      // one of several problems that share the GPU
     unsigned long long cond_loss, cond_tail;
     int ts_bs[2];                      // threads per J-plane CTA of TSTEP (128, 192, 256 or 512; mgpu_autotune)
                                        // for the pass of 2 variables (RO, ROE) and the pass of 3 (momenta)

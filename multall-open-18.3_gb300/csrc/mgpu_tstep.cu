@@ -2,8 +2,9 @@
 // SMOOTH_VAR (15352-15594) and SMOOTH_RESID (14833-14917) on the GPU.
 //
 // One call updates one conserved variable D with its SCREE history DIFF in
-// four kernels, each with one CTA per J-plane (a J-plane of the largest
-// configuration, 73 x 57 points, is 16 KB: it lives in shared memory):
+// four kernels, each but update with one CTA per J-plane (a J-plane of the
+// largest configuration, 73 x 57 points, is 16 KB: it lives in shared memory);
+// update's CTAs march along J over tiles of K:
 //   cells    tip-gap TFLUX balance, mixing-plane flux extrapolation into
 //            SOURCE, the flux sum DELTA -> STORE and DIFF, the pitchwise
 //            redistribution of STORE on the mixing-plane cells, and this
@@ -33,15 +34,17 @@ static inline unsigned grid_for(size_t n, unsigned block) { return (unsigned)((n
 
 // Threads per J-plane CTA: 128, 192, 256 (the default) or 512, chosen per
 // problem and pass by mgpu_autotune (Dev::ts_bs); each size keeps 1024
-// threads of 64 registers resident per SM (960 for 192: five CTAs).  A pass
-// of 3 x 241 CTAs fills five 192-thread slots per SM in one wave, where four
-// 256-thread slots take 1.2 waves.
+// threads of 64 registers resident per SM (960 for 192: five CTAs).  256 is
+// the best or within the noise of it on every grid tried from 7 x 50 x 9 to
+// 73 x 752 x 57: 250 us a step at 65 x 242 x 49 against 263 at 192, 259 at 512
+// and 288 at 128, although its 723 momentum CTAs take 1.2 waves.
 constexpr int TS_U = 3;          // cells per thread whose loads are issued together
 constexpr int SV_U = 3;          // points per thread whose streamwise loads are issued together
 constexpr int SM_SEG = 4;        // points per thread of one pitchwise or spanwise smoothing segment
 constexpr int SM_PAD = 2;        // floats before the plane buffers (a segment reads one before its line)
-constexpr int PR_U = 3;          // the same in prolong: five CTAs an SM at 48 registers (two cells and six CTAs: 38.9 us
-                                 // a launch against 37.6 on the 33 x 752 x 66 compressor, 16.5 against 15.8 at 65 x 242 x 49)
+constexpr int PR_U = 3;          // the same in prolong: five CTAs an SM at 48 registers (two cells and six CTAs:
+                                 // 38.9 us a launch against 37.6 on the 73 x 752 x 57 compressor, 16.5
+                                 // against 15.8 at 65 x 242 x 49)
 constexpr int TS_UG = 4;         // cells per thread whose loads the pair update issues together
 constexpr int UG_SEG = 3;        // nodes per thread of one K column in the pair update's gather
 constexpr int UP_S = 3;          // nodes along K of one thread of update
@@ -713,7 +716,7 @@ __global__ void __launch_bounds__(UP_T, 3) k_ts_update(const __grid_constant__ D
     if (act) read_cells(0, ca);
     // not unrolled: two planes an iteration save the register moves but run
     // out of the instruction cache (62.5 us a launch against 59.7 on the
-    // 73 x 712 x 57 compressor, 23.9 against 23.6 at 65 x 242 x 49)
+    // 73 x 752 x 57 compressor, 23.9 against 23.6 at 65 x 242 x 49)
 #pragma unroll 1
     for (int j = ja; j <= jb; ++j) {
         const int p = j - ja;
@@ -1171,7 +1174,7 @@ __global__ void __launch_bounds__(BS, 1024 / BS) k_ts_smooth(const __grid_consta
         // Two lines a thread, in the two halves of f32x2 operations: the pass
         // is bound by its instructions on a large grid (218 a node with one
         // line a thread), and the weights, the tests for a line's ends and the
-        // arithmetic are shared.  59.9 -> 57.3 us a launch on the 73 x 712 x 57
+        // arithmetic are shared.  59.9 -> 57.3 us a launch on the 73 x 752 x 57
         // compressor, 11.0 -> 10.5 on the 33 x 97 x 37 row, the same at
         // 65 x 242 x 49 (segments of 6 points 61.1, of 8 points 72.5: spills).
         // one segment of SM_SEG points of two lines: x(q) gives points
@@ -1400,9 +1403,9 @@ __global__ void k_copy_tm_st(const __grid_constant__ Dev d, int v0, size_t n) {
 
 // k_ts_update_pair where a 512-thread CTA covers a plane's points (TS_PAIR = 0:
 // never); the crossover lies between 63 points, where it is 4 us faster a
-// launch, and 1221, where it is 1 us slower.  In a batch, whose other problems
-// hide a launch's length, always: 64 stages 5.29 ms a step against 5.33
-static bool pair_update(const Dev &d) { return d.TS_PAIR && (d.in_batch || d.IM * d.KM <= 512); }
+// launch, and 1221, where it is 1 us slower (in a batch of 64 stages the two
+// are even)
+static bool pair_update(const Dev &d) { return d.TS_PAIR && d.IM * d.KM <= 512; }
 
 static size_t cells_smem(const Dev &d) {
     return ((size_t)d.IMM1 * d.KMM1 + 2 * d.KMM1 + d.IMM1 + (size_t)d.NIB1 * d.NKB1) * sizeof(float);
