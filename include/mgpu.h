@@ -245,9 +245,8 @@ int32_t mgpu_setup_metrics64(mgpu_handle *h, const double *x, const double *r, c
  * marching -- a Fortran driver that sized the problem to fill the device
  * from fixed COMMON extents, a monitoring thread that reports the
  * efficiency during a long run, a host whose own allocator holds the rest
- * of device memory.  mgpu_integrals_compute allocates host memory on every
- * call and overwrites the handle's node-sized work arrays; this variant
- * allocates no device or host memory (no cudaMalloc/cudaFree, no library
+ * of device memory.  mgpu_integrals_compute works in a buffer that the
+ * handle has allocated; this variant allocates no device or host memory (no cudaMalloc/cudaFree, no library
  * routine that allocates; only recording an error message for
  * mgpu_last_error may take host memory) and writes nothing of the handle's
  * arrays.  Its scratch is
@@ -278,8 +277,8 @@ int32_t mgpu_integrals_noalloc(mgpu_handle *h, mgpu_integrals *out);
 /* ---- batches of independent problems ----------------------------------- */
 /* No counterpart in the reference, which marches one problem per process.
  * A batch steps several committed handles (operating points, grids of any
- * size) with one CUDA graph launch per LOOP iteration: the graph holds one
- * branch per handle, so the kernels of all instances share the GPU at the
+ * size) with one CUDA graph launch per LOOP iteration (a graph for each
+ * kind of step: plain, LOSS, tail, both): the graph holds one branch per handle, so the kernels of all instances share the GPU at the
  * same time.  The handles must live on the current device and outlive the
  * batch; each keeps its own NSTEP, monitors and end test, and every value it
  * computes is bitwise the same as when the handle is stepped alone.  Do not
@@ -363,7 +362,7 @@ int32_t mgpu_adjoint_set(mgpu_handle *h, const char *name, const float *in, int6
 /* The reference prints "CPU TIME PER STEP" every 50 steps
  * (multall-open-18.3.f:5404-5414); these are the device-side equivalents. */
 
-/* Number of kernel launches one LOOP iteration issues from the step graph:
+/* Number of kernel launches one LOOP iteration issues from its step graph:
  * which = 0 a plain step, 1 a LOSS step, 2 a tail step (every 5th), 3 a step
  * that is both. */
 int32_t mgpu_kernels_per_step(mgpu_handle *h, int32_t which);
@@ -375,7 +374,7 @@ int32_t mgpu_kernels_per_step(mgpu_handle *h, int32_t which);
  * ms (8 entries, or NULL) = the time of one launch per candidate, the RO/ROE
  * launch's four first.  The default without tuning is 256 for both.  The
  * candidates differ in the association of per-plane sums (FP32 within a
- * thread, FP64 across threads), so a tuned handle is deterministic for its
+ * thread, double-float across threads), so a tuned handle is deterministic for its
  * choice; two choices can differ in the last bits of a value.  A member of
  * a batch keeps its own choice. */
 int32_t mgpu_autotune(mgpu_handle *h, int32_t *chosen, double *ms);

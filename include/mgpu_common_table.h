@@ -73,8 +73,9 @@
     /* time steps at their current values (frozen-turbulence stepping,    */ \
     /* the primal of the discrete adjoint)                                */ \
     M_(FROZEN,   0)                                                       \
-    /* not a COMMON variable: threads per J-plane CTA of TSTEP, 128, 256  */ \
-    /* or 512 (0: 256 until mgpu_autotune chooses)                        */ \
+    /* not a COMMON variable: threads per J-plane CTA of TSTEP, 128, 192, */ \
+    /* 256 or 512 (0: 256 until mgpu_autotune chooses); the update march  */ \
+    /* has its own size                                                   */ \
     M_(TS_THREADS, 0)                                                     \
     /* not a COMMON variable: 1 (default) runs TSTEP's damping and corner */ \
     /* gather of planes of at most 512 points over pairs of J-planes, 0   */ \

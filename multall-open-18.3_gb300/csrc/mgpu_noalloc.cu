@@ -1,9 +1,8 @@
 // mgpu_noalloc.cu -- mgpu_integrals_noalloc: the EFICOOL integrals of
 // mgpu_integrals_compute through a path that allocates nothing.
 //
-// mgpu_integrals_compute stages its node quantities in the handle's
-// node-sized work arrays (TEMP1, TMP), its per-station sums in a buffer the
-// handle allocated, and its host-side arithmetic in heap vectors.  Here one
+// mgpu_integrals_compute keeps its two stations' sums in a buffer that the
+// handle allocated and does the efficiency's arithmetic on the host.  Here one
 // kernel forms the stagnation quantities at the four corners of each face
 // on the fly and writes the four mass-weighted sums of each J station into
 // a fixed static device array; a one-thread kernel turns the two stations'
