@@ -280,8 +280,8 @@ __global__ void k_delay(long long cycles) {
 // the cell-average density and the model's own arrays, none of which the
 // inlet/exit conditions, the momentum fluxes or TSTEP of the momenta write,
 // and these read nothing it writes.  Its inlet value (4679-4689) follows the
-// conditions; the limiters, which may change the density it reads there,
-// wait for it.
+// conditions; the Mach limiter, which may change the density that it reads at
+// J = 1, waits for it (the density limiter starts at J = 3).
 struct SaBranch {
     cudaStream_t s = nullptr;
     cudaEvent_t start = nullptr, bc = nullptr, done = nullptr;
@@ -331,7 +331,6 @@ void enqueue_core(const Dev &d, Launch L, Launch Lf, cudaEvent_t join = nullptr,
     if (dens) {
         cudaEventRecord(dens->start, L.s);
         cudaStreamWaitEvent(dens->s, dens->start, 0);
-        if (sab) cudaStreamWaitEvent(dens->s, sa->done, 0);
         launch_density_fix(d, Launch{dens->s, L.sm_count, nullptr});
         cudaEventRecord(dens->done, dens->s);
     }
@@ -339,6 +338,7 @@ void enqueue_core(const Dev &d, Launch L, Launch Lf, cudaEvent_t join = nullptr,
     launch_tstep(d, L, V_ROVX, 3);
     if (dens) {
         cudaStreamWaitEvent(L.s, dens->done, 0);
+        if (sab) cudaStreamWaitEvent(L.s, sa->done, 0);
         launch_mach_limiter(d, L0);
     } else {
         launch_density_fix(d, L);

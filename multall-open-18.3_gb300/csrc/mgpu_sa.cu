@@ -495,24 +495,42 @@ __global__ void __launch_bounds__(SA_BS) k_sa_update(const __grid_constant__ Dev
         __syncthreads();
     }
     const float blk = damp_on ? s_blk[A1(d.NROW, j) - 1] : 1.0f;
-    for (int t = threadIdx.x; t < IMM1 * KMM1; t += SA_BS) {
-        const int i = t % IMM1 + 1, k = t / IMM1 + 1;
-        const int n = ix3(d, i, j, k);
-        float v = V.ST[n];
-        if (damp_on) {
-            const float FDAMP = fabsf(v) / blk;
-            v = v / (1.0f + FDAMP / DAMP);
+    // four cells at a time, loaded before the first is stored
+    constexpr int U = 4;
+    WalkN w(IMM1, d.IM * d.JM, d.IM * (j - 1), threadIdx.x, SA_BS);
+    for (int t0 = threadIdx.x; t0 < IMM1 * KMM1; t0 += U * SA_BS) {
+        float st[U], dv[U];
+        int n[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            n[u] = w.n;
+            if (t0 + u * SA_BS < IMM1 * KMM1) {
+                st[u] = V.ST[w.n];
+                dv[u] = V.D[w.n];
+            }
+            w.next();
         }
-        V.D[n] = V.D[n] + v;
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if (t0 + u * SA_BS >= IMM1 * KMM1) break;
+            float v = st[u];
+            if (damp_on) {
+                const float FDAMP = fabsf(v) / blk;
+                v = v / (1.0f + FDAMP / DAMP);
+            }
+            V.D[n[u]] = dv[u] + v;
+        }
     }
 }
 
 // the row's last plane carried across each mixing plane with the decay
-// TURBVIS_DAMP (1560-1591): one thread per (row interface, K)
+// TURBVIS_DAMP (1560-1591): one warp per (row interface, K), its lanes the
+// terms of the pitchwise sum in FP64 (one thread a line was a chain of IM
+// loads and FP64 additions, 9 us on 49 x 162 x 41)
 __global__ void k_sa_mixtransfer(const __grid_constant__ Dev d) {
     pdl_wait();
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (d.NROWS - 1) * d.KMM1) return;
+    const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (t >= (d.NROWS - 1) * d.KMM1) return;          // whole warps leave together
     const int nr = t / d.KMM1 + 1, k = t % d.KMM1 + 1;
     float *D = d.var[V_SA].D;
     const int j = A1(d.JMIX, nr);
@@ -523,11 +541,12 @@ __global__ void k_sa_mixtransfer(const __grid_constant__ Dev d) {
         for (int i = 1; i <= d.IMM1; ++i) AVG = AVG + A1(d.FP, i) * A3(D, i, j, k);
     } else {
         double s = 0.0;
-        for (int i = 1; i <= d.IMM1; ++i) s += (double)(A1(d.FP, i) * A3(D, i, j, k));
+        for (int i = lane + 1; i <= d.IMM1; i += 32) s += (double)(A1(d.FP, i) * A3(D, i, j, k));
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
         AVG = (float)s;
     }
     for (int jav = j + 1; jav <= j + 2; ++jav)
-        for (int i = 1; i <= d.IMM1; ++i) A3(D, i, jav, k) = FMULT * AVG;
+        for (int i = lane + 1; i <= d.IMM1; i += 32) A3(D, i, jav, k) = FMULT * AVG;
 }
 
 // one SMOOTH_RESID pass (14852-14910) of the transported viscosity with
@@ -574,19 +593,19 @@ __global__ void __launch_bounds__(SA_BS) k_sa_resid(const __grid_constant__ Dev 
 // averages of every (J, K) line of the transported viscosity
 __global__ void __launch_bounds__(SA_BS) k_sa_fix(const __grid_constant__ Dev d) {
     pdl_wait();
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= d.JM * d.KM) return;
-    const int j = t % d.JM + 1, k = t / d.JM + 1;
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
+    const bool on = t < d.JM * d.KM;
+    const int j = on ? t % d.JM + 1 : 1, k = on ? t / d.JM + 1 : 1;
     float *D = d.var[V_SA].D;
     const int IM = d.IM, KM = d.KM, ILAST = d.IMM1;
     const int n1 = ix3(d, 1, j, k), nl = ix3(d, ILAST, j, k);
-    if (!(A1(d.IND, j) == 1 || A1(d.INDLE, j) == 1)) {
+    if (on && !(A1(d.IND, j) == 1 || A1(d.INDLE, j) == 1)) {
         const float v = 0.5f * (D[n1] + D[nl]);
         D[n1] = v;
         D[nl] = v;
     }
     const int nr = A1(d.NROW, j);
-    if (KM != 2 && A1(d.KTIPS, nr) > 0) {
+    if (on && KM != 2 && A1(d.KTIPS, nr) > 0) {
         int K1 = A1(d.KTIPS, nr), K2 = A1(d.KTIPE, nr);
         if (K1 == 1) K2 = K2 - 1;
         if (K2 == KM) K1 = K1 + 1;
@@ -597,21 +616,29 @@ __global__ void __launch_bounds__(SA_BS) k_sa_fix(const __grid_constant__ Dev d)
         }
     }
     if (d.IFMIX == 0) return;
-    for (int r = 1; r <= d.NRWSM1; ++r) {
-        const int jx = A1(d.JMIX, r);
-        if (j != jx && j != jx + 1) continue;
+    bool line = false;
+    for (int r = 1; r <= d.NRWSM1; ++r) line = line || j == A1(d.JMIX, r) || j == A1(d.JMIX, r) + 1;
+    // the whole warp averages each of its mixing-plane lines (their threads'
+    // stores above are visible after the vote)
+    unsigned todo = __ballot_sync(0xffffffffu, on && line);
+    __syncwarp();
+    for (; todo; todo &= todo - 1) {
+        const int src = __ffs((int)todo) - 1;
+        const int jl = __shfl_sync(0xffffffffu, j, src), kl = __shfl_sync(0xffffffffu, k, src);
         float s;
         if (d.REDUCE_ORDER != 0) {
             s = 0.0f;
-            for (int i = 1; i <= d.IMM1; ++i) s = s + A1(d.FP, i) * (A3(D, i, j, k) + A3(D, i + 1, j, k));
+            for (int i = 1; i <= d.IMM1; ++i) s = s + A1(d.FP, i) * (A3(D, i, jl, kl) + A3(D, i + 1, jl, kl));
         } else {
             double s64 = 0.0;
-            for (int i = 1; i <= d.IMM1; ++i) s64 += (double)(A1(d.FP, i) * (A3(D, i, j, k) + A3(D, i + 1, j, k)));
+            for (int i = lane + 1; i <= d.IMM1; i += 32)
+                s64 += (double)(A1(d.FP, i) * (A3(D, i, jl, kl) + A3(D, i + 1, jl, kl)));
+            for (int o = 16; o > 0; o >>= 1) s64 += __shfl_xor_sync(0xffffffffu, s64, o);
             s = (float)s64;
         }
         s = 0.5f * s;
-        for (int i = 1; i <= IM; ++i) A3(D, i, j, k) = s;
-        break;
+        __syncwarp();
+        for (int i = lane + 1; i <= IM; i += 32) A3(D, i, jl, kl) = s;
     }
 }
 
@@ -656,11 +683,12 @@ void launch_sa_transport(const Dev &d, Launch L) {
     const unsigned nf = (unsigned)((d.IMM1 * d.JM * d.KMM1 + SA_BS - 1) / SA_BS);
     launchk(L, k_sa_fluxes, dim3(nf), dim3(SA_BS), 0, d);
     mark(L, "k_sa_fluxes");
+    L.pdl = !L.prof;         // the branch's edges are programmatic, as the step's are
     launch_tstep_cells_prolong(d, L, V_SA, 1);
     launchk(L, k_sa_update, dim3(d.JM - 1), dim3(SA_BS), 0, d);
     mark(L, "k_sa_update");
     if (d.NROWS > 1) {
-        launchk(L, k_sa_mixtransfer, dim3((unsigned)(((d.NROWS - 1) * d.KMM1 + 63) / 64)), dim3(64), 0, d);
+        launchk(L, k_sa_mixtransfer, dim3((unsigned)(((d.NROWS - 1) * d.KMM1 + 1) / 2)), dim3(64), 0, d);
         mark(L, "k_sa_mixtransfer");
     }
     // SMOOTH_RESID: J pass D -> TMP, I pass TMP -> D, K pass D -> TMP, and
