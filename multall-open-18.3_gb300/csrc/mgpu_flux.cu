@@ -127,8 +127,8 @@ __global__ void __launch_bounds__(PRIM_BS) k_prim(const __grid_constant__ Dev d,
         }
     }
     if (!do_tail) return;
-    df s;
-    cta_sum_key<PRIM_BS>(d.REDUCE_ORDER, df_of(eke_s), key, &s, &key);
+    double s;
+    cta_sum_key<PRIM_BS>(d.REDUCE_ORDER, eke_s, key, &s, &key);
     if (threadIdx.x == 0) {
         d.part_sum[blk] = s;
         d.part_key[blk] = key;

@@ -140,7 +140,7 @@ struct Dev {
     float *ADJ_RO_MACH;    // RO as the Mach limiter finds it
     double *BLADE_FLOW;                // (JM)
     // per-block reduction partials of the 5-step tail
-    df *part_sum;
+    double *part_sum;
     unsigned long long *part_key;
     int *part_cnt;
     int nparts;
@@ -238,36 +238,64 @@ __device__ __forceinline__ df dacc(int order, df s, df x) {
     return order == 2 ? df{s.hi + x.hi, 0.0f} : df_add(s, x);
 }
 
-// Sum of one FP32 value a thread and the largest key over a CTA of BS
-// threads, for the monitors: thread 0 receives both.  REDUCE_ORDER 2 adds in
-// FP32, the other orders in double-float, which leaves the FP64 pipe alone
-// (an FP64 tree over every node made k_prim 40 us instead of 12 on the steps
-// that run the tail, 65 x 242 x 49).  The key's halves go through the warp's
-// integer maximum.
+// Sum and largest key over a CTA, for the monitors: thread 0 receives both.
+// Each thread brings one FP32 value >= 0.  REDUCE_ORDER 2 adds in FP32; the
+// other orders form the sum to FP64's accuracy and range, with five FP64
+// instructions a CTA: an FP64 tree over every node is 53, which queue on the
+// SM's FP64 pipe.  A warp's values are integers on the scale of its largest
+// one (58 bits of it; what lies below is cut off), their sum is exact, and
+// warp 0 turns the warps' sums into FP64 and adds them.  The 31 cut-off ends
+// stay below 2^-52 of the warp's sum, five rounded FP64 additions below
+// 2^-50.7.  The keys' halves go through the warp's integer maximum.
+struct WarpSum {
+    unsigned long long m;   // the sum is m 2^(e - 184); e = 255: infinity (m = 0) or NaN
+    int e;
+};
+__device__ __forceinline__ WarpSum warp_sum(float v) {
+    const unsigned bits = __float_as_uint(v), top = __reduce_max_sync(0xffffffffu, bits);
+    if (top >= 0x7f800000u) return WarpSum{top != 0x7f800000u, 255};
+    const int e = max((int)(top >> 23), 1), x = max((int)(bits >> 23), 1);
+    const unsigned long long f = (bits & 0x7fffffu) | (bits >= 0x800000u ? 0x800000u : 0u);
+    const unsigned long long q = e - x < 58 ? (f << 34) >> (e - x) : 0ull;
+    const unsigned mask = (1u << 22) - 1;
+    const unsigned q0 = __reduce_add_sync(0xffffffffu, (unsigned)q & mask);
+    const unsigned q1 = __reduce_add_sync(0xffffffffu, (unsigned)(q >> 22) & mask);
+    const unsigned q2 = __reduce_add_sync(0xffffffffu, (unsigned)(q >> 44));
+    return WarpSum{((unsigned long long)q2 << 44) + ((unsigned long long)q1 << 22) + q0, e};
+}
+__device__ __forceinline__ double warp_sum_val(WarpSum s) {
+    if (s.e == 255) return __longlong_as_double(s.m ? 0x7ff8000000000000ll : 0x7ff0000000000000ll);
+    return (double)s.m * __longlong_as_double((long long)(s.e + 1023 - 184) << 52);
+}
 __device__ __forceinline__ unsigned long long warp_max_key(unsigned long long key) {
     const unsigned hi = (unsigned)(key >> 32), m = __reduce_max_sync(0xffffffffu, hi);
     const unsigned lo = __reduce_max_sync(0xffffffffu, hi == m ? (unsigned)key : 0u);
     return ((unsigned long long)m << 32) | lo;
 }
 template <int BS>
-__device__ __forceinline__ void cta_sum_key(int order, df s, unsigned long long key, df *out_s,
+__device__ __forceinline__ void cta_sum_key(int order, float v, unsigned long long key, double *out_s,
                                             unsigned long long *out_k) {
-    __shared__ df ss[BS / 32];
+    __shared__ WarpSum ss[BS / 32];
+    __shared__ float sf[BS / 32];
     __shared__ unsigned long long sk[BS / 32];
-    for (int o = 16; o > 0; o >>= 1) s = dacc(order, s, df_shfl_down(s, o));
-    key = warp_max_key(key);
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+    WarpSum s{0ull, 1};
+    if (order == 2)
+        for (int o = 16; o > 0; o >>= 1) v = v + __shfl_down_sync(0xffffffffu, v, o);
+    else s = warp_sum(v);
+    key = warp_max_key(key);
     if (l == 0) {
         ss[w] = s;
+        sf[w] = v;
         sk[w] = key;
     }
     __syncthreads();
     if (w == 0) {
-        s = l < BS / 32 ? ss[l] : df{0.0f, 0.0f};
+        double t = l >= BS / 32 ? 0.0 : order == 2 ? (double)sf[l] : warp_sum_val(ss[l]);
         key = l < BS / 32 ? sk[l] : 0ull;
-        for (int o = BS / 64; o > 0; o >>= 1) s = dacc(order, s, df_shfl_down(s, o));
+        for (int o = BS / 64; o > 0; o >>= 1) t = racc(order, t, __shfl_down_sync(0xffffffffu, t, o));
         key = warp_max_key(key);
-        *out_s = s;
+        *out_s = t;
         *out_k = key;
     }
 }

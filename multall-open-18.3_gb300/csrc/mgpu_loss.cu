@@ -799,26 +799,42 @@ constexpr int TAIL_BS = 256;
 // next launch that has room for it: the last CTA of the launch itself would
 // be found by a ticket (a fence and an atomic each, 3000 CTAs on the stage)
 // and would run alone, 8 us at the end of k_prim and 3 us after the node pass.
-__device__ __forceinline__ void finish_parts(const Dev &d, int n, df *s, unsigned long long *key) {
-    df t = df_of(0.0f);
+__device__ __forceinline__ void finish_parts(const Dev &d, int n, double *s, unsigned long long *key) {
+    __shared__ double ss[TAIL_BS / 32];
+    __shared__ unsigned long long sk[TAIL_BS / 32];
+    const int ro = d.REDUCE_ORDER, w = threadIdx.x >> 5, l = threadIdx.x & 31;
+    double t = 0.0;
     unsigned long long m = 0ull;
 #pragma unroll 4
     for (int p = threadIdx.x; p < n; p += TAIL_BS) {
-        t = dacc(d.REDUCE_ORDER, t, d.part_sum[p]);
+        t = racc(ro, t, d.part_sum[p]);
         const unsigned long long k2 = d.part_key[p];
         m = k2 > m ? k2 : m;
     }
-    cta_sum_key<TAIL_BS>(d.REDUCE_ORDER, t, m, s, key);
+    for (int o = 16; o > 0; o >>= 1) t = racc(ro, t, __shfl_down_sync(0xffffffffu, t, o));
+    m = warp_max_key(m);
+    if (l == 0) {
+        ss[w] = t;
+        sk[w] = m;
+    }
+    __syncthreads();
+    if (w == 0) {
+        t = l < TAIL_BS / 32 ? ss[l] : 0.0;
+        m = l < TAIL_BS / 32 ? sk[l] : 0ull;
+        for (int o = TAIL_BS / 64; o > 0; o >>= 1) t = racc(ro, t, __shfl_down_sync(0xffffffffu, t, o));
+        *s = t;
+        *key = warp_max_key(m);
+    }
 }
 
 // VREF and VMAX from k_prim's n partial sums of |W|^2
 __device__ void finish_vref(const Dev &d, int n) {
-    df s;
+    double s;
     unsigned long long key;
     finish_parts(d, n, &s, &key);
     if (threadIdx.x == 0) {
         DevCtl *c = d.ctl;
-        c->VREF = sqrtf(df_val(s) * d.RIJKM);
+        c->VREF = sqrtf((float)s * d.RIJKM);
         c->VMAX = 0.0f;
         if (key) {
             const unsigned lin = 0xFFFFFFFFu - (unsigned)(key & 0xFFFFFFFFull);
@@ -919,8 +935,8 @@ __global__ void __launch_bounds__(TAIL_BS) k_tail_nodes(const __grid_constant__ 
         }
     }
     const int ro = d.REDUCE_ORDER;
-    df s;
-    cta_sum_key<TAIL_BS>(ro, df_of(sf), key, &s, &key);
+    double s;
+    cta_sum_key<TAIL_BS>(ro, sf, key, &s, &key);
     bad = __syncthreads_count(bad & 1) + 2 * __syncthreads_count(bad & 2) + 4 * __syncthreads_count(bad & 4) +
           8 * __syncthreads_count(bad & 8);              // bad <= TAIL_NPT
     if (threadIdx.x == 0) {
@@ -958,7 +974,7 @@ __device__ void finish_tail(const Dev &d, int n) {
         se[threadIdx.x >> 5] = ek;
         sc[threadIdx.x >> 5] = bad;
     }
-    df s;
+    double s;
     unsigned long long key;
     finish_parts(d, n, &s, &key);
     if (threadIdx.x == 0) {
@@ -968,7 +984,7 @@ __device__ void finish_tail(const Dev &d, int n) {
             ke = se[w] > ke ? se[w] : ke;
             cnt += sc[w];
         }
-        const float eavg = df_val(s) / (float)(d.IM * d.JMM1 * d.KM);
+        const float eavg = (float)s / (float)(d.IM * d.JMM1 * d.KM);
         float emax = 0.0f;
         if (key) {
             unsigned lin = 0xFFFFFFFFu - (unsigned)(key & 0xFFFFFFFFull);
