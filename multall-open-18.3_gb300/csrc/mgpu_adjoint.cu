@@ -1887,25 +1887,38 @@ __global__ void rk_seed_plane(const Dev d, const Adj a, float *seed, int j,
         if (e_ != cudaSuccess) return api_fail(MGPU_E_CUDA, (std::string(#call) + ": " + cudaGetErrorString(e_)).c_str()); \
     } while (0)
 
-// Row means of |STORE| after the row mixing, as the negative feedback of the
-// recorded step formed them (1501-1525), from its per-plane sums: one CTA per
-// variable.  (Summed again over the cells in FP64 they took 1540 us at
-// 65 x 242 x 49.)
-__global__ void rk_blk(const __grid_constant__ Dev d, const __grid_constant__ Adj a) {
-    __shared__ float chg[64];
-    const VarSet &V = d.var[blockIdx.x];
-    float *blk = const_cast<float *>(a.v[blockIdx.x].tBLK);
-    const int w = threadIdx.x >> 5, l = threadIdx.x & 31, NROWS = d.NROWS, ro = d.REDUCE_ORDER;
-    if (ro == 1) {
-        for (int nr = threadIdx.x; nr < NROWS; nr += RT_BS) blk[nr] = V.AVG_BLK[nr];
-        return;
+// Row means of |STORE| of the recorded step after the row mixing (1501-1525),
+// summed over the cells in FP64: a CTA per plane and variable, then one per
+// variable (in one CTA per variable the cells took 1540 us at 65 x 242 x 49,
+// held by one SM's FP64 pipe each).  The planes' sums lie in pblk, which the
+// reverse step rewrites before it reads it.
+__global__ void __launch_bounds__(RT_BS) rk_blk_planes(const __grid_constant__ Dev d, const __grid_constant__ Adj a) {
+    __shared__ double sh[RT_BS / 32];
+    const AdjVar &V = a.v[blockIdx.y];
+    const int j = blockIdx.x + 2, nc = d.IMM1 * d.KMM1;
+    double s = 0.0;
+    WalkN w(d.IMM1, d.IM * d.JM, d.IM * (j - 1), threadIdx.x, RT_BS);
+    for (int c = threadIdx.x; c < nc; c += RT_BS, w.next()) s += (double)fabsf(V.tST[w.n]);
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = s;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double t = 0.0;
+        for (int q = 0; q < RT_BS / 32; ++q) t += sh[q];
+        V.pblk[j - 1] = t;
     }
+}
+__global__ void __launch_bounds__(RT_BS) rk_blk(const __grid_constant__ Dev d, const __grid_constant__ Adj a) {
+    __shared__ float chg[64];
+    const AdjVar &V = a.v[blockIdx.x];
+    float *blk = const_cast<float *>(V.tBLK);
+    const int w = threadIdx.x >> 5, l = threadIdx.x & 31, NROWS = d.NROWS;
     for (int nr = w + 1; nr <= NROWS; nr += RT_BS / 32) {
         const int JST = A1(d.JSTART, nr) + 1, JEN = A1(d.JMIX, nr) - 1;
-        df s = df_of(0.0f);
-        for (int jj = JST + l; jj <= JEN; jj += 32) s = dacc(ro, s, V.pabs[jj - 1]);
-        for (int o = 16; o > 0; o >>= 1) s = dacc(ro, s, df_shfl_down(s, o));
-        if (l == 0) chg[nr - 1] = df_val(s) / (float)(d.IMM1 * d.KMM1 * (JEN - JST + 1));
+        double s = 0.0;
+        for (int jj = JST + l; jj <= JEN; jj += 32) s += V.pblk[jj - 1];
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+        if (l == 0) chg[nr - 1] = (float)s / (float)(d.IMM1 * d.KMM1 * (JEN - JST + 1));
     }
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -2508,6 +2521,7 @@ int32_t mgpu_adjoint_prepare(mgpu_handle *h) {
     // the EFICOOL sums of the step's arrays (the objectives' forward values)
     double *dint = handle_int_buf(h);
     launch_station_sums(rec, L, d.NSTAGES == 1 ? 1 : 2, d.JM - 1, dint, IntLines{});
+    rk_blk_planes<<<dim3((unsigned)(d.JM - 1), NVAR), RT_BS, 0, st>>>(d, a);
     rk_blk<<<NVAR, RT_BS, 0, st>>>(d, a);
     rk_density_prep<<<gridn(np, 8), 256, 0, st>>>(d, a);
     ACK(cudaGetLastError());
