@@ -110,6 +110,7 @@ struct mgpu_batch {
     // a step that is of one kind for every member (as mgpu_handle::sg), and
     // one in which each member's own flags decide
     StepGraph sg[4], mixed;
+    std::vector<int> ts_bs;      // the members' CTA sizes that the graphs were captured with
     DevCtl **d_list = nullptr;   // the members' control blocks, their copies and the host's
     DevCtl *d_ctl = nullptr, *h_ctl = nullptr;
     void *flush_buf = nullptr;
@@ -438,6 +439,18 @@ int capture_step(mgpu_handle *h, int what) {
     return rc;
 }
 
+// Makes the captured graph g ready to launch on s: what it takes of the
+// device's memory, it takes here.
+int instantiate(StepGraph &G, cudaGraph_t g, cudaStream_t s) {
+    G.graph = g;
+    cudaError_t e = cudaGraphGetNodes(g, nullptr, &G.nodes);
+    if (e == cudaSuccess) e = cudaGraphInstantiate(&G.exec, g, 0);
+    if (e == cudaSuccess) e = cudaGraphUpload(G.exec, s);
+    if (e == cudaSuccess) return 0;
+    G.drop();
+    return fail(MGPU_E_CUDA, std::string("graph: ") + cudaGetErrorString(e));
+}
+
 // one LOOP iteration of h as a CUDA graph, by what it runs
 int build_graph(mgpu_handle *h, int what) {
     StepGraph &G = h->sg[what];
@@ -451,9 +464,24 @@ int build_graph(mgpu_handle *h, int what) {
         return rc;
     }
     if (e != cudaSuccess) return fail(MGPU_E_CUDA, std::string("graph capture: ") + cudaGetErrorString(e));
-    G.graph = g;
-    CK(cudaGraphGetNodes(g, nullptr, &G.nodes));
-    CK(cudaGraphInstantiate(&G.exec, g, 0));
+    return instantiate(G, g, h->stream);
+}
+
+// Whether a march comes to a step of kind `what` (bit 0 LOSS, bit 1 the tail,
+// as step_what).  The final step may be any, so a tail may go without LOSS.
+bool kind_occurs(const Dev &d, int what) {
+    if (d.ILOS == 0 || d.FROZEN) return !(what & 1);
+    if (d.NLOS == 1) return (what & 1) != 0;
+    return what != 1 || d.NLOS % 5 != 0;
+}
+
+// Every graph that a march of h can need, before its first step: from then on
+// the march takes no device memory and its stream does not capture, whatever
+// kind of step comes next (the final one is often the first of its kind).
+int build_graphs(mgpu_handle *h) {
+    for (int what = 0; what < 4; ++what)
+        if (kind_occurs(h->d, what))
+            if (int rc = build_graph(h, what)) return rc;
     return 0;
 }
 
@@ -508,13 +536,11 @@ int step_what(const Dev &d, const DevCtl &c, int q, bool force_end) {
 }
 
 // launches the steps that follow the mirrored control block, none of them
-// past the next tail
+// past the next tail; build_graphs has run
 int launch_steps(mgpu_handle *h, int n, bool force_end) {
     h->ctl_known = false;
     for (int q = 0; q < n; ++q) {
         const int what = step_what(h->d, *h->h_ctl, q, force_end);
-        int rc = build_graph(h, what);
-        if (rc) return rc;
         CK(cudaGraphLaunch(h->sg[what].exec, h->stream));
     }
     return 0;
@@ -1263,7 +1289,8 @@ int32_t mgpu_loss_init(mgpu_handle *h) {
 
 int32_t mgpu_step(mgpu_handle *h, int32_t force_end, mgpu_monitors *mon) {
     if (!h || !h->committed) return fail(MGPU_E_STATE, "step before commit");
-    int rc = 0;
+    int rc = build_graphs(h);
+    if (rc) return rc;
     if (!h->ctl_known && (rc = read_ctl(h))) return rc;
     int fe = force_end ? 1 : 0;
     CK(cudaMemcpyAsync(&h->d.ctl->force_end, &fe, sizeof(int), cudaMemcpyHostToDevice, h->stream));
@@ -1278,7 +1305,8 @@ int32_t mgpu_step(mgpu_handle *h, int32_t force_end, mgpu_monitors *mon) {
 int32_t mgpu_run(mgpu_handle *h, int32_t nsteps, mgpu_monitors *mon) {
     if (!h || !h->committed) return fail(MGPU_E_STATE, "run before commit");
     if (nsteps < 0) return fail(MGPU_E_ARG, "negative step count");
-    int rc = 0;
+    int rc = build_graphs(h);
+    if (rc) return rc;
     // The end test at the top of step n (3762-3764) reads NSTEP and the
     // monitors EMAX, EAVG and ECONT, which only a tail (every fifth step, or
     // the final one) rewrites.  So no step after a tail up to and including
@@ -1530,7 +1558,8 @@ int32_t mgpu_autotune(mgpu_handle *h, int32_t *chosen, double *ms) {
 
 int32_t mgpu_bench_steps(mgpu_handle *h, int32_t nsteps, int32_t flush_l2, double *total_ms) {
     if (!h || !h->committed || !total_ms || nsteps < 0) return fail(MGPU_E_ARG, "bad arguments to mgpu_bench_steps");
-    int rc = 0;
+    int rc = build_graphs(h);
+    if (rc) return rc;
     if (flush_l2 && !h->flush_buf) {
         int l2 = 0;
         cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, h->device);
@@ -1548,7 +1577,6 @@ int32_t mgpu_bench_steps(mgpu_handle *h, int32_t nsteps, int32_t flush_l2, doubl
         h->ctl_known = false;
         for (int q = 0; q < n; ++q, ++s) {
             const int what = step_what(h->d, *h->h_ctl, q, false);
-            if ((rc = build_graph(h, what))) return rc;
             if (flush_l2) CK(cudaMemsetAsync(h->flush_buf, s & 0xff, h->flush_bytes, h->stream));
             CK(cudaEventRecord(ev[2 * s], h->stream));
             CK(cudaGraphLaunch(h->sg[what].exec, h->stream));
@@ -1661,9 +1689,28 @@ int batch_graph(mgpu_batch *b, int what) {
         if (rc) return rc;
         return fail(MGPU_E_CUDA, std::string("batch capture: ") + cudaGetErrorString(e != cudaSuccess ? e : e2));
     }
-    G.graph = g;
-    CK(cudaGraphInstantiate(&G.exec, g, 0));
-    return 0;
+    return instantiate(G, g, b->stream);
+}
+
+// Every graph that a march of the batch can need, as build_graphs; a step of
+// one kind for all members where each of them comes to that kind.  Built at
+// creation, and again where a member has been tuned since: each is captured
+// with its members' CTA sizes, and all of them with the same.
+int batch_graphs(mgpu_batch *b) {
+    std::vector<int> ts;
+    for (const mgpu_handle *h : b->hs) ts.insert(ts.end(), h->d.ts_bs, h->d.ts_bs + 2);
+    if (ts != b->ts_bs) {
+        for (StepGraph &G : b->sg) G.drop();
+        b->mixed.drop();
+        b->ts_bs = ts;
+    }
+    for (int what = 0; what < 4; ++what) {
+        bool all = true;
+        for (const mgpu_handle *h : b->hs) all = all && kind_occurs(h->d, what);
+        if (all)
+            if (int rc = batch_graph(b, what)) return rc;
+    }
+    return b->hs.size() > 1 ? batch_graph(b, -1) : 0;
 }
 
 // the control blocks of a batch side by side, for one copy to the host
@@ -1725,8 +1772,7 @@ int32_t mgpu_batch_create(mgpu_handle *const *handles, int32_t n, mgpu_batch **o
     if (e == cudaSuccess) e = cudaMemcpy(b->d_list, list.data(), n * sizeof(DevCtl *), cudaMemcpyHostToDevice);
     if (e != cudaSuccess) return bail(fail(MGPU_E_NOMEM, std::string("mgpu_batch_create: ") + cudaGetErrorString(e)));
     batch_chains(b);
-    int rc = batch_graph(b, 0);
-    if (!rc) rc = batch_graph(b, 3);
+    int rc = batch_graphs(b);
     if (rc) return bail(rc);
     *out = b;
     return 0;
@@ -1776,8 +1822,8 @@ int batch_known(mgpu_batch *b) {
 // `most`: up to the first tail while each step is of one kind for every
 // member; otherwise (members at different steps, or past their end) a stretch
 // of mixed ones.  Leaves the mirrors invalid.
-int batch_plan(mgpu_batch *b, int most, std::vector<int> &plan) {
-    int n = most, rc = 0;
+void batch_plan(mgpu_batch *b, int most, std::vector<int> &plan) {
+    int n = most;
     for (mgpu_handle *h : b->hs) {
         const int k = steps_to_tail(h->d, *h->h_ctl);
         n = k < n ? k : n;
@@ -1788,22 +1834,20 @@ int batch_plan(mgpu_batch *b, int most, std::vector<int> &plan) {
         for (mgpu_handle *h : b->hs)
             if (step_what(h->d, *h->h_ctl, q, false) != what) {
                 plan.assign(most < 50 ? most : 50, -1);
-                return batch_graph(b, -1);
+                return;
             }
-        if ((rc = batch_graph(b, what))) return rc;
         plan.push_back(what);
     }
-    return 0;
 }
 }  // namespace
 
 int32_t mgpu_batch_run(mgpu_batch *b, int32_t nsteps, mgpu_monitors *mons) {
     if (!b || nsteps < 0) return fail(MGPU_E_ARG, "bad arguments to mgpu_batch_run");
     int done = 0, ended = 0, rc = 0;
-    if ((rc = batch_known(b))) return rc;
+    if ((rc = batch_graphs(b)) || (rc = batch_known(b))) return rc;
     while (done < nsteps) {
         std::vector<int> plan;
-        if ((rc = batch_plan(b, nsteps - done, plan))) return rc;
+        batch_plan(b, nsteps - done, plan);
         for (int what : plan) CK(cudaGraphLaunch((what < 0 ? b->mixed : b->sg[what]).exec, b->stream));
         done += (int)plan.size();
         if ((rc = batch_read(b, mons, &ended))) return rc;
@@ -1821,12 +1865,12 @@ int32_t mgpu_batch_bench_steps(mgpu_batch *b, int32_t nsteps, int32_t flush_l2, 
         CK(cudaMalloc(&b->flush_buf, b->flush_bytes));
     }
     int ended = 0, rc = 0;
-    if ((rc = batch_known(b))) return rc;
+    if ((rc = batch_graphs(b)) || (rc = batch_known(b))) return rc;
     std::vector<cudaEvent_t> ev((size_t)2 * nsteps);
     for (auto &e : ev) CK(cudaEventCreate(&e));
     for (int s = 0; s < nsteps;) {
         std::vector<int> plan;
-        if ((rc = batch_plan(b, nsteps - s, plan))) return rc;
+        batch_plan(b, nsteps - s, plan);
         for (int what : plan) {
             if (flush_l2) CK(cudaMemsetAsync(b->flush_buf, s & 0xff, b->flush_bytes, b->stream));
             CK(cudaEventRecord(ev[2 * s], b->stream));
