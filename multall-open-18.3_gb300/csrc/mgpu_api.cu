@@ -517,11 +517,19 @@ void fill_monitors(const DevCtl &c, mgpu_monitors *m) {
     m->flow_out = c.flow_out;
 }
 
-int read_ctl(mgpu_handle *h) {
-    CK(cudaMemcpyAsync(h->h_ctl, h->d.ctl, sizeof(DevCtl), cudaMemcpyDeviceToHost, h->stream));
+// the control block into the caller's own copy (a getter may be called on
+// another thread than a march, which plans its steps from the mirror)
+int fetch_ctl(const mgpu_handle *h, DevCtl *c) {
+    CK(cudaMemcpyAsync(c, h->d.ctl, sizeof(DevCtl), cudaMemcpyDeviceToHost, h->stream));
     CK(cudaStreamSynchronize(h->stream));
-    h->ctl_known = true;
     return 0;
+}
+
+// the control block into the mirror
+int read_ctl(mgpu_handle *h) {
+    int rc = fetch_ctl(h, h->h_ctl);
+    if (!rc) h->ctl_known = true;
+    return rc;
 }
 
 // What the step after the mirrored control block c runs, q steps on: bit 0
@@ -748,9 +756,9 @@ int32_t mgpu_get_real(mgpu_handle *h, const char *name, float *value) {
     if (h->committed && (!strcmp(name, "VISLAM") || !strcmp(name, "FTCOND") || !strcmp(name, "SFT") ||
                          !strcmp(name, "SFX") || !strcmp(name, "DAMP") || !strcmp(name, "FMIXUP") ||
                          !strcmp(name, "PDOWN_HUB") || !strcmp(name, "PDOWN_TIP") || !strcmp(name, "THROTTLE_PRES"))) {
-        int rc = read_ctl(h);
+        DevCtl c;
+        int rc = fetch_ctl(h, &c);
         if (rc) return rc;
-        const DevCtl &c = *h->h_ctl;
         if (!strcmp(name, "VISLAM")) *value = c.VISLAM;
         else if (!strcmp(name, "FTCOND")) *value = c.FTCOND;
         else if (!strcmp(name, "SFT")) *value = c.SFT;
@@ -771,9 +779,10 @@ int32_t mgpu_get_real(mgpu_handle *h, const char *name, float *value) {
 int32_t mgpu_get_int(mgpu_handle *h, const char *name, int32_t *value) {
     if (!h || !name || !value) return fail(MGPU_E_ARG, "null argument");
     if (!strcmp(name, "NSTEP") && h->committed) {
-        int rc = read_ctl(h);
+        DevCtl c;
+        int rc = fetch_ctl(h, &c);
         if (rc) return rc;
-        *value = h->h_ctl->nstep;
+        *value = c.nstep;
         return 0;
     }
 #define MGPU_GETI(n, v) if (!strcmp(name, #n)) { *value = h->d.n; return 0; }
