@@ -1852,14 +1852,17 @@ void batch_plan(mgpu_batch *b, int most, std::vector<int> &plan) {
 
 int32_t mgpu_batch_run(mgpu_batch *b, int32_t nsteps, mgpu_monitors *mons) {
     if (!b || nsteps < 0) return fail(MGPU_E_ARG, "bad arguments to mgpu_batch_run");
+    const int chunk = 50;        // a failed member ends the call, but lets the others come this far
     int done = 0, ended = 0, rc = 0;
     if ((rc = batch_graphs(b)) || (rc = batch_known(b))) return rc;
     while (done < nsteps) {
+        const int left = nsteps - done, most = chunk - done % chunk;
         std::vector<int> plan;
-        batch_plan(b, nsteps - done, plan);
+        batch_plan(b, left < most ? left : most, plan);
         for (int what : plan) CK(cudaGraphLaunch((what < 0 ? b->mixed : b->sg[what]).exec, b->stream));
         done += (int)plan.size();
-        if ((rc = batch_read(b, mons, &ended))) return rc;
+        rc = done < nsteps && done % chunk ? batch_fetch(b) : batch_read(b, mons, &ended);
+        if (rc) return rc;
     }
     if (nsteps == 0 && (rc = batch_read(b, mons, &ended))) return rc;
     return ended;
@@ -1887,7 +1890,7 @@ int32_t mgpu_batch_bench_steps(mgpu_batch *b, int32_t nsteps, int32_t flush_l2, 
             CK(cudaEventRecord(ev[2 * s + 1], b->stream));
             ++s;
         }
-        if (s < nsteps && (rc = batch_read(b, nullptr, &ended))) return rc;
+        if (s < nsteps && (rc = batch_fetch(b))) return rc;
     }
     CK(cudaStreamSynchronize(b->stream));
     double tot = 0.0;
