@@ -2206,8 +2206,12 @@ int configure(const Dev &d) {
         size_t b;
     } k[] = {{(const void *)rk_ts_smooth, smooth_bytes(d)}, {(const void *)rk_ts_gather, gather_bytes(d)},
              {(const void *)rk_ts_damp, damp_bytes(d)}, {(const void *)rk_ts_cells, cells_bytes(d)}};
+    // the limit is on what a plane takes, as in configure_bs: the smoothing
+    // weights (2.6 KB at most) come on top
+    const size_t extra = (size_t)2 * (d.IM + d.KM) * sizeof(float);
     for (auto &x : k) {
-        if (x.b > 200 * 1024) return api_fail(MGPU_E_UNSUPPORTED, "J-plane too large for the adjoint kernels");
+        if (x.b - (x.f == (const void *)rk_ts_smooth ? extra : 0) > 200 * 1024)
+            return api_fail(MGPU_E_UNSUPPORTED, "J-plane too large for the adjoint kernels");
         ACK(raise_smem(x.f, x.b));
     }
     return 0;
