@@ -12,6 +12,7 @@
 #include <cstdio>
 #include <cstring>
 #include <map>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -86,6 +87,7 @@ struct mgpu_handle {
     bool ctl_known = false;      // h_ctl mirrors the control block: nothing has run since it was read
     double *d_int = nullptr;     // launch_station_sums (INT_BUF)
     double *h_int = nullptr;     // its result, pinned (INT_OUT)
+    std::mutex int_mutex;        // held while a report uses these two
     // host copies of what the reports read of the bound data, which is fixed
     // after commit
     std::vector<int> r_nstage, r_jstart, r_jmix, r_nrow;
@@ -485,13 +487,17 @@ int build_graphs(mgpu_handle *h) {
     return 0;
 }
 
-// FP64 mass averages at stations J1 and J2 (and lines of P) into h->h_int
-int station_sums(mgpu_handle *h, int J1, int J2, const IntLines &lines) {
+// FP64 mass averages at stations J1 and J2 into out[0..7], and lines of P
+// behind them (IntLines).  The buffers are the handle's: one report at a time
+// uses them, and leaves with a copy of its own.
+int station_sums(mgpu_handle *h, int J1, int J2, const IntLines &lines, std::vector<double> &out) {
+    const size_t bytes = 8 * sizeof(double) + (size_t)lines.n * lines.n * h->d.IM * sizeof(float);
+    std::lock_guard<std::mutex> one(h->int_mutex);
     launch_station_sums(h->d, Launch{h->stream, h->sm_count}, J1, J2, h->d_int, lines);
     CK(cudaGetLastError());
-    const size_t bytes = 8 * sizeof(double) + (size_t)lines.n * lines.n * h->d.IM * sizeof(float);
     CK(cudaMemcpyAsync(h->h_int, h->d_int, bytes, cudaMemcpyDeviceToHost, h->stream));
     CK(cudaStreamSynchronize(h->stream));
+    out.assign(h->h_int, h->h_int + (bytes + sizeof(double) - 1) / sizeof(double));
     return 0;
 }
 
@@ -1361,9 +1367,9 @@ int32_t mgpu_integrals_compute(mgpu_handle *h, mgpu_integrals *out) {
     // whole-machine efficiency (11269-11394): for one stage the inlet
     // station is J=1, otherwise J=2; the exit station is JM-1
     int J1 = d.NSTAGES == 1 ? 1 : 2, J2M1 = d.JM - 1;
-    int rc = station_sums(h, J1, J2M1, IntLines{});
+    std::vector<double> v;
+    int rc = station_sums(h, J1, J2M1, IntLines{}, v);
     if (rc) return rc;
-    const double *v = h->h_int;
     auto bf = [&](int j) { return v[j == J1 ? 0 : 4]; };
     auto spo = [&](int j) { return v[j == J1 ? 1 : 5] / bf(j); };
     auto sto = [&](int j) { return v[j == J1 ? 2 : 6] / bf(j); };
@@ -1428,9 +1434,9 @@ int32_t mgpu_stage_performance(mgpu_handle *h, int32_t nstg, mgpu_stage *out) {
     const int KMID2 = d.KM / 2;
     IntLines lines{};
     if (!whole) lines = IntLines{3, {J1, JMS, J2M1}, {1, KMID2, d.KM}};
-    int rc = station_sums(h, J1, J2M1, lines);
+    std::vector<double> v;
+    int rc = station_sums(h, J1, J2M1, lines, v);
     if (rc) return rc;
-    const double *v = h->h_int;
     auto bf = [&](int j) { return v[j == J1 ? 0 : 4]; };
     auto spo = [&](int j) { return v[j == J1 ? 1 : 5] / bf(j); };
     auto sto = [&](int j) { return v[j == J1 ? 2 : 6] / bf(j); };
@@ -1445,7 +1451,7 @@ int32_t mgpu_stage_performance(mgpu_handle *h, int32_t nstg, mgpu_stage *out) {
         // pitchwise static pressures, REAL*4 in I order (11300-11349), at the
         // stations J1, JMS, J2M1 (a) and K = 1, KM/2, KM (b)
         auto pline = [&](int a, int b) {
-            const float *P = (const float *)(h->h_int + 8) + (size_t)(3 * a + b) * d.IM;
+            const float *P = (const float *)(v.data() + 8) + (size_t)(3 * a + b) * d.IM;
             float s = 0.0f;
             for (int i = 0; i < d.IMM1; ++i) s = s + 0.5f * (P[i] + P[i + 1]) * FP[i];
             return s;
