@@ -1506,8 +1506,11 @@ __global__ void __launch_bounds__(RT_BS) rk_ts_damp(const __grid_constant__ Dev 
         {
             const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
             for (int nr = w + 1; nr <= NROWS; nr += RT_BS / 32) {
+                // the planes that the row's mean damps: those of NROW, of which
+                // the last row's may lie past its JMIX
                 double s = 0.0;
-                for (int jj = max(A1(d.JSTART, nr), 2) + l; jj <= A1(d.JMIX, nr); jj += 32) s += V.pblk[jj - 1];
+                for (int jj = 2 + l; jj <= d.JM; jj += 32)
+                    if (A1(d.NROW, jj) == nr) s += V.pblk[jj - 1];
                 for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
                 if (l == 0) {
                     gblk[nr - 1] = (float)s;
