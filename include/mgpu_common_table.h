@@ -80,7 +80,12 @@
     /* not a COMMON variable: 1 (default) runs TSTEP's damping and corner */ \
     /* gather of planes of at most 512 points over pairs of J-planes, 0   */ \
     /* always marching along J; the results are bitwise the same          */ \
-    M_(TS_PAIR, 1)
+    M_(TS_PAIR, 1)                                                        \
+    /* not COMMON variables: how the march is cut, rows of K (a multiple  */ \
+    /* of 3, at most 864/IM) and planes (at most 16) of a CTA; 0 (default) */ \
+    /* by the grid's size; the results are bitwise the same               */ \
+    M_(TS_ROWS, 0)                                                        \
+    M_(TS_PLANES, 0)
 
 /* ----- REAL scalars: /BKGAS/, /BKCNTL/, /BKSMTH/, /BKLOSS/, /BKINPT/ ---- */
 #define MGPU_REAL_SCALARS(M_)                                             \

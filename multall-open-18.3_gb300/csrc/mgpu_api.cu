@@ -1261,6 +1261,8 @@ int32_t mgpu_commit(mgpu_handle *h) {
         d.TS_THREADS != 512)
         return fail(MGPU_E_ARG, "TS_THREADS must be 0, 128, 192, 256 or 512");
     if (d.TS_PAIR != 0 && d.TS_PAIR != 1) return fail(MGPU_E_ARG, "TS_PAIR must be 0 or 1");
+    if (d.TS_ROWS < 0 || d.TS_ROWS % UP_S || d.TS_ROWS / UP_S * d.IM > UP_T || d.TS_PLANES < 0 || d.TS_PLANES > UP_R)
+        return fail(MGPU_E_ARG, "TS_ROWS must be 0 or a multiple of 3 up to 864/IM, TS_PLANES 0 to 16");
     d.ts_bs[0] = d.ts_bs[1] = d.TS_THREADS ? d.TS_THREADS : 256;
     // the control block
     DevCtl c;

@@ -474,6 +474,11 @@ inline void mark(const Launch &L, const char *name) {
     }
 }
 
+// TSTEP's update march (mgpu_tstep.cu)
+constexpr int UP_S = 3;          // nodes along K of one thread of update
+constexpr int UP_T = 288;        // most threads of an update CTA (three CTAs at 72 registers)
+constexpr int UP_R = 16;         // most J planes of an update CTA
+
 void launch_step_begin(const Dev &d, Launch L);
 // what < 0: the step control has run (k_step_begin); otherwise the launch
 // runs it too, for a step of which the host knows that the tail runs (bit 1)

@@ -47,9 +47,6 @@ constexpr int PR_U = 3;          // the same in prolong: five CTAs an SM at 48 r
                                  // against 15.8 at 65 x 242 x 49)
 constexpr int TS_UG = 4;         // cells per thread whose loads the pair update issues together
 constexpr int UG_SEG = 3;        // nodes per thread of one K column in the pair update's gather
-constexpr int UP_S = 3;          // nodes along K of one thread of update
-constexpr int UP_T = 288;        // most threads of an update CTA (three CTAs at 72 registers)
-constexpr int UP_R = 16;         // most J planes of an update CTA
 
 // CTA sum of one double-float per thread (thread 0 receives it)
 template <int BS>
@@ -1021,7 +1018,8 @@ struct UpdateCut {
 static UpdateCut update_cut(const Dev &d, int sm_count, int nv) {
     UpdateCut c{};
     double best = 1e30;
-    for (int ns = 1; ns * d.IM <= UP_T && (ns == 1 || (ns - 1) * UP_S < d.KM); ++ns) {
+    for (int ns = 1; ns * d.IM <= UP_T && (ns == 1 || (ns - 1) * UP_S < d.KM || ns * UP_S <= d.TS_ROWS); ++ns) {
+        if (d.TS_ROWS && ns * UP_S != d.TS_ROWS) continue;
         const int rows = ns * UP_S, nt = (d.KM + rows - 1) / rows, th = (ns * d.IM + 31) / 32 * 32;
         const double cost = (double)nt * (rows + 1) * th / (ns * d.IM);
         if (cost < best) {
@@ -1034,6 +1032,7 @@ static UpdateCut update_cut(const Dev &d, int sm_count, int nv) {
     const long long slots = (long long)sm_count * (65536 / (72 * c.threads));
     best = 1e30;
     for (int R = 1; R <= UP_R; ++R) {
+        if (d.TS_PLANES && R != d.TS_PLANES) continue;
         const long long ctas = (long long)((d.JM + R - 1) / R) * c.ntile * nv;
         const double cost = (double)((ctas + slots - 1) / slots) * (R + 1.5);
         if (cost < best) {
