@@ -474,6 +474,7 @@ int build_graph(mgpu_handle *h, int what) {
 bool kind_occurs(const Dev &d, int what) {
     if (d.ILOS == 0 || d.FROZEN) return !(what & 1);
     if (d.NLOS == 1) return (what & 1) != 0;
+    if (d.NLOS == 5) return what == 0 || what == 3;
     return what != 1 || d.NLOS % 5 != 0;
 }
 
@@ -540,13 +541,18 @@ int read_ctl(mgpu_handle *h) {
 
 // What the step after the mirrored control block c runs, q steps on: bit 0
 // LOSS, bit 1 the tail, by the tests of step_control.  q > 0 holds only up
-// to the next tail, which rewrites what the end test reads.
+// to the next tail, which rewrites what the end test reads.  With NLOS = 5 a
+// tail without LOSS is only the final step (and what follows it): it takes the
+// graph of both, whose LOSS kernels the device's flag ends at once, rather than
+// one more graph that every march would capture for it.
 int step_what(const Dev &d, const DevCtl &c, int q, bool force_end) {
     const int n = c.nstep + 1 + q;
     const bool end = c.ifend || force_end || n == d.NSTEPS_MAX || (c.EAVG < d.CONLIM && c.ECONT < 0.01f) ||
                      (fabsf(c.EMAX) < 4.0f * d.CONLIM && c.ECONT < 0.01f);
-    const bool loss = (d.ILOS == 10 || (d.ILOS >= 100 && d.ILOS < 300)) && n % d.NLOS == 0 && !d.FROZEN;
-    return (loss ? 1 : 0) | (n % 5 == 0 || end ? 2 : 0);
+    const bool tail = n % 5 == 0 || end;
+    const bool loss = (d.ILOS == 10 || (d.ILOS >= 100 && d.ILOS < 300)) && !d.FROZEN &&
+                      (n % d.NLOS == 0 || (tail && d.NLOS == 5));
+    return (loss ? 1 : 0) | (tail ? 2 : 0);
 }
 
 // launches the steps that follow the mirrored control block, none of them
