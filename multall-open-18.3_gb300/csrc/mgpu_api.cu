@@ -1664,19 +1664,26 @@ int32_t mgpu_profile_steps(mgpu_handle *h, int32_t nsteps, mgpu_kernel_time *out
 
 namespace {
 
-// Puts the members on chains: as many side by side as hold 1.6 million nodes,
-// at least four, each member on the chain with the fewest nodes so far.  That
-// is enough to fill the GPU, and what one kernel of a member writes is still in
-// L2 when the next one reads it; with all members side by side each array went
-// through memory between two kernels.  64 stages of 258 thousand nodes, with
-// the read-out of their states: 51.0 ms for 10 steps on 64 chains, 48.2 on 16,
-// 47.6, 47.4 and 47.5 on 8, 6 and 4, 49.4 on 3 and 57.8 on 2.
+// Puts the members on chains side by side, each member on the chain with the
+// fewest nodes so far.  About 1.6 million nodes side by side fill the GPU, and
+// what one kernel of a member writes is still in L2 when the next one reads
+// it; with all members side by side each array goes through memory between two
+// kernels.  So: the members that hold 1.6 million nodes, at least four, and
+// then as few chains as leave the longest one as long (one chain longer than
+// the others runs its last member alone).  ms a step on the chains taken and on
+// as many chains as members: 32 of 236 thousand nodes 2.17 and 2.39, 12 0.81 and
+// 0.85, 8 0.55 and 0.56 (7 chains 0.60); 48 of 71 thousand 1.58 and 1.74; 32 of 325
+// thousand 2.47 and 2.68, 6 0.47 and 0.47 (5 chains 0.52); 16 of 770 thousand 2.56
+// and 2.58, 5 0.80 and 0.81 (4 chains 0.86); 8 of 3.1 million 4.81 and 4.75.
+// Small members want all of them: 128 of 3 thousand 2.11 and 2.08, on 16 chains
+// 1.56, 16 of them 0.21 on 16, 0.31 on 4.
 void batch_chains(mgpu_batch *b) {
     const size_t n = b->hs.size();
     double nodes = 0.0;
     for (mgpu_handle *h : b->hs) nodes += (double)h->d.IM * h->d.JM * h->d.KM;
     const double want = std::ceil(1.6e6 * (double)n / nodes);
-    const size_t chains = want < 4.0 ? std::min<size_t>(4, n) : want < (double)n ? (size_t)want : n;
+    const size_t fill = want < 4.0 ? std::min<size_t>(4, n) : want < (double)n ? (size_t)want : n;
+    const size_t longest = (n + fill - 1) / fill, chains = (n + longest - 1) / longest;
     std::vector<double> load(chains, 0.0);
     std::vector<int> last(chains, -1);
     b->after.assign(n, -1);
