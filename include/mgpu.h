@@ -162,7 +162,9 @@ int32_t mgpu_step(mgpu_handle *h, int32_t force_end, mgpu_monitors *mon);
  * step (IFEND: the convergence test of multall-open-18.3.f:3762-3764 met at
  * a tail, or NSTEP reaching NSTEPS_MAX), where LOOP stops (5444-5451), and
  * at once, without stepping, on a handle whose final step has run; 0 when
- * all nsteps ran without reaching it. */
+ * all nsteps ran without reaching it.  The first mgpu_step, mgpu_run or
+ * mgpu_bench_steps of a handle captures its step graphs, before any step; no
+ * later mgpu_step or mgpu_run takes device memory. */
 int32_t mgpu_run(mgpu_handle *h, int32_t nsteps, mgpu_monitors *mon);
 /* Bytes one mgpu_step() call moves between host and device: the
  * end-of-run flag it sends and the control block (monitors) it reads back. */
@@ -246,7 +248,8 @@ int32_t mgpu_setup_metrics64(mgpu_handle *h, const double *x, const double *r, c
  * from fixed COMMON extents, a monitoring thread that reports the
  * efficiency during a long run, a host whose own allocator holds the rest
  * of device memory.  mgpu_integrals_compute works in a buffer that the
- * handle has allocated; this variant allocates no device or host memory (no cudaMalloc/cudaFree, no library
+ * handle has allocated and copies its result from there; this variant
+ * allocates no device or host memory (no cudaMalloc/cudaFree, no library
  * routine that allocates; only recording an error message for
  * mgpu_last_error may take host memory) and writes nothing of the handle's
  * arrays.  Its scratch is
@@ -266,7 +269,11 @@ int32_t mgpu_setup_metrics64(mgpu_handle *h, const double *x, const double *r, c
  *    and returns 0; make it once per device before marching begins.
  *  - Every call with out != NULL synchronises the handle's stream and
  *    copies its results to the host, so it must not be made while that
- *    stream is capturing.
+ *    stream is capturing.  The library captures it only in the handle's
+ *    first mgpu_step, mgpu_run or mgpu_bench_steps after mgpu_commit or
+ *    mgpu_autotune, in mgpu_kernels_per_step, and in the creation of a batch
+ *    that the handle is in (or the batch's first call after an
+ *    mgpu_autotune).
  *  - Calls whose executions overlap in time on the same device (two host
  *    threads, or two handles on one device) share the one scratch array and
  *    race: serialise them.  The call returns only after its results are on
@@ -278,20 +285,23 @@ int32_t mgpu_integrals_noalloc(mgpu_handle *h, mgpu_integrals *out);
 /* No counterpart in the reference, which marches one problem per process.
  * A batch steps several committed handles (operating points, grids of any
  * size) with one CUDA graph launch per LOOP iteration (a graph for each
- * kind of step: plain, LOSS, tail, both): the graph holds one branch per handle, so the kernels of all instances share the GPU at the
- * same time.  The handles must live on the current device and outlive the
- * batch; each keeps its own NSTEP, monitors and end test, and every value it
- * computes is bitwise the same as when the handle is stepped alone.  Do not
- * step a member on its own while a batch call is running. */
+ * kind of step: plain, LOSS, tail, both, and one where the members differ).
+ * The members lie on a few chains side by side, one after the other on each:
+ * enough of them run at the same time to fill the GPU.  The handles must live
+ * on the current device and outlive the batch; each keeps its own NSTEP,
+ * monitors and end test, and every value it computes is bitwise the same as
+ * when the handle is stepped alone.  Do not step a member on its own while a
+ * batch call is running. */
 typedef struct mgpu_batch mgpu_batch;
 int32_t mgpu_batch_create(mgpu_handle *const *handles, int32_t n, mgpu_batch **out);
 void    mgpu_batch_destroy(mgpu_batch *b);
-/* nsteps iterations of every member, launched back to back.  mons (n
- * entries, or NULL) receives each member's control block after the last
- * step.  Returns the number of members whose end test (convergence,
+/* nsteps iterations of every member.  The control blocks are read after
+ * each tail; mons (n entries, or NULL) receives them after every 50th and the
+ * last step.  Returns the number of members whose end test (convergence,
  * NSTEPS_MAX) has been met; they keep marching with the others, so a caller
  * that wants them stopped builds a new batch without them.  Returns
- * MGPU_E_NONFINITE if a member's health check fails. */
+ * MGPU_E_NONFINITE, after every 50th or the last step, if a member's health
+ * check has failed. */
 int32_t mgpu_batch_run(mgpu_batch *b, int32_t nsteps, mgpu_monitors *mons);
 /* As mgpu_bench_steps, for the whole batch. */
 int32_t mgpu_batch_bench_steps(mgpu_batch *b, int32_t nsteps, int32_t flush_l2, double *total_ms);

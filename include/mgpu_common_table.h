@@ -65,8 +65,9 @@
     M_(IFSHROUD, 0)                                                       \
     M_(NSTEP,    0)                                                       \
     /* not a COMMON variable: order of the long reductions on the GPU,   */ \
-    /* 0 = FP64 tree sums (default), 1 = the reference's sequential REAL*4 */ \
-    /* order for the superblock and row-average sums (parity checks),    */ \
+    /* 0 = trees in double-float (TSTEP) and FP64 (default), 1 = the     */ \
+    /* reference's sequential REAL*4 order for the superblock and        */ \
+    /* row-average sums (parity checks),                                 */ \
     /* 2 = the trees of 0 with FP32 adds (the plain FP32 path)           */ \
     M_(REDUCE_ORDER, 0)                                                   \
     /* not a COMMON variable: 1 holds the LOSS body forces and the STEPUP */ \

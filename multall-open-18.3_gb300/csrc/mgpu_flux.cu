@@ -4,11 +4,12 @@
 // and Mach limiters and the mixing-plane relaxation.
 //
 // Each kernel restates one sweep of SUBROUTINE LOOP
-// (multall-open-18.3.f:3664-5463) with one thread per node and the
-// reference's floating-point expression order, so that (built without FMA
-// contraction, as the reference is) the results match REAL*4 arithmetic.
-// Periodic fix-ups that couple I=1 and I=IM are done by both end threads
-// from the same raw values, so no thread waits on another.
+// (multall-open-18.3.f:3664-5463) in the reference's floating-point
+// expression order, so that (built without FMA contraction, as the reference
+// is) the results match REAL*4 arithmetic: one thread a node, and in the flux
+// passes one thread a column of nodes, marching up K.  The periodic fix-ups
+// of the fluxes, which couple I=1 and I=IM, are done by one thread for both
+// ends, in CTAs of their own.
 #include "mgpu_internal.cuh"
 
 namespace mgpu {

@@ -317,7 +317,7 @@ __global__ void __launch_bounds__(32 * LK_W, 5) k_loss_kfaces(const __grid_const
         float WTAVG = LK(VTAVG, kq) - WREL * RAVGK[kq - 1];
         return sqrtf(LK(VXAVG, kq) * LK(VXAVG, kq) + LK(VRAVG, kq) * LK(VRAVG, kq) + WTAVG * WTAVG);
     };
-    bool walk = KMID < 2;          // a ratio that the test below does not cover
+    bool walk = false;             // a ratio that the test below does not cover (KMID >= 2: KM >= 5)
     if (col) {
         const float VISLAM = s_vis[tx];
         const float ro1 = LK(ROAVG, 1), rom = LK(ROAVG, KM);

@@ -34,10 +34,13 @@ static inline unsigned grid_for(size_t n, unsigned block) { return (unsigned)((n
 
 // Threads per J-plane CTA: 128, 192, 256 (the default) or 512, chosen per
 // problem and pass by mgpu_autotune (Dev::ts_bs); each size keeps 1024
-// threads of 64 registers resident per SM (960 for 192: five CTAs).  256 is
-// the best or within the noise of it on every grid tried from 7 x 50 x 9 to
-// 73 x 752 x 57: 250 us a step at 65 x 242 x 49 against 263 at 192, 259 at 512
-// and 288 at 128, although its 723 momentum CTAs take 1.2 waves.
+// threads of 64 registers resident per SM (960 for 192: five CTAs).  us a step
+// with both passes at 128, 192, 256 and 512: 9 x 50 x 7 72.2, 71.0, 72.6, 72.7;
+// 37 x 98 x 33 104, 97.0, 94.7, 92.4; 37 x 194 x 33 116, 111, 111, 136; 49 x 162 x 41
+// 148, 140, 137, 165; 65 x 242 x 49 244, 230, 229, 264; 73 x 752 x 57 674, 661, 659,
+// 734; 96 x 120 x 40 218, 188, 175, 182.  A pass by itself can want another size:
+// the momenta of 65 x 242 x 49 97.1 us at 192 and 99.3 at 256 (723 CTAs on 608
+// slots), a grid of fewer CTAs than SMs 512.
 constexpr int TS_U = 3;          // cells per thread whose loads are issued together
 constexpr int SV_U = 3;          // points per thread whose streamwise loads are issued together
 constexpr int SM_SEG = 4;        // points per thread of one pitchwise or spanwise smoothing segment
@@ -1401,9 +1404,11 @@ __global__ void k_copy_tm_st(const __grid_constant__ Dev d, int v0, size_t n) {
 }
 
 // k_ts_update_pair where a 512-thread CTA covers a plane's points (TS_PAIR = 0:
-// never); the crossover lies between 63 points, where it is 4 us faster a
-// launch, and 1221, where it is 1 us slower (in a batch of 64 stages the two
-// are even)
+// never).  us a step with the march and with the pair, on 98 planes: 63 points
+// 77.5 and 73.5, 130 75.6 and 73.5, 289 76.7 and 73.9, 400 77.6 and 77.0, 506 78.0
+// and 77.5, 672 78.8 and 82.1, 1221 91.1 and 93.9; on 50 and 194 planes the line
+// lies there too.  On 322 planes, more pairs than one wave, the march is the
+// faster one at every size (63 points 96.3 and 98.7, 506 109 and 113).
 static bool pair_update(const Dev &d) { return d.TS_PAIR && d.IM * d.KM <= 512; }
 
 static size_t cells_smem(const Dev &d) {
@@ -1425,8 +1430,9 @@ static cudaError_t configure_bs(const Dev &d) {
              {(const void *)k_ts_update_pair<2 * BS>, update_pair_smem(d)},
              {(const void *)k_ts_smooth<BS>, smooth_smem(d)}};
     // the limit is on what a plane takes: the smoothing weights' second copies
-    // and the paddings (9 KB at the largest IM and KM that LOSS's line arrays
-    // let through) come on top
+    // and the paddings (2.6 KB at IM = KM = 160) come on top.  The three planes
+    // of the pair update bound every problem (IMM1 KMM1 <= 17066), though the
+    // kernel itself runs on small planes only
     const size_t extra = (2 * (size_t)(d.IM + d.KM) + SM_PAD + 4 * SM_SEG) * sizeof(float);
     for (auto &x : k) {
         if (x.bytes - (x.f == (const void *)k_ts_smooth<BS> ? extra : 0) > 200 * 1024) return cudaErrorInvalidValue;
