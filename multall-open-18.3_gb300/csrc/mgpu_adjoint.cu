@@ -2492,7 +2492,6 @@ int32_t mgpu_adjoint_prepare(mgpu_handle *h) {
     ACK(cudaMemcpyAsync(s->savectl, d.ctl, sizeof(DevCtl), cudaMemcpyDeviceToDevice, st));
     // the recorded step: LOSS and STEPUP held
     Dev rec = d;
-    rec.use_cond = 0;
     rec.FROZEN = 1;
     rec.ADJ_ROIN = const_cast<float *>(a.tROIN);
     rec.ADJ_MIX = const_cast<float *>(a.tMIX);

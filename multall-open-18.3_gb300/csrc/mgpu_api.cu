@@ -70,7 +70,6 @@ struct StepGraph {
 struct mgpu_handle {
     Dev d;
     cudaStream_t stream = nullptr;
-    cudaStream_t side = nullptr;     // captures the bodies of conditional graph nodes
     cudaStream_t aux = nullptr;      // a parallel branch of the step graph (k_bc_sums)
     cudaStream_t aux2 = nullptr;     // another (the Spalart-Allmaras transport)
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
@@ -109,9 +108,11 @@ struct mgpu_batch {
     cudaStream_t stream = nullptr;
     cudaEvent_t fork = nullptr;
     std::vector<cudaEvent_t> joins;
-    // a step that is of one kind for every member (as mgpu_handle::sg), and
-    // one in which each member's own flags decide
-    StepGraph sg[4], mixed;
+    // by the kind of step (as mgpu_handle::sg), the same for every member; a
+    // step that is of several kinds takes the graph of `every`, all that any
+    // member comes to, and each member's own flags decide
+    StepGraph sg[4];
+    int every = 0;
     std::vector<int> ts_bs;      // the members' CTA sizes that the graphs were captured with
     DevCtl **d_list = nullptr;   // the members' control blocks, their copies and the host's
     DevCtl *d_ctl = nullptr, *h_ctl = nullptr;
@@ -299,12 +300,11 @@ struct DensBranch {
     cudaEvent_t start = nullptr, done = nullptr;
 };
 
-// Lf: how the first kernel follows what was launched before it
-void enqueue_core(const Dev &d, Launch L, Launch Lf, cudaEvent_t join = nullptr, const SaBranch *sa = nullptr,
+void enqueue_core(const Dev &d, Launch L, cudaEvent_t join = nullptr, const SaBranch *sa = nullptr,
                   const DensBranch *dens = nullptr) {
     Launch L0 = L;        // follows a join of two branches: plain stream order
     L0.pdl = false;
-    launch_flux_mass_energy(d, Lf);
+    launch_flux_mass_energy(d, L);
     launch_tstep(d, L, V_RO, 2);
     if (d.ILOS >= 100) launch_roavg_cell(d, L);     // 4255-4267, after TSTEP(RO)
     const bool sab = sa && sa->s && d.ILOS >= 200;
@@ -359,86 +359,35 @@ int enqueue_step(mgpu_handle *h, Prof *prof = nullptr) {
     launch_step_begin(d, L);
     launch_prim(d, L, -1);
     launch_loss(d, L, false);
-    enqueue_core(d, L, L);
+    enqueue_core(d, L);
     launch_tail(d, L);
     CK(cudaGetLastError());
     return 0;
 }
 
-// appends an IF conditional node to the graph being captured on h->stream
-// and captures its body (fn) on the side stream
-template <typename F>
-int add_conditional(mgpu_handle *h, cudaGraphConditionalHandle hnd, F fn) {
-    cudaStreamCaptureStatus st;
-    cudaGraph_t cg = nullptr;
-    const cudaGraphNode_t *deps = nullptr;
-    size_t ndeps = 0;
-    CK(cudaStreamGetCaptureInfo(h->stream, &st, nullptr, &cg, &deps, nullptr, &ndeps));
-    cudaGraphNodeParams cp = {cudaGraphNodeTypeConditional};
-    cp.conditional.handle = hnd;
-    cp.conditional.type = cudaGraphCondTypeIf;
-    cp.conditional.size = 1;
-    cudaGraphNode_t node;
-    CK(cudaGraphAddNode(&node, cg, deps, nullptr, ndeps, &cp));
-    cudaGraph_t body = cp.conditional.phGraph_out[0];
-    CK(cudaStreamBeginCaptureToGraph(h->side, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-    fn(Launch{h->side, h->sm_count, nullptr});
-    cudaGraph_t out = nullptr;
-    CK(cudaStreamEndCapture(h->side, &out));
-    CK(cudaStreamUpdateCaptureDependencies(h->stream, &node, nullptr, 1, cudaStreamSetCaptureDependencies));
-    return 0;
-}
-
 // Records one LOOP iteration of h on h->stream, which must be capturing
-// (alone, or as one branch of a batch graph).  what >= 0: the iteration that
-// runs LOSS (bit 0) and the tail (bit 1) or not, as the caller knows from
-// the control block; their kernels still test the device's own flags.
-// what < 0: the LOSS and tail kernels sit in conditional bodies that the
-// step-control kernel switches on only on the steps that need them.
+// (alone, or as one branch of a batch graph): one that runs LOSS (bit 0 of
+// what) and the tail (bit 1) or not, as the caller knows from the control
+// block.  Their kernels still test the device's own flags, so a graph of more
+// than a step runs is the same step.
 int capture_step(mgpu_handle *h, int what) {
-    cudaStreamCaptureStatus st;
-    cudaGraph_t cg = nullptr;
-    CK(cudaStreamGetCaptureInfo(h->stream, &st, nullptr, &cg, nullptr, nullptr, nullptr));
-    cudaGraphConditionalHandle hl = 0, ht = 0;
-    Dev dg = h->d;
-    if (what < 0) {
-        // every handle of a graph belongs to one conditional node: an inviscid
-        // problem (ILOS = 0), which has no LOSS node, creates no LOSS handle
-        if (h->d.ILOS != 0) CK(cudaGraphConditionalHandleCreate(&hl, cg, 0, cudaGraphCondAssignDefault));
-        CK(cudaGraphConditionalHandleCreate(&ht, cg, 0, cudaGraphCondAssignDefault));
-        dg.use_cond = 1;
-        dg.cond_loss = (unsigned long long)hl;
-        dg.cond_tail = (unsigned long long)ht;
-    }
+    const Dev &d = h->d;
     Launch L{h->stream, h->sm_count, nullptr};
-    if (what < 0) {
-        launch_step_begin(dg, L);
-        L.pdl = true;      // kernel-to-kernel edges of the step are programmatic
-    }
-    launch_prim(dg, L, what);
-    L.pdl = true;
+    launch_prim(d, L, what);
+    L.pdl = true;          // kernel-to-kernel edges of the step are programmatic
     // the exit-pressure sums depend on nothing the next kernels write, so they
     // run beside LOSS, the mass/energy fluxes and TSTEP(RO, ROE)
     CK(cudaEventRecord(h->ev_fork, h->stream));
     CK(cudaStreamWaitEvent(h->aux, h->ev_fork, 0));
-    launch_bc_sums(dg, Launch{h->aux, h->sm_count, nullptr});
+    launch_bc_sums(d, Launch{h->aux, h->sm_count, nullptr});
     CK(cudaEventRecord(h->ev_join, h->aux));
     SaBranch sab{h->aux2, h->ev_sa0, h->ev_sa1, h->ev_sa2};
     DensBranch dens{h->aux, h->ev_dens0, h->ev_dens1};
-    if (what >= 0) {
-        if (what & 1) launch_loss(dg, L, false);
-        enqueue_core(dg, L, L, h->ev_join, &sab, &dens);
-        if (what & 2) launch_tail(dg, L);
-        CK(cudaGetLastError());
-        return 0;
-    }
-    Launch L0 = L;         // follows a conditional node: plain stream order
-    L0.pdl = false;
-    // an inviscid problem (ILOS = 0) has no LOSS node
-    int rc = dg.ILOS == 0 ? 0 : add_conditional(h, hl, [&](Launch L2) { launch_loss(dg, L2, false); });
-    if (!rc) enqueue_core(dg, L, L0, h->ev_join, &sab, &dens);
-    if (!rc) rc = add_conditional(h, ht, [&](Launch L2) { launch_tail(dg, L2); });
-    return rc;
+    if (what & 1) launch_loss(d, L, false);
+    enqueue_core(d, L, h->ev_join, &sab, &dens);
+    if (what & 2) launch_tail(d, L);
+    CK(cudaGetLastError());
+    return 0;
 }
 
 // Makes the captured graph g ready to launch on s: what it takes of the
@@ -582,7 +531,7 @@ HandleView handle_view(const mgpu_handle *h) { return HandleView{&h->d, h->strea
 
 int api_fail(int code, const char *msg) { return fail(code, msg); }
 
-void enqueue_step_core(const Dev &d, Launch L) { enqueue_core(d, L, L); }
+void enqueue_step_core(const Dev &d, Launch L) { enqueue_core(d, L); }
 AdjState *&handle_adj(mgpu_handle *h) { return h->adj; }
 Dev &handle_dev(mgpu_handle *h) { return h->d; }
 int handle_sm_count(const mgpu_handle *h) { return h->sm_count; }
@@ -645,8 +594,6 @@ int32_t mgpu_create(int32_t im, int32_t jm, int32_t km, int32_t nrows, mgpu_hand
     if (e != cudaSuccess) return bail(fail(MGPU_E_CUDA, std::string("no CUDA device: ") + cudaGetErrorString(e)));
     cudaDeviceGetAttribute(&h->sm_count, cudaDevAttrMultiProcessorCount, h->device);
     e = cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking);
-    if (e != cudaSuccess) return bail(fail(MGPU_E_CUDA, cudaGetErrorString(e)));
-    e = cudaStreamCreateWithFlags(&h->side, cudaStreamNonBlocking);
     if (e != cudaSuccess) return bail(fail(MGPU_E_CUDA, cudaGetErrorString(e)));
     e = cudaStreamCreateWithFlags(&h->aux, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&h->ev_fork, cudaEventDisableTiming);
@@ -737,7 +684,6 @@ void mgpu_destroy(mgpu_handle *h) {
     if (h->h_ctl) cudaFreeHost(h->h_ctl);
     if (h->h_int) cudaFreeHost(h->h_int);
     if (h->stream) cudaStreamDestroy(h->stream);
-    if (h->side) cudaStreamDestroy(h->side);
     if (h->aux) cudaStreamDestroy(h->aux);
     if (h->aux2) cudaStreamDestroy(h->aux2);
     if (h->ev_fork) cudaEventDestroy(h->ev_fork);
@@ -1533,7 +1479,6 @@ int32_t mgpu_autotune(mgpu_handle *h, int32_t *chosen, double *ms) {
         for (int c = 0; c < NC; ++c) {
             Dev dt = d;
             dt.ts_bs[p] = cand[c];
-            dt.use_cond = 0;
             Launch L{h->stream, h->sm_count};
             for (int r = 0; r < 2; ++r) launch_tstep(dt, L, v0, nv);
             const int reps = 10;
@@ -1696,9 +1641,9 @@ void batch_chains(mgpu_batch *b) {
     }
 }
 
-// the batch's graph of a step of kind `what` (-1: mixed)
+// the batch's graph of a step of kind `what`
 int batch_graph(mgpu_batch *b, int what) {
-    StepGraph &G = what < 0 ? b->mixed : b->sg[what];
+    StepGraph &G = b->sg[what];
     if (G.exec) return 0;
     CK(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
     int rc = 0;
@@ -1722,25 +1667,29 @@ int batch_graph(mgpu_batch *b, int what) {
     return instantiate(G, g, b->stream);
 }
 
-// Every graph that a march of the batch can need, as build_graphs; a step of
-// one kind for all members where each of them comes to that kind.  Built at
-// creation, and again where a member has been tuned since: each is captured
-// with its members' CTA sizes, and all of them with the same.
+// Every graph that a march of the batch can need, as build_graphs: a step of
+// one kind for all members where each of them comes to that kind, and
+// `every`.  Built at creation, and again where a member has been tuned since:
+// each is captured with its members' CTA sizes, and all of them with the same.
 int batch_graphs(mgpu_batch *b) {
     std::vector<int> ts;
     for (const mgpu_handle *h : b->hs) ts.insert(ts.end(), h->d.ts_bs, h->d.ts_bs + 2);
     if (ts != b->ts_bs) {
         for (StepGraph &G : b->sg) G.drop();
-        b->mixed.drop();
         b->ts_bs = ts;
     }
     for (int what = 0; what < 4; ++what) {
-        bool all = true;
-        for (const mgpu_handle *h : b->hs) all = all && kind_occurs(h->d, what);
+        bool all = true, any = false;
+        for (const mgpu_handle *h : b->hs) {
+            const bool on = kind_occurs(h->d, what);
+            all = all && on;
+            any = any || on;
+        }
+        if (any) b->every |= what;
         if (all)
             if (int rc = batch_graph(b, what)) return rc;
     }
-    return b->hs.size() > 1 ? batch_graph(b, -1) : 0;
+    return batch_graph(b, b->every);
 }
 
 // the control blocks of a batch side by side, for one copy to the host
@@ -1758,7 +1707,6 @@ void mgpu_batch_destroy(mgpu_batch *b) {
     if (b->stream) cudaStreamSynchronize(b->stream);
     if (b->flush_buf) cudaFree(b->flush_buf);
     for (StepGraph &G : b->sg) G.drop();
-    b->mixed.drop();
     if (b->d_list) cudaFree(b->d_list);
     if (b->d_ctl) cudaFree(b->d_ctl);
     if (b->h_ctl) cudaFreeHost(b->h_ctl);
@@ -1851,7 +1799,7 @@ int batch_known(mgpu_batch *b) {
 // The steps to launch before the control blocks are read again, at most
 // `most`: up to the first tail while each step is of one kind for every
 // member; otherwise (members at different steps, or past their end) a stretch
-// of mixed ones.  Leaves the mirrors invalid.
+// of steps that are all of them.  Leaves the mirrors invalid.
 void batch_plan(mgpu_batch *b, int most, std::vector<int> &plan) {
     int n = most;
     for (mgpu_handle *h : b->hs) {
@@ -1863,7 +1811,7 @@ void batch_plan(mgpu_batch *b, int most, std::vector<int> &plan) {
         const int what = step_what(b->hs[0]->d, *b->hs[0]->h_ctl, q, false);
         for (mgpu_handle *h : b->hs)
             if (step_what(h->d, *h->h_ctl, q, false) != what) {
-                plan.assign(most < 50 ? most : 50, -1);
+                plan.assign(most < 50 ? most : 50, b->every);
                 return;
             }
         plan.push_back(what);
@@ -1880,7 +1828,7 @@ int32_t mgpu_batch_run(mgpu_batch *b, int32_t nsteps, mgpu_monitors *mons) {
         const int left = nsteps - done, most = chunk - done % chunk;
         std::vector<int> plan;
         batch_plan(b, left < most ? left : most, plan);
-        for (int what : plan) CK(cudaGraphLaunch((what < 0 ? b->mixed : b->sg[what]).exec, b->stream));
+        for (int what : plan) CK(cudaGraphLaunch(b->sg[what].exec, b->stream));
         done += (int)plan.size();
         rc = done < nsteps && done % chunk ? batch_fetch(b) : batch_read(b, mons, &ended);
         if (rc) return rc;
@@ -1907,7 +1855,7 @@ int32_t mgpu_batch_bench_steps(mgpu_batch *b, int32_t nsteps, int32_t flush_l2, 
         for (int what : plan) {
             if (flush_l2) CK(cudaMemsetAsync(b->flush_buf, s & 0xff, b->flush_bytes, b->stream));
             CK(cudaEventRecord(ev[2 * s], b->stream));
-            CK(cudaGraphLaunch((what < 0 ? b->mixed : b->sg[what]).exec, b->stream));
+            CK(cudaGraphLaunch(b->sg[what].exec, b->stream));
             CK(cudaEventRecord(ev[2 * s + 1], b->stream));
             ++s;
         }

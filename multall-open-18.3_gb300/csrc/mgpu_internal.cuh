@@ -156,10 +156,6 @@ struct Dev {
     int *MG12;                         // (NIB1*NKB1) level-2 block of each level-1 block, where nested
     int mg_nested;                     // every level-2 block is a union of level-1 blocks (in I and in K)
     DevCtl *ctl;
-    // graph conditionals selecting the LOSS and 5-step tail bodies (set by
-    // the step-control kernel when the step runs from the CUDA graph)
-    int use_cond;
-    unsigned long long cond_loss, cond_tail;
     int ts_bs[2];                      // threads per J-plane CTA of TSTEP (128, 192, 256 or 512; mgpu_autotune)
                                        // for the pass of 2 variables (RO, ROE) and the pass of 3 (momenta)
 };
