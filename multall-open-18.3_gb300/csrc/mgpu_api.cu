@@ -1613,29 +1613,38 @@ namespace {
 // fewest nodes so far.  About 1.6 million nodes side by side fill the GPU, and
 // what one kernel of a member writes is still in L2 when the next one reads
 // it; with all members side by side each array goes through memory between two
-// kernels.  So: the members that hold 1.6 million nodes, at least four, and
-// then as few chains as leave the longest one as long (one chain longer than
-// the others runs its last member alone).  ms a step on the chains taken and on
-// as many chains as members: 32 of 236 thousand nodes 2.17 and 2.39, 12 0.81 and
-// 0.85, 8 0.55 and 0.56 (7 chains 0.60); 48 of 71 thousand 1.58 and 1.74; 32 of 325
-// thousand 2.47 and 2.68, 6 0.47 and 0.47 (5 chains 0.52); 16 of 770 thousand 2.56
-// and 2.58, 5 0.80 and 0.81 (4 chains 0.86); 8 of 3.1 million 4.81 and 4.75.
-// Small members want all of them: 128 of 3 thousand 2.11 and 2.08, on 16 chains
-// 1.56, 16 of them 0.21 on 16, 0.31 on 4.
+// kernels.  So: as many chains as members hold 1.6 million nodes, at least four;
+// and where the members are equal, as few as leave the longest chain as long
+// (one longer than the others runs its last member alone).
+// ms a step on the chains taken and on as many chains as members.  Equal members:
+// 32 of 236 thousand nodes 2.17 and 2.39, 12 0.81 and 0.85, 8 0.55 and 0.56 (7 chains
+// 0.60); 48 of 71 thousand 1.58 and 1.74; 32 of 325 thousand 2.47 and 2.68, 6 0.47
+// and 0.47 (5 chains 0.52); 16 of 770 thousand 2.56 and 2.58, 5 0.80 and 0.81 (4
+// chains 0.86); 8 of 3.1 million 4.81 and 4.75; 128 of 3 thousand 2.11 and 2.08 (16
+// chains 1.56).  Members of 139 to 484 thousand nodes, four mixes: 40 2.85, 2.37,
+// 2.62, 2.39 and 3.02, 2.52, 2.75, 2.54; 16 1.18, 0.97, 1.05, 0.98 and 1.20, 0.98, 1.08,
+// 0.99; 8 0.60, 0.48, 0.57, 0.53 and 0.59, 0.48, 0.53, 0.48: where a chain more or less
+// decides, it is the mix that says which, and evening them out by number lost
+// as often (12 members 0.74 for 0.70) as it won.
 void batch_chains(mgpu_batch *b) {
     const size_t n = b->hs.size();
     double nodes = 0.0;
-    for (mgpu_handle *h : b->hs) nodes += (double)h->d.IM * h->d.JM * h->d.KM;
+    bool equal = true;
+    auto size = [](const mgpu_handle *h) { return (double)h->d.IM * h->d.JM * h->d.KM; };
+    for (const mgpu_handle *h : b->hs) {
+        nodes += size(h);
+        equal = equal && size(h) == size(b->hs[0]);
+    }
     const double want = std::ceil(1.6e6 * (double)n / nodes);
     const size_t fill = want < 4.0 ? std::min<size_t>(4, n) : want < (double)n ? (size_t)want : n;
-    const size_t longest = (n + fill - 1) / fill, chains = (n + longest - 1) / longest;
+    const size_t longest = (n + fill - 1) / fill, chains = equal ? (n + longest - 1) / longest : fill;
     std::vector<double> load(chains, 0.0);
     std::vector<int> last(chains, -1);
     b->after.assign(n, -1);
     for (size_t i = 0; i < n; ++i) {
         const size_t c = (size_t)(std::min_element(load.begin(), load.end()) - load.begin());
         const mgpu_handle *h = b->hs[i];
-        load[c] += (double)h->d.IM * h->d.JM * h->d.KM;
+        load[c] += size(h);
         b->after[i] = last[c];
         last[c] = (int)i;
     }
