@@ -551,7 +551,7 @@ cudaError_t configure_kernels(const Dev &d);
 cudaError_t configure_loss_kernels(const Dev &d);
 cudaError_t configure_flux_kernels(const Dev &d);
 
-// one LOOP iteration without the LOSS and tail bodies, eager launches on
+// one LOOP iteration without LOSS and the tail, eager launches on
 // L.s (mgpu_api.cu)
 void enqueue_step_core(const Dev &d, Launch L);
 

@@ -401,9 +401,9 @@ class Problem:
 
 
 class Batch:
-    """Several Problems stepped by one CUDA graph launch per iteration (one
-    graph branch per problem); each problem's results are the same as when
-    it is stepped alone."""
+    """Several Problems stepped by one CUDA graph launch per iteration (on a
+    few chains side by side); each problem's results are the same as when it
+    is stepped alone."""
 
     def __init__(self, problems):
         L = load()
